@@ -1,0 +1,676 @@
+// A recurrence over a per-request state in chunks of 64 tokens, float arithmetic throughout, for long portions:
+//     S_t = diag(a_t) S_(t-1) + k_t u_t^T,   o_t = S_t^T q_t (+ skip v_t)
+// with u_t = beta_t (v_t - (diag(a_t) S_(t-1))^T k_t) (DELTA) or f_t v_t, decays per key channel (PERCH) or per head. With a
+// BONUS b a token reads the state before it and its own product times b: o_t = S_(t-1)^T q_t + v_t sum_c q_t b k_t.
+//
+// Token by token this is one chain: a token's sums over the channels wait for the one before. Inside a chunk, with P_t the
+// product of the decays up to t and P_t / P_j that of the decays after j (always formed as a product of factors, never as a
+// quotient, so that nothing overflows where the decays are strong), everything is a product of matrices:
+//     (I + L) U = diag(beta) (V - (P k) S_0),   L[t][j] = beta_t sum_c k_t k_j P_t / P_j  for j < t
+//     O = (P q) S_0 + M U,                      M[t][j] = sum_c q_t k_j P_t / P_j         for j <= t
+//     S_end = diag(P_end) S_0 + (k P_end / P)^T U
+//   chunk_prep_kernel   a CTA a (chunk, head), all chunks side by side: M, P q, k P_end / P, and for DELTA W = (I + L)^-1 beta P k
+//                       and (I + L)^-1 beta V, the inverse by blocks of 16 (what is left of U is - W S_0).
+//   chunk_carry_kernel  a CTA a (sequence, head, NC value columns) walks the chunks: keeps the state it meets for the last
+//                       kernel, U -= W S, S = P_end S + (k P_end / P)^T U. The next chunk's rows travel meanwhile (cp.async).
+//   chunk_out_kernel    a CTA a (chunk, head, 64 value columns), all side by side: O.
+// Decays per channel do not factor out of M and L. Blocks of 16 x 16 below the diagonal are a product of rows scaled by the
+// decays since their own block's beginning with rows scaled by the decays up to it (both at most 1); the ones on the diagonal
+// are summed with a running product per channel.
+// What bounds it: the FMA units (a token costs a head about 73,000 FMAs at 128 x 128, no fewer than token by token), not a
+// chain; a product's operands come from shared memory in tiles of 32 x 16 a warp, 64 FMAs for 8 loads of 16 bytes.
+// 64 tokens: with 32 the walk over the chunks has twice the barriers for the same FMAs, with 128 the triangles cost more than
+// the rest. Sums are grouped differently than token by token, within float rounding.
+#pragma once
+#include "common.cuh"
+
+namespace rllm {
+namespace chunked {
+
+constexpr int C = 64;      // tokens a chunk
+constexpr int SB = 16;     // tokens a block of the triangles
+constexpr int LC = C + 4;  // row stride of a [64][64] matrix in shared memory
+constexpr int THREADS = 256;
+
+struct Args {
+  const void* q; const void* k; const void* v;        // rows of TI, column offset folded in
+  long long q_ld, k_ld, v_ld;
+  int q_heads, k_heads;
+  float qscale;
+  const float* decay;                                 // [T, H * D] (PERCH) or [T, H]
+  const void* beta; long long beta_ld; int beta_bf16; // logits (DELTA)
+  const float* vscale;                                // [T, H] or null
+  const float* skip;                                  // [H] or null
+  const float* bonus;                                 // [H, D] (BONUS)
+  int H, vdim;
+  const int* cu_q; int num_seqs; const int* state_slots;
+  int long_from;                                      // sequences with fewer rows are left to another kernel
+  float* state;                                       // [slots, H, D, vdim]
+  float* out;                                         // [T, H, vdim]
+  float* scratch;                                     // per (chunk, head): see Place
+};
+
+// One (chunk, head)'s share of the scratch.
+template <int D>
+struct Place {
+  float *m, *qd, *kt, *w, *u, *s, *pc;
+  __host__ __device__ static long long floats(int vdim, bool delta) {
+    return (long long)C * C + 2 * C * D + (delta ? C * D : 0) + (long long)C * vdim + (long long)D * vdim + D;
+  }
+  __device__ Place(float* base, long long x, int vdim, bool delta) {
+    m = base + x * floats(vdim, delta);
+    qd = m + C * C;
+    kt = qd + C * D;
+    w = kt + C * D;
+    u = w + (delta ? C * D : 0);
+    s = u + (long long)C * vdim;
+    pc = s + (long long)D * vdim;
+  }
+};
+
+// Chunks of a sequence of n rows; which sequence and chunk a CTA has (false: none).
+__device__ __forceinline__ int chunks_of(int n, int long_from) { return n < long_from ? 0 : (n + C - 1) / C; }
+__device__ __forceinline__ bool find_chunk(const Args& a, int b, int& row0, int& n) {
+  int at = 0;
+  for (int s = 0; s < a.num_seqs; ++s) {
+    const int r0 = a.cu_q[s], rows = a.cu_q[s + 1] - r0, cs = chunks_of(rows, a.long_from);
+    if (b < at + cs) { row0 = r0 + (b - at) * C; n = min(C, rows - (b - at) * C); return true; }
+    at += cs;
+  }
+  return false;
+}
+
+__device__ __forceinline__ void copy16(float* smem, const float* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+  const uint2 x = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// acc[i][4 n + c] += sum_k A[row + 8 i][k] B[k][col + 16 n + c]: a warp's tile of 32 x 16 NT, `row` = first row + lane / 4,
+// `col` = first column + 4 (lane % 4). K a multiple of 4; A's rows 16 bytes apart in bank phase (stride 4 mod 32).
+template <int NT>
+__device__ __forceinline__ void tile_product(float (&acc)[4][4 * NT], const float* A, int lda, const float* B, int ldb, int K) {
+  for (int k = 0; k < K; k += 4) {
+    float4 x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(A + 8 * i * lda + k);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float4 y[NT];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) y[n] = *reinterpret_cast<const float4*>(B + (k + e) * ldb + 16 * n);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          acc[i][4 * n] = fmaf(xv, y[n].x, acc[i][4 * n]);
+          acc[i][4 * n + 1] = fmaf(xv, y[n].y, acc[i][4 * n + 1]);
+          acc[i][4 * n + 2] = fmaf(xv, y[n].z, acc[i][4 * n + 2]);
+          acc[i][4 * n + 3] = fmaf(xv, y[n].w, acc[i][4 * n + 3]);
+        }
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
+  return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
+}
+
+// X (lower triangular, [64][LC]) = (I + L)^-1, L strictly lower [64][LC]; tmp: 3 x 16 x 17 floats. Blocks of 16 on the diagonal
+// column by column, then the block diagonals below: X_IJ = -X_II sum_K L_IK X_KJ.
+__device__ __forceinline__ void unit_lower_inverse(const float* L, float* X, float* tmp) {
+  const int tid = threadIdx.x;
+  for (int x = tid; x < C * C; x += THREADS) {
+    const int t = x / C, j = x % C;
+    if ((t / SB) != (j / SB)) X[t * LC + j] = 0.f;
+  }
+  if (tid < C) {
+    const int b = tid / SB * SB, j = tid % SB;
+    float x[SB];
+#pragma unroll
+    for (int t = 0; t < SB; ++t) {
+      float r = t == j ? 1.f : 0.f;
+#pragma unroll
+      for (int m = 0; m < t; ++m) r = fmaf(-L[(b + t) * LC + b + m], x[m], r);
+      x[t] = r;
+    }
+#pragma unroll
+    for (int t = 0; t < SB; ++t) X[(b + t) * LC + b + j] = x[t];
+  }
+  __syncthreads();
+  const int t = tid / SB, j = tid % SB;
+#pragma unroll
+  for (int d = 1; d < C / SB; ++d) {
+#pragma unroll
+    for (int J = 0; J < C / SB - d; ++J) {
+      const int I = J + d;
+      float y = 0.f;
+#pragma unroll
+      for (int m = 0; m < SB * d; m += 4) {
+        const float4 l = *reinterpret_cast<const float4*>(L + (I * SB + t) * LC + J * SB + m);
+        const float* xc = X + (J * SB + m) * LC + J * SB + j;
+        y = fmaf(l.x, xc[0], y); y = fmaf(l.y, xc[LC], y); y = fmaf(l.z, xc[2 * LC], y); y = fmaf(l.w, xc[3 * LC], y);
+      }
+      tmp[(J * SB + t) * (SB + 1) + j] = y;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int J = 0; J < C / SB - d; ++J) {
+      const int I = J + d;
+      float x = 0.f;
+#pragma unroll
+      for (int m = 0; m < SB; ++m) x = fmaf(X[(I * SB + t) * LC + I * SB + m], tmp[(J * SB + m) * (SB + 1) + j], x);
+      X[(I * SB + t) * LC + J * SB + j] = -x;
+    }
+    __syncthreads();
+  }
+}
+
+template <typename TI, int D, bool PERCH, bool DELTA, bool BONUS>
+__global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_kernel(Args a) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int LDD = D + 4, NV = D / 4;
+  extern __shared__ __align__(16) float sm[];
+  float* Q = sm;                                        // [C][LDD] each
+  float* K = Q + C * LDD;
+  float* A = K + C * LDD;                               // decays per channel, later k scaled up to the next block
+  float* G1 = PERCH ? A + C * LDD : A;                  // [C][LC] ratios of decays (per head), later the inverse
+  float* G2 = G1 + C * LC;                              // [C][LC] L (DELTA)
+  float* few = G1 + (DELTA ? 2 : PERCH ? 0 : 1) * C * LC;   // [C] decays, [C] beta or value scales
+  float* blk = few + 2 * C;                             // per channel: [4][D] a block's product; scalar: scratch
+  int row0, n;
+  if (!find_chunk(a, blockIdx.x, row0, n)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int H = a.H, h = blockIdx.y, V = a.vdim;
+  const Place<D> to(a.scratch, (long long)blockIdx.x * H + h, V, DELTA);
+  const TI* qg = reinterpret_cast<const TI*>(a.q) + (h / (H / a.q_heads)) * D;
+  const TI* kg = reinterpret_cast<const TI*>(a.k) + (h / (H / a.k_heads)) * D;
+  const TI* vg = reinterpret_cast<const TI*>(a.v) + (long long)h * V;
+  for (int x = tid; x < C * NV; x += THREADS) {
+    const int t = x / NV, c = x % NV * 4;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q, d = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (t < n) {
+      const long long r = row0 + t;
+      q = load4(qg + r * a.q_ld + c);
+      k = load4(kg + r * a.k_ld + c);
+      if (PERCH) d = load4(a.decay + (r * H + h) * D + c);
+      q.x *= a.qscale; q.y *= a.qscale; q.z *= a.qscale; q.w *= a.qscale;
+    }
+    *reinterpret_cast<float4*>(Q + t * LDD + c) = q;
+    *reinterpret_cast<float4*>(K + t * LDD + c) = k;
+    if (PERCH) *reinterpret_cast<float4*>(A + t * LDD + c) = d;
+  }
+  if (tid < C) {
+    const long long r = row0 + tid;
+    if (!PERCH) few[tid] = tid < n ? a.decay[r * H + h] : 1.f;
+    float b = 0.f;
+    if (tid < n) {
+      if (DELTA) {
+        const float z = a.beta_bf16 ? to_f32(reinterpret_cast<const bf16*>(a.beta)[r * a.beta_ld + h])
+                                    : reinterpret_cast<const float*>(a.beta)[r * a.beta_ld + h];
+        b = 1.f / (1.f + expf(-z));
+      } else {
+        b = a.vscale ? a.vscale[r * H + h] : 1.f;
+      }
+    }
+    few[C + tid] = b;
+  }
+  __syncthreads();
+  const float* beta = few + C;
+
+  if constexpr (!PERCH) {
+    // one decay a head: the ratios of products are a matrix of their own, G1[t][j] = a_(j+1) ... a_t
+    if (tid < C) {
+      float r = 1.f;
+      G1[tid * LC + tid] = 1.f;
+      for (int t = tid + 1; t < C; ++t) { r *= few[t]; G1[t * LC + tid] = r; }
+    }
+    __syncthreads();
+    const float first = few[0];
+    const int r0 = (warp >> 1) * 16 + (lane >> 3), c0 = (warp & 1) * 32 + (lane & 7);
+    float m[4][4] = {}, l[4][4] = {};
+    if ((warp & 1) * 32 < (warp >> 1) * 16 + 16) {      // else wholly above the diagonal
+      for (int c = 0; c < D; c += 4) {
+        float4 q[4], k[4], kc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          q[i] = *reinterpret_cast<const float4*>(Q + (r0 + 4 * i) * LDD + c);
+          if (DELTA) k[i] = *reinterpret_cast<const float4*>(K + (r0 + 4 * i) * LDD + c);
+          kc[i] = *reinterpret_cast<const float4*>(K + (c0 + 8 * i) * LDD + c);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            m[i][j] = dot4(q[i], kc[j], m[i][j]);
+            if (DELTA) l[i][j] = dot4(k[i], kc[j], l[i][j]);
+          }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = r0 + 4 * i, s = c0 + 8 * j;
+        const float r = s <= t ? G1[t * LC + s] : 0.f;
+        to.m[t * C + s] = s <= t ? m[i][j] * r : 0.f;
+        if (DELTA) G2[t * LC + s] = s < t ? beta[t] * l[i][j] * r : 0.f;
+      }
+    // P q and k P_end / P; what K holds afterwards is k P (times beta) for the last product
+    for (int x = tid; x < C * NV; x += THREADS) {
+      const int t = x / NV, c = x % NV * 4;
+      const float p = first * G1[t * LC], e = G1[(C - 1) * LC + t];
+      float4 q = *reinterpret_cast<float4*>(Q + t * LDD + c), k = *reinterpret_cast<float4*>(K + t * LDD + c);
+      *reinterpret_cast<float4*>(to.qd + t * D + c) = make_float4(q.x * p, q.y * p, q.z * p, q.w * p);
+      *reinterpret_cast<float4*>(to.kt + t * D + c) = make_float4(k.x * e, k.y * e, k.z * e, k.w * e);
+    }
+    if (tid < D) to.pc[tid] = first * G1[(C - 1) * LC];
+    if (DELTA) {
+      __syncthreads();
+      for (int x = tid; x < C * NV; x += THREADS) {
+        const int t = x / NV, c = x % NV * 4;
+        const float p = first * G1[t * LC] * beta[t];
+        float4* k = reinterpret_cast<float4*>(K + t * LDD + c);
+        *k = make_float4(k->x * p, k->y * p, k->z * p, k->w * p);
+      }
+    }
+  } else {
+    // blocks on the diagonal: a thread has key token j of a block and every fourth group of four channels, and walks the
+    // tokens after it with the running product of the decays
+    {
+      const int b = (tid >> 6) * SB, j = (tid >> 2) & 15, s = tid & 3;
+      float m[SB], l[DELTA ? SB : 1];
+#pragma unroll
+      for (int e = 0; e < SB; ++e) { m[e] = 0.f; if (DELTA) l[e] = 0.f; }
+      for (int c = 4 * s; c < D; c += 16) {
+        float4 x = *reinterpret_cast<const float4*>(K + (b + j) * LDD + c);
+        if (BONUS) {
+          const float4 u = load4(a.bonus + (long long)h * D + c);
+          const float4 q = *reinterpret_cast<const float4*>(Q + (b + j) * LDD + c);
+          m[0] = fmaf(q.x * x.x, u.x, fmaf(q.y * x.y, u.y, fmaf(q.z * x.z, u.z, fmaf(q.w * x.w, u.w, m[0]))));
+        } else {
+          m[0] = dot4(*reinterpret_cast<const float4*>(Q + (b + j) * LDD + c), x, m[0]);
+        }
+#pragma unroll
+        for (int e = 1; e < SB; ++e) {
+          if (j + e < SB) {
+            const int t = (b + j + e) * LDD + c;
+            const float4 d = *reinterpret_cast<const float4*>(A + t);
+            if (BONUS) m[e] = dot4(*reinterpret_cast<const float4*>(Q + t), x, m[e]);
+            x.x *= d.x; x.y *= d.y; x.z *= d.z; x.w *= d.w;
+            if (!BONUS) m[e] = dot4(*reinterpret_cast<const float4*>(Q + t), x, m[e]);
+            if (DELTA) l[e] = dot4(*reinterpret_cast<const float4*>(K + t), x, l[e]);
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < SB; ++e) {
+        m[e] += __shfl_xor_sync(0xffffffffu, m[e], 1);
+        m[e] += __shfl_xor_sync(0xffffffffu, m[e], 2);
+        if (DELTA) { l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1); l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2); }
+      }
+      if (s == 0) {
+#pragma unroll
+        for (int e = 0; e < SB; ++e) {
+          if (j + e < SB) {
+            to.m[(b + j + e) * C + b + j] = m[e];
+            if (DELTA) G2[(b + j + e) * LC + b + j] = e ? beta[b + j + e] * l[e] : 0.f;
+          }
+        }
+      }
+    }
+    for (int x = tid; x < C * C; x += THREADS) {           // nothing above the diagonal
+      const int t = x / C, j = x % C;
+      if (j > t) { to.m[x] = 0.f; if (DELTA) G2[t * LC + j] = 0.f; }
+    }
+    __syncthreads();
+    // rows scaled by the decays since their block's beginning (q, k), and k by those up to the block's end (in A's place)
+    for (int x = tid; x < (C / SB) * D; x += THREADS) {
+      const int b = x / D, c = x % D;
+      float d[SB];
+#pragma unroll
+      for (int t = 0; t < SB; ++t) d[t] = A[(b * SB + t) * LDD + c];
+      float p = 1.f;
+#pragma unroll
+      for (int t = SB - 1; t >= 0; --t) {
+        A[(b * SB + t) * LDD + c] = K[(b * SB + t) * LDD + c] * p;
+        p *= d[t];
+      }
+      blk[x] = p;
+      p = 1.f;
+#pragma unroll
+      for (int t = 0; t < SB; ++t) {
+        const int at = (b * SB + t) * LDD + c;
+        if (BONUS) Q[at] *= p;
+        p *= d[t];
+        if (!BONUS) Q[at] *= p;
+        if (DELTA) K[at] *= p;
+      }
+    }
+    __syncthreads();
+    const int t = tid >> 4, j = tid & 15;
+#pragma unroll
+    for (int I = 1; I < C / SB; ++I) {
+      float m[C / SB - 1] = {}, l[C / SB - 1] = {};
+      for (int c = 0; c < D; c += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(Q + (I * SB + t) * LDD + c);
+        float4 k;
+        if (DELTA) k = *reinterpret_cast<const float4*>(K + (I * SB + t) * LDD + c);
+#pragma unroll
+        for (int J = 0; J < I; ++J) {
+          const float4 x = *reinterpret_cast<const float4*>(A + (J * SB + j) * LDD + c);
+          m[J] = dot4(q, x, m[J]);
+          if (DELTA) l[J] = dot4(k, x, l[J]);
+        }
+      }
+#pragma unroll
+      for (int J = 0; J < I; ++J) {
+        to.m[(I * SB + t) * C + J * SB + j] = m[J];
+        if (DELTA) G2[(I * SB + t) * LC + J * SB + j] = beta[I * SB + t] * l[J];
+      }
+      __syncthreads();
+      for (int x = tid; x < I * SB * NV; x += THREADS) {   // up to the end of block I
+        const int c = x % NV * 4;
+        float4* y = reinterpret_cast<float4*>(A + x / NV * LDD + c);
+        const float4 d = *reinterpret_cast<const float4*>(blk + I * D + c);
+        *y = make_float4(y->x * d.x, y->y * d.y, y->z * d.z, y->w * d.w);
+      }
+      __syncthreads();
+    }
+    for (int x = tid; x < C * NV; x += THREADS) {
+      const int t2 = x / NV, c = x % NV * 4;
+      float4 p = make_float4(1.f, 1.f, 1.f, 1.f);
+      for (int b = 0; b < t2 / SB; ++b) {
+        const float4 d = *reinterpret_cast<const float4*>(blk + b * D + c);
+        p = make_float4(p.x * d.x, p.y * d.y, p.z * d.z, p.w * d.w);
+      }
+      const float4 q = *reinterpret_cast<const float4*>(Q + t2 * LDD + c);
+      *reinterpret_cast<float4*>(to.qd + t2 * D + c) = make_float4(q.x * p.x, q.y * p.y, q.z * p.z, q.w * p.w);
+      *reinterpret_cast<float4*>(to.kt + t2 * D + c) = *reinterpret_cast<const float4*>(A + t2 * LDD + c);
+      if (DELTA) {
+        float4* k = reinterpret_cast<float4*>(K + t2 * LDD + c);
+        const float b = beta[t2];
+        *k = make_float4(k->x * p.x * b, k->y * p.y * b, k->z * p.z * b, k->w * p.w * b);
+      }
+    }
+    if (tid < D) to.pc[tid] = blk[tid] * blk[D + tid] * blk[2 * D + tid] * blk[3 * D + tid];
+  }
+
+  if constexpr (!DELTA) {
+    for (int x = tid; x < C * (V / 4); x += THREADS) {
+      const int t = x / (V / 4), c = x % (V / 4) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < n) v = load4(vg + (long long)(row0 + t) * a.v_ld + c);
+      const float f = beta[t];
+      *reinterpret_cast<float4*>(to.u + (long long)t * V + c) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+    }
+  } else {
+    __syncthreads();                                       // Q is done with, L and K are whole
+    unit_lower_inverse(G2, G1, PERCH ? A : blk);
+    // W = X (beta P k), then X (beta v), D value columns at a time in Q's place
+    const int rl = (warp & 1) * 32 + (lane >> 2), cl = (warp >> 1) * 16 + 4 * (lane & 3);
+    const int kk = (warp & 1) ? C : C / 2;                 // the upper rows meet the first half only
+    for (int c = 0; c < D; c += 64) {
+      float acc[4][4] = {};
+      tile_product<1>(acc, G1 + rl * LC, LC, K + c + cl, LDD, kk);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4*>(to.w + (rl + 8 * i) * D + c + cl) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+    for (int v0 = 0; v0 < V; v0 += D) {
+      const int nv = min(D, V - v0);
+      __syncthreads();
+      for (int x = tid; x < C * (nv / 4); x += THREADS) {
+        const int t = x / (nv / 4), c = x % (nv / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n) v = load4(vg + (long long)(row0 + t) * a.v_ld + v0 + c);
+        const float f = beta[t];
+        *reinterpret_cast<float4*>(Q + t * LDD + c) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+      }
+      __syncthreads();
+      for (int c = 0; c + (warp >> 1) * 16 < nv; c += 64) {
+        float acc[4][4] = {};
+        tile_product<1>(acc, G1 + rl * LC, LC, Q + c + cl, LDD, kk);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float4*>(to.u + (long long)(rl + 8 * i) * V + v0 + c + cl) =
+              make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      }
+    }
+  }
+}
+
+// NC value columns a CTA (16, or 32 where there are CTAs enough): 8 warps, for U two halves of the rows x four quarters of the
+// channels, for S a quarter of the channels (32; at D = 64 an eighth of the work each: two x four) x halves of the tokens.
+template <int D, int NC, bool DELTA>
+__global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int LDW = D + 4, NT = NC / 16, RG = D / 32, JG = 8 / RG;     // S: RG groups of 32 channels x JG parts of the tokens
+  constexpr int STAGE = (DELTA ? C * LDW : 0) + C * D + C * NC + D;
+  extern __shared__ __align__(16) float sm[];
+  float* S = sm + 2 * STAGE;                             // [D][NC]
+  float* part = S + D * NC;                              // [4][C][NC] sums of U, or [JG - 1][D][NC] of S
+  const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * NC, H = a.H, V = a.vdim;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n = a.cu_q[seq + 1] - a.cu_q[seq], chunks = chunks_of(n, a.long_from);
+  if (chunks == 0) return;
+  int base = 0;
+  for (int s = 0; s < seq; ++s) base += chunks_of(a.cu_q[s + 1] - a.cu_q[s], a.long_from);
+  const int slot = a.state_slots ? a.state_slots[seq] : -1;
+  float* sp = a.state + ((long long)(slot < 0 ? 0 : slot) * H + h) * D * V + v0;
+  auto issue = [&](int ci, int stage) {
+    const Place<D> in(a.scratch, (long long)(base + ci) * H + h, V, DELTA);
+    float* ws = sm + stage * STAGE;
+    float* ks = ws + (DELTA ? C * LDW : 0);
+    float* us = ks + C * D;
+    float* ps = us + C * NC;
+    for (int x = tid; x < C * (D / 4); x += THREADS) {
+      if (DELTA) copy16(ws + x / (D / 4) * LDW + x % (D / 4) * 4, in.w + 4 * x);
+      copy16(ks + 4 * x, in.kt + 4 * x);
+    }
+    for (int x = tid; x < C * (NC / 4); x += THREADS)
+      copy16(us + 4 * x, in.u + (long long)(x / (NC / 4)) * V + v0 + x % (NC / 4) * 4);
+    if (tid < D / 4) copy16(ps + 4 * tid, in.pc + 4 * tid);
+  };
+  issue(0, 0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int x = tid; x < D * (NC / 4); x += THREADS) {
+    const int k = x / (NC / 4), c = x % (NC / 4) * 4;
+    *reinterpret_cast<float4*>(S + k * NC + c) =
+        slot >= 0 ? *reinterpret_cast<const float4*>(sp + (long long)k * V + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int ci = 0; ci < chunks; ++ci) {
+    const Place<D> in(a.scratch, (long long)(base + ci) * H + h, V, DELTA);
+    if (ci + 1 < chunks) issue(ci + 1, (ci + 1) & 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    float* ws = sm + (ci & 1) * STAGE;
+    float* ks = ws + (DELTA ? C * LDW : 0);
+    float* us = ks + C * D;
+    const float* ps = us + C * NC;
+    for (int x = tid; x < D * (NC / 4); x += THREADS)     // the state that the chunk meets
+      *reinterpret_cast<float4*>(in.s + (long long)(x / (NC / 4)) * V + v0 + x % (NC / 4) * 4) = *reinterpret_cast<const float4*>(S + 4 * x);
+    if (DELTA) {
+      const int r = (warp & 1) * 32 + (lane >> 2), k0 = (warp >> 1) * (D / 4), c = 4 * (lane & 3);
+      float acc[4][4 * NT] = {};
+      tile_product<NT>(acc, ws + r * LDW + k0, LDW, S + k0 * NC + c, NC, D / 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          *reinterpret_cast<float4*>(part + ((warp >> 1) * C + r + 8 * i) * NC + c + 16 * t) =
+              make_float4(acc[i][4 * t], acc[i][4 * t + 1], acc[i][4 * t + 2], acc[i][4 * t + 3]);
+      __syncthreads();
+      for (int x = tid; x < C * (NC / 4); x += THREADS) {
+        const float4 p0 = *reinterpret_cast<const float4*>(part + 4 * x), p1 = *reinterpret_cast<const float4*>(part + C * NC + 4 * x);
+        const float4 p2 = *reinterpret_cast<const float4*>(part + 2 * C * NC + 4 * x), p3 = *reinterpret_cast<const float4*>(part + 3 * C * NC + 4 * x);
+        float4 u = *reinterpret_cast<const float4*>(us + 4 * x);
+        u.x -= (p0.x + p1.x) + (p2.x + p3.x); u.y -= (p0.y + p1.y) + (p2.y + p3.y);
+        u.z -= (p0.z + p1.z) + (p2.z + p3.z); u.w -= (p0.w + p1.w) + (p2.w + p3.w);
+        *reinterpret_cast<float4*>(us + 4 * x) = u;
+        *reinterpret_cast<float4*>(in.u + (long long)(x / (NC / 4)) * V + v0 + x % (NC / 4) * 4) = u;
+      }
+      __syncthreads();
+    }
+    {
+      const int k = (warp % RG) * 32 + 4 * (lane >> 2), jg = warp / RG, c = 4 * (lane & 3);
+      float acc[4][4 * NT] = {};
+#pragma unroll 8
+      for (int j = jg * (C / JG); j < (jg + 1) * (C / JG); ++j) {
+        const float4 x = *reinterpret_cast<const float4*>(ks + j * D + k);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const float4 y = *reinterpret_cast<const float4*>(us + j * NC + c + 16 * t);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[i][4 * t] = fmaf(xs[i], y.x, acc[i][4 * t]);
+            acc[i][4 * t + 1] = fmaf(xs[i], y.y, acc[i][4 * t + 1]);
+            acc[i][4 * t + 2] = fmaf(xs[i], y.z, acc[i][4 * t + 2]);
+            acc[i][4 * t + 3] = fmaf(xs[i], y.w, acc[i][4 * t + 3]);
+          }
+        }
+      }
+      if (jg > 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+            *reinterpret_cast<float4*>(part + ((jg - 1) * D + k + i) * NC + c + 16 * t) =
+                make_float4(acc[i][4 * t], acc[i][4 * t + 1], acc[i][4 * t + 2], acc[i][4 * t + 3]);
+      }
+      __syncthreads();
+      if (jg == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float p = ps[k + i];
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            float4 s = *reinterpret_cast<float4*>(S + (k + i) * NC + c + 16 * t);
+            float4 x = make_float4(acc[i][4 * t], acc[i][4 * t + 1], acc[i][4 * t + 2], acc[i][4 * t + 3]);
+#pragma unroll
+            for (int g = 0; g < JG - 1; ++g) {
+              const float4 y = *reinterpret_cast<const float4*>(part + (g * D + k + i) * NC + c + 16 * t);
+              x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+            }
+            *reinterpret_cast<float4*>(S + (k + i) * NC + c + 16 * t) =
+                make_float4(fmaf(p, s.x, x.x), fmaf(p, s.y, x.y), fmaf(p, s.z, x.z), fmaf(p, s.w, x.w));
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (slot >= 0)
+    for (int x = tid; x < D * (NC / 4); x += THREADS)
+      *reinterpret_cast<float4*>(sp + (long long)(x / (NC / 4)) * V + x % (NC / 4) * 4) = *reinterpret_cast<const float4*>(S + 4 * x);
+}
+
+// O of a chunk: [64][D + 64] x [D + 64][64], the rows of the second operand being the state the chunk meets and U.
+template <typename TI, int D, bool DELTA>
+__global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Args a) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int LDA = D + C + 4, NB = 64;
+  extern __shared__ __align__(16) float sm[];
+  float* A = sm;                                         // [C][LDA]: P q | M
+  float* B = A + C * LDA;                                // [D + C][NB]
+  int row0, n;
+  if (!find_chunk(a, blockIdx.x, row0, n)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int H = a.H, h = blockIdx.y, V = a.vdim, v0 = blockIdx.z * NB, nv = min(NB, V - v0);
+  const Place<D> in(a.scratch, (long long)blockIdx.x * H + h, V, DELTA);
+  for (int x = tid; x < C * (D / 4); x += THREADS) copy16(A + x / (D / 4) * LDA + x % (D / 4) * 4, in.qd + 4 * x);
+  for (int x = tid; x < C * (C / 4); x += THREADS) copy16(A + x / (C / 4) * LDA + D + x % (C / 4) * 4, in.m + 4 * x);
+  for (int x = tid; x < D * (nv / 4); x += THREADS) {
+    const int k = x / (nv / 4), c = x % (nv / 4) * 4;
+    copy16(B + k * NB + c, in.s + (long long)k * V + v0 + c);
+  }
+  for (int x = tid; x < C * (nv / 4); x += THREADS) {
+    const int k = x / (nv / 4), c = x % (nv / 4) * 4;
+    copy16(B + (D + k) * NB + c, in.u + (long long)k * V + v0 + c);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int r = (warp & 1) * 32 + (lane >> 2), c = (warp >> 1) * 16 + 4 * (lane & 3);
+  if ((warp >> 1) * 16 >= nv) return;
+  float acc[4][4] = {};
+  tile_product<1>(acc, A + r * LDA, LDA, B + c, NB, (warp & 1) ? D + C : D + C / 2);     // M is zero right of the diagonal
+  const float skip = a.skip ? a.skip[h] : 0.f;
+  const TI* vg = reinterpret_cast<const TI*>(a.v) + (long long)h * V + v0 + c;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = r + 8 * i;
+    if (t >= n) continue;
+    float4 o = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    if (a.skip) {
+      const float4 v = load4(vg + (long long)(row0 + t) * a.v_ld);
+      o.x = fmaf(skip, v.x, o.x); o.y = fmaf(skip, v.y, o.y); o.z = fmaf(skip, v.z, o.z); o.w = fmaf(skip, v.w, o.w);
+    }
+    *reinterpret_cast<float4*>(a.out + ((long long)(row0 + t) * H + h) * V + v0 + c) = o;
+  }
+}
+
+// Sizes and alignments that the kernels take: heads of 64 or 128 key channels, value heads a multiple of 16, rows of four
+// neighbouring numbers on a boundary of their size.
+template <typename TI>
+inline bool takes(const Args& a, int dim) {
+  auto fits = [](const void* p, long long ld) { return !((uintptr_t)p % (4 * sizeof(TI))) && ld % 4 == 0; };
+  return (dim == 64 || dim == 128) && a.vdim > 0 && a.vdim % 16 == 0 && fits(a.q, a.q_ld) && fits(a.k, a.k_ld) && fits(a.v, a.v_ld) &&
+         !((uintptr_t)a.decay & 15) && !((uintptr_t)a.state & 15) && !((uintptr_t)a.out & 15) && !((uintptr_t)a.bonus & 15) &&
+         !((uintptr_t)a.scratch & 15) && a.H <= 65535 && a.vdim / 16 <= 65535;
+}
+
+inline long long scratch_floats(int T, int S, int H, int dim, int vdim, bool delta) {
+  return (long long)(T / C + S) * H * (dim == 64 ? Place<64>::floats(vdim, delta) : Place<128>::floats(vdim, delta));
+}
+
+template <typename TI, int D, bool PERCH, bool DELTA, bool BONUS>
+int launch(const Args& a, int T, cudaStream_t s) {
+  constexpr int LDD = D + 4;
+  constexpr int BLK = PERCH ? 4 * D : 3 * SB * (SB + 1);
+  constexpr size_t prep = sizeof(float) * ((PERCH ? 3 : 2) * C * LDD + (DELTA ? 2 : PERCH ? 0 : 1) * C * LC + 2 * C + BLK);
+  constexpr size_t outs = sizeof(float) * (C * (D + C + 4) + (D + C) * 64);
+  static bool ok_prep[64], ok_out[64], ok_16[64], ok_32[64];
+  const unsigned chunks = (unsigned)(T / C + a.num_seqs);
+  auto prep_k = chunk_prep_kernel<TI, D, PERCH, DELTA, BONUS>;
+  int rc = allow_dynamic_smem(prep_k, (int)prep, ok_prep);
+  if (rc) return rc;
+  rc = launch_ex(prep_k, dim3(chunks, a.H), dim3(THREADS), prep, s, 1, a);
+  if (rc) return rc;
+  auto carry = [&](auto kernel, int nc, bool (&ok)[64]) {
+    constexpr int RG = D / 32, JG = 8 / RG;
+    const size_t stage = (DELTA ? C * (D + 4) : 0) + C * D + C * nc + D;
+    const size_t part = (size_t)nc * (DELTA && 4 * C > (JG - 1) * D ? 4 * C : (JG - 1) * D);
+    const size_t bytes = sizeof(float) * (2 * stage + D * nc + part);
+    const int rc2 = allow_dynamic_smem(kernel, (int)bytes, ok);
+    return rc2 ? rc2 : launch_ex(kernel, dim3(a.num_seqs, a.H, a.vdim / nc), dim3(THREADS), bytes, s, 1, a);
+  };
+  // 16 columns a CTA put twice as many CTAs on the walk; 32 read the rows of W and k half as often. The line is the number
+  // of SMs: with more CTAs than that a walk of 16 columns is two waves long.
+  if (a.vdim % 32 == 0 && (long long)a.num_seqs * a.H * (a.vdim / 16) > 148)
+    rc = carry(chunk_carry_kernel<D, 32, DELTA>, 32, ok_32);
+  else
+    rc = carry(chunk_carry_kernel<D, 16, DELTA>, 16, ok_16);
+  if (rc) return rc;
+  auto out_k = chunk_out_kernel<TI, D, DELTA>;
+  rc = allow_dynamic_smem(out_k, (int)outs, ok_out);
+  if (rc) return rc;
+  return launch_ex(out_k, dim3(chunks, a.H, (a.vdim + 63) / 64), dim3(THREADS), outs, s, 1, a);
+}
+
+}  // namespace chunked
+}  // namespace rllm

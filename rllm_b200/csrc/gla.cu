@@ -21,9 +21,11 @@
 //   (S_start of each chunk, the final state into the slot), pass FINAL runs each chunk again from its
 //   S_start and writes the outputs. Twice the arithmetic, chunks-fold the parallelism; sums are grouped
 //   differently than token by token, within float rounding.
+//   bfloat16 projections with heads of 64 or 128 key channels run long portions as products of matrices (chunk_scan.cuh).
 // gla_finish: one warp per (token, head): o / sqrt(mean(o^2) + eps) * w over vdim (w shared by the heads, or each head's
 //   own), times silu(gate).
 #include "common.cuh"
+#include "chunk_scan.cuh"
 using namespace rllm;
 
 namespace {
@@ -60,7 +62,7 @@ gla_scan_kernel(const TI* __restrict__ proj, long long ld, int q_off, int k_off,
                 const float* __restrict__ alpha, float qscale, int H, int dim, int vdim,
                 const int* __restrict__ cu_q, int num_seqs, const int* __restrict__ state_slots,
                 float* __restrict__ state, float* __restrict__ out, int chunk, float* __restrict__ chunk_state,
-                float* __restrict__ chunk_decay, int ch, const float* __restrict__ bonus) {
+                float* __restrict__ chunk_decay, int ch, const float* __restrict__ bonus, int long_from) {
   pdl_launch();
   pdl_wait();
   extern __shared__ __align__(16) float staged[];              // queries, keys, decays: [ch][dimp] each
@@ -73,6 +75,7 @@ gla_scan_kernel(const TI* __restrict__ proj, long long ld, int q_off, int k_off,
   if (MODE != WHOLE && !find_chunk(cu_q, num_seqs, chunk, blockIdx.x, seq, c, base)) return;
   int row0 = cu_q[seq], row1 = cu_q[seq + 1];
   if (MODE != WHOLE) { row0 += c * chunk; row1 = min(row1, row0 + chunk); }
+  else if (long_from > 0 && row1 - row0 >= long_from) return;          // another kernel's
   const int slot = (MODE == WHOLE && state_slots) ? state_slots[seq] : -1;
   const int dimp = (dim + 3) & ~3;               // a staged row, padded to 16 bytes
   float* qs = staged;
@@ -268,14 +271,14 @@ gla_finish_kernel(const float* __restrict__ o, const float* __restrict__ w, int 
 template <typename TI, int MODE, bool BONUS>
 int scan(dim3 grid, cudaStream_t s, const void* proj, long long ld, int q_off, int k_off, int v_off, const float* alpha,
          float qscale, int H, int dim, int vdim, const int* cu_q, int num_seqs, const int* state_slots, float* state,
-         float* out, int chunk, float* chunk_state, float* chunk_decay, int T, const float* bonus) {
+         float* out, int chunk, float* chunk_state, float* chunk_decay, int T, const float* bonus, int long_from) {
   const int kp = (dim + 3) / 4;
   // tokens staged at a time: 16 (8 for wide heads), 2 for steps of single tokens (the room goes to more CTAs an SM)
   const int ch = T <= 2 * num_seqs ? 2 : (dim <= 128 ? CH : CH / 2);
   const size_t smem = (size_t)3 * ch * ((dim + 3) & ~3) * sizeof(float);                             // at most 24 KB
 #define GO(KP)                                                                                                        \
   return launch_ex(gla_scan_kernel<TI, KP, MODE, BONUS>, grid, dim3(128), smem, s, 1, (const TI*)proj, ld, q_off, k_off, v_off, \
-                   alpha, qscale, H, dim, vdim, cu_q, num_seqs, state_slots, state, out, chunk, chunk_state, chunk_decay, ch, bonus)
+                   alpha, qscale, H, dim, vdim, cu_q, num_seqs, state_slots, state, out, chunk, chunk_state, chunk_decay, ch, bonus, long_from)
   if (kp <= 8) GO(8);
   if (kp <= 16) GO(16);
   if (kp <= 32) GO(32);
@@ -302,18 +305,36 @@ RLLM_API int rllm_gla_decay(float* z, const float* bias, int T, int n, float tau
 RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, int k_off, int v_off, const float* alpha,
                            float qscale, int T, int S, int H, int dim, int vdim, const int* cu_q,
                            const int* state_slots, float* state, float* out, int chunk, float* chunk_state,
-                           float* chunk_decay, const float* bonus, void* stream) {
+                           float* chunk_decay, const float* bonus, int long_from, int any_short, float* scratch, void* stream) {
   if (S <= 0 || T <= 0) return 0;
   if (H <= 0 || dim <= 0 || dim > MAX_DIM || vdim <= 0) return ERR_BAD_SIZE;
   if (H > 65535 || (vdim + 31) / 32 > 65535) return ERR_TOO_LARGE;
   if (dt != DT_F32 && dt != DT_BF16) return ERR_BAD_DTYPE;
   cudaStream_t s = (cudaStream_t)stream;
   const int vb = (vdim + 31) / 32;
+  if (scratch != nullptr && long_from > 0 && dt == DT_BF16) {
+    const bf16* p = (const bf16*)proj;
+    chunked::Args c = {};
+    c.q = p + q_off; c.k = p + k_off; c.v = p + v_off; c.q_ld = c.k_ld = c.v_ld = ld; c.q_heads = c.k_heads = H;
+    c.qscale = qscale; c.decay = alpha; c.bonus = bonus; c.H = H; c.vdim = vdim; c.cu_q = cu_q; c.num_seqs = S;
+    c.state_slots = state_slots; c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch;
+    if (chunked::takes<bf16>(c, dim)) {
+      const int rc = dim == 64 ? (bonus ? chunked::launch<bf16, 64, true, false, true>(c, T, s) : chunked::launch<bf16, 64, true, false, false>(c, T, s))
+                               : (bonus ? chunked::launch<bf16, 128, true, false, true>(c, T, s) : chunked::launch<bf16, 128, true, false, false>(c, T, s));
+      if (rc || !any_short) return rc;
+      chunk = 0;                                                       // the short sequences, row by row
+    } else {
+      long_from = 0;
+      if (!chunk_state) chunk = 0;
+    }
+  } else {
+    long_from = 0;
+  }
 #define SCAN_B(MODE, BONUS, GRID)                                                                                       \
   (dt == DT_F32 ? scan<float, MODE, BONUS>(GRID, s, proj, ld, q_off, k_off, v_off, alpha, qscale, H, dim, vdim, cu_q, S, \
-                                           state_slots, state, out, chunk, chunk_state, chunk_decay, T, bonus)          \
+                                           state_slots, state, out, chunk, chunk_state, chunk_decay, T, bonus, long_from)          \
                 : scan<bf16, MODE, BONUS>(GRID, s, proj, ld, q_off, k_off, v_off, alpha, qscale, H, dim, vdim, cu_q, S,  \
-                                          state_slots, state, out, chunk, chunk_state, chunk_decay, T, bonus))
+                                          state_slots, state, out, chunk, chunk_state, chunk_decay, T, bonus, long_from))
 #define SCAN(MODE, GRID) (bonus ? SCAN_B(MODE, true, GRID) : SCAN_B(MODE, false, GRID))
   if (chunk <= 0) return SCAN(WHOLE, dim3(S, H, vb));
   if (!chunk_state || !chunk_decay) return ERR_BAD_SIZE;
@@ -327,6 +348,14 @@ RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, in
   return SCAN(FINAL, dim3(chunks, H, vb));
 #undef SCAN
 #undef SCAN_B
+}
+
+// Floats of scratch that a (chunk of 64 rows, head) takes in the form for bfloat16 and heads of 64 or 128 (chunk_scan.cuh), asked
+// for by `scratch` and `long_from`: sequences of at least so many rows run in it, the others (any_short) row by row. 0: not taken.
+RLLM_API int rllm_gla_chunk_floats(int dim, int vdim) {
+  if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % 16) return 0;
+  const long long n = chunked::scratch_floats(0, 1, 1, dim, vdim, false);
+  return n < 2147483647LL ? (int)n : 0;
 }
 
 // o float [T, H, vdim]; w float [vdim], or [H * vdim] with w_heads; gate in proj at g_off (H x vdim, storage type); out [T, H * vdim].

@@ -17,9 +17,11 @@
 //   join their sums by shuffles); it keeps its share of S in registers while it walks the sequence's tokens, a few
 //   at a time through shared memory. The order of every sum depends on the sizes only, so a position's result is
 //   the same bits however its tokens were cut into steps. Queries and keys may be shared by groups of heads.
+//   Where the caller says so (`long_from`), sequences of at least that many rows run in chunks instead (chunk_scan.cuh).
 // gated_norm: per (token, group of columns) y / sqrt(mean(y^2) + eps) * w, with a gate act(g) applied to y before
 //   the norm or to the result after it; act silu or sigmoid.
 #include "common.cuh"
+#include "chunk_scan.cuh"
 using namespace rllm;
 
 namespace {
@@ -126,6 +128,7 @@ struct ScanArgs {
   const float* vscale;                                // [T, H] or null
   const float* skip;                                  // [H] or null
   int H, dim, vdim, split, ch, beta_bf16;
+  int long_from;                                      // sequences of at least so many rows are another kernel's (0: none)
   const int* cu_q; const int* state_slots;
   float* state;                                       // [slots, H, dim, vdim]
   float* out;                                         // [T, H, vdim]
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(128) state_scan_kernel(ScanArgs a) {
   const int v = blockIdx.z * cols + col;
   const bool vok = v < vdim;
   const int row0 = a.cu_q[seq], row1 = a.cu_q[seq + 1];
+  if (a.long_from > 0 && row1 - row0 >= a.long_from) return;
   const int slot = a.state_slots ? a.state_slots[seq] : -1;
   const int qh = h / (H / a.q_heads), kh = h / (H / a.k_heads);
   float S[R];
@@ -278,6 +282,7 @@ __global__ void __launch_bounds__(128) state_scan_fast_kernel(ScanArgs a) {
   const int v = blockIdx.z * COLS + col;
   const bool vok = v < vdim;
   const int row0 = a.cu_q[seq], row1 = a.cu_q[seq + 1];
+  if (a.long_from > 0 && row1 - row0 >= a.long_from) return;
   const int slot = a.state_slots ? a.state_slots[seq] : -1;
   const int qh = h / (H / a.q_heads), kh = h / (H / a.k_heads);
   float S[R];
@@ -472,6 +477,22 @@ RLLM_API int rllm_softplus_decay(int dt, const void* z, long long ld, int col0, 
   return ERR_BAD_DTYPE;
 }
 
+// Floats of scratch that a (chunk of 64 rows, head) of the chunked form takes; 0: these sizes do not run in chunks.
+RLLM_API int rllm_state_scan_chunk_floats(int dim, int vdim, int delta) {
+  if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % 16) return 0;
+  const long long n = chunked::scratch_floats(0, 1, 1, dim, vdim, delta != 0);
+  return n < 2147483647LL ? (int)n : 0;
+}
+
+static int launch_chunked(const chunked::Args& c, int dim, bool perch, bool delta, int T, cudaStream_t s) {
+#define RLLM_CH(D, P, DL) \
+  if (dim == D && perch == P && delta == DL) return chunked::launch<float, D, P, DL, false>(c, T, s)
+  RLLM_CH(64, false, false); RLLM_CH(64, false, true); RLLM_CH(64, true, false); RLLM_CH(64, true, true);
+  RLLM_CH(128, false, false); RLLM_CH(128, false, true); RLLM_CH(128, true, false); RLLM_CH(128, true, true);
+#undef RLLM_CH
+  return ERR_BAD_SIZE;
+}
+
 // How the key channels of a head are dealt to lanes: `split` neighbouring lanes share a value column.
 RLLM_API int rllm_state_scan_split(int dim) {
   int split = 1;
@@ -493,7 +514,7 @@ RLLM_API int rllm_state_scan(int beta_dt, const float* q, long long q_ld, int q_
                              int k_heads, const float* v, long long v_ld, const float* decay, int decay_per_channel,
                              const void* beta, long long beta_ld, const float* vscale, const float* skip, int S, int H,
                              int dim, int vdim, const int* cu_q, const int* state_slots, float* state, float* out,
-                             int channels, void* stream) {
+                             int channels, int T, int long_from, int any_short, float* scratch, void* stream) {
   if (S <= 0) return 0;
   if (H <= 0 || dim <= 0 || dim > 1024 || vdim <= 0 || q_heads <= 0 || k_heads <= 0 || H % q_heads || H % k_heads)
     return ERR_BAD_SIZE;
@@ -506,6 +527,19 @@ RLLM_API int rllm_state_scan(int beta_dt, const float* q, long long q_ld, int q_
   a.beta_bf16 = beta != nullptr && beta_dt == DT_BF16;
   if (beta != nullptr && beta_dt != DT_BF16 && beta_dt != DT_F32) return ERR_BAD_DTYPE;
   cudaStream_t s = (cudaStream_t)stream;
+  a.long_from = 0;
+  if (long_from > 0 && scratch != nullptr) {
+    chunked::Args c = {};
+    c.q = q; c.k = k; c.v = v; c.q_ld = q_ld; c.k_ld = k_ld; c.v_ld = v_ld; c.q_heads = q_heads; c.k_heads = k_heads;
+    c.qscale = 1.f; c.decay = decay; c.beta = beta; c.beta_ld = beta_ld; c.beta_bf16 = a.beta_bf16; c.vscale = vscale;
+    c.skip = skip; c.H = H; c.vdim = vdim; c.cu_q = cu_q; c.num_seqs = S; c.state_slots = state_slots;
+    c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch;
+    if (chunked::takes<float>(c, dim)) {
+      const int rc = launch_chunked(c, dim, decay_per_channel != 0, beta != nullptr, T, s);
+      if (rc || !any_short) return rc;
+      a.long_from = long_from;
+    }
+  }
   if (const int r = scan_fast_channels(dim, channels)) {
     a.split = dim / r;
     const int fcols = 128 / a.split, ldk = a.split * (r + 4);

@@ -16,6 +16,11 @@ class GroupView:
     page_size: int
 
 
+# Rows of a portion from which a recurrence runs in chunks: three launches cost some 50 us at 64 rows (16 heads of 128 x 128,
+# delta rule) where row by row takes 31, 63 against 72 at 128 rows, 341 against 1,058 at 2,048
+LONG_FROM = 128
+
+
 @dataclass
 class StepContext:
     """One batch: T tokens of S sequences, rows of a sequence adjacent and in order.
@@ -50,3 +55,10 @@ class StepContext:
     @property
     def all_decode(self) -> bool:
         return self.max_q_len == 1
+
+    def long_rows(self) -> dict:
+        """What a recurrence's scan is told about a step with long portions: from how many rows on a sequence runs in
+        chunks of 64 as products of matrices, and whether there are shorter ones beside it."""
+        if self.graph_safe or self.max_q_len < LONG_FROM:
+            return {}
+        return {"long_from": LONG_FROM, "any_short": min(self.q_lens_host) < LONG_FROM}

@@ -522,8 +522,10 @@ class Backend:
         return self._hy.softplus_decay(*a, **k)
 
     def state_scan(self, q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx, state, beta=None, vscale=None, skip=None):
+        # the 32-bit run's results are the same bits however a sequence is cut into steps: row by row
+        long = ctx.long_rows() if self.dtype == torch.bfloat16 else {}
         return self._hy.state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx.cu_q, ctx.num_seqs,
-                                   ctx.state_slots, state, beta, vscale, skip)
+                                   ctx.state_slots, state, beta, vscale, skip, **long)
 
     def gated_norm(self, y, gate, gate_col0, weight, eps, groups, gate_first, act):
         return self._hy.gated_norm(y, gate, gate_col0, weight, eps, groups, self.dtype, gate_first, act)

@@ -71,7 +71,7 @@ class GatedLinearAttention(Part):
         z = be.linear_f32(proj[:, self._a1_off:], self.w_a2)             # float decay logits [T, H * dim]
         alpha = be.gla_decay(z, self._b_f32, self.tau)                   # in place
         o = be.gla_scan(proj, 0, H * d, 2 * H * d, alpha, d ** -0.5, H, d, v, ctx.cu_q, ctx.num_seqs,
-                        ctx.state_slots, cache.state["S"], scan_chunk(ctx, self.chunk))
+                        ctx.state_slots, cache.state["S"], scan_chunk(ctx, self.chunk), **ctx.long_rows())
         att = be.gla_finish(o, self._norm_f32, self.eps, proj, 2 * H * d + H * v)
         if residual is None:
             return be.linear_f32(att, self.w_o)
@@ -120,7 +120,7 @@ class TimeMixing(Part):
         proj = be.linear_mixes(x, self.w_in, C, tag="in")                # [T, r | k | v | g | w1]
         decay = be.lowrank_decay(proj[:, 4 * C:], self._w2_t, self._w0)   # float [T, C]
         o = be.gla_scan(proj, 0, C, 2 * C, decay, 1.0, H, d, d, ctx.cu_q, ctx.num_seqs, ctx.state_slots, cache.state["S"],
-                        scan_chunk(ctx, self.chunk), bonus=self._u)
+                        scan_chunk(ctx, self.chunk), bonus=self._u, **ctx.long_rows())
         return be.linear_f32(be.gla_finish(o, self._norm_f32, self.eps, proj, 3 * C), self.w_o, tag="o"), n2
 
 

@@ -1,0 +1,125 @@
+"""Recurrences in chunks of 64 rows as products of matrices (csrc/chunk_scan.cuh) against the recurrence itself in 64 bits,
+token by token, beside the row-by-row kernels on the same inputs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+def rnd(*shape, seed, scale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(DEV)
+
+
+def decays(*shape, seed):
+    """Mostly near one, some strong, some so strong that a few of them leave nothing."""
+    g = torch.Generator().manual_seed(seed)
+    x = torch.rand(*shape, generator=g)
+    return torch.where(x < 0.85, 1 - 0.05 * x, torch.where(x < 0.97, x - 0.8, torch.where(x < 0.99, 1e-20, 0.0))).to(DEV)
+
+
+def recurrence(q, k, v, a, S, beta=None, bonus=None):
+    """One sequence in 64 bits: q, k, a [n, H, d] (a of 1 or d channels), v [n, H, dv], S [H, d, dv]."""
+    S, out = S.clone(), []
+    for t in range(q.shape[0]):
+        before = S
+        S = a[t][:, :, None] * S
+        u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        kv = k[t][:, :, None] * u[:, None]
+        S = S + kv
+        out.append(torch.einsum("hkv,hk->hv", S if bonus is None else before + bonus[:, :, None] * kv, q[t]))
+    return torch.stack(out), S
+
+
+def layout(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return cu, torch.tensor(cu, dtype=torch.int32, device=DEV)
+
+
+# lengths at the edges of blocks of 16 and chunks of 64, beside rows that stay with the other kernel
+LENS = [(64,), (65, 1, 130), (127, 3, 64, 81), (512, 66)]
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("dim,vdim,H,G", [(128, 128, 4, 2), (64, 48, 6, 3), (128, 64, 8, 2), (128, 16, 40, 40)])
+@pytest.mark.parametrize("channel", [True, False])
+@pytest.mark.parametrize("delta", [True, False])
+def test_state_scan_in_chunks(lens, dim, vdim, H, G, channel, delta):
+    from rllm_b200.kernels import hybrid
+    cu, cud = layout(lens)
+    T, S = cu[-1], len(lens)
+    q = torch.nn.functional.normalize(rnd(T, G, dim, seed=1), dim=-1)
+    k = torch.nn.functional.normalize(rnd(T, G, dim, seed=2), dim=-1)
+    v = rnd(T, H * vdim, seed=3)
+    a = decays(T, H, dim if channel else 1, seed=4)
+    beta = rnd(T, H + 3, seed=5)[:, :H] if delta else None
+    vs, skip = (None, None) if delta else (rnd(T, H, seed=6), rnd(H, seed=7))
+    slots = torch.tensor([-1 if s == 1 else S - s for s in range(S)], dtype=torch.int32, device=DEV)
+    state = rnd(S + 1, H, dim, vdim, seed=8)
+    got = {}
+    for name, long in (("chunks", dict(long_from=64, any_short=min(lens) < 64)), ("rows", {})):
+        st = state.clone()
+        o = hybrid.state_scan(q.view(T, -1), G, k.view(T, -1), G, v, a.view(T, -1), H, dim, vdim, cud, S, slots, st, beta=beta,
+                              vscale=vs, skip=skip, **long)
+        got[name] = (o, st)
+    d = lambda x: x.double()
+    which = torch.arange(H, device=DEV) // (H // G)
+    keep = state.double()
+    want = []
+    for s, n in enumerate(lens):
+        r, sl = slice(cu[s], cu[s + 1]), int(slots[s])
+        u = d(v[r]).view(n, H, vdim)
+        o, end = recurrence(d(q[r])[:, which], d(k[r])[:, which], u if delta else u * d(vs[r])[:, :, None], d(a[r]),
+                            keep[sl] if sl >= 0 else torch.zeros_like(keep[0]), torch.sigmoid(d(beta[r])) if delta else None)
+        want.append(o if delta else o + d(skip)[:, None] * u)
+        if sl >= 0:
+            keep[sl] = end
+    want = torch.cat(want)
+    e = {name: (rel(o, want), rel(st, keep)) for name, (o, st) in got.items()}
+    # sums of up to 128 + 64 products in float: some 5e-7 either way
+    assert e["chunks"][0] < 2e-6 and e["chunks"][1] < 2e-6, e
+    assert torch.equal(got["chunks"][1][0], state[0])                      # a slot of nobody's
+    if min(lens) < 64:
+        s = min(range(S), key=lambda i: lens[i])
+        assert torch.equal(got["chunks"][0][cu[s]: cu[s + 1]], got["rows"][0][cu[s]: cu[s + 1]])
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("dim,vdim,H", [(128, 128, 3), (64, 80, 5), (64, 16, 160)])
+@pytest.mark.parametrize("bonus", [True, False])
+def test_gated_linear_attention_in_chunks(lens, dim, vdim, H, bonus):
+    from rllm_b200.kernels import mix
+    cu, cud = layout(lens)
+    T, S = cu[-1], len(lens)
+    proj = rnd(T, 8 + H * (2 * dim + vdim), seed=1).bfloat16()
+    a, u = decays(T, H * dim, seed=2), rnd(H, dim, seed=3) if bonus else None
+    slots = torch.tensor([-1 if s == 1 else S - s for s in range(S)], dtype=torch.int32, device=DEV)
+    state = rnd(S + 1, H, dim, vdim, seed=4)
+    got = {}
+    for name, long in (("chunks", dict(long_from=64, any_short=min(lens) < 64)), ("rows", {})):
+        st = state.clone()
+        o = mix.gla_scan(proj, 8, 8 + H * dim, 8 + 2 * H * dim, a, dim ** -0.5, H, dim, vdim, cud, S, slots, st, bonus=u, **long)
+        got[name] = (o, st)
+    p, keep, want = proj.double(), state.double(), []
+    for s, n in enumerate(lens):
+        r, sl = slice(cu[s], cu[s + 1]), int(slots[s])
+        q, k = (p[r, 8 + i * H * dim: 8 + (i + 1) * H * dim].view(n, H, dim) for i in (0, 1))
+        o, end = recurrence(q * dim ** -0.5, k, p[r, 8 + 2 * H * dim:].view(n, H, vdim), a[r].double().view(n, H, dim),
+                            keep[sl] if sl >= 0 else torch.zeros_like(keep[0]), bonus=u.double() if bonus else None)
+        want.append(o)
+        if sl >= 0:
+            keep[sl] = end
+    want = torch.cat(want)
+    e = {name: (rel(o, want), rel(st, keep)) for name, (o, st) in got.items()}
+    assert e["chunks"][0] < 2e-6 and e["chunks"][1] < 2e-6, e
+    assert torch.equal(got["chunks"][1][0], state[0])
+    if min(lens) < 64:
+        s = min(range(S), key=lambda i: lens[i])
+        assert torch.equal(got["chunks"][0][cu[s]: cu[s + 1]], got["rows"][0][cu[s]: cu[s + 1]])
