@@ -59,29 +59,31 @@ constexpr int THREADS = (LOADERS + 1 + 4 * RT) * 32;
 // registers per thread: 168 each at launch (65,536 / 384, in eights); then 4 warps keep 56 and 8 warps have 224
 constexpr int REGS_LOW = 56, REGS_HIGH = 224;
 static_assert(SOFTMAX_WARP0 * 32 * REGS_LOW + 4 * RT * 32 * REGS_HIGH <= 168 * THREADS, "more registers than the launch has");
-constexpr int KV_TILE_BYTES = 16384;             // one K or V tile: 128 keys of 64 values, or 64 keys of 128
-constexpr int KVS = 4;           // K/V stages with TMA (one loader, tile after tile). Without TMA only LOADERS of them
+                                 // K/V stages with TMA (one loader, tile after tile): Shape::KVS. Without TMA only LOADERS of them
                                  // are used: loader warp w always fills stage w (tiles w, w + 3, ...), so its waits
                                  // on that stage's barriers follow one another phase by phase; a warp that moved
                                  // between stages could be two phases ahead, which a parity cannot tell
 constexpr int SB = 3;            // S accumulators: one per row tile in its softmax, one being computed ahead
 constexpr int TMEM_COLS = 512;
 
-// Sizes that follow from the head size (64 or 128). Operands lie in shared memory as "atoms" of
-// 128-byte rows (64 values), swizzled: a tile wider than 64 values is several atoms one after the other.
-template <int HD> struct Shape {
-  static_assert(HD == 64 || HD == 128, "head sizes 64 and 128");
-  static constexpr int PN = HD == 64 ? 128 : 64;     // keys per tile (a K or V tile is 16 KB either way)
-  static constexpr int HA = HD / 64;                 // atoms along the head dimension (Q, K, V)
+// Sizes that follow from the head sizes: keys of KD and values of VD numbers, 64 / 64, 128 / 128 or 192 / 128. Operands lie in
+// shared memory as "atoms" of 128-byte rows (64 values), swizzled: a tile wider than 64 values is several atoms one after
+// the other. With keys of 192 the queries leave room for two stages.
+template <int KD, int VD> struct Shape {
+  static_assert((KD == 64 && VD == 64) || (KD == 128 && VD == 128) || (KD == 192 && VD == 128), "head sizes");
+  static constexpr int PN = KD == 64 ? 128 : 64;     // keys per tile (a V tile is 16 KB either way)
+  static constexpr int KVS = KD == 192 ? 2 : 4;      // K/V stages
+  static constexpr int HA = KD / 64;                 // atoms along the head dimension (Q, K)
+  static constexpr int VA = VD / 64;                 // (V)
   static constexpr int KA = PN / 64;                 // atoms along the keys (P)
   static constexpr int ATOM_ROWS = PM * 128;         // bytes of one atom of Q or P (128 rows)
   static constexpr int ATOM_KEYS = PN * 128;         // bytes of one atom of K or V (PN rows)
+  static constexpr int K_BYTES = HA * ATOM_KEYS, V_BYTES = VA * ATOM_KEYS;     // one tile
   static constexpr int Q_BYTES = HA * ATOM_ROWS;     // one row tile of Q
   static constexpr int P_BYTES = KA * ATOM_ROWS;     // one row tile of P
-  static constexpr int SMEM_BYTES = 1024 + RT * Q_BYTES + 2 * KVS * KV_TILE_BYTES + RT * P_BYTES;   // Q[2], K[KVS], V[KVS], P[2]
+  static constexpr int SMEM_BYTES = 1024 + RT * Q_BYTES + KVS * (K_BYTES + V_BYTES) + RT * P_BYTES;   // Q[2], K[KVS], V[KVS], P[2]
   static constexpr int S_COL = 0, O_COL = SB * PN;   // TMEM: three S accumulators, then the output of both row tiles
-  static_assert(O_COL + RT * HD <= TMEM_COLS, "S and the outputs must fit in TMEM");
-  static_assert(HA * ATOM_KEYS == KV_TILE_BYTES, "a K or V tile is 16 KB");
+  static_assert(O_COL + RT * VD <= TMEM_COLS, "S and the outputs must fit in TMEM");
 };
 
 struct PfParams {
@@ -101,6 +103,15 @@ struct PfParams {
   float cap_z;           // scale / cap
   int box_rows;          // TMA variant: keys per copy = min(page size, 128)
   int row_pairs, num_seqs, sm_count;
+  int long_from;         // sequences with fewer rows are left out (another kernel's)
+  float* cross;          // not null: every query head meets every kv head's values, and the output is the floats
+                         // [token][query head][kv head of the values][VD] here
+  // DENSE: keys and values of a sequence lie one after the other (a row per position, the sequences that are not left out
+  // in order), the maps see them as [heads][rows][128]; with KD 192 the last 64 numbers of a key are shared by the heads
+  // (map tmap_r) and those of a query lie in rows of their own
+  int q_head;            // numbers between a row's query heads
+  const bf16* q2; long long q2_stride; int q2_head;
+  const bf16* gate_h; int gate_h_ld, gate_cols;   // logits [T, gate_h_ld] or null: a column per head, or (gate_cols) per output
   float scale_log2e;
   int* err;
 };
@@ -165,10 +176,14 @@ __device__ __forceinline__ void softcap_poly2(uint32_t& x0, uint32_t& x1, float 
 
 // TMA: the K and V tiles come by tensor copies over the caches seen as [pages * kv heads][page size][HD].
 // CAP: scores are bounded (p.cap).
-template <int HD, bool TMA, bool CAP>
+// DENSE: keys and values as in PfParams, by tensor copies of whole tiles.
+template <int KD, int VD, bool TMA, bool CAP, bool DENSE>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                       const PfParams p) {
+                       const __grid_constant__ CUtensorMap tmap_r, const PfParams p) {
+  static_assert(TMA || !DENSE, "dense keys come by tensor copies");
+  typedef Shape<KD, VD> C;
+  constexpr int KVS = C::KVS;
   extern __shared__ uint8_t pf_smem_raw[];
   __shared__ __align__(8) uint64_t kv_full[KVS], kv_empty[KVS], s_full[SB], s_free[SB], p_full[RT], pv_full[RT], q_full;
   __shared__ uint32_t tmem_base_slot;
@@ -176,10 +191,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* smem = (uint8_t*)(((uintptr_t)pf_smem_raw + 1023) & ~(uintptr_t)1023);
-  typedef Shape<HD> C;
   constexpr int PN = C::PN;
   const uint32_t q_s = smem_u32(smem);
-  const uint32_t k_s = q_s + RT * C::Q_BYTES, v_s = k_s + KVS * KV_TILE_BYTES, p_s = v_s + KVS * KV_TILE_BYTES;
+  const uint32_t k_s = q_s + RT * C::Q_BYTES, v_s = k_s + KVS * C::K_BYTES, p_s = v_s + KVS * C::V_BYTES;
 
   const int G = p.nh / p.nkv;
   constexpr int NST = TMA ? KVS : LOADERS;              // K/V stages in use
@@ -190,7 +204,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     // an earlier kernel left here need not be zero: start from zeros (later leftovers are keys).
     if (warp == 0 && lane == 0) { prefetch_tensormap(&tmap_k); prefetch_tensormap(&tmap_v); }
     uint4* kv = reinterpret_cast<uint4*>(smem + RT * C::Q_BYTES);
-    for (int i = threadIdx.x; i < 2 * KVS * KV_TILE_BYTES / 16; i += THREADS) kv[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < KVS * (C::K_BYTES + C::V_BYTES) / 16; i += THREADS) kv[i] = make_uint4(0, 0, 0, 0);
     fence_proxy_async();
   }
   if (warp == MMA_WARP) { tmem_alloc(&tmem_base_slot, TMEM_COLS); tmem_relinquish(); }
@@ -210,14 +224,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   // walks the items in its own copy of the loop (the block-wide barriers are the same ones).
   auto walk = [&](auto softmax_side) {
   constexpr bool SOFTMAX = decltype(softmax_side)::value;
-  const int items = p.row_pairs * p.nkv * p.num_seqs;
+  const int vheads = p.cross ? p.nkv : 1;
+  const int items = p.row_pairs * p.nkv * vheads * p.num_seqs;
   for (int round = 0;; ++round) {
   const int item = round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
   if (item >= items) break;
-  const int tile0 = (p.row_pairs - 1 - item / (p.nkv * p.num_seqs)) * RT;      // first of the item's row tiles
-  const int kvh = item % p.nkv, seq = (item / p.nkv) % p.num_seqs;
+  const int tile0 = (p.row_pairs - 1 - item / (p.nkv * vheads * p.num_seqs)) * RT;      // first of the item's row tiles
+  const int kvh = item % p.nkv, seq = (item / (p.nkv * vheads)) % p.num_seqs;
+  const int vh = p.cross ? item / p.nkv % p.nkv : kvh;                         // the kv head of the values
   // an item beyond its sequence's rows (a short portion beside long ones) is skipped by all threads alike
-  if (tile0 * PM >= (p.cu_q[seq + 1] - p.cu_q[seq]) * G) continue;
+  if (tile0 * PM >= (p.cu_q[seq + 1] - p.cu_q[seq]) * G || p.cu_q[seq + 1] - p.cu_q[seq] < p.long_from) continue;
   __syncthreads();                                      // everybody has left the item before
   if (threadIdx.x == 0) {
     for (int i = 0; i < KVS; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
@@ -265,7 +281,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       const int row = tile0 * PM + r;
       const bool valid = row < rows_total;
       const int tok = valid ? row / G : 0, head = kvh * G + (valid ? row % G : 0);
-      const bf16* src = p.q + (size_t)(q0 + tok) * p.q_stride + (size_t)head * HD + ch * 8;
+      const bf16* src = p.q + (size_t)(q0 + tok) * p.q_stride + (size_t)head * KD + ch * 8;
       const uint32_t dst = q_s + (uint32_t)((r / PM) * C::Q_BYTES + (r % PM) * 128 + ((ch ^ (r & 7)) << 4));
 #pragma unroll
       for (int a = 0; a < C::HA; ++a) cp_async16z(dst + (uint32_t)(a * C::ATOM_ROWS), src + a * 64, valid);
@@ -296,10 +312,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       abort_flag = 1; record_failure(p.err, 22, t); ok = false; return;
     }
     tc_fence_after();
-    const uint64_t dq = dq0 + (uint64_t)(g * (C::Q_BYTES >> 4)), dk = dk0 + (uint64_t)(ks * (KV_TILE_BYTES >> 4));
+    const uint64_t dq = dq0 + (uint64_t)(g * (C::Q_BYTES >> 4)), dk = dk0 + (uint64_t)(ks * (C::K_BYTES >> 4));
     const uint32_t acc = tmem_base + C::S_COL + (uint32_t)(k % SB) * PN;
 #pragma unroll
-    for (int kk = 0; kk < HD / 16; ++kk)                // 16 values a product: atom kk / 4, 32 bytes on within it
+    for (int kk = 0; kk < KD / 16; ++kk)                // 16 values a product: atom kk / 4, 32 bytes on within it
       umma_bf16(acc, dq + (uint64_t)((kk >> 2) * (C::ATOM_ROWS >> 4) + (kk & 3) * 2),
                 dk + (uint64_t)((kk >> 2) * (C::ATOM_KEYS >> 4) + (kk & 3) * 2), id_s, kk > 0);
     umma_commit(&s_full[k % SB]);
@@ -312,10 +328,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       abort_flag = 1; record_failure(p.err, 23, t); ok = false; return;
     }
     tc_fence_after();
-    const uint64_t dp = dp0 + (uint64_t)(g * (C::P_BYTES >> 4)), dv = dv0 + (uint64_t)((t % NST) * (KV_TILE_BYTES >> 4));
-    const uint32_t acc = tmem_base + C::O_COL + (uint32_t)g * HD;
+    const uint64_t dp = dp0 + (uint64_t)(g * (C::P_BYTES >> 4)), dv = dv0 + (uint64_t)((t % NST) * (C::V_BYTES >> 4));
+    const uint32_t acc = tmem_base + C::O_COL + (uint32_t)g * VD;
 #pragma unroll
-    for (int a = 0; a < C::HA; ++a)                     // 64 output values = one atom of V
+    for (int a = 0; a < C::VA; ++a)                     // 64 output values = one atom of V
 #pragma unroll
       for (int ks = 0; ks < PN / 16; ++ks) {
         // P: K-major, atoms of 64 keys, 32 bytes per 16 keys; V: MN-major, 16 key rows = 2 KB per step
@@ -330,7 +346,31 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     // Lane c looks up the page of the tile's c-th copy; lane 0 tells the stage's barrier how many
     // bytes are coming; every lane with a page issues its two copies. Nothing waits for a tile to
     // land: up to NST tiles are on their way.
-    if (warp == 0) {
+    if (warp == 0 && DENSE) {
+      // a lane a copy: the atoms of K that are the head's own, those of V, the one of K that the heads share
+      int base = 0;                                        // the sequence's first row: the keys of those before it
+      for (int i = lane; i < seq; i += 32) base += p.cu_q[i + 1] - p.cu_q[i] < p.long_from ? 0 : p.kv_lens[i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+      constexpr int KO = KD == 192 ? 2 : C::HA;
+      for (int t = 0; t < n_tiles; ++t) {
+        const int s = t % NST;
+        if (t >= NST) {
+          int w_ok = 1;
+          if (lane == 0 && !mbar_wait(&kv_empty[s], (uint32_t)(t / NST - 1) & 1u, &abort_flag)) {
+            abort_flag = 1; record_failure(p.err, 21, t); w_ok = 0;
+          }
+          if (__shfl_sync(0xffffffffu, w_ok, 0) == 0) break;
+        }
+        if (lane == 0) mbar_expect_tx(&kv_full[s], C::K_BYTES + C::V_BYTES);
+        __syncwarp();
+        const int row = base + tile_first(t);
+        const uint32_t kd = k_s + (uint32_t)(s * C::K_BYTES), vd = v_s + (uint32_t)(s * C::V_BYTES);
+        if (lane < KO) tma_load_3d(kd + (uint32_t)(lane * C::ATOM_KEYS), &tmap_k, &kv_full[s], lane * 64, row, kvh);
+        else if (lane < KO + C::VA) tma_load_3d(vd + (uint32_t)((lane - KO) * C::ATOM_KEYS), &tmap_v, &kv_full[s], (lane - KO) * 64, row, kvh);
+        else if (KD == 192 && lane == KO + C::VA) tma_load_3d(kd + (uint32_t)(2 * C::ATOM_KEYS), &tmap_r, &kv_full[s], 0, row, 0);
+      }
+    } else if (warp == 0) {
       const int* bt = p.block_table + (size_t)seq * p.bt_stride;
       const int copies = PN / p.box_rows;                  // runs of keys per tile; each is one copy per atom and cache
       const uint32_t copy_bytes = (uint32_t)p.box_rows * 128;
@@ -351,10 +391,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         if (lane == 0) mbar_expect_tx(&kv_full[s], 2 * n * copy_bytes);
         __syncwarp();
         if (mine) {
-          const uint32_t dst = (uint32_t)s * KV_TILE_BYTES + (uint32_t)at * C::ATOM_KEYS + (uint32_t)cp * copy_bytes;
+          const uint32_t dst = (uint32_t)(s * C::K_BYTES) + (uint32_t)at * C::ATOM_KEYS + (uint32_t)cp * copy_bytes;
           const int off = j & (p.page_size - 1);
           tma_load_3d(k_s + dst, &tmap_k, &kv_full[s], at * 64, off, page * p.nkv + kvh);
-          tma_load_3d(v_s + dst, &tmap_v, &kv_full[s], at * 64, off, page * p.nkv + kvh);
+          tma_load_3d(v_s + dst, &tmap_v, &kv_full[s], at * 64, off, page * p.nkv + vh);
         }
       }
     } else if (warp == 2) {
@@ -385,7 +425,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       }
       if (t == 0) load_q(0, RT * PM);                     // lands with the tile, announced by its barrier
       const int j0 = tile_first(t);
-      const uint32_t kd = k_s + (uint32_t)s * KV_TILE_BYTES, vd = v_s + (uint32_t)s * KV_TILE_BYTES;
+      const uint32_t kd = k_s + (uint32_t)(s * C::K_BYTES), vd = v_s + (uint32_t)(s * C::V_BYTES);
 #pragma unroll 1
       for (int i0 = 0; i0 < PN / 4; i0 += 8) {
         int page[8];
@@ -401,7 +441,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           const int j = j0 + r;
           const int off = p.page_shift >= 0 ? (j & (p.page_size - 1)) : j % p.page_size;
           const bool valid = page[i] >= 0;
-          const size_t src = valid ? ((((size_t)page[i] * p.nkv + kvh) * p.page_size + off) * HD + ch * 8) : 0;
+          const size_t src = valid ? ((((size_t)page[i] * p.nkv + kvh) * p.page_size + off) * KD + ch * 8) : 0;
           const uint32_t dst = (uint32_t)(r * 128 + ((ch ^ (r & 7)) << 4));
 #pragma unroll
           for (int a = 0; a < C::HA; ++a) {
@@ -450,13 +490,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     if (TMA) {
       // this thread's own row of Q into the A-operand layout (rows beyond the sequence zero), while the
       // first K and V tiles are on their way
-      const bf16* src = p.q + (size_t)(q0 + tok) * p.q_stride + (size_t)head * HD;
+      const bf16* src = p.q + (size_t)(q0 + tok) * p.q_stride + (size_t)head * (DENSE ? p.q_head : KD);
+      const bf16* src2 = KD == 192 ? p.q2 + (size_t)(q0 + tok) * p.q2_stride + (size_t)head * p.q2_head : src;
       const uint32_t drow = q_s + (uint32_t)(g * C::Q_BYTES + r * 128);
 #pragma unroll
       for (int a = 0; a < C::HA; ++a)
 #pragma unroll
         for (int ch = 0; ch < 8; ++ch)
-          cp_async16z(drow + (uint32_t)(a * C::ATOM_ROWS) + (uint32_t)((ch ^ (r & 7)) << 4), src + a * 64 + ch * 8, valid);
+          cp_async16z(drow + (uint32_t)(a * C::ATOM_ROWS) + (uint32_t)((ch ^ (r & 7)) << 4), (KD == 192 && a == 2 ? src2 : src + a * 64) + ch * 8, valid);
       cp_async_commit();
       cp_async_wait<0>();
       fence_proxy_async();
@@ -464,7 +505,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       if (lane == 0) mbar_arrive(&q_full);
     }
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t pv_addr = lane_addr + C::O_COL + (uint32_t)g * HD;
+    const uint32_t pv_addr = lane_addr + C::O_COL + (uint32_t)g * VD;
     const uint32_t prow = p_s + (uint32_t)g * C::P_BYTES + (uint32_t)(r * 128);
     constexpr int NC = PN / 32;                           // the row's scores come 32 at a time
     const float sl = CAP ? 1.f : p.scale_log2e;        // bounded scores leave the bound in the log2 domain
@@ -549,7 +590,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         if (__any_sync(0xffffffffu, move)) {
           tc_fence_after();
 #pragma unroll
-          for (int c = 0; c < HD / 16; ++c) {
+          for (int c = 0; c < VD / 16; ++c) {
             uint32_t ov[16];
             tmem_ld16(pv_addr + 16 * c, ov);
             tmem_ld_wait();
@@ -598,13 +639,38 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       tc_fence_after();
       float inv = sig ? 1.f : (l > 0.f ? 1.f / l : 0.f);
       if (p.gate && valid) inv *= 1.f / (1.f + __expf(-p.gate[(size_t)(q0 + tok) * p.gate_ld + head]));
-      bf16* dst = p.out + (size_t)(q0 + tok) * p.out_stride + (size_t)head * HD;
+      const bf16* gh = nullptr;
+      if (DENSE && p.gate_h && valid) {
+        gh = p.gate_h + (size_t)(q0 + tok) * p.gate_h_ld + (p.gate_cols ? head * VD : head);
+        if (!p.gate_cols) { inv *= 1.f / (1.f + __expf(-__bfloat162float(*gh))); gh = nullptr; }
+      }
+      bf16* dst = p.out + (size_t)(q0 + tok) * p.out_stride + (size_t)head * VD;
+      float* fdst = p.cross ? p.cross + (((size_t)(q0 + tok) * p.nh + head) * p.nkv + vh) * VD : nullptr;
 #pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
+      for (int c = 0; c < VD / 32; ++c) {
         uint32_t ov[32];
         tmem_ld32(pv_addr + 32 * c, ov);
         tmem_ld_wait();
-        if (valid) {
+        if (valid && fdst) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(fdst + 32 * c + i) =
+                make_float4(__uint_as_float(ov[i]) * inv, __uint_as_float(ov[i + 1]) * inv, __uint_as_float(ov[i + 2]) * inv,
+                            __uint_as_float(ov[i + 3]) * inv);
+        } else if (valid) {
+          if (DENSE && gh) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              const uint4 g8 = *reinterpret_cast<const uint4*>(gh + 32 * c + i);
+              const uint32_t gw[4] = {g8.x, g8.y, g8.z, g8.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gw[e]));
+                ov[i + 2 * e] = __float_as_uint(__uint_as_float(ov[i + 2 * e]) / (1.f + __expf(-z.x)));
+                ov[i + 2 * e + 1] = __float_as_uint(__uint_as_float(ov[i + 2 * e + 1]) / (1.f + __expf(-z.y)));
+              }
+            }
+          }
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
             uint4 w;
@@ -654,19 +720,23 @@ struct MapHash {
 };
 std::unordered_map<MapKey, CUtensorMap, MapHash> g_maps;
 
+int find_encode() {                                      // under g_mu
+  if (g_encode) return 0;
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
+      qres != cudaDriverEntryPointSuccess || !fn) {
+    cudaGetLastError();
+    return -5;
+  }
+  g_encode = (EncodeTiledFn)fn;
+  return 0;
+}
+
 // cache [planes = pages * kv heads][page_size][hd] bf16; a copy brings 64 values of box_rows keys of one plane
 int cache_map(CUtensorMap* out, const void* ptr, long long planes, int page_size, int hd, int box_rows) {
   std::lock_guard<std::mutex> lk(g_mu);
-  if (!g_encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess || !fn) {
-      cudaGetLastError();
-      return -5;
-    }
-    g_encode = (EncodeTiledFn)fn;
-  }
+  if (find_encode()) return -5;
   MapKey key{ptr, planes, page_size, hd};
   auto it = g_maps.find(key);
   if (it == g_maps.end()) {
@@ -685,16 +755,44 @@ int cache_map(CUtensorMap* out, const void* ptr, long long planes, int page_size
   return 0;
 }
 
-template <int HD, bool TMA, bool CAP>
-int launch_pf_c(const CUtensorMap& mk, const CUtensorMap& mv, const PfParams& p, int ctas, cudaStream_t s) {
+template <int KD, int VD, bool TMA, bool CAP, bool DENSE>
+int launch_pf_c(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, const PfParams& p, int ctas, cudaStream_t s) {
   static bool configured[64] = {};
-  if (allow_dynamic_smem(attn_prefill_tc_kernel<HD, TMA, CAP>, Shape<HD>::SMEM_BYTES, configured)) return -5;
-  return launch_ex(attn_prefill_tc_kernel<HD, TMA, CAP>, dim3(ctas), dim3(THREADS), Shape<HD>::SMEM_BYTES, s, 1, mk, mv, p);
+  constexpr int smem = Shape<KD, VD>::SMEM_BYTES;
+  if (allow_dynamic_smem(attn_prefill_tc_kernel<KD, VD, TMA, CAP, DENSE>, smem, configured)) return -5;
+  return launch_ex(attn_prefill_tc_kernel<KD, VD, TMA, CAP, DENSE>, dim3(ctas), dim3(THREADS), smem, s, 1, mk, mv, mr, p);
 }
 
 template <int HD, bool TMA>
 int launch_pf(const CUtensorMap& mk, const CUtensorMap& mv, const PfParams& p, int ctas, cudaStream_t s) {
-  return p.cap.c > 0.f ? launch_pf_c<HD, TMA, true>(mk, mv, p, ctas, s) : launch_pf_c<HD, TMA, false>(mk, mv, p, ctas, s);
+  return p.cap.c > 0.f ? launch_pf_c<HD, HD, TMA, true, false>(mk, mv, mk, p, ctas, s)
+                       : launch_pf_c<HD, HD, TMA, false, false>(mk, mv, mk, p, ctas, s);
+}
+
+// Rows of 128 (or the heads' shared 64) numbers by tensor copies of 64 rows: [heads][rows][n], strides in numbers.
+int dense_map(CUtensorMap* out, const void* ptr, int n, long long rows, long long row_stride, int heads, long long head_stride) {
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (find_encode()) return -5;
+  }
+  cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)rows, (cuuint64_t)heads};
+  cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)head_stride * 2};
+  cuuint32_t box[3] = {64, 64, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -5;
+}
+
+int multiprocessors(int asked, int& sms) {
+  sms = asked;
+  if (sms > 0) return 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return -5;
+  }
+  return 0;
 }
 
 }  // namespace
@@ -704,19 +802,22 @@ int launch_pf(const CUtensorMap& mk, const CUtensorMap& mv, const PfParams& p, i
 // max_q_len: the longest portion in the batch (sizes the list of work items). Head sizes 64 and 128.
 // chunk > 0: a query sees only the keys of its own block of `chunk` positions (blocks counted from position 0);
 // sinks: float [nh] or null; gate: float logits [T, gate_ld] or null (see PfParams); keep_first, sigmoid: see PfParams.
-// softcap > 0: bounded scores. sm_count: CTAs to launch at most (0: asked from the device).
+// softcap > 0: bounded scores. long_from: sequences with fewer rows are left out. cross: see PfParams. sm_count: CTAs to launch at most (0: asked from the device).
 RLLM_API int rllm_attention_prefill_tc(const void* q, int q_stride, const void* kcache, const void* vcache,
                                        void* out, int out_stride, const int* cu_q, const int* kv_lens,
                                        const int* block_table, int bt_stride, int num_seqs, int max_q_len,
                                        int num_pages, int nh, int nkv, int hd, int page_size, float scale, int window,
                                        int chunk, const float* sinks, const float* gate, int gate_ld,
-                                       int keep_first, int sigmoid, float softcap, int* err, int sm_count, void* stream) {
+                                       int keep_first, int sigmoid, float softcap, int long_from, float* cross, int* err,
+                                       int sm_count, void* stream) {
   if (num_seqs <= 0 || max_q_len <= 0) return 0;
   if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv || page_size <= 0 || num_pages <= 0 || keep_first < 0 || scale <= 0.f)
     return ERR_BAD_SIZE;
   if (q_stride % 8 || out_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) ||
       ((uintptr_t)kcache & 15) || ((uintptr_t)vcache & 15)) return ERR_BAD_ALIGN;
-  PfParams p;
+  if (cross && (softcap > 0.f || sigmoid || gate || ((uintptr_t)cross & 15))) return ERR_BAD_SIZE;
+  PfParams p = {};
+  p.long_from = long_from; p.cross = cross;
   p.q = (const bf16*)q; p.q_stride = q_stride; p.kc = (const bf16*)kcache; p.vc = (const bf16*)vcache;
   p.out = (bf16*)out; p.out_stride = out_stride; p.cu_q = cu_q; p.kv_lens = kv_lens;
   p.block_table = block_table; p.bt_stride = bt_stride; p.nh = nh; p.nkv = nkv; p.page_size = page_size;
@@ -727,31 +828,64 @@ RLLM_API int rllm_attention_prefill_tc(const void* q, int q_stride, const void* 
   p.window = window; p.scale_log2e = scale * 1.4426950408889634f; p.err = err;
   const int G = nh / nkv;
   p.row_pairs = (max_q_len * G + RT * PM - 1) / (RT * PM); p.num_seqs = num_seqs;
-  const long long items = (long long)p.row_pairs * nkv * num_seqs;
+  const long long items = (long long)p.row_pairs * nkv * (cross ? nkv : 1) * num_seqs;
   if (items > 2147483647LL) return ERR_TOO_LARGE;
-  int sms = sm_count;
-  if (sms <= 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-      cudaGetLastError();
-      return -5;
-    }
-  }
+  int sms;
+  if (int rc = multiprocessors(sm_count, sms)) return rc;
   const int ctas = items < sms ? (int)items : sms;
   // pages of a power of two from 8 keys up (whole 1 KB swizzle atoms) come by tensor copies
   const bool tma = p.page_shift >= 3 && (long long)num_pages * nkv <= 2147483647LL;
   CUtensorMap mk, mv;
   cudaStream_t s = (cudaStream_t)stream;
   if (tma) {
-    const int pn = hd == 64 ? Shape<64>::PN : Shape<128>::PN;
+    const int pn = hd == 64 ? Shape<64, 64>::PN : Shape<128, 128>::PN;
     p.box_rows = page_size < pn ? page_size : pn;
     int rc;
     if ((rc = cache_map(&mk, kcache, (long long)num_pages * nkv, page_size, hd, p.box_rows))) return rc;
     if ((rc = cache_map(&mv, vcache, (long long)num_pages * nkv, page_size, hd, p.box_rows))) return rc;
     return hd == 64 ? launch_pf<64, true>(mk, mv, p, ctas, s) : launch_pf<128, true>(mk, mv, p, ctas, s);
   }
+  if (cross) return ERR_BAD_SIZE;                        // only where tensor copies bring the pages
   p.box_rows = 0;
   memset(&mk, 0, sizeof(mk));
   mv = mk;
   return hd == 64 ? launch_pf<64, false>(mk, mv, p, ctas, s) : launch_pf<128, false>(mk, mv, p, ctas, s);
+}
+
+// The same attention over keys and values that lie in rows, a key and a value per query head (PfParams, DENSE): k at
+// row * kv_stride + head * k_head, v likewise, `rows` of them; keys of 128 numbers, or (r not null) 192, of which the last 64 are
+// r's row. q [T, ...]: head h at h * q_head, its last 64 of 192 at q2 + h * q2_head. Values of 128. gate: bf16 logits or null.
+RLLM_API int rllm_attention_prefill_dense(const void* q, int q_stride, int q_head, const void* q2, long long q2_stride, int q2_head,
+                                          const void* k, const void* v, long long kv_stride, int k_head, int v_head, const void* r,
+                                          int r_stride, long long rows, void* out, int out_stride, const int* cu_q,
+                                          const int* kv_lens, int num_seqs, int max_q_len, int nh, float scale, int window,
+                                          const void* gate, int gate_ld, int gate_cols, int long_from, int* err, int sm_count,
+                                          void* stream) {
+  if (num_seqs <= 0 || max_q_len <= 0 || rows <= 0) return 0;
+  if (nh <= 0 || scale <= 0.f || rows > 2147483647LL || (r && !q2)) return ERR_BAD_SIZE;
+  if (q_stride % 8 || q_head % 8 || q2_stride % 8 || q2_head % 8 || kv_stride % 8 || k_head % 8 || v_head % 8 || r_stride % 8 ||
+      out_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)q2 & 15) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15) ||
+      ((uintptr_t)r & 15) || ((uintptr_t)out & 15) || (gate_cols && (gate_ld % 8 || ((uintptr_t)gate & 15)))) return ERR_BAD_ALIGN;
+  PfParams p = {};
+  p.q = (const bf16*)q; p.q_stride = q_stride; p.q_head = q_head;
+  p.q2 = (const bf16*)q2; p.q2_stride = q2_stride; p.q2_head = q2_head;
+  p.out = (bf16*)out; p.out_stride = out_stride; p.cu_q = cu_q; p.kv_lens = kv_lens;
+  p.nh = p.nkv = nh; p.page_size = 1; p.page_shift = 0; p.window = window;
+  p.gate_h = (const bf16*)gate; p.gate_h_ld = gate_ld; p.gate_cols = gate_cols; p.long_from = long_from;
+  p.scale_log2e = scale * 1.4426950408889634f; p.err = err;
+  p.row_pairs = (max_q_len + RT * PM - 1) / (RT * PM); p.num_seqs = num_seqs;
+  const long long items = (long long)p.row_pairs * nh * num_seqs;
+  if (items > 2147483647LL) return ERR_TOO_LARGE;
+  int sms;
+  if (int rc = multiprocessors(sm_count, sms)) return rc;
+  const int ctas = items < sms ? (int)items : sms;
+  CUtensorMap mk, mv, mr;
+  int rc;
+  if ((rc = dense_map(&mk, k, 128, rows, kv_stride, nh, k_head))) return rc;
+  if ((rc = dense_map(&mv, v, 128, rows, kv_stride, nh, v_head))) return rc;
+  mr = mk;
+  if (r && (rc = dense_map(&mr, r, 64, rows, r_stride, 1, rows * r_stride))) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  return r ? launch_pf_c<192, 128, true, false, true>(mk, mv, mr, p, ctas, s)
+           : launch_pf_c<128, 128, true, false, true>(mk, mv, mr, p, ctas, s);
 }

@@ -13,6 +13,10 @@
 //   the rotated query parts are a second call without a latent.
 //   Rotation: pairs (2i, 2i+1), i < dims/2, by the angle of the step's table (cos, sin per token and i);
 //   dimensions from `dims` on pass unchanged.
+// Long portions in bfloat16 with heads of 128 (and 64 rotated) numbers go the other way: their sequences' rows are gathered
+//   (latent_gather), one product turns them into every head's keys and values, and the attention kernel of prompt portions
+//   runs over those (attn_prefill_tc.cu, DENSE). A pair of query and key costs a head 640 or 512 multiplications there, 2,176
+//   or 2,048 here, against some 4 million a key for its expansion at 16 heads.
 // latent_attention (one CTA a query token and group of up to 8 heads, a warp a head): keys j with
 //   max(0, pos - window + 1) <= j <= pos (window <= 0: from 0), taken 32 at a time in position order from
 //   the paged cache, staged once in shared memory for all the CTA's heads; running maximum and sum. A
@@ -209,13 +213,18 @@ static inline int mma_row_pad(int dk, int nh) {          // numbers per shared-m
   return (a > b ? a : b) + 8;
 }
 
+// Row tiles of a sequence; one of at least `skip_from` (> 0) tokens is another kernel's.
+__device__ __forceinline__ int row_tiles(int tokens, int H, int rows, int skip_from) {
+  return skip_from > 0 && tokens >= skip_from ? 0 : (tokens * H + rows - 1) / rows;
+}
+
 template <int NH>     // value columns per half = 8 * NH; rank <= 16 * NH
 __global__ void __launch_bounds__(256, 1)
 latent_attention_mma_kernel(const bf16* __restrict__ qfull, const bf16* __restrict__ cache, bf16* __restrict__ out,
                             const int* __restrict__ cu_q, const int* __restrict__ positions,
                             const int* __restrict__ block_table, int bt_stride, int num_seqs, int H, int rank, int dk,
                             int ld, int page_size, float scale, int window, int splits, float* __restrict__ pacc,
-                            float* __restrict__ pml) {
+                            float* __restrict__ pml, int skip_from) {
   pdl_launch();
   pdl_wait();
   // which sequence and which 64 of its (token, head) rows
@@ -223,7 +232,7 @@ latent_attention_mma_kernel(const bf16* __restrict__ qfull, const bf16* __restri
   {
     int at = 0;
     for (int s = 0; s < num_seqs; ++s) {
-      const int n = ((cu_q[s + 1] - cu_q[s]) * H + QROWS - 1) / QROWS;
+      const int n = row_tiles(cu_q[s + 1] - cu_q[s], H, QROWS, skip_from);
       if ((int)blockIdx.x < at + n) { seq = s; tile = blockIdx.x - at; break; }
       at += n;
     }
@@ -583,18 +592,39 @@ latent_attention_few_kernel(const bf16* __restrict__ qfull, const bf16* __restri
 }
 
 // The splits' parts of every row, merged in split order: out = sum_s e^(m_s - M) acc_s / sum_s e^(m_s - M) l_s.
+// A warp a cached position of the sequences of at least `long_from` rows: their rows one after the other, sequence by sequence
+// in order (pages given back: zeros). Pieces of 16 bytes; grid.x covers the longest sequence, grid.y the sequences.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const uint4* __restrict__ cache, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ cu_q,
+                     const int* __restrict__ kv_lens, int long_from, int page_size, int pieces, uint4* __restrict__ out) {
+  pdl_launch();
+  pdl_wait();
+  const int seq = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * 8 + warp;
+  if (cu_q[seq + 1] - cu_q[seq] < long_from || j >= kv_lens[seq]) return;
+  int base = 0;
+  for (int i = lane; i < seq; i += 32) base += cu_q[i + 1] - cu_q[i] < long_from ? 0 : kv_lens[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+  const int page = block_table[(long long)seq * bt_stride + j / page_size];
+  const uint4* src = cache + ((long long)(page < 0 ? 0 : page) * page_size + j % page_size) * pieces;
+  uint4* dst = out + (long long)(base + j) * pieces;
+  for (int i = lane; i < pieces; i += 32) dst[i] = page < 0 ? make_uint4(0, 0, 0, 0) : src[i];
+}
+
 // grid.x: the row tiles (of `qrows` rows) as in the kernel that left the parts; grid.y: blocks of 32 columns; a
 // warp takes rows, its lanes the columns, all splits' values asked for at once.
 __global__ void __launch_bounds__(256)
 latent_merge_kernel(const float* __restrict__ pacc, const float* __restrict__ pml, bf16* __restrict__ out,
-                    const int* __restrict__ cu_q, int num_seqs, int H, int rank, int splits, int qrows) {
+                    const int* __restrict__ cu_q, int num_seqs, int H, int rank, int splits, int qrows,
+                    int skip_from) {
   pdl_launch();
   pdl_wait();
   int seq = -1, tile = 0;
   {
     int at = 0;
     for (int s = 0; s < num_seqs; ++s) {
-      const int n = ((cu_q[s + 1] - cu_q[s]) * H + qrows - 1) / qrows;
+      const int n = row_tiles(cu_q[s + 1] - cu_q[s], H, qrows, skip_from);
       if ((int)blockIdx.x < at + n) { seq = s; tile = blockIdx.x - at; break; }
       at += n;
     }
@@ -654,11 +684,12 @@ RLLM_API int rllm_latent_prepare(int dt, const void* proj, long long ld, int q_o
 // splits > 1 (tensor-core kernels only): the keys of every row tile are dealt out to that many CTAs; pacc: float
 // [row tiles, splits, rows, rank], pml: float [row tiles, splits, rows, 2], rows = 64 a tile, or 16 with `few`
 // (the shape for steps of a token or two per sequence; taken when rank is a multiple of 128), row tiles =
-// ceil(T * H / rows) + num_seqs.
+// ceil(T * H / rows) + num_seqs. skip_from > 0: sequences of at least so many rows may be left out (their outputs are then not
+// written), where the tensor-core kernel runs.
 RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache, void* out, const int* token_seq,
                                    const int* positions, const int* block_table, int bt_stride, int T, int H, int rank,
                                    int dk, int page_size, float scale, int window, const int* cu_q, int num_seqs,
-                                   int tc, int splits, int few, float* pacc, float* pml, void* stream) {
+                                   int tc, int splits, int few, int skip_from, float* pacc, float* pml, void* stream) {
   if (T <= 0) return 0;
   if (H <= 0 || rank <= 0 || rank > MAX_RANK || dk < rank || page_size <= 0) return ERR_BAD_SIZE;
   if (tc && dt == DT_BF16 && cu_q && num_seqs > 0 && dk % 8 == 0 && rank % 16 == 0 && rank <= 512 &&
@@ -682,7 +713,7 @@ RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache,
                              bt_stride, num_seqs, H, rank, dk, ld, page_size, scale, window, splits, pacc, pml);        \
     if (rl || splits == 1) return rl;                                                                                   \
     return launch_ex(latent_merge_kernel, dim3((unsigned)blocks, (rank + 31) / 32), dim3(256), 0, s, 1,                 \
-                     (const float*)pacc, (const float*)pml, (bf16*)out, cu_q, num_seqs, H, rank, splits, FROWS);        \
+                     (const float*)pacc, (const float*)pml, (bf16*)out, cu_q, num_seqs, H, rank, splits, FROWS, 0);        \
   } while (0)
         if (nw == 2) GO(2);
         if (nw == 4) GO(4);
@@ -702,10 +733,10 @@ RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache,
     if (rc) return rc;                                                                                                  \
     const int rl = launch_ex(latent_attention_mma_kernel<NH>, dim3((unsigned)blocks, splits), dim3(256), (size_t)smem,  \
                              s, 1, (const bf16*)qfull, (const bf16*)cache, (bf16*)out, cu_q, positions, block_table,    \
-                             bt_stride, num_seqs, H, rank, dk, ld, page_size, scale, window, splits, pacc, pml);        \
+                             bt_stride, num_seqs, H, rank, dk, ld, page_size, scale, window, splits, pacc, pml, skip_from);        \
     if (rl || splits == 1) return rl;                                                                                   \
     return launch_ex(latent_merge_kernel, dim3((unsigned)blocks, (rank + 31) / 32), dim3(256), 0, s, 1,                 \
-                     (const float*)pacc, (const float*)pml, (bf16*)out, cu_q, num_seqs, H, rank, splits, QROWS);        \
+                     (const float*)pacc, (const float*)pml, (bf16*)out, cu_q, num_seqs, H, rank, splits, QROWS, skip_from);        \
   } while (0)
       if (nh == 4) GO(4);
       if (nh == 8) GO(8);
@@ -744,4 +775,15 @@ RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache,
 #undef BY_RANK
 #undef GO
   return ERR_BAD_DTYPE;
+}
+
+// The cached rows (of `width` bfloat16 numbers) of every sequence that brings at least long_from rows, out: [sum of their
+// kv_lens, width]. max_kv: the longest sequence.
+RLLM_API int rllm_latent_gather(const void* cache, const int* block_table, int bt_stride, const int* cu_q, const int* kv_lens,
+                                int num_seqs, int long_from, int page_size, int width, int max_kv, void* out, void* stream) {
+  if (num_seqs <= 0 || max_kv <= 0) return 0;
+  if (page_size <= 0 || width <= 0 || width % 8 || num_seqs > 65535) return ERR_BAD_SIZE;
+  if (((uintptr_t)cache & 15) || ((uintptr_t)out & 15)) return ERR_BAD_ALIGN;
+  return launch_ex(latent_gather_kernel, dim3((max_kv + 7) / 8, num_seqs), dim3(256), 0, (cudaStream_t)stream, 1, (const uint4*)cache,
+                   block_table, bt_stride, cu_q, kv_lens, long_from, page_size, width / 8, (uint4*)out);
 }

@@ -68,6 +68,7 @@ struct Args {
   int window, chunk;
   const float* sinks;
   int page_shift;              // log2(page_size), or -1 when it is no power of two
+  int skip_from;               // > 0: sequences of at least so many rows are another kernel's (attn_prefill_tc.cu, `cross`)
 };
 
 __device__ __forceinline__ int first_key(int pos, int window, int chunk) {
@@ -99,7 +100,8 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
     int base = 0;
     for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
       const int i = s0 + lane;
-      const int nt = i < p.num_seqs ? ((p.cu_q[i + 1] - p.cu_q[i]) * Gq + ROWS - 1) / ROWS : 0;
+      const int ntok = i < p.num_seqs ? p.cu_q[i + 1] - p.cu_q[i] : 0;
+      const int nt = p.skip_from > 0 && ntok >= p.skip_from ? 0 : (ntok * Gq + ROWS - 1) / ROWS;
       int inc = nt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -376,12 +378,13 @@ RLLM_API int rllm_talk_attention_mma_supported(int dt, int nh, int kd, int vd, i
 }
 
 // As rllm_talk_attention_simt, bfloat16 only. cu_q [num_seqs + 1]: the row range of each sequence (rows of a sequence
-// adjacent, positions ascending); parts: float scratch [n_tokens, nh, nkv, vd]; out [n_tokens, nh * vd], contiguous.
+// adjacent, positions ascending); skip_from > 0: the parts of sequences of at least so many rows are there already (any_short 0:
+// all of them); parts: float scratch [n_tokens, nh, nkv, vd]; out [n_tokens, nh * vd], contiguous.
 RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const void* kcache, const void* vcache, void* out,
                                      float* parts, const int* positions, const int* cu_q, const int* block_table,
                                      int bt_stride, int num_seqs, int n_tokens, int max_q_len, int nh, int nkv, int kd, int vd,
                                      int page_size, float scale, int window, int chunk, const float* mix, const float* sinks,
-                                     void* stream) {
+                                     int skip_from, int any_short, void* stream) {
   using namespace talkmma;
   if (n_tokens <= 0 || num_seqs <= 0) return 0;
   if (!rllm_talk_attention_mma_supported(DT_BF16, nh, kd, vd, page_size) || nkv <= 0 || nh % nkv) return ERR_BAD_SIZE;
@@ -390,21 +393,22 @@ RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const vo
   const long long tiles = ((long long)n_tokens * Gq + ROWS - 1) / ROWS + num_seqs;
   if (tiles > 2147483647LL || nkv > 65535) return ERR_TOO_LARGE;
   Args a = {(const bf16*)q, q_stride, (const bf16*)kcache, (const bf16*)vcache, parts, positions, cu_q, block_table,
-            bt_stride, num_seqs, nh, nkv, kd, vd, page_size, scale * 1.4426950408889634f, window, chunk, sinks, -1};
+            bt_stride, num_seqs, nh, nkv, kd, vd, page_size, scale * 1.4426950408889634f, window, chunk, sinks, -1, skip_from};
   for (int sft = 0; sft < 31; ++sft) if ((1 << sft) == page_size) a.page_shift = sft;
   cudaStream_t s = (cudaStream_t)stream;
   const dim3 grid((unsigned)tiles, (unsigned)nkv, (unsigned)nkv);
   const int dp = (kd <= 64 && vd <= 64) ? 64 : 128;
   const int smem = 2 * STAGES * KEYS * (dp + 8) * (int)sizeof(bf16);     // also holds the FEW join: 4 x 16 x (dp + 2) floats
   const bool few = (long long)max_q_len * Gq <= 16;             // every sequence's rows fit one warp's 16
-  int rc;
+  int rc = 0;
 #define GO(D, F)                                                                                     \
   {                                                                                                  \
     static bool done[64] = {};                                                                       \
     if ((rc = allow_dynamic_smem(talk_attention_mma_kernel<D, F>, smem, done))) return rc;           \
     rc = launch_ex(talk_attention_mma_kernel<D, F>, grid, dim3(THREADS), (size_t)smem, s, 1, a);     \
   }
-  if (dp == 64) { if (few) GO(64, true) else GO(64, false) }
+  if (!any_short) {}
+  else if (dp == 64) { if (few) GO(64, true) else GO(64, false) }
   else { if (few) GO(128, true) else GO(128, false) }
 #undef GO
   if (rc) return rc;

@@ -16,6 +16,10 @@ import torch
 from . import ops
 
 
+# Rows of a portion from which attention over latents or with mixed heads runs in the tcgen05 kernel of prompt portions
+LATENT_LONG = TALK_LONG = 128
+
+
 class Normed:
     """An RMSNorm that has not run yet: rows of the float residual stream, the norm's weight and
     eps. A product that can take the norm in front of it in one kernel consumes it as it is;
@@ -400,7 +404,32 @@ class Backend:
     def latent_prepare(self, *a, **k):
         return self._mix.latent_prepare(*a, **k)
 
-    def latent_attention(self, qfull, cache, ctx, rank, scale, window):
+    def latent_expanded(self, ctx, heads, dim, rot, vdim, rank, window, scale):
+        """Portions whose latent attention runs over expanded keys and values: (rows a portion has at least, their cached
+        positions, whether there are shorter portions beside them), or None. A pair of query and key costs 0.26 ns less then
+        (16 heads, measured: 590 us against 39 for 2,048 tokens) and a cached position 4.6 ns for its expansion, hence from 32
+        visible queries a key on it pays with a margin; the expansion may take 2 GB."""
+        if not self.fast or ctx.graph_safe or ctx.max_q_len < LATENT_LONG or dim != 128 or vdim != 128 or rot not in (0, 64) \
+                or rank % 64 or scale <= 0 or os.environ.get("RLLM_B200_NO_TC_ATTENTION") == "1":
+            return None
+        long = [(q, n) for q, n in zip(ctx.q_lens_host, ctx.kv_lens_host) if q >= LATENT_LONG]
+        rows = sum(n for _, n in long)
+        if rows * heads * (dim + vdim) * 2 > 2 << 30 or 32 * rows > sum(q * min(n, window or n) for q, n in long):
+            return None
+        return LATENT_LONG, rows, len(long) < ctx.num_seqs
+
+    def latent_attention_expanded(self, q, qfull, cache, ctx, w_ukv, heads, dim, rot, rank, scale, window, long, out, gate, gate_cols):
+        """The long portions' rows of `out` [T, heads * 128]: their sequences' cached rows, every head's keys and values from
+        them (`w_ukv`: W_uk over W_uv), attention, the gate."""
+        long_from, rows, _ = long
+        c = self._mix.latent_gather(cache.tensors["kv"], cache.block_table, ctx.cu_q, ctx.kv_lens, ctx.num_seqs, long_from, rows,
+                                    ctx.max_kv_len)
+        kv = self.linear(c[:, :rank], w_ukv)
+        return self._sm100.attention_prefill_dense(
+            q, dim + rot, qfull[:, :, rank:] if rot else None, kv, 0, heads * dim, c[:, rank:] if rot else None, ctx.cu_q,
+            ctx.kv_lens, ctx.max_q_len, heads, scale, window, out, long_from, gate, gate_cols)
+
+    def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0):
         # Steps of few rows (decoding) have fewer row tiles than the GPU has SMs: the keys of a tile are then
         # dealt out to several CTAs, at least four key tiles (128 keys) each; steps of a token or two per
         # sequence take the kernel shape with 16 rows a CTA. Everything this depends on is known when a decode
@@ -408,13 +437,15 @@ class Backend:
         T, H = qfull.shape[0], qfull.shape[1]
         few = ctx.max_q_len <= 2 and rank % 128 == 0
         rows = 16 if few else 64
+        if skip_from:
+            T = sum(q for q in ctx.q_lens_host if q < skip_from)
         tiles = max(1, T * H // rows)               # row tiles the step has at least
         keys = min(window, ctx.max_kv_len) if window else ctx.max_kv_len
         splits = max(1, min(16, self.sm_count // tiles, keys // 128))
         return self._mix.latent_attention(qfull, cache.tensors["kv"], ctx.token_seq, ctx.positions,
                                           cache.block_table, rank, scale, window, cu_q=ctx.cu_q, num_seqs=ctx.num_seqs,
                                           tensor_cores=self.fast and os.environ.get("RLLM_B200_NO_TC_ATTENTION") != "1",
-                                          splits=splits, few=few)
+                                          splits=splits, few=few, skip_from=skip_from)
 
     def gla_decay(self, z, bias, tau):
         return self._mix.gla_decay(z, bias, tau)
@@ -541,6 +572,17 @@ class Backend:
         kd, vd = cache.k.shape[3], cache.v.shape[3]
         if self.fast and os.environ.get("RLLM_B200_NO_TC_ATTENTION") != "1" \
                 and hy.talk_mma_supported(q.dtype, nh, kd, vd, cache.page_size):
+            page = cache.page_size
+            if not ctx.graph_safe and ctx.max_q_len >= TALK_LONG and kd == vd and page >= 8 and page & (page - 1) == 0 and scale > 0 \
+                    and self._sm100.prefill_tc_supported(q, cache.k):
+                # every head over every kv head's values is ordinary attention: the tcgen05 kernel of prompt portions for
+                # the long ones (16 heads of 128 over 4 kv heads, 2,048 tokens: 515 us with mma.sync), the rest as ever
+                parts = torch.empty((q.shape[0], nh, cache.k.shape[1], vd), dtype=torch.float32, device=q.device)
+                self._sm100.attention_prefill_tc(q, cache.k, cache.v, ctx.cu_q, ctx.kv_lens, cache.block_table, ctx.max_q_len, nh,
+                                                 scale, window, chunk=chunk, sinks=sinks, long_from=TALK_LONG, cross=parts)
+                return hy.talk_attention_mma(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, ctx.cu_q,
+                                             ctx.num_seqs, ctx.max_q_len, nh, scale, mix, window, chunk, sinks, parts=parts,
+                                             skip_from=TALK_LONG, any_short=min(ctx.q_lens_host) < TALK_LONG)
             return hy.talk_attention_mma(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, ctx.cu_q,
                                          ctx.num_seqs, ctx.max_q_len, nh, scale, mix, window, chunk, sinks)
         return hy.talk_attention_simt(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, nh, scale,

@@ -38,7 +38,8 @@ ops.register_signatures("mix", {
     "rllm_latent_prepare": [c_int, _P, _LL, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, _P,
                             _P, _P, _P, c_int, c_int, _P, _P, _P],
     "rllm_latent_attention": [c_int, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
-                              c_int, _P, c_int, c_int, c_int, c_int, _P, _P, _P],
+                              c_int, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, _P],
+    "rllm_latent_gather": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "rllm_gla_decay": [_P, _P, c_int, c_int, c_float, _P],
     "rllm_gla_scan": [c_int, _P, _LL, c_int, c_int, c_int, _P, c_float, c_int, c_int, c_int, c_int, c_int, _P, _P, _P,
                       _P, c_int, _P, _P, _P, c_int, c_int, _P, _P],
@@ -318,12 +319,13 @@ def latent_prepare(proj: torch.Tensor, q_off: int, dkv_off: int, heads: int, dim
 def latent_attention(qfull: torch.Tensor, cache: torch.Tensor, token_seq: torch.Tensor, positions: torch.Tensor,
                      block_table: torch.Tensor, rank: int, scale: float, window: int | None,
                      cu_q: torch.Tensor | None = None, num_seqs: int = 0, tensor_cores: bool = True,
-                     splits: int = 1, few: bool = False) -> torch.Tensor:
+                     splits: int = 1, few: bool = False, skip_from: int = 0) -> torch.Tensor:
     """qfull [T, heads, dk]; cache [pages, page, dk] -> [T, heads, rank] of qfull's dtype. With `cu_q`
     (int32 [num_seqs + 1], the row range of each sequence) bfloat16 problems of fitting sizes run on the
     tensor cores (`tensor_cores` False: never); `splits` > 1 there deals a row tile's keys out to that many
     CTAs and merges their parts (steps of few rows); `few` asks for the kernel shape with 16 rows a CTA (a
-    token or two per sequence; taken where the rank is a multiple of 128)."""
+    token or two per sequence; taken where the rank is a multiple of 128). `skip_from` > 0: the outputs of sequences of
+    at least so many rows may stay unwritten (they are another kernel's)."""
     _cuda(qfull, "qfull"); _cuda(cache, "cache")
     T, H, dk = qfull.shape
     if not qfull.is_contiguous() or not cache.is_contiguous() or cache.dtype != qfull.dtype or cache.dim() != 3 \
@@ -350,7 +352,22 @@ def latent_attention(qfull: torch.Tensor, cache: torch.Tensor, token_seq: torch.
         _dt(qfull, "qfull"), qfull.data_ptr(), cache.data_ptr(), out.data_ptr(), token_seq.data_ptr(),
         positions.data_ptr(), block_table.data_ptr(), block_table.stride(0), T, H, rank, dk, cache.shape[1],
         float(scale), int(window or 0), _ptr(cu_q), int(num_seqs), int(bool(tensor_cores)), splits, int(few),
-        _ptr(pacc), _ptr(pml), _stream()), "latent_attention", 2 if splits > 1 else 1)
+        int(skip_from), _ptr(pacc), _ptr(pml), _stream()), "latent_attention", 2 if splits > 1 else 1)
+    return out
+
+
+def latent_gather(cache, block_table, cu_q, kv_lens, num_seqs, long_from, rows, max_kv) -> torch.Tensor:
+    """The cached rows of every sequence that brings at least `long_from` rows, one after the other: [rows, width]."""
+    _cuda(cache, "cache")
+    if cache.dtype != torch.bfloat16 or cache.dim() != 3 or not cache.is_contiguous() or cache.shape[2] % 8:
+        raise KernelError("the latent cache must be contiguous bfloat16 [pages, page, a multiple of 8]")
+    if block_table.dtype != torch.int32 or block_table.dim() != 2 or block_table.stride(1) != 1:
+        raise KernelError("block_table must be int32 [sequences, pages] with unit inner stride")
+    _i32(cu_q, "cu_q", num_seqs + 1); _i32(kv_lens, "kv_lens", num_seqs)
+    out = torch.empty((rows, cache.shape[2]), dtype=cache.dtype, device=cache.device)
+    _check(_fn("mix", "rllm_latent_gather")(cache.data_ptr(), block_table.data_ptr(), block_table.stride(0), cu_q.data_ptr(),
+                                            kv_lens.data_ptr(), int(num_seqs), int(long_from), cache.shape[1], cache.shape[2],
+                                            int(max_kv), out.data_ptr(), _stream()), "latent_gather")
     return out
 
 

@@ -31,7 +31,9 @@ ops.register_signatures("sm100", {
     "rllm_attention_fa": [_P, c_int, _P, _P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
                           c_int, c_int, c_float, c_int, c_int, _P, _P, _P],
     "rllm_attention_prefill_tc": [_P, c_int, _P, _P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
-                                  c_int, c_int, c_float, c_int, c_int, _P, _P, c_int, c_int, c_int, c_float, _P, c_int, _P],
+                                  c_int, c_int, c_float, c_int, c_int, _P, _P, c_int, c_int, c_int, c_float, c_int, _P, _P, c_int, _P],
+    "rllm_attention_prefill_dense": [_P, c_int, c_int, _P, c_longlong, c_int, _P, _P, c_longlong, c_int, c_int, _P, c_int, c_longlong, _P,
+                                     c_int, _P, _P, c_int, c_int, c_int, c_float, c_int, _P, c_int, c_int, c_int, _P, c_int, _P],
     "rllm_attention_decode": [_P, c_int, _P, _P, c_longlong, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int,
                               c_int, c_float, c_int, c_int, _P, _P, c_int, c_float, c_int, _P, _P],
 })
@@ -379,26 +381,66 @@ def _extras(chunk, sinks, gate, nh, rows):
 
 
 def attention_prefill_tc(q, kcache, vcache, cu_q, kv_lens, block_table, max_q_len, nh, scale, window, out=None,
-                         chunk=None, sinks=None, gate=None, keep_first=0, sigmoid=False, softcap=None):
+                         chunk=None, sinks=None, gate=None, keep_first=0, sigmoid=False, softcap=None, long_from=0,
+                         cross=None):
     """Prefill attention on the tcgen05 tensor cores (bf16, head size 64 or 128): tiles of 128 rows x
     128 (64) keys, both products with their accumulators in TMEM. `chunk`: a query sees only the keys of its
     own block of that many positions; `sinks` float [nh]: exp(sink) joins a row's denominator; `gate` float
     logits [T, >= nh]: head h's output times sigmoid(gate[t, h]); `keep_first`: positions below it are seen whatever
     the window says; `sigmoid`: no softmax, a visible key's weight is sigmoid(score + sinks[head]); `softcap`: scores
-    bounded, softcap * tanh(score / softcap)."""
+    bounded, softcap * tanh(score / softcap). `long_from`: sequences with fewer rows are left out. `cross` float32
+    [T, nh, nkv, hd]: every query head meets every kv head's values and the float outputs go there (pages of a power of two
+    from 8 keys on; no gate, bound or sigmoid)."""
     if not prefill_tc_supported(q, kcache):
         raise ops.KernelError("attention_prefill_tc: bfloat16, head size 64 or 128, rows 16-byte aligned")
     st = init(q.device)
     _, nkv, page_size, hd = kcache.shape
+    if cross is not None:
+        if cross.dtype != torch.float32 or not cross.is_contiguous() or tuple(cross.shape) != (q.shape[0], nh, nkv, hd) or not cross.is_cuda:
+            raise ops.KernelError(f"attention_prefill_tc: cross must be contiguous float32 [{q.shape[0]}, {nh}, {nkv}, {hd}]")
+        out = cross.view(torch.bfloat16).view(-1, 8)[:1] if out is None else out      # not written
     if out is None:
         out = torch.empty((q.shape[0], nh * hd), dtype=torch.bfloat16, device=q.device)
     rc = ops._fn("sm100", "rllm_attention_prefill_tc")(
         q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), out.data_ptr(), out.stride(0),
         cu_q.data_ptr(), kv_lens.data_ptr(), block_table.data_ptr(), block_table.stride(0), kv_lens.numel(),
         max_q_len, kcache.shape[0], nh, nkv, hd, page_size, float(scale), int(window or 0),
-        *_extras(chunk, sinks, gate, nh, q.shape[0]), int(keep_first or 0), int(bool(sigmoid)), float(softcap or 0.0), st.err.data_ptr(),
-        st.sm_count, ops._stream())
+        *_extras(chunk, sinks, gate, nh, q.shape[0]), int(keep_first or 0), int(bool(sigmoid)), float(softcap or 0.0), int(long_from),
+        None if cross is None else cross.data_ptr(), st.err.data_ptr(), st.sm_count, ops._stream())
     ops._check(rc, "attention_prefill_tc")
+    return out if cross is None else cross
+
+
+def attention_prefill_dense(q, q_head, q2, kv, k_off, v_off, r, cu_q, kv_lens, max_q_len, nh, scale, window, out, long_from,
+                            gate=None, gate_cols=False):
+    """Prefill attention with a key and a value per query head that lie in rows instead of pages: kv bf16 [rows, ...], head h's
+    key of 128 numbers at column k_off + 128 h, its value at v_off + 128 h; r (bf16 [rows, 64] or None): 64 more numbers of every
+    head's key. The rows are those of the sequences that bring at least `long_from` rows, one sequence's after the other's (the
+    others are left out). q [T, ...]: head h at h * q_head; with r its last 64 numbers are q2[:, h] (bf16 [T, nh, 64], any
+    strides). gate: bf16 logits [T, >= nh] (or [T, >= nh * 128] with `gate_cols`, one per output). out [T, nh * 128]."""
+    for t, name in ((q, "q"), (kv, "kv"), (out, "out")) + (((r, "r"), (q2, "q2")) if r is not None else ()) \
+            + (((gate, "gate"),) if gate is not None else ()):
+        if t.dtype != torch.bfloat16 or not t.is_cuda or t.stride(-1) != 1:
+            raise ops.KernelError(f"attention_prefill_dense: {name} must be bfloat16 on the device with unit inner stride")
+    T, rows = q.shape[0], kv.shape[0]
+    if q.shape[1] < (nh - 1) * q_head + 128 or kv.shape[1] < max(k_off, v_off) + nh * 128 or tuple(out.shape) != (T, nh * 128):
+        raise ops.KernelError("attention_prefill_dense: q, kv or out too narrow for its heads")
+    if r is not None and (tuple(r.shape) != (rows, 64) or tuple(q2.shape) != (T, nh, 64)):
+        raise ops.KernelError(f"attention_prefill_dense: r must be [{rows}, 64] and q2 [{T}, {nh}, 64]")
+    if gate is not None and (gate.shape[0] != T or gate.shape[1] < (nh * 128 if gate_cols else nh)):
+        raise ops.KernelError("attention_prefill_dense: the gate is too small")
+    for t, n in ((cu_q, kv_lens.numel() + 1), (kv_lens, 1)):
+        if t.dtype != torch.int32 or not t.is_contiguous() or t.numel() < n:
+            raise ops.KernelError("attention_prefill_dense: cu_q and kv_lens must be contiguous int32 vectors")
+    st, es = init(q.device), 2
+    rc = ops._fn("sm100", "rllm_attention_prefill_dense")(
+        q.data_ptr(), q.stride(0), int(q_head), None if r is None else q2.data_ptr(), 0 if r is None else q2.stride(0),
+        0 if r is None else q2.stride(1), kv.data_ptr() + es * k_off, kv.data_ptr() + es * v_off, kv.stride(0), 128, 128,
+        None if r is None else r.data_ptr(), 0 if r is None else r.stride(0), rows, out.data_ptr(), out.stride(0), cu_q.data_ptr(),
+        kv_lens.data_ptr(), kv_lens.numel(), int(max_q_len), int(nh), float(scale), int(window or 0),
+        None if gate is None else gate.data_ptr(), 0 if gate is None else gate.stride(0), int(bool(gate_cols)), int(long_from),
+        st.err.data_ptr(), st.sm_count, ops._stream())
+    ops._check(rc, "attention_prefill_dense")
     return out
 
 

@@ -12,7 +12,8 @@ a `window` allows (None: all earlier ones); each head's output is multiplied by 
 projected from h, one number per head (`gate` "head", or True), or one per output of every head (`gate` "full"; False:
 there is none); W_o follows. `q_rank`: the queries come out of a latent of their own, q = W_uq RMSnorm(W_dq h). `rot_dim` 0
 with `position` None: no rotated part, positions do not enter the scores. Scores, softmax, the latents' norms and the
-rotation are float.
+rotation are float. Long portions in bfloat16 expand their sequence's latents after all (`Backend.latent_expanded` says when
+and why): with hundreds of queries a key the expansion is the smaller cost.
 """
 from __future__ import annotations
 
@@ -80,6 +81,7 @@ class LatentAttention(Part):
         # per head: [kv_rank, dim] so that the fold is a product with K = dim; [vdim, kv_rank] as stored
         self._uk_t = self.w_uk.view(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
         self._uv = self.w_uv.view(H, self.vdim, self.kv_rank)
+        self._ukv = torch.cat([self.w_uk, self.w_uv], 0)          # every head's keys and values out of a latent
         self._norm_f32 = self.w_latent_norm.float().contiguous()
         self._q_norm_f32 = None if self.w_q_norm is None else self.w_q_norm.float().contiguous()
 
@@ -106,11 +108,17 @@ class LatentAttention(Part):
             q = be.linear(cq, self.w_uq, tag="uq")
             if self.rot_dim:
                 be.latent_prepare(q, 0, 0, H, self.dim, self.rot_dim, self.kv_rank, dims, None, self.eps, table, None, None, qfull)
-        be.linear_heads(q, self.dim + self.rot_dim, self._uk_t, qfull.view(T, H * dk), dk)
-        o = be.latent_attention(qfull, cache, ctx, self.kv_rank, self.scale, self.window)
         att = torch.empty((T, H * self.vdim), dtype=proj.dtype, device=proj.device)
-        be.linear_heads(o.view(T, H * self.kv_rank), self.kv_rank, self._uv, att, self.vdim,
-                        gate=proj[:, q_cols + dk:] if self.gate else None, gate_cols=self.gate == "full")
+        gate, gate_cols = proj[:, q_cols + dk:] if self.gate else None, self.gate == "full"
+        # long portions over expanded keys and values, the others (decoded tokens beside them) over the latents themselves
+        long = be.latent_expanded(ctx, H, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.window, self.scale)
+        if long is None or long[2]:
+            be.linear_heads(q, self.dim + self.rot_dim, self._uk_t, qfull.view(T, H * dk), dk)
+            o = be.latent_attention(qfull, cache, ctx, self.kv_rank, self.scale, self.window, skip_from=long[0] if long else 0)
+            be.linear_heads(o.view(T, H * self.kv_rank), self.kv_rank, self._uv, att, self.vdim, gate=gate, gate_cols=gate_cols)
+        if long is not None:
+            be.latent_attention_expanded(q, qfull, cache, ctx, self._ukv, H, self.dim, self.rot_dim, self.kv_rank, self.scale,
+                                         self.window, long, att, gate, gate_cols)
         if residual is None:
             return be.linear_f32(att, self.w_o, tag="o")
         be.linear_residual(att, self.w_o, residual)
