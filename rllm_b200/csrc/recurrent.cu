@@ -66,6 +66,63 @@ __global__ void short_conv_kernel(const TI* __restrict__ x, long long ld, int co
   out[(long long)t * C + c] = silu ? acc / (1.f + expf(-acc)) : acc;
 }
 
+// Four taps (what every configuration here has), four neighbouring channels a thread, RUN tokens one after the other with
+// the last three inputs in registers: an input is read 1 + 3 / RUN times instead of four, in pieces of 8 or 16 bytes. The sums'
+// order is the kernel's above, so the bits are too. Bound by its bytes (2 or 4 in, 4 out a value): 2,048 tokens x 6,144 channels
+// of bfloat16 70.7 us with a token and a channel a thread.
+template <typename TI, int RUN>
+__global__ void __launch_bounds__(128) short_conv4_kernel(const TI* __restrict__ x, long long ld, int col0, int C,
+                                                          const float* __restrict__ w, const float* __restrict__ bias,
+                                                          const int* __restrict__ token_seq, const int* __restrict__ positions,
+                                                          const int* __restrict__ cu_q, const int* __restrict__ state_slots,
+                                                          const float* __restrict__ tail, float* __restrict__ out, int T, int silu) {
+  pdl_launch();
+  pdl_wait();
+  const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+  if (c >= C) return;
+  const int t0 = blockIdx.x * RUN, t1 = min(T, t0 + RUN);
+  float wt[4][4], b[4];                                   // [channel][tap]
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float4 v = *reinterpret_cast<const float4*>(w + (long long)(c + e) * 4);
+    wt[e][0] = v.x; wt[e][1] = v.y; wt[e][2] = v.z; wt[e][3] = v.w;
+    b[e] = bias ? bias[c + e] : 0.f;
+  }
+  const TI* xc = x + col0 + c;
+  auto row = [&](int r) { return chunked::load4(xc + (long long)r * ld); };
+  float4 in[4];                                           // inputs of rows t - 3 .. t
+  in[0] = t0 >= 3 ? row(t0 - 3) : make_float4(0.f, 0.f, 0.f, 0.f);
+  in[1] = t0 >= 2 ? row(t0 - 2) : make_float4(0.f, 0.f, 0.f, 0.f);
+  in[2] = t0 >= 1 ? row(t0 - 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < RUN; ++i) {
+    const int t = t0 + i;
+    if (t >= t1) break;
+    in[3] = row(t);
+    const int s = token_seq[t], row0 = cu_q[s], pos = positions[t];
+    const int slot = state_slots ? state_slots[s] : -1;
+    float a[4] = {b[0], b[1], b[2], b[3]};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int back = 3 - j;
+      if (pos - back < 0) continue;
+      float4 v = in[j];
+      if (t - back < row0) {                              // before the portion: the tail, or nothing
+        v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (slot >= 0) v = *reinterpret_cast<const float4*>(tail + ((long long)slot * 3 + (3 - (row0 - (t - back)))) * C + c);
+      }
+      a[0] = fmaf(wt[0][j], v.x, a[0]); a[1] = fmaf(wt[1][j], v.y, a[1]);
+      a[2] = fmaf(wt[2][j], v.z, a[2]); a[3] = fmaf(wt[3][j], v.w, a[3]);
+    }
+    if (silu) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = a[e] / (1.f + expf(-a[e]));
+    }
+    *reinterpret_cast<float4*>(out + (long long)t * C + c) = make_float4(a[0], a[1], a[2], a[3]);
+    in[0] = in[1]; in[1] = in[2]; in[2] = in[3];
+  }
+}
+
 template <typename TI>
 __global__ void short_conv_keep_kernel(const TI* __restrict__ x, long long ld, int col0, int C, int taps,
                                        const int* __restrict__ cu_q, const int* __restrict__ state_slots,
@@ -107,16 +164,24 @@ __global__ void unit_heads_kernel(float* __restrict__ x, long long ld, int col0,
 template <typename TI>
 __global__ void softplus_decay_kernel(const TI* __restrict__ z, long long ld, int col0, const float* __restrict__ bias,
                                       const float* __restrict__ a_log, int n, int per_head, float* __restrict__ step,
-                                      float* __restrict__ decay, long long total) {
+                                      float* __restrict__ decay, int T) {
   pdl_launch();
   pdl_wait();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / n;
-    const int c = (int)(i % n);
-    const float d = softplus_f(to_f32(z[t * ld + col0 + c]) + (bias ? bias[c] : 0.f));
-    if (step) step[i] = d;
-    if (decay) decay[i] = expf(-expf(a_log[c / per_head]) * d);
+  // a thread stays with its column, so that what belongs to the column is worked out once and nothing is divided per value
+  const int c = blockIdx.y * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const float b = bias ? bias[c] : 0.f, rate = decay ? -expf(a_log[c / per_head]) : 0.f;
+  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
+    const float d = softplus_f(to_f32(z[t * ld + col0 + c]) + b);
+    if (step) step[t * n + c] = d;
+    if (decay) decay[t * n + c] = expf(rate * d);
   }
+}
+
+__device__ __forceinline__ void store4(float* p, const float (&o)[4]) { *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]); }
+__device__ __forceinline__ void store4(bf16* p, const float (&o)[4]) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(o[0], o[1]), b = __floats2bfloat162_rn(o[2], o[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
 struct ScanArgs {
@@ -227,6 +292,51 @@ __global__ void __launch_bounds__(128) state_scan_kernel(ScanArgs a) {
   }
 }
 
+// The same for parts of 128 V numbers (1 <= V <= 8), a warp a (token, part) with its share in registers, four neighbouring
+// numbers a load: one pass over y and the gate. (A CTA a part: 70 us for 2,047 tokens x 32 parts of 128.)
+template <typename TG, typename TO, int V>
+__global__ void __launch_bounds__(128) gated_norm_warp_kernel(const float* __restrict__ y, const TG* __restrict__ gate, long long g_ld,
+                                                              const float* __restrict__ w, int w_period, float eps,
+                                                              TO* __restrict__ out, int groups, long long parts, int gate_first, int act) {
+  pdl_launch();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const long long part = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (part >= parts) return;
+  constexpr int G = 128 * V;
+  const long long t = part / groups;
+  const int g0 = (int)(part % groups) * G;
+  const float* yr = y + part * G;
+  float v[4 * V], g[4 * V], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = i * 128 + lane * 4;
+    const float4 a = *reinterpret_cast<const float4*>(yr + c);
+    v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = a.z; v[4 * i + 3] = a.w;
+    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (gate) z = chunked::load4(gate + t * g_ld + g0 + c);
+    g[4 * i] = z.x; g[4 * i + 1] = z.y; g[4 * i + 2] = z.z; g[4 * i + 3] = z.w;
+  }
+#pragma unroll
+  for (int i = 0; i < 4 * V; ++i) {
+    g[i] = !gate ? 1.f : act == 0 ? g[i] / (1.f + expf(-g[i])) : 1.f / (1.f + expf(-g[i]));
+    if (gate_first) v[i] *= g[i];
+    ss = fmaf(v[i], v[i], ss);
+  }
+  ss = warp_sum(ss);
+  const float r = 1.f / sqrtf(ss / (float)G + eps);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = i * 128 + lane * 4;
+    const float4 wv = *reinterpret_cast<const float4*>(w + (g0 + c) % w_period);
+    const float ws[4] = {wv.x, wv.y, wv.z, wv.w};
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = gate_first ? v[4 * i + e] * r * ws[e] : v[4 * i + e] * r * ws[e] * g[4 * i + e];
+    store4(out + part * G + c, o);
+  }
+}
+
 // One CTA per (token, group). gate: logits [T, >= cols] with row stride g_ld, of type TG.
 template <typename TG, typename TO>
 __global__ void gated_norm_kernel(const float* __restrict__ y, const TG* __restrict__ gate, long long g_ld,
@@ -259,8 +369,6 @@ __global__ void gated_norm_kernel(const float* __restrict__ y, const TG* __restr
     o[i] = from_f32<TO>(v);
   }
 }
-
-inline unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256 > 65535 * 8 ? 65535 * 8 : (n + 255) / 256); }
 
 // The same recurrence for heads of R * SPLIT key channels (32 to 256) with R = 32, 16 or 8 channels a thread, the sizes
 // known when compiled: a thread's channels are neighbours (sub * R ...), so queries, keys and decays come from shared
@@ -439,7 +547,19 @@ RLLM_API int rllm_short_conv(int dt, const void* x, long long ld, int col0, int 
   const dim3 grid((unsigned)T, (unsigned)((C + threads - 1) / threads));
   if (grid.y > 65535) return ERR_TOO_LARGE;
   int rc;
-  if (dt == DT_F32)
+  // four channels a thread where rows, weights and tail let them be read together; runs of 8 tokens from 512 tokens on, below
+  // that single ones, so that there are threads enough
+  const size_t es = dt == DT_F32 ? 4 : 2;
+  const bool wide = taps == 4 && C % 4 == 0 && col0 % 4 == 0 && ld % 4 == 0 && !((uintptr_t)x % (4 * es)) && !((uintptr_t)w & 15) &&
+                    !((uintptr_t)tail & 15) && !((uintptr_t)out & 15) && (dt == DT_F32 || dt == DT_BF16);
+  if (wide) {
+    const int run = T >= 512 ? 8 : 1;
+    const dim3 g4((unsigned)((T + run - 1) / run), (unsigned)((C / 4 + 127) / 128));
+#define RLLM_SC(TI, RUN) launch_ex(short_conv4_kernel<TI, RUN>, g4, dim3(128), 0, s, 1, (const TI*)x, ld, col0, C, w, bias, token_seq,  \
+                                   positions, cu_q, state_slots, (const float*)tail, out, T, silu)
+    rc = dt == DT_F32 ? (run == 8 ? RLLM_SC(float, 8) : RLLM_SC(float, 1)) : (run == 8 ? RLLM_SC(bf16, 8) : RLLM_SC(bf16, 1));
+#undef RLLM_SC
+  } else if (dt == DT_F32)
     rc = launch_ex(short_conv_kernel<float>, grid, dim3(threads), 0, s, 1, (const float*)x, ld, col0, C, taps, w, bias,
                    token_seq, positions, cu_q, state_slots, (const float*)tail, out, silu);
   else if (dt == DT_BF16)
@@ -466,14 +586,16 @@ RLLM_API int rllm_softplus_decay(int dt, const void* z, long long ld, int col0, 
                                  int n, int per_head, float* step, float* decay, void* stream) {
   if (T <= 0 || n <= 0) return 0;
   if (per_head <= 0 || n % per_head) return ERR_BAD_SIZE;
-  const long long total = (long long)T * n;
   cudaStream_t s = (cudaStream_t)stream;
+  const int threads = n >= 128 ? 128 : n > 32 ? 64 : 32, cols = (n + threads - 1) / threads;
+  if (cols > 65535) return ERR_TOO_LARGE;
+  const dim3 grid(T < 4096 / cols + 1 ? T : 4096 / cols + 1, cols);        // some thirty CTAs an SM, rows dealt out to them
   if (dt == DT_F32)
-    return launch_ex(softplus_decay_kernel<float>, dim3(blocks_for(total)), dim3(256), 0, s, 1, (const float*)z, ld, col0, bias,
-                     a_log, n, per_head, step, decay, total);
+    return launch_ex(softplus_decay_kernel<float>, grid, dim3(threads), 0, s, 1, (const float*)z, ld, col0, bias, a_log, n, per_head,
+                     step, decay, T);
   if (dt == DT_BF16)
-    return launch_ex(softplus_decay_kernel<bf16>, dim3(blocks_for(total)), dim3(256), 0, s, 1, (const bf16*)z, ld, col0, bias,
-                     a_log, n, per_head, step, decay, total);
+    return launch_ex(softplus_decay_kernel<bf16>, grid, dim3(threads), 0, s, 1, (const bf16*)z, ld, col0, bias, a_log, n, per_head,
+                     step, decay, T);
   return ERR_BAD_DTYPE;
 }
 
@@ -570,6 +692,24 @@ RLLM_API int rllm_gated_norm(const float* y, const void* gate, int gate_dt, long
   if (groups <= 0 || gsize <= 0 || w_period <= 0 || act < 0 || act > 1) return ERR_BAD_SIZE;
   const dim3 grid((unsigned)((long long)T * groups)), block(gsize >= 512 ? 256 : gsize >= 128 ? 128 : 64);
   cudaStream_t s = (cudaStream_t)stream;
+  const size_t gb = gate_dt == DT_F32 ? 16 : 8, ob = out_dt == DT_F32 ? 16 : 8;
+  if ((gsize == 128 || gsize == 256 || gsize == 512 || gsize == 1024) && w_period % 4 == 0 && g_ld % 4 == 0 && !((uintptr_t)y & 15) &&
+      !((uintptr_t)w & 15) && !((uintptr_t)gate % gb) && !((uintptr_t)out % ob)) {
+    const long long parts = (long long)T * groups;
+    const dim3 gw((unsigned)((parts + 3) / 4));
+#define RLLM_GV(TG, TO, V) \
+  return launch_ex(gated_norm_warp_kernel<TG, TO, V>, gw, dim3(128), 0, s, 1, y, (const TG*)gate, g_ld, w, w_period, eps, (TO*)out, groups, \
+                   parts, gate_first, act)
+#define RLLM_GW(TG, TO) \
+  do { if (gsize == 128) RLLM_GV(TG, TO, 1); if (gsize == 256) RLLM_GV(TG, TO, 2); if (gsize == 512) RLLM_GV(TG, TO, 4); RLLM_GV(TG, TO, 8); } while (0)
+    if (gate_dt == DT_F32 && out_dt == DT_F32) RLLM_GW(float, float);
+    if (gate_dt == DT_F32 && out_dt == DT_BF16) RLLM_GW(float, bf16);
+    if (gate_dt == DT_BF16 && out_dt == DT_BF16) RLLM_GW(bf16, bf16);
+    if (gate_dt == DT_BF16 && out_dt == DT_F32) RLLM_GW(bf16, float);
+#undef RLLM_GW
+#undef RLLM_GV
+    return ERR_BAD_DTYPE;
+  }
 #define RLLM_GN(TG, TO) \
   return launch_ex(gated_norm_kernel<TG, TO>, grid, block, 0, s, 1, y, (const TG*)gate, g_ld, w, w_period, eps, (TO*)out, groups, \
                    gsize, gate_first, act)

@@ -445,19 +445,45 @@ template <typename T>
 __global__ void add_bias_kernel(T* __restrict__ y, const T* __restrict__ bias, int rows, int N, long long ld) {
   pdl_launch();
   pdl_wait();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)rows * N) return;
-  const int n = (int)(i % N);
-  T* p = y + (size_t)(i / N) * ld + n;
-  *p = from_f32<T>(to_f32(*p) + to_f32(bias[n]));
+  const int n = blockIdx.y * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const float b = to_f32(bias[n]);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    T* p = y + (size_t)r * ld + n;
+    *p = from_f32<T>(to_f32(*p) + b);
+  }
+}
+// Eight bfloat16 a thread, rows and bias on 16-byte boundaries (2,048 x 3,072: 27 us a value a thread with a division each).
+__global__ void add_bias8_kernel(bf16* __restrict__ y, const bf16* __restrict__ bias, int rows, int N, long long ld) {
+  pdl_launch();
+  pdl_wait();
+  const int n = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (n >= N) return;
+  const uint4 bv = *reinterpret_cast<const uint4*>(bias + n);
+  const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    uint4* p = reinterpret_cast<uint4*>(y + (size_t)r * ld + n);
+    uint4 v = *p;
+    __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = __bfloat1622float2(v2[e]), c = __bfloat1622float2(b2[e]);
+      v2[e] = __floats2bfloat162_rn(a.x + c.x, a.y + c.y);
+    }
+    *p = v;
+  }
 }
 RLLM_API int rllm_add_bias(void* y, const void* bias, int dt, int rows, int N, long long ld, void* stream) {
   if (rows <= 0 || N <= 0) return 0;
-  const int threads = 256;
-  const unsigned blocks = (unsigned)(((size_t)rows * N + threads - 1) / threads);
+  const int threads = 128;
   cudaStream_t s = (cudaStream_t)stream;
-  if (dt == DT_F32) return launch_ex(add_bias_kernel<float>, dim3(blocks), dim3(threads), 0, s, 1, (float*)y, (const float*)bias, rows, N, ld);
-  if (dt == DT_BF16) return launch_ex(add_bias_kernel<bf16>, dim3(blocks), dim3(threads), 0, s, 1, (bf16*)y, (const bf16*)bias, rows, N, ld);
+  const int per = dt == DT_BF16 && N % 8 == 0 && ld % 8 == 0 && !((uintptr_t)y & 15) && !((uintptr_t)bias & 15) ? 8 : 1;
+  const int cols = (N / per + threads - 1) / threads;
+  if (cols > 65535) return ERR_TOO_LARGE;
+  const dim3 grid(rows < 4096 / cols + 1 ? rows : 4096 / cols + 1, cols);   // some thirty CTAs an SM, rows dealt out to them
+  if (per == 8) return launch_ex(add_bias8_kernel, grid, dim3(threads), 0, s, 1, (bf16*)y, (const bf16*)bias, rows, N, ld);
+  if (dt == DT_F32) return launch_ex(add_bias_kernel<float>, grid, dim3(threads), 0, s, 1, (float*)y, (const float*)bias, rows, N, ld);
+  if (dt == DT_BF16) return launch_ex(add_bias_kernel<bf16>, grid, dim3(threads), 0, s, 1, (bf16*)y, (const bf16*)bias, rows, N, ld);
   return ERR_BAD_DTYPE;
 }
 

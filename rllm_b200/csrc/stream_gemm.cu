@@ -80,7 +80,7 @@ struct Params {
   void* C;                  // output [T][N] (type by epilogue), row stride ldc
   long long ldc;
   int T;
-  int act;                  // store epilogue only: 1 stores max(value, 0)^2, 2 gelu(value) in its tanh form, 3 in its erf form
+  int act;                  // gate/up epilogue: 2 gelu in its tanh form for silu; store epilogue: 1 stores max(value, 0)^2, 2 gelu(value) in its tanh form, 3 in its erf form
   int njobs;
   int nchw;                 // chunks per warp and tile
   RopeArgs rope;
@@ -335,7 +335,8 @@ stream_gemm_kernel(const Params p) {
         }
         else if (EPI == EPI_STORE_F32) ((float*)p.C)[o] = s0;
         else if (EPI == EPI_ACCUM_F32) ((float*)p.C)[o] += s0;
-        else if (EPI == EPI_SWIGLU) ((bf16*)p.C)[o] = __float2bfloat16_rn(s0 / (1.f + expf(-s0)) * s1);
+        else if (EPI == EPI_SWIGLU) ((bf16*)p.C)[o] = __float2bfloat16_rn(
+            s0 / (1.f + expf(p.act == 2 ? -1.5957691216057308f * (s0 + 0.044715f * s0 * s0 * s0) : -s0)) * s1);
       }
     }
     if (batch0 + BATCH < my_jobs) __syncthreads();      // the parts are read before the next batch overwrites them
@@ -423,7 +424,7 @@ RLLM_API int rllm_stream_gemm(int epi, const void* X, long long ldx, const float
                               int T, int N, int K, int sm_count, void* stream) {
   const int act = epi >> 8;                       // as in rllm_tc_gemm: 0 | 1 << 8 stores max(value, 0)^2, 0 | 2 << 8 gelu(value), 0 | 3 << 8 its erf form
   epi &= 0xff;
-  if (epi < 0 || epi > EPI_SWIGLU || act > 3 || (act && epi != EPI_STORE)) return ERR_BAD_SIZE;
+  if (epi < 0 || epi > EPI_SWIGLU || act > 3 || (act && epi != EPI_STORE && !(epi == EPI_SWIGLU && act == 2))) return ERR_BAD_SIZE;
   const bool norm = X == nullptr;
   if (norm && (!h || !g || (g_dt != DT_F32 && g_dt != DT_BF16))) return ERR_BAD_SIZE;
   Params p = {};

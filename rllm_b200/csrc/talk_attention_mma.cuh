@@ -338,10 +338,11 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
   }
 }
 
-// One CTA per token, a thread per (kv head c, value column d): it reads A[g, c][d] of every head g once and adds it
-// into the outputs of the heads that use kv head c, HB of them at a time.
-constexpr int HB = 8;
-__global__ void __launch_bounds__(256) talk_mix_kernel(const float* __restrict__ parts, const float* __restrict__ mix,
+// One CTA per token, a thread per (kv head c, four value columns): it reads A[g, c] of every head g once and adds it into
+// the outputs of the heads that use kv head c, HB of them at a time, each sum in the order of the heads. Bound by the parts'
+// bytes (2,048 tokens x 16 heads x 512: 29 us with a column a thread).
+constexpr int HB = 4;
+__global__ void __launch_bounds__(128) talk_mix_kernel(const float* __restrict__ parts, const float* __restrict__ mix,
                                                        bf16* __restrict__ out, int nh, int nkv, int vd) {
   pdl_launch();
   pdl_wait();
@@ -351,21 +352,28 @@ __global__ void __launch_bounds__(256) talk_mix_kernel(const float* __restrict__
   const int t = blockIdx.x, rep = nh / nkv;
   const float* A = parts + (size_t)t * nh * nkv * vd;
   bf16* o = out + (size_t)t * nh * vd;
-  for (int x = threadIdx.x; x < nkv * vd; x += blockDim.x) {
-    const int c = x / vd, d = x % vd;
+  for (int x = threadIdx.x; x < nkv * vd / 4; x += blockDim.x) {
+    const int c = 4 * x / vd, d = 4 * x % vd;
     for (int h0 = 0; h0 < rep; h0 += HB) {
-      float acc[HB];
+      float4 acc[HB];
 #pragma unroll
-      for (int i = 0; i < HB; ++i) acc[i] = 0.f;
+      for (int i = 0; i < HB; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
       for (int g = 0; g < nh; ++g) {
-        const float a = A[((size_t)g * nkv + c) * vd + d];
+        const float4 a = *reinterpret_cast<const float4*>(A + ((size_t)g * nkv + c) * vd + d);
 #pragma unroll
         for (int i = 0; i < HB; ++i)
-          if (h0 + i < rep) acc[i] = fmaf(msm[(c * rep + h0 + i) * nh + g], a, acc[i]);
+          if (h0 + i < rep) {
+            const float m = msm[(c * rep + h0 + i) * nh + g];
+            acc[i].x = fmaf(m, a.x, acc[i].x); acc[i].y = fmaf(m, a.y, acc[i].y);
+            acc[i].z = fmaf(m, a.z, acc[i].z); acc[i].w = fmaf(m, a.w, acc[i].w);
+          }
       }
 #pragma unroll
       for (int i = 0; i < HB; ++i)
-        if (h0 + i < rep) o[(size_t)(c * rep + h0 + i) * vd + d] = __float2bfloat16_rn(acc[i]);
+        if (h0 + i < rep)
+          *reinterpret_cast<uint2*>(o + (size_t)(c * rep + h0 + i) * vd + d) =
+              make_uint2(pack_bf16(acc[i].x, acc[i].y), pack_bf16(acc[i].z, acc[i].w));
     }
   }
 }
@@ -412,6 +420,6 @@ RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const vo
   else { if (few) GO(128, true) else GO(128, false) }
 #undef GO
   if (rc) return rc;
-  return launch_ex(talk_mix_kernel, dim3((unsigned)n_tokens), dim3(256), sizeof(float) * nh * nh, s, 1, (const float*)parts,
+  return launch_ex(talk_mix_kernel, dim3((unsigned)n_tokens), dim3(128), sizeof(float) * nh * nh, s, 1, (const float*)parts,
                    mix, (bf16*)out, nh, nkv, vd);
 }

@@ -155,7 +155,8 @@ struct Params {
   int bn;             // persistent kernel: tokens per tile (a multiple of 16, at most the template's BN)
   int* err;           // device error word (0 = fine)
   int x_rows, x_gs;   // x_rows > 0: weight rows in groups of that many (a multiple of BM), group g reads X's columns from g * x_gs on
-  int act;            // store epilogue only: 0 the value as it is, 1 max(value, 0)^2, 2 gelu in its tanh form, 3 gelu in its erf form
+  int act;            // store epilogue: 0 the value as it is, 1 max(value, 0)^2, 2 gelu in its tanh form, 3 gelu in its erf form;
+                      // gate/up epilogue: what the gate passes, 0 silu, 2 gelu in its tanh form
   RopeArgs rope;
   NormArgs norm;      // NORM variants only
 };
@@ -193,7 +194,10 @@ __device__ __forceinline__ void emit(const Params& p, int t, int n, float v, flo
   if (EPI == EPI_STORE) ((bf16*)p.C)[o] = __float2bfloat16_rn(store_act(p, v));
   else if (EPI == EPI_STORE_F32) ((float*)p.C)[o] = v;
   else if (EPI == EPI_ACCUM_F32) ((float*)p.C)[o] += v;
-  else if (EPI == EPI_SWIGLU) ((bf16*)p.C)[o] = __float2bfloat16_rn(__fdividef(v, 1.f + __expf(-v)) * u);   // float, rounded once to bfloat16
+  else if (EPI == EPI_SWIGLU) {
+    if (p.act == 2) v = store_act(p, v); else v = __fdividef(v, 1.f + __expf(-v));
+    ((bf16*)p.C)[o] = __float2bfloat16_rn(v * u);                // float, rounded once to bfloat16
+  }
 }
 
 // (cos, sin) of a token's angle at one frequency, when the caller gave no table. Not inlined and returned
@@ -883,11 +887,19 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               if (n0 + c0 + 8 * q >= p.N) break;
-              float h[8];
+              float h[8];                                         // float, rounded once to bfloat16
+              if (p.act == 2) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float gv = __uint_as_float(g[8 * q + e]);
-                h[e] = __fdividef(gv, 1.f + __expf(-gv)) * __uint_as_float(u[8 * q + e]);   // float, rounded once to bfloat16
+                for (int e = 0; e < 8; ++e) {
+                  const float gv = __uint_as_float(g[8 * q + e]);
+                  h[e] = __fdividef(gv, 1.f + __expf(-1.5957691216057308f * (gv + 0.044715f * gv * gv * gv))) * __uint_as_float(u[8 * q + e]);
+                }
+              } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  const float gv = __uint_as_float(g[8 * q + e]);
+                  h[e] = __fdividef(gv, 1.f + __expf(-gv)) * __uint_as_float(u[8 * q + e]);
+                }
               }
               uint4 pk;
               pk.x = pack_bf16x2(h[0], h[1]); pk.y = pack_bf16x2(h[2], h[3]);
@@ -1499,7 +1511,7 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   else if ((rc = make_map(&mx, X, T, x_rows ? (long long)((N - 1) / x_rows) * x_gs + K : K, ldx, pair ? bn / 2 : bn))) return rc;
   Params p;
   p.C = Cout; p.ldc = (int)ldc; p.T = T; p.N = N; p.K = K; p.up_row0 = N; p.splits = splits; p.err = err; p.bn = bn;
-  p.act = epi == EPI_STORE ? t_store_act : 0;
+  p.act = epi == EPI_STORE || epi == EPI_SWIGLU ? t_store_act : 0;
   p.x_rows = x_rows; p.x_gs = x_gs;
   p.rope = rope ? *rope : RopeArgs{};
   p.norm = norm ? *norm : NormArgs{};
@@ -1563,11 +1575,14 @@ RLLM_API int rllm_tc_gemm_set_pairs(int on) { g_pairs = on != 0; return 0; }
 RLLM_API int rllm_tc_gemm_set_token_rows(int on) { g_token_rows = on != 0; return 0; }
 
 // The store epilogue (0) may carry an activation in the bits above the epilogue's number: epi = 0 | 1 << 8 stores
-// max(value, 0)^2, 0 | 2 << 8 gelu(value) in its tanh form, 0 | 3 << 8 in its erf form. The launcher's own state for one call:
+// max(value, 0)^2, 0 | 2 << 8 gelu(value) in its tanh form, 0 | 3 << 8 in its erf form; the gate/up epilogue (3) gelu in its
+// tanh form for silu, 3 | 2 << 8. The launcher's own state for one call:
 struct StoreAct {
   explicit StoreAct(int& epi) {
-    t_store_act = (epi & 0xff) == EPI_STORE ? (epi >> 8) : 0;
-    epi = ((epi >> 8) > 3 || ((epi >> 8) && (epi & 0xff) != EPI_STORE)) ? -1 : (epi & 0xff);
+    const int act = epi >> 8, e = epi & 0xff;
+    const bool fine = act == 0 || (e == EPI_STORE && act <= 3) || (e == EPI_SWIGLU && act == 2);
+    t_store_act = fine ? act : 0;
+    epi = fine ? e : -1;
   }
   ~StoreAct() { t_store_act = 0; }
 };

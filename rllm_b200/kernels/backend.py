@@ -504,9 +504,15 @@ class Backend:
 
     def linear_glu(self, x, w_gate_up, act, limit=0.0, alpha=1.0):
         """act(x Wg^T, x Wu^T) with w_gate_up = [Wg; Wu] in the run dtype; the two products stay float until the
-        activation has run."""
+        activation has run: in the product's epilogue where a tensor-core kernel takes it."""
         if act == "silu":
             return self.linear_swiglu(x, w_gate_up)
+        if act == "gelu_tanh":
+            if self._fused_norm(x, w_gate_up, gate_up=True):
+                return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows, gelu_gate=True)
+            x = x.tensor() if isinstance(x, Normed) else x
+            if self._tc(x, w_gate_up):
+                return self._sm100.gemm(x, w_gate_up, ops.EPI_SWIGLU, gelu_gate=True)
         return self._hy.glu_act(self.linear_f32(x, w_gate_up, tag="gate_up"), self.dtype, act, limit, alpha)
 
     def experts_glu_up(self, x, w_gate_up, plan, act, limit=0.0, alpha=1.0, block=None):

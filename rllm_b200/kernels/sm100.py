@@ -140,15 +140,18 @@ STORE_ACTS = {None: 0, "relu2": ACT_RELU2, "gelu_tanh": ACT_GELU_TANH, "gelu_erf
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, epilogue: int, out: torch.Tensor | None = None,
-         split: bool = True, relu2: bool = False, act: str | None = None) -> torch.Tensor:
+         split: bool = True, relu2: bool = False, act: str | None = None, gelu_gate: bool = False) -> torch.Tensor:
     """C = X W^T on the tensor cores. x [T, K] bf16 (unit inner stride); w [N, K] bf16 ([2N, K] with
     the SwiGLU epilogue). `out` is required for the accumulate epilogue (the float residual). `act`
     (store epilogue only; `relu2` True is act "relu2"): the activation of the float result is what is rounded and
-    stored: "relu2" max(., 0)^2, "gelu_tanh" gelu in its tanh form, "gelu_erf" in its erf form."""
+    stored: "relu2" max(., 0)^2, "gelu_tanh" gelu in its tanh form, "gelu_erf" in its erf form. `gelu_gate` (SwiGLU epilogue
+    only): the gate passes gelu in its tanh form instead of silu."""
+    if gelu_gate and epilogue != ops.EPI_SWIGLU:
+        raise ops.KernelError("tc gemm: gelu_gate goes with the SwiGLU epilogue only")
     act = "relu2" if relu2 else act
     if act is not None and (epilogue != ops.EPI_STORE or act not in STORE_ACTS):
         raise ops.KernelError("tc gemm: an activation (relu2, gelu_tanh, gelu_erf) goes with the store epilogue only")
-    code = epilogue | STORE_ACTS[act]
+    code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0)
     if not gemm_supported(x, w):
         raise ops.KernelError("tc gemm: operands must be bfloat16, K a multiple of 8, 16-byte aligned")
     st = init(x.device)
@@ -220,8 +223,11 @@ def norm_supported(h: torch.Tensor, g: torch.Tensor, w: torch.Tensor, rows: torc
 
 
 def gemm_norm(h: torch.Tensor, g: torch.Tensor, eps: float, w: torch.Tensor, epilogue: int,
-              rows: torch.Tensor | None = None, split: bool = True, act: str | None = None) -> torch.Tensor:
-    """C = rmsnorm(h[rows]; g, eps) W^T in one kernel (store, store-float or SwiGLU epilogue; `act` as in `gemm`)."""
+              rows: torch.Tensor | None = None, split: bool = True, act: str | None = None, gelu_gate: bool = False) -> torch.Tensor:
+    """C = rmsnorm(h[rows]; g, eps) W^T in one kernel (store, store-float or SwiGLU epilogue; `act` and `gelu_gate` as in
+    `gemm`)."""
+    if gelu_gate and epilogue != ops.EPI_SWIGLU:
+        raise ops.KernelError("tc gemm with norm: gelu_gate goes with the SwiGLU epilogue only")
     if act is not None and (epilogue != ops.EPI_STORE or act not in STORE_ACTS):
         raise ops.KernelError("tc gemm with norm: an activation (relu2, gelu_tanh, gelu_erf) goes with the store epilogue only")
     if not norm_supported(h, g, w, rows):
@@ -229,6 +235,7 @@ def gemm_norm(h: torch.Tensor, g: torch.Tensor, eps: float, w: torch.Tensor, epi
                               f"{norm_max_tokens()} tokens, bfloat16 weights, 16-byte aligned")
     if epilogue not in (ops.EPI_STORE, ops.EPI_STORE_F32, ops.EPI_SWIGLU):
         raise ops.KernelError("tc gemm with norm: epilogue must be store, store-float or SwiGLU")
+    code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0)
     st = init(h.device)
     T = h.shape[0] if rows is None else rows.numel()
     K = h.shape[1]
@@ -237,12 +244,12 @@ def gemm_norm(h: torch.Tensor, g: torch.Tensor, eps: float, w: torch.Tensor, epi
                       device=h.device)
     if split and stream_supported(epilogue, True, T, N, K):
         rc = ops._fn("sm100", "rllm_stream_gemm")(
-            epilogue | STORE_ACTS[act], None, 0, h.data_ptr(), h.stride(0), ops._ptr(rows), g.data_ptr(), ops._dt(g, "norm weight"),
+            code, None, 0, h.data_ptr(), h.stride(0), ops._ptr(rows), g.data_ptr(), ops._dt(g, "norm weight"),
             float(eps), w.data_ptr(), out.data_ptr(), out.stride(0), T, N, K, st.sm_count, ops._stream())
         ops._check(rc, "stream_gemm_norm")
         return out
     rc = ops._fn("sm100", "rllm_tc_gemm_norm")(
-        epilogue | STORE_ACTS[act], h.data_ptr(), h.stride(0), ops._ptr(rows), g.data_ptr(), ops._dt(g, "norm weight"), float(eps),
+        code, h.data_ptr(), h.stride(0), ops._ptr(rows), g.data_ptr(), ops._dt(g, "norm weight"), float(eps),
         w.data_ptr(), out.data_ptr(), out.stride(0), T, N, K, int(split), st.err.data_ptr(), st.sm_count,
         ops._stream())
     ops._check(rc, "tc_gemm_norm")
