@@ -103,7 +103,7 @@ struct PfParams {
   float cap_z;           // scale / cap
   int box_rows;          // TMA variant: keys per copy = min(page size, 128)
   int row_pairs, num_seqs, sm_count;
-  int long_from;         // sequences with fewer rows are left out (another kernel's)
+  int long_from;         // CROSS, DENSE: sequences with fewer rows are left out (another kernel's)
   float* cross;          // not null: every query head meets every kv head's values, and the output is the floats
                          // [token][query head][kv head of the values][VD] here
   // DENSE: keys and values of a sequence lie one after the other (a row per position, the sequences that are not left out
@@ -176,12 +176,15 @@ __device__ __forceinline__ void softcap_poly2(uint32_t& x0, uint32_t& x1, float 
 
 // TMA: the K and V tiles come by tensor copies over the caches seen as [pages * kv heads][page size][HD].
 // CAP: scores are bounded (p.cap).
-// DENSE: keys and values as in PfParams, by tensor copies of whole tiles.
-template <int KD, int VD, bool TMA, bool CAP, bool DENSE>
+// MODE PLAIN: pages. CROSS: pages, every head over every kv head's values, float outputs (PfParams). DENSE: keys and values in
+// rows, by tensor copies of whole tiles.
+enum : int { PLAIN = 0, CROSS = 1, DENSE_ROWS = 2 };
+template <int KD, int VD, bool TMA, bool CAP, int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                        const __grid_constant__ CUtensorMap tmap_r, const PfParams p) {
-  static_assert(TMA || !DENSE, "dense keys come by tensor copies");
+  constexpr bool DENSE = MODE == DENSE_ROWS;
+  static_assert(TMA || MODE == PLAIN, "the other forms come by tensor copies");
   typedef Shape<KD, VD> C;
   constexpr int KVS = C::KVS;
   extern __shared__ uint8_t pf_smem_raw[];
@@ -224,16 +227,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   // walks the items in its own copy of the loop (the block-wide barriers are the same ones).
   auto walk = [&](auto softmax_side) {
   constexpr bool SOFTMAX = decltype(softmax_side)::value;
-  const int vheads = p.cross ? p.nkv : 1;
+  const int vheads = MODE == CROSS ? p.nkv : 1;
   const int items = p.row_pairs * p.nkv * vheads * p.num_seqs;
   for (int round = 0;; ++round) {
   const int item = round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
   if (item >= items) break;
   const int tile0 = (p.row_pairs - 1 - item / (p.nkv * vheads * p.num_seqs)) * RT;      // first of the item's row tiles
   const int kvh = item % p.nkv, seq = (item / (p.nkv * vheads)) % p.num_seqs;
-  const int vh = p.cross ? item / p.nkv % p.nkv : kvh;                         // the kv head of the values
+  const int vh = MODE == CROSS ? item / p.nkv % p.nkv : kvh;                         // the kv head of the values
   // an item beyond its sequence's rows (a short portion beside long ones) is skipped by all threads alike
-  if (tile0 * PM >= (p.cu_q[seq + 1] - p.cu_q[seq]) * G || p.cu_q[seq + 1] - p.cu_q[seq] < p.long_from) continue;
+  if (tile0 * PM >= (p.cu_q[seq + 1] - p.cu_q[seq]) * G) continue;
+  if (MODE != PLAIN && p.cu_q[seq + 1] - p.cu_q[seq] < p.long_from) continue;
   __syncthreads();                                      // everybody has left the item before
   if (threadIdx.x == 0) {
     for (int i = 0; i < KVS; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
@@ -645,13 +649,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         if (!p.gate_cols) { inv *= 1.f / (1.f + __expf(-__bfloat162float(*gh))); gh = nullptr; }
       }
       bf16* dst = p.out + (size_t)(q0 + tok) * p.out_stride + (size_t)head * VD;
-      float* fdst = p.cross ? p.cross + (((size_t)(q0 + tok) * p.nh + head) * p.nkv + vh) * VD : nullptr;
+      float* fdst = MODE == CROSS ? p.cross + (((size_t)(q0 + tok) * p.nh + head) * p.nkv + vh) * VD : nullptr;
 #pragma unroll
       for (int c = 0; c < VD / 32; ++c) {
         uint32_t ov[32];
         tmem_ld32(pv_addr + 32 * c, ov);
         tmem_ld_wait();
-        if (valid && fdst) {
+        if (MODE == CROSS) {
+          if (!valid) continue;
 #pragma unroll
           for (int i = 0; i < 32; i += 4)
             *reinterpret_cast<float4*>(fdst + 32 * c + i) =
@@ -755,18 +760,21 @@ int cache_map(CUtensorMap* out, const void* ptr, long long planes, int page_size
   return 0;
 }
 
-template <int KD, int VD, bool TMA, bool CAP, bool DENSE>
+template <int KD, int VD, bool TMA, bool CAP, int MODE>
 int launch_pf_c(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, const PfParams& p, int ctas, cudaStream_t s) {
   static bool configured[64] = {};
   constexpr int smem = Shape<KD, VD>::SMEM_BYTES;
-  if (allow_dynamic_smem(attn_prefill_tc_kernel<KD, VD, TMA, CAP, DENSE>, smem, configured)) return -5;
-  return launch_ex(attn_prefill_tc_kernel<KD, VD, TMA, CAP, DENSE>, dim3(ctas), dim3(THREADS), smem, s, 1, mk, mv, mr, p);
+  if (allow_dynamic_smem(attn_prefill_tc_kernel<KD, VD, TMA, CAP, MODE>, smem, configured)) return -5;
+  return launch_ex(attn_prefill_tc_kernel<KD, VD, TMA, CAP, MODE>, dim3(ctas), dim3(THREADS), smem, s, 1, mk, mv, mr, p);
 }
 
 template <int HD, bool TMA>
 int launch_pf(const CUtensorMap& mk, const CUtensorMap& mv, const PfParams& p, int ctas, cudaStream_t s) {
-  return p.cap.c > 0.f ? launch_pf_c<HD, HD, TMA, true, false>(mk, mv, mk, p, ctas, s)
-                       : launch_pf_c<HD, HD, TMA, false, false>(mk, mv, mk, p, ctas, s);
+  if constexpr (TMA) {
+    if (p.cross) return launch_pf_c<HD, HD, true, false, CROSS>(mk, mv, mk, p, ctas, s);
+  }
+  return p.cap.c > 0.f ? launch_pf_c<HD, HD, TMA, true, PLAIN>(mk, mv, mk, p, ctas, s)
+                       : launch_pf_c<HD, HD, TMA, false, PLAIN>(mk, mv, mk, p, ctas, s);
 }
 
 // Rows of 128 (or the heads' shared 64) numbers by tensor copies of 64 rows: [heads][rows][n], strides in numbers.
@@ -802,7 +810,7 @@ int multiprocessors(int asked, int& sms) {
 // max_q_len: the longest portion in the batch (sizes the list of work items). Head sizes 64 and 128.
 // chunk > 0: a query sees only the keys of its own block of `chunk` positions (blocks counted from position 0);
 // sinks: float [nh] or null; gate: float logits [T, gate_ld] or null (see PfParams); keep_first, sigmoid: see PfParams.
-// softcap > 0: bounded scores. long_from: sequences with fewer rows are left out. cross: see PfParams. sm_count: CTAs to launch at most (0: asked from the device).
+// softcap > 0: bounded scores. cross, long_from: see PfParams. sm_count: CTAs to launch at most (0: asked from the device).
 RLLM_API int rllm_attention_prefill_tc(const void* q, int q_stride, const void* kcache, const void* vcache,
                                        void* out, int out_stride, const int* cu_q, const int* kv_lens,
                                        const int* block_table, int bt_stride, int num_seqs, int max_q_len,
@@ -815,6 +823,7 @@ RLLM_API int rllm_attention_prefill_tc(const void* q, int q_stride, const void* 
     return ERR_BAD_SIZE;
   if (q_stride % 8 || out_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) ||
       ((uintptr_t)kcache & 15) || ((uintptr_t)vcache & 15)) return ERR_BAD_ALIGN;
+  if (long_from > 0 && !cross) return ERR_BAD_SIZE;
   if (cross && (softcap > 0.f || sigmoid || gate || ((uintptr_t)cross & 15))) return ERR_BAD_SIZE;
   PfParams p = {};
   p.long_from = long_from; p.cross = cross;
@@ -886,6 +895,6 @@ RLLM_API int rllm_attention_prefill_dense(const void* q, int q_stride, int q_hea
   mr = mk;
   if (r && (rc = dense_map(&mr, r, 64, rows, r_stride, 1, rows * r_stride))) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  return r ? launch_pf_c<192, 128, true, false, true>(mk, mv, mr, p, ctas, s)
-           : launch_pf_c<128, 128, true, false, true>(mk, mv, mr, p, ctas, s);
+  return r ? launch_pf_c<192, 128, true, false, DENSE_ROWS>(mk, mv, mr, p, ctas, s)
+           : launch_pf_c<128, 128, true, false, DENSE_ROWS>(mk, mv, mr, p, ctas, s);
 }

@@ -12,17 +12,24 @@
 //   chunk_prep_kernel   a CTA a (chunk, head), all chunks side by side: M, P q, k P_end / P, and for DELTA W = (I + L)^-1 beta P k
 //                       and (I + L)^-1 beta V, the inverse by blocks of 16 (what is left of U is - W S_0).
 //   chunk_carry_kernel  a CTA a (sequence, head, NC value columns) walks the chunks: keeps the state it meets for the last
-//                       kernel, U -= W S, S = P_end S + (k P_end / P)^T U. The next chunk's rows travel meanwhile (cp.async).
+//                       kernel, U -= W S, S = P_end S + (k P_end / P)^T U. The rows of the chunk after the next travel meanwhile.
 //   chunk_out_kernel    a CTA a (chunk, head, 64 value columns), all side by side: O.
+// What a kernel leaves for the next lies in the scratch as the next one's shared memory holds it (rows padded, value columns
+// in tiles of 16), so that a few bulk copies by one thread bring it (16-byte copies by all threads cost as much as the sums).
 // Decays per channel do not factor out of M and L. Blocks of 16 x 16 below the diagonal are a product of rows scaled by the
 // decays since their own block's beginning with rows scaled by the decays up to it (both at most 1); the ones on the diagonal
 // are summed with a running product per channel.
-// What bounds it: the FMA units (a token costs a head about 73,000 FMAs at 128 x 128, no fewer than token by token), not a
-// chain; a product's operands come from shared memory in tiles of 32 x 16 a warp, 64 FMAs for 8 loads of 16 bytes.
+// What bounds it: FMAs and the shared memory that feeds them (a token costs a head about 73,000 FMAs at 128 x 128, no fewer
+// than token by token), no longer a chain; a product's operands come in tiles of 32 x 16 a warp, 64 FMAs for 8 loads of 16
+// bytes (8 x 8 outputs a thread, half the loads: level, and 85 us against 59 where a CTA's sum is short).
+// 2,048 tokens, bfloat16 runs, us (token by token before): delta rule with decays per channel, 16 heads of 128 x 128
+// 275 (1,061); with a decay per head, 32 heads 430 (1,050); state space, 32 heads of 128 x 64 200 (745); gated linear attention,
+// 16 heads 215 (405 in three passes over chunks).
 // 64 tokens: with 32 the walk over the chunks has twice the barriers for the same FMAs, with 128 the triangles cost more than
 // the rest. Sums are grouped differently than token by token, within float rounding.
 #pragma once
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace rllm {
 namespace chunked {
@@ -48,21 +55,23 @@ struct Args {
   float* state;                                       // [slots, H, D, vdim]
   float* out;                                         // [T, H, vdim]
   float* scratch;                                     // per (chunk, head): see Place
+  int* err;                                           // device word that a wait which runs out leaves its mark in
 };
 
-// One (chunk, head)'s share of the scratch.
+// One (chunk, head)'s share of the scratch: M [C][LC], P q [C][D + 4], k P_end / P [C][D], W [C][D + 4] (DELTA), U and the state the
+// chunk meets in tiles of 16 columns, [C][16] and [D][16] each, P_end [D]. Every piece a multiple of 16 bytes.
 template <int D>
 struct Place {
   float *m, *qd, *kt, *w, *u, *s, *pc;
   __host__ __device__ static long long floats(int vdim, bool delta) {
-    return (long long)C * C + 2 * C * D + (delta ? C * D : 0) + (long long)C * vdim + (long long)D * vdim + D;
+    return (long long)C * LC + C * (D + 4) + C * D + (delta ? C * (D + 4) : 0) + (long long)C * vdim + (long long)D * vdim + D;
   }
   __device__ Place(float* base, long long x, int vdim, bool delta) {
     m = base + x * floats(vdim, delta);
-    qd = m + C * C;
-    kt = qd + C * D;
+    qd = m + C * LC;
+    kt = qd + C * (D + 4);
     w = kt + C * D;
-    u = w + (delta ? C * D : 0);
+    u = w + (delta ? C * (D + 4) : 0);
     s = u + (long long)C * vdim;
     pc = s + (long long)D * vdim;
   }
@@ -80,8 +89,22 @@ __device__ __forceinline__ bool find_chunk(const Args& a, int b, int& row0, int&
   return false;
 }
 
-__device__ __forceinline__ void copy16(float* smem, const float* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+// n floats (a multiple of 4) into shared memory, counted by the barrier; one thread.
+__device__ __forceinline__ void bulk(float* smem, const float* gmem, int n, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm100::smem_u32(smem)),
+               "l"(gmem), "r"(4 * n), "r"(sm100::smem_u32(bar)) : "memory");
+}
+// All threads wait for a barrier's phase. A wait that runs out leaves its mark, waits once more (a copy may still be on its way
+// into this CTA's memory) and ends the CTA's work.
+__device__ __forceinline__ bool landed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err, int role) {
+  bool ok = sm100::mbar_wait(bar, parity, abort_flag);
+  if (!ok) {
+    *abort_flag = 1;
+    sm100::record_failure(err, role);
+    volatile int none = 0;
+    sm100::mbar_wait(bar, parity, &none);
+  }
+  return __syncthreads_and(ok);
 }
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -96,6 +119,7 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 // `col` = first column + 4 (lane % 4). K a multiple of 4; A's rows 16 bytes apart in bank phase (stride 4 mod 32).
 template <int NT>
 __device__ __forceinline__ void tile_product(float (&acc)[4][4 * NT], const float* A, int lda, const float* B, int ldb, int K) {
+#pragma unroll 2
   for (int k = 0; k < K; k += 4) {
     float4 x[4];
 #pragma unroll
@@ -175,18 +199,20 @@ __device__ __forceinline__ void unit_lower_inverse(const float* L, float* X, flo
 }
 
 template <typename TI, int D, bool PERCH, bool DELTA, bool BONUS>
-__global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_kernel(Args a) {
+__global__ void __launch_bounds__(THREADS, 2) chunk_prep_kernel(Args a) {
   pdl_launch();
   pdl_wait();
   constexpr int LDD = D + 4, NV = D / 4;
   extern __shared__ __align__(16) float sm[];
-  float* Q = sm;                                        // [C][LDD] each
+  float* few = sm;                                      // [C] decays, [C] beta or value scales
+  float* Q = few + 2 * C;                               // [C][LDD] each
   float* K = Q + C * LDD;
-  float* A = K + C * LDD;                               // decays per channel, later k scaled up to the next block
-  float* G1 = PERCH ? A + C * LDD : A;                  // [C][LC] ratios of decays (per head), later the inverse
-  float* G2 = G1 + C * LC;                              // [C][LC] L (DELTA)
-  float* few = G1 + (DELTA ? 2 : PERCH ? 0 : 1) * C * LC;   // [C] decays, [C] beta or value scales
-  float* blk = few + 2 * C;                             // per channel: [4][D] a block's product; scalar: scratch
+  float* A = K + C * LDD;                               // PERCH: decays, later k scaled up to the next block, later L and the inverse
+  float* blk = A + C * LDD;                             // PERCH: [4][D] products of blocks
+  float* G2 = A;                                        // [C][LC] L (DELTA)
+  float* G1 = A + (DELTA ? C * LC : 0);                 // [C][LC] ratios of decays (per head); the inverse (DELTA)
+  float* tmp = G1 + C * LC;                             // 3 x 16 x 17 for the inverse, or 5 x 64 products (per head)
+  // L of the decays per channel waits in W's place of the scratch until A's is free (a second CTA fits the SM that way)
   int row0, n;
   if (!find_chunk(a, blockIdx.x, row0, n)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -228,11 +254,32 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
   const float* beta = few + C;
 
   if constexpr (!PERCH) {
-    // one decay a head: the ratios of products are a matrix of their own, G1[t][j] = a_(j+1) ... a_t
+    // one decay a head: the ratios of products are a matrix of their own, G1[t][j] = a_(j+1) ... a_t: inside a block of 16 one by
+    // one, below as (up to the end of j's block) (the blocks between) (from the beginning of t's block)
+    float* upto = tmp;                                   // [C] from the block's beginning
+    float* rest = tmp + C;                               // [C] to the block's end
     if (tid < C) {
+      const int b = tid & ~(SB - 1), j = tid;
       float r = 1.f;
-      G1[tid * LC + tid] = 1.f;
-      for (int t = tid + 1; t < C; ++t) { r *= few[t]; G1[t * LC + tid] = r; }
+      for (int t = b; t <= j; ++t) r *= few[t];
+      upto[j] = r;
+      r = 1.f;
+#pragma unroll
+      for (int e = 0; e < SB; ++e) {
+        const int t = b + e;
+        if (t > j) r *= few[t];
+        G1[t * LC + j] = r;                              // 1 where t <= j
+      }
+      rest[j] = r;
+    }
+    __syncthreads();
+    for (int x = tid; x < C * C; x += THREADS) {
+      const int t = x / C, j = x % C, I = t / SB, J = j / SB;
+      if (J < I) {
+        float r = rest[j];
+        for (int b = J + 1; b < I; ++b) r *= upto[b * SB + SB - 1];
+        G1[t * LC + j] = r * upto[t];
+      }
     }
     __syncthreads();
     const float first = few[0];
@@ -262,7 +309,7 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
       for (int j = 0; j < 4; ++j) {
         const int t = r0 + 4 * i, s = c0 + 8 * j;
         const float r = s <= t ? G1[t * LC + s] : 0.f;
-        to.m[t * C + s] = s <= t ? m[i][j] * r : 0.f;
+        to.m[t * LC + s] = s <= t ? m[i][j] * r : 0.f;
         if (DELTA) G2[t * LC + s] = s < t ? beta[t] * l[i][j] * r : 0.f;
       }
     // P q and k P_end / P; what K holds afterwards is k P (times beta) for the last product
@@ -270,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
       const int t = x / NV, c = x % NV * 4;
       const float p = first * G1[t * LC], e = G1[(C - 1) * LC + t];
       float4 q = *reinterpret_cast<float4*>(Q + t * LDD + c), k = *reinterpret_cast<float4*>(K + t * LDD + c);
-      *reinterpret_cast<float4*>(to.qd + t * D + c) = make_float4(q.x * p, q.y * p, q.z * p, q.w * p);
+      *reinterpret_cast<float4*>(to.qd + t * LDD + c) = make_float4(q.x * p, q.y * p, q.z * p, q.w * p);
       *reinterpret_cast<float4*>(to.kt + t * D + c) = make_float4(k.x * e, k.y * e, k.z * e, k.w * e);
     }
     if (tid < D) to.pc[tid] = first * G1[(C - 1) * LC];
@@ -322,15 +369,15 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
 #pragma unroll
         for (int e = 0; e < SB; ++e) {
           if (j + e < SB) {
-            to.m[(b + j + e) * C + b + j] = m[e];
-            if (DELTA) G2[(b + j + e) * LC + b + j] = e ? beta[b + j + e] * l[e] : 0.f;
+            to.m[(b + j + e) * LC + b + j] = m[e];
+            if (DELTA) to.w[(b + j + e) * LC + b + j] = e ? beta[b + j + e] * l[e] : 0.f;
           }
         }
       }
     }
     for (int x = tid; x < C * C; x += THREADS) {           // nothing above the diagonal
       const int t = x / C, j = x % C;
-      if (j > t) { to.m[x] = 0.f; if (DELTA) G2[t * LC + j] = 0.f; }
+      if (j > t) { to.m[t * LC + j] = 0.f; if (DELTA) to.w[t * LC + j] = 0.f; }
     }
     __syncthreads();
     // rows scaled by the decays since their block's beginning (q, k), and k by those up to the block's end (in A's place)
@@ -374,8 +421,8 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
       }
 #pragma unroll
       for (int J = 0; J < I; ++J) {
-        to.m[(I * SB + t) * C + J * SB + j] = m[J];
-        if (DELTA) G2[(I * SB + t) * LC + J * SB + j] = beta[I * SB + t] * l[J];
+        to.m[(I * SB + t) * LC + J * SB + j] = m[J];
+        if (DELTA) to.w[(I * SB + t) * LC + J * SB + j] = beta[I * SB + t] * l[J];
       }
       __syncthreads();
       for (int x = tid; x < I * SB * NV; x += THREADS) {   // up to the end of block I
@@ -394,7 +441,7 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
         p = make_float4(p.x * d.x, p.y * d.y, p.z * d.z, p.w * d.w);
       }
       const float4 q = *reinterpret_cast<const float4*>(Q + t2 * LDD + c);
-      *reinterpret_cast<float4*>(to.qd + t2 * D + c) = make_float4(q.x * p.x, q.y * p.y, q.z * p.z, q.w * p.w);
+      *reinterpret_cast<float4*>(to.qd + t2 * LDD + c) = make_float4(q.x * p.x, q.y * p.y, q.z * p.z, q.w * p.w);
       *reinterpret_cast<float4*>(to.kt + t2 * D + c) = *reinterpret_cast<const float4*>(A + t2 * LDD + c);
       if (DELTA) {
         float4* k = reinterpret_cast<float4*>(K + t2 * LDD + c);
@@ -411,11 +458,15 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (t < n) v = load4(vg + (long long)(row0 + t) * a.v_ld + c);
       const float f = beta[t];
-      *reinterpret_cast<float4*>(to.u + (long long)t * V + c) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+      *reinterpret_cast<float4*>(to.u + (c / 16 * C + t) * 16 + c % 16) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
     }
   } else {
     __syncthreads();                                       // Q is done with, L and K are whole
-    unit_lower_inverse(G2, G1, PERCH ? A : blk);
+    if (PERCH) {
+      for (int x = tid; x < C * LC / 4; x += THREADS) *reinterpret_cast<float4*>(G2 + 4 * x) = *reinterpret_cast<const float4*>(to.w + 4 * x);
+      __syncthreads();
+    }
+    unit_lower_inverse(G2, G1, tmp);
     // W = X (beta P k), then X (beta v), D value columns at a time in Q's place
     const int rl = (warp & 1) * 32 + (lane >> 2), cl = (warp >> 1) * 16 + 4 * (lane & 3);
     const int kk = (warp & 1) ? C : C / 2;                 // the upper rows meet the first half only
@@ -424,7 +475,7 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
       tile_product<1>(acc, G1 + rl * LC, LC, K + c + cl, LDD, kk);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float4*>(to.w + (rl + 8 * i) * D + c + cl) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        *reinterpret_cast<float4*>(to.w + (rl + 8 * i) * LDD + c + cl) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     }
     for (int v0 = 0; v0 < V; v0 += D) {
       const int nv = min(D, V - v0);
@@ -442,24 +493,29 @@ __global__ void __launch_bounds__(THREADS, (PERCH && DELTA) ? 1 : 2) chunk_prep_
         tile_product<1>(acc, G1 + rl * LC, LC, Q + c + cl, LDD, kk);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<float4*>(to.u + (long long)(rl + 8 * i) * V + v0 + c + cl) =
+          *reinterpret_cast<float4*>(to.u + ((v0 + c + cl) / 16 * C + rl + 8 * i) * 16 + cl % 16) =
               make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
       }
     }
   }
 }
 
-// NC value columns a CTA (16, or 32 where there are CTAs enough): 8 warps, for U two halves of the rows x four quarters of the
-// channels, for S a quarter of the channels (32; at D = 64 an eighth of the work each: two x four) x halves of the tokens.
+// NC value columns a CTA (16, or 32 where there are CTAs enough), eight warps: for U two halves of the rows x four quarters of
+// the channels, for S groups of 32 channels x parts of the tokens, tiles of 4 x 4 (x 2) a thread, partial sums joined through
+// shared memory. (A row of U and two channels of S a thread over whole sums, without joining: 141 us against 109 at 16 heads
+// of 128 x 128 and 2,048 tokens. What counts is the bytes that a sum's operands move out of shared memory: 128 a cycle, so
+// that a 16-byte load costs a warp four cycles whether its lanes share addresses or not.)
 template <int D, int NC, bool DELTA>
 __global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
   pdl_launch();
   pdl_wait();
   constexpr int LDW = D + 4, NT = NC / 16, RG = D / 32, JG = 8 / RG;     // S: RG groups of 32 channels x JG parts of the tokens
   constexpr int STAGE = (DELTA ? C * LDW : 0) + C * D + C * NC + D;
-  extern __shared__ __align__(16) float sm[];
-  float* S = sm + 2 * STAGE;                             // [D][NC]
-  float* part = S + D * NC;                              // [4][C][NC] sums of U, or [JG - 1][D][NC] of S
+  extern __shared__ __align__(128) float sm[];
+  __shared__ __align__(8) uint64_t full[2];
+  __shared__ int abort_flag;
+  float* S = sm + 2 * STAGE;                             // [NT][D][16]
+  float* part = S + D * NC;                              // [4][NT][C][16] sums of U, or [JG - 1][NT][D][16] of S
   const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * NC, H = a.H, V = a.vdim;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = a.cu_q[seq + 1] - a.cu_q[seq], chunks = chunks_of(n, a.long_from);
@@ -468,49 +524,70 @@ __global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
   for (int s = 0; s < seq; ++s) base += chunks_of(a.cu_q[s + 1] - a.cu_q[s], a.long_from);
   const int slot = a.state_slots ? a.state_slots[seq] : -1;
   float* sp = a.state + ((long long)(slot < 0 ? 0 : slot) * H + h) * D * V + v0;
-  auto issue = [&](int ci, int stage) {
-    const Place<D> in(a.scratch, (long long)(base + ci) * H + h, V, DELTA);
-    float* ws = sm + stage * STAGE;
-    float* ks = ws + (DELTA ? C * LDW : 0);
-    float* us = ks + C * D;
-    float* ps = us + C * NC;
-    for (int x = tid; x < C * (D / 4); x += THREADS) {
-      if (DELTA) copy16(ws + x / (D / 4) * LDW + x % (D / 4) * 4, in.w + 4 * x);
-      copy16(ks + 4 * x, in.kt + 4 * x);
-    }
-    for (int x = tid; x < C * (NC / 4); x += THREADS)
-      copy16(us + 4 * x, in.u + (long long)(x / (NC / 4)) * V + v0 + x % (NC / 4) * 4);
-    if (tid < D / 4) copy16(ps + 4 * tid, in.pc + 4 * tid);
-  };
-  issue(0, 0);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int x = tid; x < D * (NC / 4); x += THREADS) {
-    const int k = x / (NC / 4), c = x % (NC / 4) * 4;
-    *reinterpret_cast<float4*>(S + k * NC + c) =
-        slot >= 0 ? *reinterpret_cast<const float4*>(sp + (long long)k * V + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid == 0) {
+    abort_flag = 0;
+    sm100::mbar_init(&full[0], 1);
+    sm100::mbar_init(&full[1], 1);
+    sm100::fence_barrier_init();
   }
-  for (int ci = 0; ci < chunks; ++ci) {
+  auto issue = [&](int ci) {                             // one thread
     const Place<D> in(a.scratch, (long long)(base + ci) * H + h, V, DELTA);
-    if (ci + 1 < chunks) issue(ci + 1, (ci + 1) & 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
     float* ws = sm + (ci & 1) * STAGE;
     float* ks = ws + (DELTA ? C * LDW : 0);
-    float* us = ks + C * D;
+    uint64_t* bar = &full[ci & 1];
+    sm100::mbar_expect_tx(bar, STAGE * 4);
+    if (DELTA) bulk(ws, in.w, C * LDW, bar);
+    bulk(ks, in.kt, C * D, bar);
+    bulk(ks + C * D, in.u + (long long)(v0 / 16) * C * 16, C * NC, bar);
+    bulk(ks + C * D + C * NC, in.pc, D, bar);
+  };
+  if (tid == 0) {
+    issue(0);
+    if (chunks > 1) issue(1);
+  }
+  const int c = 4 * (lane & 3);
+  for (int x = tid; x < D * (NC / 4); x += THREADS) {
+    const int k = x / (NC / 4), v = x % (NC / 4) * 4;
+    *reinterpret_cast<float4*>(S + (v / 16 * D + k) * 16 + v % 16) =
+        slot >= 0 ? *reinterpret_cast<const float4*>(sp + (long long)k * V + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __syncthreads();
+  for (int ci = 0; ci < chunks; ++ci) {
+    const Place<D> in(a.scratch, (long long)(base + ci) * H + h, V, DELTA);
+    float* ws = sm + (ci & 1) * STAGE;
+    const float* ks = ws + (DELTA ? C * LDW : 0);
+    float* us = ws + (DELTA ? C * LDW : 0) + C * D;      // [NT][C][16]
     const float* ps = us + C * NC;
-    for (int x = tid; x < D * (NC / 4); x += THREADS)     // the state that the chunk meets
-      *reinterpret_cast<float4*>(in.s + (long long)(x / (NC / 4)) * V + v0 + x % (NC / 4) * 4) = *reinterpret_cast<const float4*>(S + 4 * x);
+    for (int x = tid; x < D * (NC / 4); x += THREADS)    // the state that the chunk meets
+      *reinterpret_cast<float4*>(in.s + (long long)(v0 / 16) * D * 16 + 4 * x) = *reinterpret_cast<const float4*>(S + 4 * x);
+    if (!landed(&full[ci & 1], (uint32_t)(ci >> 1) & 1u, &abort_flag, a.err, 41)) return;
     if (DELTA) {
-      const int r = (warp & 1) * 32 + (lane >> 2), k0 = (warp >> 1) * (D / 4), c = 4 * (lane & 3);
-      float acc[4][4 * NT] = {};
-      tile_product<NT>(acc, ws + r * LDW + k0, LDW, S + k0 * NC + c, NC, D / 4);
+      const int r = (warp & 1) * 32 + (lane >> 2), k0 = (warp >> 1) * (D / 4);
+      float acc[NT][4][4] = {};
+#pragma unroll 2
+      for (int k = k0; k < k0 + D / 4; k += 4) {
+        float4 x[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(ws + (r + 8 * i) * LDW + k);
 #pragma unroll
-        for (int t = 0; t < NT; ++t)
-          *reinterpret_cast<float4*>(part + ((warp >> 1) * C + r + 8 * i) * NC + c + 16 * t) =
-              make_float4(acc[i][4 * t], acc[i][4 * t + 1], acc[i][4 * t + 2], acc[i][4 * t + 3]);
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const float4 y = *reinterpret_cast<const float4*>(S + (t * D + k + e) * 16 + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+              acc[t][i][0] = fmaf(xv, y.x, acc[t][i][0]); acc[t][i][1] = fmaf(xv, y.y, acc[t][i][1]);
+              acc[t][i][2] = fmaf(xv, y.z, acc[t][i][2]); acc[t][i][3] = fmaf(xv, y.w, acc[t][i][3]);
+            }
+          }
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float4*>(part + (((warp >> 1) * NT + t) * C + r + 8 * i) * 16 + c) =
+              make_float4(acc[t][i][0], acc[t][i][1], acc[t][i][2], acc[t][i][3]);
       __syncthreads();
       for (int x = tid; x < C * (NC / 4); x += THREADS) {
         const float4 p0 = *reinterpret_cast<const float4*>(part + 4 * x), p1 = *reinterpret_cast<const float4*>(part + C * NC + 4 * x);
@@ -519,98 +596,105 @@ __global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
         u.x -= (p0.x + p1.x) + (p2.x + p3.x); u.y -= (p0.y + p1.y) + (p2.y + p3.y);
         u.z -= (p0.z + p1.z) + (p2.z + p3.z); u.w -= (p0.w + p1.w) + (p2.w + p3.w);
         *reinterpret_cast<float4*>(us + 4 * x) = u;
-        *reinterpret_cast<float4*>(in.u + (long long)(x / (NC / 4)) * V + v0 + x % (NC / 4) * 4) = u;
+        *reinterpret_cast<float4*>(in.u + (long long)(v0 / 16) * C * 16 + 4 * x) = u;
       }
       __syncthreads();
     }
-    {
-      const int k = (warp % RG) * 32 + 4 * (lane >> 2), jg = warp / RG, c = 4 * (lane & 3);
-      float acc[4][4 * NT] = {};
+    const int k = (warp % RG) * 32 + 4 * (lane >> 2), jg = warp / RG;
+    float acc[NT][4][4] = {};
 #pragma unroll 8
-      for (int j = jg * (C / JG); j < (jg + 1) * (C / JG); ++j) {
-        const float4 x = *reinterpret_cast<const float4*>(ks + j * D + k);
-        const float xs[4] = {x.x, x.y, x.z, x.w};
+    for (int j = jg * (C / JG); j < (jg + 1) * (C / JG); ++j) {
+      const float4 x = *reinterpret_cast<const float4*>(ks + j * D + k);
+      const float xs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const float4 y = *reinterpret_cast<const float4*>(us + j * NC + c + 16 * t);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            acc[i][4 * t] = fmaf(xs[i], y.x, acc[i][4 * t]);
-            acc[i][4 * t + 1] = fmaf(xs[i], y.y, acc[i][4 * t + 1]);
-            acc[i][4 * t + 2] = fmaf(xs[i], y.z, acc[i][4 * t + 2]);
-            acc[i][4 * t + 3] = fmaf(xs[i], y.w, acc[i][4 * t + 3]);
-          }
-        }
-      }
-      if (jg > 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int t = 0; t < NT; ++t)
-            *reinterpret_cast<float4*>(part + ((jg - 1) * D + k + i) * NC + c + 16 * t) =
-                make_float4(acc[i][4 * t], acc[i][4 * t + 1], acc[i][4 * t + 2], acc[i][4 * t + 3]);
-      }
-      __syncthreads();
-      if (jg == 0) {
+      for (int t = 0; t < NT; ++t) {
+        const float4 y = *reinterpret_cast<const float4*>(us + (t * C + j) * 16 + c);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float p = ps[k + i];
-#pragma unroll
-          for (int t = 0; t < NT; ++t) {
-            float4 s = *reinterpret_cast<float4*>(S + (k + i) * NC + c + 16 * t);
-            float4 x = make_float4(acc[i][4 * t], acc[i][4 * t + 1], acc[i][4 * t + 2], acc[i][4 * t + 3]);
-#pragma unroll
-            for (int g = 0; g < JG - 1; ++g) {
-              const float4 y = *reinterpret_cast<const float4*>(part + (g * D + k + i) * NC + c + 16 * t);
-              x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-            }
-            *reinterpret_cast<float4*>(S + (k + i) * NC + c + 16 * t) =
-                make_float4(fmaf(p, s.x, x.x), fmaf(p, s.y, x.y), fmaf(p, s.z, x.z), fmaf(p, s.w, x.w));
-          }
+          acc[t][i][0] = fmaf(xs[i], y.x, acc[t][i][0]); acc[t][i][1] = fmaf(xs[i], y.y, acc[t][i][1]);
+          acc[t][i][2] = fmaf(xs[i], y.z, acc[t][i][2]); acc[t][i][3] = fmaf(xs[i], y.w, acc[t][i][3]);
         }
       }
-      __syncthreads();
+    }
+    if (jg > 0) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float4*>(part + (((jg - 1) * NT + t) * D + k + i) * 16 + c) =
+              make_float4(acc[t][i][0], acc[t][i][1], acc[t][i][2], acc[t][i][3]);
+    }
+    __syncthreads();
+    if (jg == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float p = ps[k + i];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          float4* sv = reinterpret_cast<float4*>(S + (t * D + k + i) * 16 + c);
+          float4 x = make_float4(acc[t][i][0], acc[t][i][1], acc[t][i][2], acc[t][i][3]);
+#pragma unroll
+          for (int g = 0; g < JG - 1; ++g) {
+            const float4 y = *reinterpret_cast<const float4*>(part + ((g * NT + t) * D + k + i) * 16 + c);
+            x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+          }
+          *sv = make_float4(fmaf(p, sv->x, x.x), fmaf(p, sv->y, x.y), fmaf(p, sv->z, x.z), fmaf(p, sv->w, x.w));
+        }
+      }
+    }
+    __syncthreads();                                     // this stage is done with, S is whole
+    if (tid == 0 && ci + 2 < chunks) {
+      sm100::fence_proxy_async();
+      issue(ci + 2);
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (slot >= 0)
-    for (int x = tid; x < D * (NC / 4); x += THREADS)
-      *reinterpret_cast<float4*>(sp + (long long)(x / (NC / 4)) * V + x % (NC / 4) * 4) = *reinterpret_cast<const float4*>(S + 4 * x);
+    for (int x = tid; x < D * (NC / 4); x += THREADS) {
+      const int k = x / (NC / 4), v = x % (NC / 4) * 4;
+      *reinterpret_cast<float4*>(sp + (long long)k * V + v) = *reinterpret_cast<const float4*>(S + (v / 16 * D + k) * 16 + v % 16);
+    }
 }
 
-// O of a chunk: [64][D + 64] x [D + 64][64], the rows of the second operand being the state the chunk meets and U.
+// O of a chunk: M U, then (P q) S on top, 64 value columns a CTA; the first product's operands (the smaller ones) land first.
 template <typename TI, int D, bool DELTA>
 __global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Args a) {
   pdl_launch();
   pdl_wait();
-  constexpr int LDA = D + C + 4, NB = 64;
-  extern __shared__ __align__(16) float sm[];
-  float* A = sm;                                         // [C][LDA]: P q | M
-  float* B = A + C * LDA;                                // [D + C][NB]
+  constexpr int LDD = D + 4;
+  extern __shared__ __align__(128) float sm[];
+  __shared__ __align__(8) uint64_t full[2];
+  __shared__ int abort_flag;
+  float* M = sm;                                         // [C][LC]
+  float* Q = M + C * LC;                                 // [C][LDD]
+  float* U = Q + C * LDD;                                // [4][C][16]
+  float* S = U + 4 * C * 16;                             // [4][D][16]
   int row0, n;
   if (!find_chunk(a, blockIdx.x, row0, n)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int H = a.H, h = blockIdx.y, V = a.vdim, v0 = blockIdx.z * NB, nv = min(NB, V - v0);
-  const Place<D> in(a.scratch, (long long)blockIdx.x * H + h, V, DELTA);
-  for (int x = tid; x < C * (D / 4); x += THREADS) copy16(A + x / (D / 4) * LDA + x % (D / 4) * 4, in.qd + 4 * x);
-  for (int x = tid; x < C * (C / 4); x += THREADS) copy16(A + x / (C / 4) * LDA + D + x % (C / 4) * 4, in.m + 4 * x);
-  for (int x = tid; x < D * (nv / 4); x += THREADS) {
-    const int k = x / (nv / 4), c = x % (nv / 4) * 4;
-    copy16(B + k * NB + c, in.s + (long long)k * V + v0 + c);
+  const int H = a.H, h = blockIdx.y, V = a.vdim, v0 = blockIdx.z * 64, tiles = min(4, (V - v0) / 16);
+  if (tid == 0) {
+    abort_flag = 0;
+    sm100::mbar_init(&full[0], 1);
+    sm100::mbar_init(&full[1], 1);
+    sm100::fence_barrier_init();
+    const Place<D> in(a.scratch, (long long)blockIdx.x * H + h, V, DELTA);
+    sm100::mbar_expect_tx(&full[0], 4 * (C * LC + tiles * C * 16));
+    bulk(M, in.m, C * LC, &full[0]);
+    bulk(U, in.u + (long long)(v0 / 16) * C * 16, tiles * C * 16, &full[0]);
+    sm100::mbar_expect_tx(&full[1], 4 * (C * LDD + tiles * D * 16));
+    bulk(Q, in.qd, C * LDD, &full[1]);
+    bulk(S, in.s + (long long)(v0 / 16) * D * 16, tiles * D * 16, &full[1]);
   }
-  for (int x = tid; x < C * (nv / 4); x += THREADS) {
-    const int k = x / (nv / 4), c = x % (nv / 4) * 4;
-    copy16(B + (D + k) * NB + c, in.u + (long long)k * V + v0 + c);
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  const int r = (warp & 1) * 32 + (lane >> 2), c = (warp >> 1) * 16 + 4 * (lane & 3);
-  if ((warp >> 1) * 16 >= nv) return;
+  const int tile = warp >> 1, r = (warp & 1) * 32 + (lane >> 2), c = 4 * (lane & 3);
   float acc[4][4] = {};
-  tile_product<1>(acc, A + r * LDA, LDA, B + c, NB, (warp & 1) ? D + C : D + C / 2);     // M is zero right of the diagonal
+  const bool ok0 = landed(&full[0], 0, &abort_flag, a.err, 42);
+  if (ok0 && tile < tiles)
+    tile_product<1>(acc, M + r * LC, LC, U + tile * C * 16 + c, 16, (warp & 1) ? C : C / 2);       // M is zero right of the diagonal
+  if (!landed(&full[1], 0, &abort_flag, a.err, 43) || !ok0 || tile >= tiles) return;
+  tile_product<1>(acc, Q + r * LDD, LDD, S + tile * D * 16 + c, 16, D);
   const float skip = a.skip ? a.skip[h] : 0.f;
-  const TI* vg = reinterpret_cast<const TI*>(a.v) + (long long)h * V + v0 + c;
+  const TI* vg = reinterpret_cast<const TI*>(a.v) + (long long)h * V + v0 + tile * 16 + c;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = r + 8 * i;
@@ -620,7 +704,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Args a) {
       const float4 v = load4(vg + (long long)(row0 + t) * a.v_ld);
       o.x = fmaf(skip, v.x, o.x); o.y = fmaf(skip, v.y, o.y); o.z = fmaf(skip, v.z, o.z); o.w = fmaf(skip, v.w, o.w);
     }
-    *reinterpret_cast<float4*>(a.out + ((long long)(row0 + t) * H + h) * V + v0 + c) = o;
+    *reinterpret_cast<float4*>(a.out + ((long long)(row0 + t) * H + h) * V + v0 + tile * 16 + c) = o;
   }
 }
 
@@ -629,7 +713,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Args a) {
 template <typename TI>
 inline bool takes(const Args& a, int dim) {
   auto fits = [](const void* p, long long ld) { return !((uintptr_t)p % (4 * sizeof(TI))) && ld % 4 == 0; };
-  return (dim == 64 || dim == 128) && a.vdim > 0 && a.vdim % 16 == 0 && fits(a.q, a.q_ld) && fits(a.k, a.k_ld) && fits(a.v, a.v_ld) &&
+  return a.err != nullptr && (dim == 64 || dim == 128) && a.vdim > 0 && a.vdim % 16 == 0 && fits(a.q, a.q_ld) && fits(a.k, a.k_ld) && fits(a.v, a.v_ld) &&
          !((uintptr_t)a.decay & 15) && !((uintptr_t)a.state & 15) && !((uintptr_t)a.out & 15) && !((uintptr_t)a.bonus & 15) &&
          !((uintptr_t)a.scratch & 15) && a.H <= 65535 && a.vdim / 16 <= 65535;
 }
@@ -641,9 +725,10 @@ inline long long scratch_floats(int T, int S, int H, int dim, int vdim, bool del
 template <typename TI, int D, bool PERCH, bool DELTA, bool BONUS>
 int launch(const Args& a, int T, cudaStream_t s) {
   constexpr int LDD = D + 4;
-  constexpr int BLK = PERCH ? 4 * D : 3 * SB * (SB + 1);
-  constexpr size_t prep = sizeof(float) * ((PERCH ? 3 : 2) * C * LDD + (DELTA ? 2 : PERCH ? 0 : 1) * C * LC + 2 * C + BLK);
-  constexpr size_t outs = sizeof(float) * (C * (D + C + 4) + (D + C) * 64);
+  constexpr int INV = 3 * SB * (SB + 1), MATS = DELTA ? 2 * C * LC + INV : PERCH ? 0 : C * LC + 2 * C;    // from A on
+  constexpr int OWN = PERCH ? C * LDD + 4 * D : 0;                                                        // A and blk
+  constexpr size_t prep = sizeof(float) * (2 * C + 2 * C * LDD + (MATS > OWN ? MATS : OWN));
+  constexpr size_t outs = sizeof(float) * (C * LC + C * LDD + 4 * C * 16 + 4 * D * 16);
   static bool ok_prep[64], ok_out[64], ok_16[64], ok_32[64];
   const unsigned chunks = (unsigned)(T / C + a.num_seqs);
   auto prep_k = chunk_prep_kernel<TI, D, PERCH, DELTA, BONUS>;
@@ -652,8 +737,8 @@ int launch(const Args& a, int T, cudaStream_t s) {
   rc = launch_ex(prep_k, dim3(chunks, a.H), dim3(THREADS), prep, s, 1, a);
   if (rc) return rc;
   auto carry = [&](auto kernel, int nc, bool (&ok)[64]) {
-    constexpr int RG = D / 32, JG = 8 / RG;
     const size_t stage = (DELTA ? C * (D + 4) : 0) + C * D + C * nc + D;
+    constexpr int RG = D / 32, JG = 8 / RG;
     const size_t part = (size_t)nc * (DELTA && 4 * C > (JG - 1) * D ? 4 * C : (JG - 1) * D);
     const size_t bytes = sizeof(float) * (2 * stage + D * nc + part);
     const int rc2 = allow_dynamic_smem(kernel, (int)bytes, ok);

@@ -305,7 +305,7 @@ RLLM_API int rllm_gla_decay(float* z, const float* bias, int T, int n, float tau
 RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, int k_off, int v_off, const float* alpha,
                            float qscale, int T, int S, int H, int dim, int vdim, const int* cu_q,
                            const int* state_slots, float* state, float* out, int chunk, float* chunk_state,
-                           float* chunk_decay, const float* bonus, int long_from, int any_short, float* scratch, void* stream) {
+                           float* chunk_decay, const float* bonus, int long_from, int any_short, float* scratch, int* err, void* stream) {
   if (S <= 0 || T <= 0) return 0;
   if (H <= 0 || dim <= 0 || dim > MAX_DIM || vdim <= 0) return ERR_BAD_SIZE;
   if (H > 65535 || (vdim + 31) / 32 > 65535) return ERR_TOO_LARGE;
@@ -317,7 +317,7 @@ RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, in
     chunked::Args c = {};
     c.q = p + q_off; c.k = p + k_off; c.v = p + v_off; c.q_ld = c.k_ld = c.v_ld = ld; c.q_heads = c.k_heads = H;
     c.qscale = qscale; c.decay = alpha; c.bonus = bonus; c.H = H; c.vdim = vdim; c.cu_q = cu_q; c.num_seqs = S;
-    c.state_slots = state_slots; c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch;
+    c.state_slots = state_slots; c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch; c.err = err;
     if (chunked::takes<bf16>(c, dim)) {
       const int rc = dim == 64 ? (bonus ? chunked::launch<bf16, 64, true, false, true>(c, T, s) : chunked::launch<bf16, 64, true, false, false>(c, T, s))
                                : (bonus ? chunked::launch<bf16, 128, true, false, true>(c, T, s) : chunked::launch<bf16, 128, true, false, false>(c, T, s));

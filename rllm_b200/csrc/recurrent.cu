@@ -636,7 +636,7 @@ RLLM_API int rllm_state_scan(int beta_dt, const float* q, long long q_ld, int q_
                              int k_heads, const float* v, long long v_ld, const float* decay, int decay_per_channel,
                              const void* beta, long long beta_ld, const float* vscale, const float* skip, int S, int H,
                              int dim, int vdim, const int* cu_q, const int* state_slots, float* state, float* out,
-                             int channels, int T, int long_from, int any_short, float* scratch, void* stream) {
+                             int channels, int T, int long_from, int any_short, float* scratch, int* err, void* stream) {
   if (S <= 0) return 0;
   if (H <= 0 || dim <= 0 || dim > 1024 || vdim <= 0 || q_heads <= 0 || k_heads <= 0 || H % q_heads || H % k_heads)
     return ERR_BAD_SIZE;
@@ -655,7 +655,7 @@ RLLM_API int rllm_state_scan(int beta_dt, const float* q, long long q_ld, int q_
     c.q = q; c.k = k; c.v = v; c.q_ld = q_ld; c.k_ld = k_ld; c.v_ld = v_ld; c.q_heads = q_heads; c.k_heads = k_heads;
     c.qscale = 1.f; c.decay = decay; c.beta = beta; c.beta_ld = beta_ld; c.beta_bf16 = a.beta_bf16; c.vscale = vscale;
     c.skip = skip; c.H = H; c.vdim = vdim; c.cu_q = cu_q; c.num_seqs = S; c.state_slots = state_slots;
-    c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch;
+    c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch; c.err = err;
     if (chunked::takes<float>(c, dim)) {
       const int rc = launch_chunked(c, dim, decay_per_channel != 0, beta != nullptr, T, s);
       if (rc || !any_short) return rc;

@@ -451,7 +451,7 @@ class Backend:
         return self._mix.gla_decay(z, bias, tau)
 
     def gla_scan(self, *a, **k):
-        return self._mix.gla_scan(*a, **k)
+        return self._mix.gla_scan(*a, err=self._sm100.init(self.device).err if self.fast else None, **k)
 
     def gla_finish(self, *a, **k):
         return self._mix.gla_finish(*a, **k)
@@ -560,7 +560,7 @@ class Backend:
 
     def state_scan(self, q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx, state, beta=None, vscale=None, skip=None):
         # the 32-bit run's results are the same bits however a sequence is cut into steps: row by row
-        long = ctx.long_rows() if self.dtype == torch.bfloat16 else {}
+        long = dict(ctx.long_rows(), err=self._sm100.init(self.device).err) if self.fast else {}
         return self._hy.state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx.cu_q, ctx.num_seqs,
                                    ctx.state_slots, state, beta, vscale, skip, **long)
 

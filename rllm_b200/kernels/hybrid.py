@@ -21,7 +21,7 @@ ops.register_signatures("recurrent", {
     "rllm_softplus_decay": [c_int, _P, _LL, c_int, _P, _P, c_int, c_int, c_int, _P, _P, _P],
     "rllm_state_scan_split": [c_int],
     "rllm_state_scan": [c_int, _P, _LL, c_int, _P, _LL, c_int, _P, _LL, _P, c_int, _P, _LL, _P, _P, c_int, c_int, c_int,
-                        c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P],
+                        c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P],
     "rllm_state_scan_chunk_floats": [c_int, c_int, c_int],
     "rllm_gated_norm": [_P, _P, c_int, _LL, _P, c_int, c_float, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P],
 })
@@ -300,12 +300,14 @@ def softplus_decay(z, col0, n, bias, a_log, want_step=False):
 
 
 def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seqs, state_slots, state, beta=None, vscale=None,
-               skip=None, channels: int = 0, long_from: int = 0, any_short: bool = True) -> torch.Tensor:
+               skip=None, channels: int = 0, long_from: int = 0, any_short: bool = True, err=None) -> torch.Tensor:
     """See csrc/recurrent.cu. q [T, q_heads * dim], k [T, k_heads * dim], v [T, heads * vdim]: float32 views with unit
     inner stride; decay float32 [T, heads * dim] (per channel) or [T, heads]; beta: logits [T, heads] of the
     projection's type (delta rule) or None (plain); vscale float32 [T, heads]; skip float32 [heads].
     -> float32 [T, heads, vdim]; `state` float32 [slots, heads, dim, vdim] is updated. `channels` (32, 16 or 8): key
-    channels a thread where the kernel with compiled sizes runs, for measurements; 0: chosen from the sizes."""
+    a thread where the kernel with compiled sizes runs, for measurements; 0: chosen from the sizes. `long_from` > 0: sequences
+    of at least so many rows run in chunks (csrc/chunk_scan.cuh) where the sizes allow; `any_short`: there are others; `err`:
+    the device's error word, without which nothing runs in chunks."""
     T = q.shape[0]
     for t, n, c in ((q, "q", q_heads * dim), (k, "k", k_heads * dim), (v, "v", heads * vdim)):
         _rows(t, n, c)
@@ -329,14 +331,14 @@ def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seq
         _f32(skip, "skip", (heads,))
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
     scratch = None
-    if long_from > 0 and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
+    if long_from > 0 and err is not None and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
         scratch = torch.empty((T // 64 + num_seqs) * heads * per, dtype=torch.float32, device=q.device)
     _check(_fn("recurrent", "rllm_state_scan")(
         _dt(beta, "beta") if beta is not None else 0, q.data_ptr(), q.stride(0), int(q_heads), k.data_ptr(), k.stride(0),
         int(k_heads), v.data_ptr(), v.stride(0), decay.data_ptr(), int(per_channel), _ptr(beta),
         beta.stride(0) if beta is not None else 0, _ptr(vscale), _ptr(skip), int(num_seqs), int(heads), int(dim), int(vdim),
         cu_q.data_ptr(), _ptr(state_slots), state.data_ptr(), out.data_ptr(), int(channels), T, int(long_from), int(any_short),
-        _ptr(scratch), _stream()), "state_scan", 1 if scratch is None else 3 + int(any_short))
+        _ptr(scratch), _ptr(err), _stream()), "state_scan", 1 if scratch is None else 3 + int(any_short))
     return out
 
 

@@ -395,9 +395,9 @@ def attention_prefill_tc(q, kcache, vcache, cu_q, kv_lens, block_table, max_q_le
     own block of that many positions; `sinks` float [nh]: exp(sink) joins a row's denominator; `gate` float
     logits [T, >= nh]: head h's output times sigmoid(gate[t, h]); `keep_first`: positions below it are seen whatever
     the window says; `sigmoid`: no softmax, a visible key's weight is sigmoid(score + sinks[head]); `softcap`: scores
-    bounded, softcap * tanh(score / softcap). `long_from`: sequences with fewer rows are left out. `cross` float32
-    [T, nh, nkv, hd]: every query head meets every kv head's values and the float outputs go there (pages of a power of two
-    from 8 keys on; no gate, bound or sigmoid)."""
+    bounded, softcap * tanh(score / softcap). `cross` float32 [T, nh, nkv, hd]: every query head meets every kv head's
+    values and the float outputs go there (pages of a power of two from 8 keys on; no gate, bound or sigmoid); sequences with
+    fewer than `long_from` rows are then left out."""
     if not prefill_tc_supported(q, kcache):
         raise ops.KernelError("attention_prefill_tc: bfloat16, head size 64 or 128, rows 16-byte aligned")
     st = init(q.device)

@@ -7,6 +7,11 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
+def ERR():
+    from rllm_b200.kernels import sm100
+    return sm100.init(torch.device(DEV)).err
+
+
 def rel(a, b):
     return float((a.double() - b).norm() / b.norm())
 
@@ -64,7 +69,7 @@ def test_state_scan_in_chunks(lens, dim, vdim, H, G, channel, delta):
     slots = torch.tensor([-1 if s == 1 else S - s for s in range(S)], dtype=torch.int32, device=DEV)
     state = rnd(S + 1, H, dim, vdim, seed=8)
     got = {}
-    for name, long in (("chunks", dict(long_from=64, any_short=min(lens) < 64)), ("rows", {})):
+    for name, long in (("chunks", dict(long_from=64, any_short=min(lens) < 64, err=ERR())), ("rows", {})):
         st = state.clone()
         o = hybrid.state_scan(q.view(T, -1), G, k.view(T, -1), G, v, a.view(T, -1), H, dim, vdim, cud, S, slots, st, beta=beta,
                               vscale=vs, skip=skip, **long)
@@ -103,7 +108,7 @@ def test_gated_linear_attention_in_chunks(lens, dim, vdim, H, bonus):
     slots = torch.tensor([-1 if s == 1 else S - s for s in range(S)], dtype=torch.int32, device=DEV)
     state = rnd(S + 1, H, dim, vdim, seed=4)
     got = {}
-    for name, long in (("chunks", dict(long_from=64, any_short=min(lens) < 64)), ("rows", {})):
+    for name, long in (("chunks", dict(long_from=64, any_short=min(lens) < 64, err=ERR())), ("rows", {})):
         st = state.clone()
         o = mix.gla_scan(proj, 8, 8 + H * dim, 8 + 2 * H * dim, a, dim ** -0.5, H, dim, vdim, cud, S, slots, st, bonus=u, **long)
         got[name] = (o, st)
