@@ -13,18 +13,25 @@
 //               16-byte cp.async, the three warps taking turns tile by tile, one stage each;
 //   warp 3      one thread issues the products of both row tiles in turn:  S = Q K^T  (M 128,
 //               N 128 keys, K 64) into the row tile's S accumulator, and  PV = P V  (M 128, N 64,
-//               K 128 keys) with P read from shared memory and V as it lies in the cache tile (an
+//               K 128 keys) with P read from TMEM and V as it lies in the cache tile (an
 //               MN-major operand: the contraction runs over key rows);
 //   warps 4..7  the softmax of the first row tile, one thread per row; warps 8..11 of the second.
 //               A thread reads its row of S (128 scores) from TMEM, takes the maximum, exp2 and
-//               the sum in float and writes P as bf16 in the swizzled layout of an A operand.
+//               the sum in float (scale, subtraction and sum two scores an instruction) and writes P
+//               as bf16 over the scores' own columns, two keys a column. P used to go through shared
+//               memory, in the swizzled layout of an A operand and behind a proxy fence, and a step
+//               waited for the PV product before it with its exponentials: 595 us at 8,192 tokens (32 / 8
+//               heads of 64) against 431, 58 against 49 at 2,048; heads of 128 688 against 626, 60 against 55.
+//               What bounds a step is what its two warps a scheduler issue and wait for, not the
+//               exponentials' unit: a quarter of them on the FMA pipe (a polynomial) cost 441 and 689 us,
+//               an S accumulator a row tile with P beside it and the wait behind the packed results 471 and 646.
 //               The row's output stays in TMEM, where PV of tile after tile is added up. The
 //               exponentials are taken against a maximum that is moved only when the true one
 //               has grown by more than 2^8 since (P then stays below 2^8, which bf16 holds as
 //               well as values below 1); when it moves, the thread scales its row of the output
 //               in TMEM (tcgen05.ld / st) before the next PV is added.
 // The (row tile, K tile) steps are numbered k = 0, 1, ... in the order A0 B0 A1 B1 ...; S of step k
-// lands in accumulator k % 3, so while both row tiles are in their softmax the scores of the step
+// lands in accumulator k % 3 once PV of step k - 3, whose P lay there, is complete, so while both row tiles are in their softmax the scores of the step
 // after are computed already, and a row tile that has written its P goes on at once: the four warp
 // schedulers always have a warp with work (two warps each, one of either tile).
 // TMEM: three S accumulators and PV of both tiles, 512 columns.
@@ -68,21 +75,19 @@ constexpr int TMEM_COLS = 512;
 
 // Sizes that follow from the head sizes: keys of KD and values of VD numbers, 64 / 64, 128 / 128 or 192 / 128. Operands lie in
 // shared memory as "atoms" of 128-byte rows (64 values), swizzled: a tile wider than 64 values is several atoms one after
-// the other. With keys of 192 the queries leave room for two stages.
+// the other. With keys of 192 the queries leave room for three stages.
 template <int KD, int VD> struct Shape {
   static_assert((KD == 64 && VD == 64) || (KD == 128 && VD == 128) || (KD == 192 && VD == 128), "head sizes");
   static constexpr int PN = KD == 64 ? 128 : 64;     // keys per tile (a V tile is 16 KB either way)
-  static constexpr int KVS = KD == 192 ? 2 : 4;      // K/V stages
+  static constexpr int KVS = KD == 192 ? 3 : 4;      // K/V stages
   static constexpr int HA = KD / 64;                 // atoms along the head dimension (Q, K)
   static constexpr int VA = VD / 64;                 // (V)
-  static constexpr int KA = PN / 64;                 // atoms along the keys (P)
-  static constexpr int ATOM_ROWS = PM * 128;         // bytes of one atom of Q or P (128 rows)
+  static constexpr int ATOM_ROWS = PM * 128;         // bytes of one atom of Q (128 rows)
   static constexpr int ATOM_KEYS = PN * 128;         // bytes of one atom of K or V (PN rows)
   static constexpr int K_BYTES = HA * ATOM_KEYS, V_BYTES = VA * ATOM_KEYS;     // one tile
   static constexpr int Q_BYTES = HA * ATOM_ROWS;     // one row tile of Q
-  static constexpr int P_BYTES = KA * ATOM_ROWS;     // one row tile of P
-  static constexpr int SMEM_BYTES = 1024 + RT * Q_BYTES + KVS * (K_BYTES + V_BYTES) + RT * P_BYTES;   // Q[2], K[KVS], V[KVS], P[2]
-  static constexpr int S_COL = 0, O_COL = SB * PN;   // TMEM: three S accumulators, then the output of both row tiles
+  static constexpr int SMEM_BYTES = 1024 + RT * Q_BYTES + KVS * (K_BYTES + V_BYTES);   // Q[2], K[KVS], V[KVS]
+  static constexpr int S_COL = 0, O_COL = SB * PN;   // TMEM: three S accumulators (P of a step in S's place), then the output of both row tiles
   static_assert(O_COL + RT * VD <= TMEM_COLS, "S and the outputs must fit in TMEM");
 };
 
@@ -151,6 +156,9 @@ __device__ __forceinline__ uint64_t f32x2(float a, float b) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
   return d;
 }
+__device__ __forceinline__ void split2(uint64_t d, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
+}
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -159,6 +167,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 __device__ __forceinline__ void softcap_poly2(uint32_t& x0, uint32_t& x1, float zscale, float c) {
@@ -196,7 +209,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   uint8_t* smem = (uint8_t*)(((uintptr_t)pf_smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int PN = C::PN;
   const uint32_t q_s = smem_u32(smem);
-  const uint32_t k_s = q_s + RT * C::Q_BYTES, v_s = k_s + KVS * C::K_BYTES, p_s = v_s + KVS * C::V_BYTES;
+  const uint32_t k_s = q_s + RT * C::Q_BYTES, v_s = k_s + KVS * C::K_BYTES;
 
   const int G = p.nh / p.nkv;
   constexpr int NST = TMA ? KVS : LOADERS;              // K/V stages in use
@@ -241,7 +254,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   __syncthreads();                                      // everybody has left the item before
   if (threadIdx.x == 0) {
     for (int i = 0; i < KVS; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
-    for (int i = 0; i < SB; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); }
+    for (int i = 0; i < SB; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 1); }
     for (int i = 0; i < RT; ++i) { mbar_init(&p_full[i], 4); mbar_init(&pv_full[i], 1); }
     mbar_init(&q_full, TMA ? 4 * RT : RT);             // TMA: one arrival per softmax warp, which brings its own rows of Q
     fence_barrier_init();
@@ -300,14 +313,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     if (k < 2 * n_both) { g = k & 1; t = k >> 1; } else { g = g_long; t = n_both + (k - 2 * n_both); }
   };
   // descriptors move with the address: 16 bytes are one unit of the start-address field
-  const uint64_t dq0 = umma_desc_sw128(q_s), dk0 = umma_desc_sw128(k_s), dv0 = umma_desc_sw128(v_s),
-                 dp0 = umma_desc_sw128(p_s);
+  const uint64_t dq0 = umma_desc_sw128(q_s), dk0 = umma_desc_sw128(k_s), dv0 = umma_desc_sw128(v_s);
   auto issue_s = [&](int k, bool& ok) {                 // S = Q K^T of step k (one thread)
     int g, t;
     step(k, g, t);
     const int ks = t % NST;
     if (k >= SB) {
-      // the accumulator's scores of step k - 3 are in their threads' registers
+      // the PV product of step k - 3 is complete: its P lay in the accumulator's place
       if (!mbar_wait(&s_free[k % SB], (uint32_t)(k / SB - 1) & 1u, &abort_flag)) {
         abort_flag = 1; record_failure(p.err, 28, k); ok = false; return;
       }
@@ -332,17 +344,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       abort_flag = 1; record_failure(p.err, 23, t); ok = false; return;
     }
     tc_fence_after();
-    const uint64_t dp = dp0 + (uint64_t)(g * (C::P_BYTES >> 4)), dv = dv0 + (uint64_t)((t % NST) * (C::V_BYTES >> 4));
-    const uint32_t acc = tmem_base + C::O_COL + (uint32_t)g * VD;
+    const uint64_t dv = dv0 + (uint64_t)((t % NST) * (C::V_BYTES >> 4));
+    const uint32_t acc = tmem_base + C::O_COL + (uint32_t)g * VD, pa = tmem_base + C::S_COL + (uint32_t)(k % SB) * PN;
 #pragma unroll
     for (int a = 0; a < C::VA; ++a)                     // 64 output values = one atom of V
 #pragma unroll
-      for (int ks = 0; ks < PN / 16; ++ks) {
-        // P: K-major, atoms of 64 keys, 32 bytes per 16 keys; V: MN-major, 16 key rows = 2 KB per step
-        umma_bf16(acc + (uint32_t)(a * 64), dp + (uint64_t)((ks >> 2) * (C::ATOM_ROWS >> 4) + (ks & 3) * 2),
-                  dv + (uint64_t)(a * (C::ATOM_KEYS >> 4) + ks * (2048 >> 4)), id_pv, t > 0 || ks > 0);
-      }
+      for (int ks = 0; ks < PN / 16; ++ks)
+        // P: 16 keys are 8 columns; V: MN-major, 16 key rows = 2 KB per step
+        umma_bf16_ts(acc + (uint32_t)(a * 64), pa + (uint32_t)(ks * 8), dv + (uint64_t)(a * (C::ATOM_KEYS >> 4) + ks * (2048 >> 4)),
+                     id_pv, t > 0 || ks > 0);
     umma_commit(&pv_full[g]);
+    umma_commit(&s_free[k % SB]);
     if (g == 1 || t >= n_both) umma_commit(&kv_empty[t % NST]);     // the last reader of this K and V stage
   };
   if (warp < LOADERS && TMA) {
@@ -472,6 +484,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         if (!TMA && ok && k + SB < n_steps) issue_s(k + SB, ok);
       }
       // nothing of this item may still be on its way to a barrier when the next item sets them up again
+      for (int k = max(0, n_steps - SB); k < n_steps && ok; ++k)
+        if (!mbar_wait(&s_free[k % SB], (uint32_t)(k / SB) & 1u, &abort_flag)) {
+          abort_flag = 1; record_failure(p.err, 29, k); ok = false;
+        }
       for (int t = max(0, n_tiles - NST); t < n_tiles && ok; ++t)
         if (!mbar_wait(&kv_empty[t % NST], (uint32_t)(t / NST) & 1u, &abort_flag)) {
           abort_flag = 1; record_failure(p.err, 26, t); ok = false;
@@ -510,7 +526,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     }
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     const uint32_t pv_addr = lane_addr + C::O_COL + (uint32_t)g * VD;
-    const uint32_t prow = p_s + (uint32_t)g * C::P_BYTES + (uint32_t)(r * 128);
     constexpr int NC = PN / 32;                           // the row's scores come 32 at a time
     const float sl = CAP ? 1.f : p.scale_log2e;        // bounded scores leave the bound in the log2 domain
     // m: what the exponentials are taken against, up to 2^8 behind the true maximum. A sink opens the row's
@@ -539,9 +554,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
 #pragma unroll
       for (int c = 0; c < NC; ++c) tmem_ld32(s_addr + 32 * c, v[c]);
       tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_free[k % SB]);        // the accumulator may take the scores of step k + 3
       if (CAP) {
         float far[NC];
 #pragma unroll
@@ -565,7 +577,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
             for (int i = 0; i < 32; ++i) v[c][i] = __float_as_uint(softcap_log2(__uint_as_float(v[c][i]), p.cap));
         }
       }
-      if (!valid || j0 + PN - 1 > pos || (j0 < lo && j0 + PN > kf)) {        // some key is hidden from this row
+      const bool hides = !valid || j0 + PN - 1 > pos || (j0 < lo && j0 + PN > kf);      // some key is hidden from this row
+      if (hides) {
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -588,10 +601,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       const bool move = !sig && cand > m + 8.f;           // also the first visible key (m = -inf)
       float corr = 1.f;
       if (move) { corr = fast_exp2(m - cand); m = cand; l *= corr; }      // exp2(-inf) = 0
-      if (t > 0) {
-        // the PV of the tile before is complete: P may be written again, the output may be touched
-        if (!wait_on(&pv_full[g], (uint32_t)(t - 1) & 1u, 25, t)) { ok = false; break; }
-        if (__any_sync(0xffffffffu, move)) {
+      // PV of the tile before has to be complete only where the output is touched; else the wait comes behind the
+      // exponentials (a phase is never skipped, so that a parity says which one it is)
+      auto pv_before = [&]() { return t == 0 || wait_on(&pv_full[g], (uint32_t)(t - 1) & 1u, 25, t); };
+      const bool moves = __any_sync(0xffffffffu, move);
+      if (moves) {
+        if (!pv_before()) { ok = false; break; }
+        if (t > 0) {
           tc_fence_after();
 #pragma unroll
           for (int c = 0; c < VD / 16; ++c) {
@@ -602,42 +618,47 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
             for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
             tmem_st16(pv_addr + 16 * c, ov);
           }
-          tmem_st_wait();
         }
       }
-      // ---- exponentials, their sum, P as bf16 into the A-operand layout
+      // ---- exponentials, their sum, P as bf16 into the scores' place, two keys a column
       const float use = (m == -INFINITY) ? 0.f : m;
-      float lq[8];                                        // partial sums side by side, added up in a fixed order
+      // two scores an instruction where the pipe takes two: what bounds a step is the instructions its warps issue
+      const uint64_t sl2 = f32x2(sl, sl), use2 = f32x2(-use, -use);
+      uint64_t lq[4];                                     // eight partial sums side by side, added up in a fixed order
 #pragma unroll
-      for (int i = 0; i < 8; ++i) lq[i] = 0.f;
+      for (int i = 0; i < 4; ++i) lq[i] = f32x2(0.f, 0.f);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const uint32_t base = prow + (uint32_t)(c >> 1) * C::ATOM_ROWS;    // an atom of 64 keys
+        uint32_t pk[16];
+        if (sig) {
+          // sigmoid(x) = 1 / (1 + 2^(-x log2 e)); hidden keys hold -inf: 1 / (1 + inf) = 0
 #pragma unroll
-        for (int q8 = 0; q8 < 4; ++q8) {                  // 8 keys = one 16-byte chunk
-          float e[8];
-          if (sig) {
-            // sigmoid(x) = 1 / (1 + 2^(-x log2 e)); hidden keys hold -inf: 1 / (1 + inf) = 0
-#pragma unroll
-            for (int i = 0; i < 8; ++i) e[i] = fast_rcp(1.f + fast_exp2(-fmaf(__uint_as_float(v[c][8 * q8 + i]), sl, sb)));
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              e[i] = fast_exp2(fmaf(__uint_as_float(v[c][8 * q8 + i]), sl, -use));      // hidden keys hold -inf: 0
-              lq[i] += e[i];
-            }
+          for (int i = 0; i < 16; ++i) {
+            const float e0 = fast_rcp(1.f + fast_exp2(-fmaf(__uint_as_float(v[c][2 * i]), sl, sb)));
+            const float e1 = fast_rcp(1.f + fast_exp2(-fmaf(__uint_as_float(v[c][2 * i + 1]), sl, sb)));
+            pk[i] = pack_bf16(e0, e1);
           }
-          const int ch = (c & 1) * 4 + q8;
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (uint32_t)((ch ^ (r & 7)) << 4)),
-                       "r"(pack_bf16(e[0], e[1])), "r"(pack_bf16(e[2], e[3])), "r"(pack_bf16(e[4], e[5])),
-                       "r"(pack_bf16(e[6], e[7])) : "memory");
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float e0, e1;
+            split2(fma2(f32x2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), sl2, use2), e0, e1);
+            e0 = fast_exp2(e0); e1 = fast_exp2(e1);         // hidden keys hold -inf: 0
+            lq[i & 3] = add2(lq[i & 3], f32x2(e0, e1));
+            pk[i] = pack_bf16(e0, e1);
+          }
         }
+        tmem_st16(s_addr + 16 * c, pk);
       }
+      tmem_st_wait();
+      if (!moves && !pv_before()) { ok = false; break; }
       tc_fence_before();
-      fence_proxy_async();                                // P is read by the tensor core's proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[g]);
-      l += ((lq[0] + lq[1]) + (lq[2] + lq[3])) + ((lq[4] + lq[5]) + (lq[6] + lq[7]));
+      float ls[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split2(lq[i], ls[2 * i], ls[2 * i + 1]);
+      l += ((ls[0] + ls[1]) + (ls[2] + ls[3])) + ((ls[4] + ls[5]) + (ls[6] + ls[7]));
     }
     if (ok && wait_on(&pv_full[g], (uint32_t)(n_mine - 1) & 1u, 25, n_mine)) {
       tc_fence_after();
