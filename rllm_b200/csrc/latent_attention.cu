@@ -427,14 +427,14 @@ latent_attention_few_kernel(const bf16* __restrict__ qfull, const bf16* __restri
                             const int* __restrict__ cu_q, const int* __restrict__ positions,
                             const int* __restrict__ block_table, int bt_stride, int num_seqs, int H, int rank, int dk,
                             int ld, int page_size, float scale, int window, int splits, float* __restrict__ pacc,
-                            float* __restrict__ pml) {
+                            float* __restrict__ pml, int skip_from) {
   pdl_launch();
   pdl_wait();
   int seq = -1, tile = 0;
   {
     int at = 0;
     for (int s = 0; s < num_seqs; ++s) {
-      const int n = ((cu_q[s + 1] - cu_q[s]) * H + FROWS - 1) / FROWS;
+      const int n = row_tiles(cu_q[s + 1] - cu_q[s], H, FROWS, skip_from);
       if ((int)blockIdx.x < at + n) { seq = s; tile = blockIdx.x - at; break; }
       at += n;
     }
@@ -710,10 +710,10 @@ RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache,
     if (rc) return rc;                                                                                                  \
     const int rl = launch_ex(latent_attention_few_kernel<NW>, dim3((unsigned)blocks, splits), dim3(256), (size_t)smem,  \
                              s, 1, (const bf16*)qfull, (const bf16*)cache, (bf16*)out, cu_q, positions, block_table,    \
-                             bt_stride, num_seqs, H, rank, dk, ld, page_size, scale, window, splits, pacc, pml);        \
+                             bt_stride, num_seqs, H, rank, dk, ld, page_size, scale, window, splits, pacc, pml, skip_from);        \
     if (rl || splits == 1) return rl;                                                                                   \
     return launch_ex(latent_merge_kernel, dim3((unsigned)blocks, (rank + 31) / 32), dim3(256), 0, s, 1,                 \
-                     (const float*)pacc, (const float*)pml, (bf16*)out, cu_q, num_seqs, H, rank, splits, FROWS, 0);        \
+                     (const float*)pacc, (const float*)pml, (bf16*)out, cu_q, num_seqs, H, rank, splits, FROWS, skip_from);        \
   } while (0)
         if (nw == 2) GO(2);
         if (nw == 4) GO(4);

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
   // counts one sequence's tiles, a warp scan finds the one that holds tile blockIdx.x (every warp for itself).
   int b = blockIdx.x, s = -1;
   if (FEW) {
-    if (b < p.num_seqs) { s = b; b = 0; }
+    if (b < p.num_seqs && !(p.skip_from > 0 && p.cu_q[b + 1] - p.cu_q[b] >= p.skip_from)) { s = b; b = 0; }
   } else {
     int base = 0;
     for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
@@ -387,7 +387,7 @@ RLLM_API int rllm_talk_attention_mma_supported(int dt, int nh, int kd, int vd, i
 
 // As rllm_talk_attention_simt, bfloat16 only. cu_q [num_seqs + 1]: the row range of each sequence (rows of a sequence
 // adjacent, positions ascending); skip_from > 0: the parts of sequences of at least so many rows are there already (any_short 0:
-// all of them); parts: float scratch [n_tokens, nh, nkv, vd]; out [n_tokens, nh * vd], contiguous.
+// all of them) and max_q_len is the longest of the others; parts: float scratch [n_tokens, nh, nkv, vd]; out [n_tokens, nh * vd], contiguous.
 RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const void* kcache, const void* vcache, void* out,
                                      float* parts, const int* positions, const int* cu_q, const int* block_table,
                                      int bt_stride, int num_seqs, int n_tokens, int max_q_len, int nh, int nkv, int kd, int vd,

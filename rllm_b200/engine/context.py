@@ -16,9 +16,13 @@ class GroupView:
     page_size: int
 
 
-# Rows of a portion from which a recurrence runs in chunks: three launches cost some 50 us at 64 rows (16 heads of 128 x 128,
-# delta rule) where row by row takes 31, 63 against 72 at 128 rows, 341 against 1,058 at 2,048
-LONG_FROM = 128
+# Steps whose longest portion has this many rows run their recurrences in chunks of 64, portions of CHUNK_FROM rows and more,
+# the shorter ones row by row beside them. Measured, row by row against chunks, us: 16 heads of 128 x 128, delta rule with
+# decays per channel 64 rows 35 / 56, 128 rows 68 / 59, 256 rows 128 / 83, 512 rows 253 / 96, portions of 281, 199 and 117 rows
+# 221 / 126 (199 with the last one row by row), 17 single tokens beside 256 rows 210 / 111; gated linear attention 57 / 50 at 128
+# rows, 109 / 57 at 256; state space with 32 heads 49 / 37 and 95 / 44. Four portions of 128 rows with 32 heads are level. Below 256
+# rows a step waits for its launches, of which chunks take three.
+LONG_FROM, CHUNK_FROM = 256, 64
 
 
 @dataclass
@@ -57,8 +61,8 @@ class StepContext:
         return self.max_q_len == 1
 
     def long_rows(self) -> dict:
-        """What a recurrence's scan is told about a step with long portions: from how many rows on a sequence runs in
-        chunks of 64 as products of matrices, and whether there are shorter ones beside it."""
+        """What a recurrence's scan is told about a step with a long portion: from how many rows on a sequence runs in
+        chunks as products of matrices, and whether there are shorter ones beside it."""
         if self.graph_safe or self.max_q_len < LONG_FROM:
             return {}
-        return {"long_from": LONG_FROM, "any_short": min(self.q_lens_host) < LONG_FROM}
+        return {"long_from": CHUNK_FROM, "any_short": min(self.q_lens_host) < CHUNK_FROM}

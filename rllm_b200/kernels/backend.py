@@ -16,8 +16,10 @@ import torch
 from . import ops
 
 
-# Rows of a portion from which attention over latents or with mixed heads runs in the tcgen05 kernel of prompt portions
-LATENT_LONG = TALK_LONG = 128
+# Rows that a step's longest portion has where attention over latents runs over expanded keys and values, and rows from which
+# a portion beside it does too; rows of a portion from which attention with mixed heads runs in the tcgen05 kernel
+LATENT_LONG, LATENT_FROM, TALK_LONG = 256, 32, 128
+TALK_PAIRS = 384 * 384       # pairs of query and key that mixed heads have at least there (`talk_attention` says why)
 
 
 class Normed:
@@ -49,11 +51,11 @@ class Backend:
             raise ops.KernelError("the engine runs on a CUDA device only (there is no CPU path)")
         self.fast = dtype == torch.bfloat16 and os.environ.get("RLLM_B200_GENERIC_ONLY") != "1"
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
-        self._sm100 = None
+        self._sm100 = self._err = None
         if self.fast:
             from . import sm100          # builds/loads the tcgen05 library, or raises
             self._sm100 = sm100
-            sm100.init(self.device)
+            self._err = sm100.init(self.device).err      # the device's error word
 
     # ---- element-wise / row-wise
     def embed(self, ids, table, err=None, scale=1.0):
@@ -408,15 +410,16 @@ class Backend:
         """Portions whose latent attention runs over expanded keys and values: (rows a portion has at least, their cached
         positions, whether there are shorter portions beside them), or None. A pair of query and key costs 0.26 ns less then
         (16 heads, measured: 590 us against 39 for 2,048 tokens) and a cached position 4.6 ns for its expansion, hence from 32
-        visible queries a key on it pays with a margin; the expansion may take 2 GB."""
+        visible queries a key on it pays with a margin; the expansion may take 2 GB. Steps whose longest portion has fewer
+        than 256 rows wait for their launches and stay as they are."""
         if not self.fast or ctx.graph_safe or ctx.max_q_len < LATENT_LONG or dim != 128 or vdim != 128 or rot not in (0, 64) \
                 or rank % 64 or scale <= 0 or os.environ.get("RLLM_B200_NO_TC_ATTENTION") == "1":
             return None
-        long = [(q, n) for q, n in zip(ctx.q_lens_host, ctx.kv_lens_host) if q >= LATENT_LONG]
+        long = [(q, n) for q, n in zip(ctx.q_lens_host, ctx.kv_lens_host) if q >= LATENT_FROM]
         rows = sum(n for _, n in long)
         if rows * heads * (dim + vdim) * 2 > 2 << 30 or 32 * rows > sum(q * min(n, window or n) for q, n in long):
             return None
-        return LATENT_LONG, rows, len(long) < ctx.num_seqs
+        return LATENT_FROM, rows, len(long) < ctx.num_seqs
 
     def latent_attention_expanded(self, q, qfull, cache, ctx, w_ukv, heads, dim, rot, rank, scale, window, long, out, gate, gate_cols):
         """The long portions' rows of `out` [T, heads * 128]: their sequences' cached rows, every head's keys and values from
@@ -435,7 +438,8 @@ class Backend:
         # sequence take the kernel shape with 16 rows a CTA. Everything this depends on is known when a decode
         # graph is captured (rows, sequences, the longest portion, the bound of the key count).
         T, H = qfull.shape[0], qfull.shape[1]
-        few = ctx.max_q_len <= 2 and rank % 128 == 0
+        longest = max((n for n in ctx.q_lens_host if n < skip_from), default=0) if skip_from else ctx.max_q_len
+        few = longest <= 2 and rank % 128 == 0
         rows = 16 if few else 64
         if skip_from:
             T = sum(q for q in ctx.q_lens_host if q < skip_from)
@@ -451,7 +455,7 @@ class Backend:
         return self._mix.gla_decay(z, bias, tau)
 
     def gla_scan(self, *a, **k):
-        return self._mix.gla_scan(*a, err=self._sm100.init(self.device).err if self.fast else None, **k)
+        return self._mix.gla_scan(*a, err=self._err, **k)
 
     def gla_finish(self, *a, **k):
         return self._mix.gla_finish(*a, **k)
@@ -560,7 +564,9 @@ class Backend:
 
     def state_scan(self, q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx, state, beta=None, vscale=None, skip=None):
         # the 32-bit run's results are the same bits however a sequence is cut into steps: row by row
-        long = dict(ctx.long_rows(), err=self._sm100.init(self.device).err) if self.fast else {}
+        long = ctx.long_rows() if self.fast else {}
+        if long:
+            long["err"] = self._err
         return self._hy.state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx.cu_q, ctx.num_seqs,
                                    ctx.state_slots, state, beta, vscale, skip, **long)
 
@@ -578,17 +584,21 @@ class Backend:
         kd, vd = cache.k.shape[3], cache.v.shape[3]
         if self.fast and os.environ.get("RLLM_B200_NO_TC_ATTENTION") != "1" \
                 and hy.talk_mma_supported(q.dtype, nh, kd, vd, cache.page_size):
+            # Every head over every kv head's values is ordinary attention: portions of 128 rows and more go to the tcgen05
+            # kernel of prompt portions where they have pairs enough to outweigh its start. Measured at 16 heads of 128 over
+            # 4 kv heads, mma.sync against tcgen05, us: 256 rows x 256 keys 25 / 37, 384 x 384 39 / 39, 512 x 512 55 / 38,
+            # 128 x 1,500 92 / 47, 2,048 x 2,048 515 / 127.
             page = cache.page_size
-            if not ctx.graph_safe and ctx.max_q_len >= TALK_LONG and kd == vd and page >= 8 and page & (page - 1) == 0 and scale > 0 \
+            pairs = 0 if ctx.graph_safe else sum(n * k for n, k in zip(ctx.q_lens_host, ctx.kv_lens_host) if n >= TALK_LONG)
+            if pairs >= TALK_PAIRS and kd == vd and page >= 8 and page & (page - 1) == 0 and scale > 0 \
                     and self._sm100.prefill_tc_supported(q, cache.k):
-                # every head over every kv head's values is ordinary attention: the tcgen05 kernel of prompt portions for
-                # the long ones (16 heads of 128 over 4 kv heads, 2,048 tokens: 515 us with mma.sync), the rest as ever
                 parts = torch.empty((q.shape[0], nh, cache.k.shape[1], vd), dtype=torch.float32, device=q.device)
                 self._sm100.attention_prefill_tc(q, cache.k, cache.v, ctx.cu_q, ctx.kv_lens, cache.block_table, ctx.max_q_len, nh,
                                                  scale, window, chunk=chunk, sinks=sinks, long_from=TALK_LONG, cross=parts)
+                short = max((n for n in ctx.q_lens_host if n < TALK_LONG), default=0)
                 return hy.talk_attention_mma(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, ctx.cu_q,
-                                             ctx.num_seqs, ctx.max_q_len, nh, scale, mix, window, chunk, sinks, parts=parts,
-                                             skip_from=TALK_LONG, any_short=min(ctx.q_lens_host) < TALK_LONG)
+                                             ctx.num_seqs, short, nh, scale, mix, window, chunk, sinks, parts=parts,
+                                             skip_from=TALK_LONG, any_short=short > 0)
             return hy.talk_attention_mma(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, ctx.cu_q,
                                          ctx.num_seqs, ctx.max_q_len, nh, scale, mix, window, chunk, sinks)
         return hy.talk_attention_simt(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, nh, scale,

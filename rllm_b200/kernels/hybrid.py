@@ -437,7 +437,8 @@ def talk_attention_mma(q, kcache, vcache, token_seq, positions, block_table, cu_
     values: a first kernel leaves, as floats, every head's weights summed over every kv head's values ([T, nh, nkv,
     vd], one pass with a running softmax), a second one adds them by `mix` and rounds once. `cu_q` int32
     [num_seqs + 1]: each sequence's rows; `max_q_len`: the longest portion of the step. `parts`, `skip_from`: what the first
-    kernel leaves is there already for sequences of at least so many rows; `any_short`: there are others."""
+    kernel leaves is there already for sequences of at least so many rows; `any_short`: there are others, and `max_q_len` is the
+    longest of them."""
     _cuda(q, "q")
     T = q.shape[0]
     nkv = kcache.shape[1]
