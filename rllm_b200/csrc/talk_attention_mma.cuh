@@ -69,6 +69,8 @@ struct Args {
   const float* sinks;
   int page_shift;              // log2(page_size), or -1 when it is no power of two
   int skip_from;               // > 0: sequences of at least so many rows are another kernel's (attn_prefill_tc.cu, `cross`)
+  int splits, n_tokens;        // FEW: ranges that a sequence's keys are cut into, a CTA each; > 1: parts are not normalised,
+  float* ml;                   // [split][token][head][..], and (maximum, sum) per [split][token][head] go here
 };
 
 __device__ __forceinline__ int first_key(int pos, int window, int chunk) {
@@ -79,7 +81,9 @@ __device__ __forceinline__ int first_key(int pos, int window, int chunk) {
 
 // FEW: the step's sequences bring at most 16 rows each (single tokens with up to 16 heads a kv head). The four warps
 // then all hold the tile's 16 rows and split each tile's 64 keys between them (16 keys a warp), each with a running
-// softmax of its own; the four are joined in warp order through shared memory at the end.
+// softmax of its own; the four are joined in warp order through shared memory at the end. A CTA walks its keys at
+// some 1.7 us a tile whatever else runs, so few sequences are cut into ranges of keys (8 sequences of 1,100 keys, 16 heads of
+// 128 over 4 kv heads: 30 us as one range each), which talk_mix_kernel joins in their order.
 template <int DP, bool FEW>
 __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args p) {
   pdl_launch();
@@ -95,7 +99,8 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
   // counts one sequence's tiles, a warp scan finds the one that holds tile blockIdx.x (every warp for itself).
   int b = blockIdx.x, s = -1;
   if (FEW) {
-    if (b < p.num_seqs && !(p.skip_from > 0 && p.cu_q[b + 1] - p.cu_q[b] >= p.skip_from)) { s = b; b = 0; }
+    const int sq = b / p.splits;
+    if (sq < p.num_seqs && !(p.skip_from > 0 && p.cu_q[sq + 1] - p.cu_q[sq] >= p.skip_from)) { s = sq; b = 0; }
   } else {
     int base = 0;
     for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
@@ -124,7 +129,13 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
   const int tok_lo = row_base / Gq, tok_hi = min(ql - 1, (row_base + ROWS - 1) / Gq);
   const int pos_lo = p.positions[q0 + tok_lo], pos_hi = p.positions[q0 + tok_hi];
   const int key_lo = first_key(pos_lo, p.window, p.chunk);
-  const int tile0 = key_lo / KEYS, tile1 = pos_hi / KEYS + 1;     // key tiles [tile0, tile1)
+  int tile0 = key_lo / KEYS, tile1 = pos_hi / KEYS + 1;           // key tiles [tile0, tile1)
+  const int split = FEW ? blockIdx.x % p.splits : 0;
+  if (FEW && p.splits > 1) {
+    const int per = (tile1 - tile0 + p.splits - 1) / p.splits;
+    tile0 += split * per;                                         // an empty range leaves a maximum of -inf
+    tile1 = min(tile1, tile0 + per);
+  }
   const int* bt = p.block_table + (size_t)s * p.bt_stride;
 
   // zero the tiles once where a head is narrower than DP: the columns beyond kd / vd are never copied into
@@ -181,7 +192,7 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
   float o[DP / 8][4];
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  const bool with_sink = p.sinks && (!FEW || warp == 0);
+  const bool with_sink = p.sinks && (!FEW || (warp == 0 && split == 0));
   float m0 = (with_sink && v0) ? p.sinks[h0] * 1.4426950408889634f : -INFINITY, l0 = (with_sink && v0) ? 1.f : 0.f;
   float m1 = (with_sink && v1) ? p.sinks[h1] * 1.4426950408889634f : -INFINITY, l1 = (with_sink && v1) ? 1.f : 0.f;
 
@@ -316,8 +327,10 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
         const float2 ov = *reinterpret_cast<const float2*>(po + (w * 16 + r) * DP + c);
         a0 = fmaf(ov.x, f, a0); a1 = fmaf(ov.y, f, a1);
       }
-      const float f = L > 0.f ? 1.f / L : 0.f;
-      *reinterpret_cast<float2*>(p.parts + (((size_t)t * p.nh + h) * p.nkv + cv) * p.vd + c) = make_float2(a0 * f, a1 * f);
+      const float f = p.splits > 1 ? 1.f : L > 0.f ? 1.f / L : 0.f;
+      const size_t row_of = (size_t)split * p.n_tokens + t;
+      *reinterpret_cast<float2*>(p.parts + ((row_of * p.nh + h) * p.nkv + cv) * p.vd + c) = make_float2(a0 * f, a1 * f);
+      if (p.splits > 1 && cv == 0 && c == 0) *reinterpret_cast<float2*>(p.ml + (row_of * p.nh + h) * 2) = make_float2(M, L);
     }
     return;
   }
@@ -343,13 +356,27 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
 // bytes (2,048 tokens x 16 heads x 512: 29 us with a column a thread).
 constexpr int HB = 4;
 __global__ void __launch_bounds__(128) talk_mix_kernel(const float* __restrict__ parts, const float* __restrict__ mix,
-                                                       bf16* __restrict__ out, int nh, int nkv, int vd) {
+                                                       bf16* __restrict__ out, int nh, int nkv, int vd, int splits, int n_tokens,
+                                                       const float* __restrict__ ml) {
   pdl_launch();
   pdl_wait();
-  extern __shared__ float msm[];                    // [nh][nh]
+  extern __shared__ float msm[];                    // [nh][nh], with ranges of keys their factors [splits][nh] behind
   for (int i = threadIdx.x; i < nh * nh; i += blockDim.x) msm[i] = mix[i];
-  __syncthreads();
   const int t = blockIdx.x, rep = nh / nkv;
+  float* fac = msm + nh * nh;
+  if (splits > 1)
+    for (int g = threadIdx.x; g < nh; g += blockDim.x) {
+      float M = -INFINITY, L = 0.f;
+      for (int s = 0; s < splits; ++s) M = fmaxf(M, ml[(((size_t)s * n_tokens + t) * nh + g) * 2]);
+      for (int s = 0; s < splits; ++s) {
+        const float2 x = *reinterpret_cast<const float2*>(ml + (((size_t)s * n_tokens + t) * nh + g) * 2);
+        const float f = x.x == -INFINITY ? 0.f : fast_exp2(x.x - M);
+        fac[s * nh + g] = f;
+        L = fmaf(x.y, f, L);
+      }
+      for (int s = 0; s < splits; ++s) fac[s * nh + g] *= L > 0.f ? 1.f / L : 0.f;
+    }
+  __syncthreads();
   const float* A = parts + (size_t)t * nh * nkv * vd;
   bf16* o = out + (size_t)t * nh * vd;
   for (int x = threadIdx.x; x < nkv * vd / 4; x += blockDim.x) {
@@ -360,7 +387,16 @@ __global__ void __launch_bounds__(128) talk_mix_kernel(const float* __restrict__
       for (int i = 0; i < HB; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
       for (int g = 0; g < nh; ++g) {
-        const float4 a = *reinterpret_cast<const float4*>(A + ((size_t)g * nkv + c) * vd + d);
+        float4 a = *reinterpret_cast<const float4*>(A + ((size_t)g * nkv + c) * vd + d);
+        if (splits > 1) {
+          const float f0 = fac[g];
+          a = make_float4(a.x * f0, a.y * f0, a.z * f0, a.w * f0);
+          for (int s = 1; s < splits; ++s) {
+            const float f = fac[s * nh + g];
+            const float4 x = *reinterpret_cast<const float4*>(A + (((size_t)s * n_tokens * nh + g) * nkv + c) * vd + d);
+            a.x = fmaf(x.x, f, a.x); a.y = fmaf(x.y, f, a.y); a.z = fmaf(x.z, f, a.z); a.w = fmaf(x.w, f, a.w);
+          }
+        }
 #pragma unroll
         for (int i = 0; i < HB; ++i)
           if (h0 + i < rep) {
@@ -387,12 +423,13 @@ RLLM_API int rllm_talk_attention_mma_supported(int dt, int nh, int kd, int vd, i
 
 // As rllm_talk_attention_simt, bfloat16 only. cu_q [num_seqs + 1]: the row range of each sequence (rows of a sequence
 // adjacent, positions ascending); skip_from > 0: the parts of sequences of at least so many rows are there already (any_short 0:
-// all of them) and max_q_len is the longest of the others; parts: float scratch [n_tokens, nh, nkv, vd]; out [n_tokens, nh * vd], contiguous.
+// all of them) and max_q_len is the longest of the others; splits > 1 (steps of at most 16 rows a sequence and kv head): ranges of
+// keys, ml: float scratch [splits, n_tokens, nh, 2] and parts splits times as large; parts: float scratch [n_tokens, nh, nkv, vd]; out [n_tokens, nh * vd], contiguous.
 RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const void* kcache, const void* vcache, void* out,
                                      float* parts, const int* positions, const int* cu_q, const int* block_table,
                                      int bt_stride, int num_seqs, int n_tokens, int max_q_len, int nh, int nkv, int kd, int vd,
                                      int page_size, float scale, int window, int chunk, const float* mix, const float* sinks,
-                                     int skip_from, int any_short, void* stream) {
+                                     int skip_from, int any_short, int splits, float* ml, void* stream) {
   using namespace talkmma;
   if (n_tokens <= 0 || num_seqs <= 0) return 0;
   if (!rllm_talk_attention_mma_supported(DT_BF16, nh, kd, vd, page_size) || nkv <= 0 || nh % nkv) return ERR_BAD_SIZE;
@@ -401,13 +438,17 @@ RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const vo
   const long long tiles = ((long long)n_tokens * Gq + ROWS - 1) / ROWS + num_seqs;
   if (tiles > 2147483647LL || nkv > 65535) return ERR_TOO_LARGE;
   Args a = {(const bf16*)q, q_stride, (const bf16*)kcache, (const bf16*)vcache, parts, positions, cu_q, block_table,
-            bt_stride, num_seqs, nh, nkv, kd, vd, page_size, scale * 1.4426950408889634f, window, chunk, sinks, -1, skip_from};
+            bt_stride, num_seqs, nh, nkv, kd, vd, page_size, scale * 1.4426950408889634f, window, chunk, sinks, -1, skip_from, 1, n_tokens, ml};
   for (int sft = 0; sft < 31; ++sft) if ((1 << sft) == page_size) a.page_shift = sft;
   cudaStream_t s = (cudaStream_t)stream;
-  const dim3 grid((unsigned)tiles, (unsigned)nkv, (unsigned)nkv);
   const int dp = (kd <= 64 && vd <= 64) ? 64 : 128;
   const int smem = 2 * STAGES * KEYS * (dp + 8) * (int)sizeof(bf16);     // also holds the FEW join: 4 x 16 x (dp + 2) floats
   const bool few = (long long)max_q_len * Gq <= 16;             // every sequence's rows fit one warp's 16
+  if (splits > 1) {
+    if (!few || !ml || skip_from > 0 || splits > 64) return ERR_BAD_SIZE;
+    a.splits = splits;
+  }
+  const dim3 grid((unsigned)(few ? (long long)num_seqs * a.splits : tiles), (unsigned)nkv, (unsigned)nkv);
   int rc = 0;
 #define GO(D, F)                                                                                     \
   {                                                                                                  \
@@ -420,6 +461,6 @@ RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const vo
   else { if (few) GO(128, true) else GO(128, false) }
 #undef GO
   if (rc) return rc;
-  return launch_ex(talk_mix_kernel, dim3((unsigned)n_tokens), dim3(128), sizeof(float) * nh * nh, s, 1, (const float*)parts,
-                   mix, (bf16*)out, nh, nkv, vd);
+  return launch_ex(talk_mix_kernel, dim3((unsigned)n_tokens), dim3(128), sizeof(float) * (nh * nh + (a.splits > 1 ? a.splits * nh : 0)), s, 1,
+                   (const float*)parts, mix, (bf16*)out, nh, nkv, vd, a.splits, n_tokens, (const float*)ml);
 }

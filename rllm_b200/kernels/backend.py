@@ -599,8 +599,13 @@ class Backend:
                 return hy.talk_attention_mma(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, ctx.cu_q,
                                              ctx.num_seqs, short, nh, scale, mix, window, chunk, sinks, parts=parts,
                                              skip_from=TALK_LONG, any_short=short > 0)
+            splits, nkv = 1, cache.k.shape[1]
+            if ctx.max_q_len * (nh // nkv) <= 16:
+                # a step of single tokens: ranges of at least four tiles of 64 keys while there are places (three CTAs an SM)
+                keys = min(ctx.max_kv_len, window or ctx.max_kv_len, chunk or ctx.max_kv_len)
+                splits = max(1, min(8, 3 * self.sm_count // (ctx.num_seqs * nkv * nkv), keys // 256))
             return hy.talk_attention_mma(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, ctx.cu_q,
-                                         ctx.num_seqs, ctx.max_q_len, nh, scale, mix, window, chunk, sinks)
+                                         ctx.num_seqs, ctx.max_q_len, nh, scale, mix, window, chunk, sinks, splits=splits)
         return hy.talk_attention_simt(q, cache.k, cache.v, ctx.token_seq, ctx.positions, cache.block_table, nh, scale,
                                             mix, window, chunk, sinks)
 

@@ -42,7 +42,7 @@ ops.register_signatures("hybrid", {
     "rllm_mingru_scan": [_P, _LL, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P,
                          _P, _P],
     "rllm_talk_attention_mma": [_P, _LL, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                c_int, c_float, c_int, c_int, _P, _P, c_int, c_int, _P],
+                                c_int, c_float, c_int, c_int, _P, _P, c_int, c_int, c_int, _P, _P],
 })
 
 GLU_ACTS = {"silu": 0, "gelu_tanh": 1, "swish_clamped": 2}
@@ -432,13 +432,14 @@ def _dt_of(dtype) -> int:
 
 
 def talk_attention_mma(q, kcache, vcache, token_seq, positions, block_table, cu_q, num_seqs, max_q_len, nh, scale, mix,
-                       window=None, chunk=None, sinks=None, parts=None, skip_from: int = 0, any_short: bool = True) -> torch.Tensor:
+                       window=None, chunk=None, sinks=None, parts=None, skip_from: int = 0, any_short: bool = True,
+                       splits: int = 1) -> torch.Tensor:
     """The same attention in bfloat16 on the tensor cores (`mma.sync`, float softmax). The mix is applied after the
     values: a first kernel leaves, as floats, every head's weights summed over every kv head's values ([T, nh, nkv,
     vd], one pass with a running softmax), a second one adds them by `mix` and rounds once. `cu_q` int32
     [num_seqs + 1]: each sequence's rows; `max_q_len`: the longest portion of the step. `parts`, `skip_from`: what the first
     kernel leaves is there already for sequences of at least so many rows; `any_short`: there are others, and `max_q_len` is the
-    longest of them."""
+    longest of them. `splits` > 1 (at most 16 rows a sequence and kv head): ranges that a sequence's keys are cut into."""
     _cuda(q, "q")
     T = q.shape[0]
     nkv = kcache.shape[1]
@@ -456,13 +457,18 @@ def talk_attention_mma(q, kcache, vcache, token_seq, positions, block_table, cu_
     _f32(mix, "head mix", (nh, nh))
     if sinks is not None:
         _f32(sinks, "sinks", (nh,))
-    if parts is None:
+    ml = None
+    if splits > 1:
+        parts = torch.empty((splits, T, nh, nkv, vd), dtype=torch.float32, device=q.device)
+        ml = torch.empty((splits, T, nh, 2), dtype=torch.float32, device=q.device)
+    elif parts is None:
         parts = torch.empty((T, nh, nkv, vd), dtype=torch.float32, device=q.device)
-    _f32(parts, "parts", (T, nh, nkv, vd))
+    else:
+        _f32(parts, "parts", (T, nh, nkv, vd))
     out = torch.empty((T, nh * vd), dtype=q.dtype, device=q.device)
     _check(_fn("hybrid", "rllm_talk_attention_mma")(
         q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), out.data_ptr(), parts.data_ptr(), positions.data_ptr(),
         cu_q.data_ptr(), block_table.data_ptr(), block_table.stride(0), int(num_seqs), T, int(max_q_len), nh, nkv, kd, vd,
         page_size, float(scale), int(window or 0), int(chunk or 0), mix.data_ptr(), _ptr(sinks), int(skip_from), int(any_short),
-        _stream()), "talk_attention_mma", 2 if any_short else 1)
+        int(splits), _ptr(ml), _stream()), "talk_attention_mma", 2 if any_short else 1)
     return out

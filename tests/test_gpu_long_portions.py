@@ -145,3 +145,19 @@ def test_latents_beside_long_portions(lens, splits):
         sc = torch.einsum("ihd,jd->hij", qfull[mine].double(), c) * scale
         p = torch.softmax(sc.masked_fill(~visible(r, n, None), float("-inf")), -1)
         assert rel(got[mine], torch.einsum("hij,jd->ihd", p, c[:, :rank])) < 8e-3
+
+
+@pytest.mark.parametrize("splits", [2, 3, 8])
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 8, 2), (48, 3, 1)])
+@pytest.mark.parametrize("window", [None, 70])
+def test_mixed_heads_of_single_tokens_over_ranges_of_keys(splits, hd, nh, nkv, window):
+    """Sequences shorter than a range, ranges that the window empties, one that ends at a tile's edge."""
+    from rllm_b200.kernels import hybrid
+    lens = [(1, 1), (1, 64), (2, 130), (1, 700)]
+    cu, cud, _, seq, pos, table, pages = batch(lens, 16, hd, 1)
+    q = rnd(cu[-1], nh * hd, seed=3).bfloat16()
+    kc, vc = rnd(pages, nkv, 16, hd, seed=4).bfloat16(), rnd(pages, nkv, 16, hd, seed=5).bfloat16()
+    args = (q, kc, vc, seq, pos, table, cud, len(lens), 2, nh, hd ** -0.5, rnd(nh, nh, seed=6), window, None, rnd(nh, seed=7))
+    one, got = hybrid.talk_attention_mma(*args), hybrid.talk_attention_mma(*args, splits=splits)
+    # the weights of a range are rounded to bfloat16 against its own maximum: 2^-9 each, as the one range's are
+    assert rel(got, one.double()) < 6e-3
