@@ -421,13 +421,20 @@ class Backend:
             return None
         return LATENT_FROM, rows, len(long) < ctx.num_seqs
 
-    def latent_attention_expanded(self, q, qfull, cache, ctx, w_ukv, heads, dim, rot, rank, scale, window, long, out, gate, gate_cols):
-        """The long portions' rows of `out` [T, heads * 128]: their sequences' cached rows, every head's keys and values from
-        them (`w_ukv`: W_uk over W_uv), attention, the gate."""
+    def latent_expand(self, cache, ctx, w_ukv, rank, long):
+        """The cached rows of the long portions' sequences, and every head's keys and values from them (`w_ukv`: W_uk over
+        W_uv); None where the memory left does not hold them."""
         long_from, rows, _ = long
-        c = self._mix.latent_gather(cache.tensors["kv"], cache.block_table, ctx.cu_q, ctx.kv_lens, ctx.num_seqs, long_from, rows,
-                                    ctx.max_kv_len)
-        kv = self.linear(c[:, :rank], w_ukv)
+        try:
+            c = self._mix.latent_gather(cache.tensors["kv"], cache.block_table, ctx.cu_q, ctx.kv_lens, ctx.num_seqs, long_from,
+                                        rows, ctx.max_kv_len)
+            return c, self.linear(c[:, :rank], w_ukv)
+        except torch.OutOfMemoryError:
+            return None
+
+    def latent_attention_expanded(self, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, out, gate, gate_cols):
+        """The long portions' rows of `out` [T, heads * 128]: attention over the expanded keys and values, the gate."""
+        (c, kv), long_from = expanded, long[0]
         return self._sm100.attention_prefill_dense(
             q, dim + rot, qfull[:, :, rank:] if rot else None, kv, 0, heads * dim, c[:, rank:] if rot else None, ctx.cu_q,
             ctx.kv_lens, ctx.max_q_len, heads, scale, window, out, long_from, gate, gate_cols)

@@ -11,7 +11,7 @@ from ctypes import c_float, c_int, c_longlong
 import torch
 
 from . import ops
-from .ops import KernelError, _check, _cuda, _dt, _fn, _ptr, _stream
+from .ops import KernelError, _check, _cuda, _dt, _fn, _ptr, _scratch, _stream
 
 _P, _LL = ops._P, c_longlong
 
@@ -332,7 +332,7 @@ def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seq
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
     scratch = None
     if long_from > 0 and err is not None and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
-        scratch = torch.empty((T // 64 + num_seqs) * heads * per, dtype=torch.float32, device=q.device)
+        scratch = _scratch((T // 64 + num_seqs) * heads * per, q.device)
     _check(_fn("recurrent", "rllm_state_scan")(
         _dt(beta, "beta") if beta is not None else 0, q.data_ptr(), q.stride(0), int(q_heads), k.data_ptr(), k.stride(0),
         int(k_heads), v.data_ptr(), v.stride(0), decay.data_ptr(), int(per_channel), _ptr(beta),

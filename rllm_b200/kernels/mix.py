@@ -13,7 +13,7 @@ from ctypes import c_float, c_int, c_longlong
 import torch
 
 from . import ops
-from .ops import KernelError, _check, _cuda, _dt, _fn, _ptr, _stream
+from .ops import KernelError, _check, _cuda, _dt, _fn, _ptr, _scratch, _stream
 
 _P, _LL = ops._P, c_longlong
 GEPI_STORE, GEPI_STORE_F32, GEPI_RELU2, GEPI_SILU_GATED = 0, 1, 2, 3
@@ -405,8 +405,8 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torc
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=proj.device)
     cs = cd = scratch = None
     if long_from > 0 and err is not None and proj.dtype == torch.bfloat16 and (per := _fn("mix", "rllm_gla_chunk_floats")(int(dim), int(vdim))):
-        scratch = torch.empty((T // 64 + num_seqs) * heads * per, dtype=torch.float32, device=proj.device)
-    elif chunk > 0:
+        scratch = _scratch((T // 64 + num_seqs) * heads * per, proj.device)
+    if chunk > 0 and scratch is None:
         n = T // chunk + num_seqs
         cs = torch.empty((n, heads, dim, vdim), dtype=torch.float32, device=proj.device)
         cd = torch.empty((n, heads, dim), dtype=torch.float32, device=proj.device)

@@ -109,6 +109,14 @@ def _dt(t: torch.Tensor, name: str) -> int:
         raise KernelError(f"{name}: dtype {t.dtype} is not supported (float32 or bfloat16)") from None
 
 
+def _scratch(n: int, device) -> torch.Tensor | None:
+    """Float scratch of a faster form of a kernel, or None where the memory left does not hold it: the other form runs then."""
+    try:
+        return torch.empty(n, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 

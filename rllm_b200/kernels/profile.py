@@ -238,11 +238,11 @@ class OpProfile:
     def latent_prepare(self, proj, *a, **k):
         return self._timed("latent_prepare", 2 * _nbytes(proj), 0, self._be.latent_prepare, proj, *a, **k)
 
-    def latent_attention_expanded(self, q, qfull, cache, ctx, w_ukv, heads, dim, rot, rank, scale, window, long, *a):
+    def latent_attention_expanded(self, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, *a):
         lens = [(n, L) for n, L in zip(ctx.q_lens_host, ctx.kv_lens_host) if n >= long[0]]
         pairs = sum(n * ((min(L, window + n - 1) if window else L) - n) + n * (n + 1) // 2 for n, L in lens)
         return self._timed("latent_attention", long[1] * (rank + rot) * 2 + _nbytes(q), 2 * heads * (dim + rot + 128) * pairs,
-                           self._be.latent_attention_expanded, q, qfull, cache, ctx, w_ukv, heads, dim, rot, rank, scale, window, long, *a)
+                           self._be.latent_attention_expanded, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, *a)
 
     def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0):
         T, H, dk = qfull.shape

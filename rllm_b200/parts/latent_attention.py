@@ -112,13 +112,16 @@ class LatentAttention(Part):
         gate, gate_cols = proj[:, q_cols + dk:] if self.gate else None, self.gate == "full"
         # long portions over expanded keys and values, the others (decoded tokens beside them) over the latents themselves
         long = be.latent_expanded(ctx, H, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.window, self.scale)
+        expanded = None
+        if long is not None and (expanded := be.latent_expand(cache, ctx, self._ukv, self.kv_rank, long)) is None:
+            long = None                                              # no memory for the expansion
         if long is None or long[2]:
             be.linear_heads(q, self.dim + self.rot_dim, self._uk_t, qfull.view(T, H * dk), dk)
             o = be.latent_attention(qfull, cache, ctx, self.kv_rank, self.scale, self.window, skip_from=long[0] if long else 0)
             be.linear_heads(o.view(T, H * self.kv_rank), self.kv_rank, self._uv, att, self.vdim, gate=gate, gate_cols=gate_cols)
         if long is not None:
-            be.latent_attention_expanded(q, qfull, cache, ctx, self._ukv, H, self.dim, self.rot_dim, self.kv_rank, self.scale,
-                                         self.window, long, att, gate, gate_cols)
+            be.latent_attention_expanded(q, qfull, expanded, ctx, H, self.dim, self.rot_dim, self.kv_rank, self.scale, self.window,
+                                         long, att, gate, gate_cols)
         if residual is None:
             return be.linear_f32(att, self.w_o, tag="o")
         be.linear_residual(att, self.w_o, residual)
