@@ -406,14 +406,16 @@ class Backend:
     def latent_prepare(self, *a, **k):
         return self._mix.latent_prepare(*a, **k)
 
-    def latent_expanded(self, ctx, heads, dim, rot, vdim, rank, window, scale):
+    def latent_expanded(self, ctx, q, gate, gate_cols, heads, dim, rot, vdim, rank, window, scale):
         """Portions whose latent attention runs over expanded keys and values: (rows a portion has at least, their cached
         positions, whether there are shorter portions beside them), or None. A pair of query and key costs 0.26 ns less then
         (16 heads, measured: 590 us against 39 for 2,048 tokens) and a cached position 4.6 ns for its expansion, hence from 32
         visible queries a key on it pays with a margin; the expansion may take 2 GB. Steps whose longest portion has fewer
-        than 256 rows wait for their launches and stay as they are."""
+        than 256 rows wait for their launches and stay as they are, and so do queries and gates whose rows the attention
+        kernel cannot copy in pieces of 16 bytes."""
         if not self.fast or ctx.graph_safe or ctx.max_q_len < LATENT_LONG or dim != 128 or vdim != 128 or rot not in (0, 64) \
-                or rank % 64 or scale <= 0 or os.environ.get("RLLM_B200_NO_TC_ATTENTION") == "1":
+                or rank % 64 or scale <= 0 or not self._sm100.prefill_dense_supported(q, gate, gate_cols) \
+                or os.environ.get("RLLM_B200_NO_TC_ATTENTION") == "1":
             return None
         long = [(q, n) for q, n in zip(ctx.q_lens_host, ctx.kv_lens_host) if q >= LATENT_FROM]
         rows = sum(n for _, n in long)

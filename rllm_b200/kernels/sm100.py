@@ -418,6 +418,13 @@ def attention_prefill_tc(q, kcache, vcache, cu_q, kv_lens, block_table, max_q_le
     return out if cross is None else cross
 
 
+def prefill_dense_supported(q, gate=None, gate_cols=False) -> bool:
+    """Do the rows of the queries, and of a gate per output, start where copies of 16 bytes may? (A projection's rows are as
+    wide as its parts together: 12 heads of 128 + 64 with a latent of 512 + 64 and a gate a head are 2,892 numbers.)"""
+    rows = (q,) if gate is None or not gate_cols else (q, gate)
+    return all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in rows)
+
+
 def attention_prefill_dense(q, q_head, q2, kv, k_off, v_off, r, cu_q, kv_lens, max_q_len, nh, scale, window, out, long_from,
                             gate=None, gate_cols=False):
     """Prefill attention with a key and a value per query head that lie in rows instead of pages: kv bf16 [rows, ...], head h's

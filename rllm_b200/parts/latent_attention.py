@@ -111,7 +111,7 @@ class LatentAttention(Part):
         att = torch.empty((T, H * self.vdim), dtype=proj.dtype, device=proj.device)
         gate, gate_cols = proj[:, q_cols + dk:] if self.gate else None, self.gate == "full"
         # long portions over expanded keys and values, the others (decoded tokens beside them) over the latents themselves
-        long = be.latent_expanded(ctx, H, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.window, self.scale)
+        long = be.latent_expanded(ctx, q, gate, gate_cols, H, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.window, self.scale)
         expanded = None
         if long is not None and (expanded := be.latent_expand(cache, ctx, self._ukv, self.kv_rank, long)) is None:
             long = None                                              # no memory for the expansion

@@ -1,0 +1,74 @@
+"""Attention over latents as a part, with heads of 128 and prompt portions long enough for expanded keys and values: whole,
+behind a cached context, beside single tokens and short portions, against the plain implementations; with row widths that
+the expanded form's copies cannot start on, and beside a request whose numbers are not finite."""
+import pytest
+import torch
+
+import plain_zufotar as PF
+import plain_zukotar as PK
+import zufotar_tiny as ZF
+import zukotar_tiny as ZK
+from test_gpu_zufotar import lat_weights
+from test_gpu_zukotar import DEV, DT, Harness, as_stored, bind, latent_weights, rel, rnd
+
+pytestmark = pytest.mark.gpu
+W, EPS, ROWS = 64, 1e-6, 300
+
+
+def built(heads, rot, rank, window=None, q_rank=None):
+    """(part, weights, plain implementation) of a layer with a gate a head, or (q_rank) a query latent and a gate an output."""
+    from rllm_b200.parts import InterleavedRotary, LatentAttention
+    scale = (128 + rot) ** -0.5
+    position = InterleavedRotary(rot, 10000.0, rot) if rot else None
+    if q_rank is None:
+        m = ZK.latent(heads, 128, rot, 128, rank, scale, 10000.0, rot, window)
+        w = latent_weights(W, m, seed=3)
+        plain = lambda x, st: PK.latent_attention(x, st, "x.", m, EPS)
+    else:
+        m = ZF.lat(heads, 128, rot, 128, q_rank, rank, scale, None, (10000.0, rot, None) if rot else None)["mixer"]
+        w = lat_weights(W, m, seed=3)
+        plain = lambda x, st: PF.latent_attention(x, st, "x.", m, EPS)
+    part = LatentAttention(W, heads, 128, rot, 128, rank, scale, position, window=window, eps=EPS,
+                           gate="head" if q_rank is None else "full", q_rank=q_rank)
+    # keys, queries and values of some size: weights a tenth of the tiny models'
+    w = {k: v if k.endswith("norm") else v * 0.4 for k, v in w.items()}
+    return part, w, plain
+
+
+def steps(part, w, plan, src, spoil=None):
+    """Run `plan` (a list of steps {request: rows}) in bfloat16; -> each request's outputs, steps that ran expanded, backend."""
+    bind(part, w, "bfloat16", "x.")
+    hs = Harness("bfloat16", [part.cache_spec()], page_size=16, pages=160, slots=len(src))
+    real, expanded = hs.backend.latent_attention_expanded, []
+    hs.backend.latent_attention_expanded = lambda *a, **k: (expanded.append(True), real(*a, **k))[1]
+    at, got = {k: 0 for k in src}, {k: [] for k in src}
+    for st in plan:
+        rows = torch.cat([src[k][at[k]: at[k] + n] for k, n in st.items()])
+        y = hs.run(list(st.items()), lambda ctx, cache: part.forward(rows, ctx, cache))
+        o = 0
+        for k, n in st.items():
+            got[k].append(y[o: o + n]); o += n; at[k] += n
+        hs.engine.check()
+    return {k: torch.cat(v) for k, v in got.items()}, len(expanded), hs
+
+
+PLAN = [{"a": ROWS}, {"b": 40, "a": 1, "c": ROWS}, {"a": 2, "b": ROWS, "c": 1}, {"a": 1, "b": 1, "c": 1}]
+
+
+@pytest.mark.parametrize("heads,rot,rank,window,q_rank,fits", [
+    (8, 64, 64, None, None, True),       # 8 * 192 + 64 + 64 + 8 columns: rows start on 16 bytes
+    (12, 64, 64, None, None, False),     # ... + 12 columns: they do not
+    (8, 64, 128, 70, None, True),
+    (3, 64, 128, None, None, False),
+    (3, 64, 64, None, 104, True),
+    (3, 64, 64, None, 100, False),       # the gate begins at column 100 + 64 + 64
+    (2, 0, 64, None, 48, True),
+])
+def test_long_portions_beside_others(heads, rot, rank, window, q_rank, fits):
+    part, w, plain = built(heads, rot, rank, window, q_rank)
+    src = {k: rnd(sum(st.get(k, 0) for st in PLAN), W, seed=i).bfloat16() for i, k in enumerate("abc")}
+    got, expanded, _ = steps(part, w, PLAN, {k: x.to(DEV) for k, x in src.items()})
+    assert expanded == (3 if fits else 0)
+    for k, x in src.items():
+        # projections, latents, weights and outputs rounded to bfloat16, as the part's other bfloat16 tests have it
+        assert rel(got[k], plain(x.double(), as_stored(w, "bfloat16"))) < 4e-2, k
