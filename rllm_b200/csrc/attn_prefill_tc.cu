@@ -586,6 +586,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
             const int j = j0 + 32 * c + i;
             if (!(valid && j <= pos && (j >= lo || j < kf))) v[c][i] = 0xff800000u;
           }
+        // The copies of the last tile brought rows beyond the sequence: another request's, or what a page's last holder left.
+        // Their weights are zero, but zero times an infinity is not: those rows of V become zeros before the product reads them
+        // (both row tiles' threads may write the same zeros; V landed with K, whose product is done). Every row has hidden keys in
+        // such a tile; in front of `p_full` instead, or by a loader's warp, 8,192 tokens cost 1 to 4 % more.
+        if (TMA && j0 + PN > kv_len) {
+          if (r < PN && j0 + r >= kv_len) {
+            const uint32_t vrow = v_s + (uint32_t)(t % NST * C::V_BYTES + r * 128);
+#pragma unroll 1
+            for (int i = 0; i < C::VA * 8; ++i)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(vrow + (uint32_t)((i >> 3) * C::ATOM_KEYS + (i & 7) * 16)), "r"(0) : "memory");
+          }
+          fence_proxy_async();
+        }
       }
       float mq[NC];                                       // chains side by side, not one of 64 links
 #pragma unroll

@@ -72,3 +72,17 @@ def test_long_portions_beside_others(heads, rot, rank, window, q_rank, fits):
     for k, x in src.items():
         # projections, latents, weights and outputs rounded to bfloat16, as the part's other bfloat16 tests have it
         assert rel(got[k], plain(x.double(), as_stored(w, "bfloat16"))) < 4e-2, k
+
+
+@pytest.mark.parametrize("order", ["ab", "ba"])
+@pytest.mark.parametrize("rot", [0, 64])
+def test_a_request_beside_one_that_is_not_finite(order, rot):
+    """Sequences lie one after the other in the expanded rows: a tile's rows beyond its own sequence are the next one's."""
+    part, w, _ = built(8, rot, 64)
+    src = {k: rnd(ROWS, W, seed=i).bfloat16().to(DEV) for i, k in enumerate("ab")}
+    plan = [{k: ROWS for k in order}]
+    want, expanded, _ = steps(part, w, plan, src)
+    src["b"][:20] = float("inf")
+    got, _, _ = steps(part, w, plan, src)
+    assert expanded == 1 and not bool(got["b"].isfinite().any())
+    assert bool(want["a"].isfinite().all()) and torch.equal(got["a"], want["a"])

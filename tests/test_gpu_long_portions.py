@@ -161,3 +161,26 @@ def test_mixed_heads_of_single_tokens_over_ranges_of_keys(splits, hd, nh, nkv, w
     one, got = hybrid.talk_attention_mma(*args), hybrid.talk_attention_mma(*args, splits=splits)
     # the weights of a range are rounded to bfloat16 against its own maximum: 2^-9 each, as the one range's are
     assert rel(got, one.double()) < 6e-3
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("cross", [True, False])
+@pytest.mark.parametrize("page", [16, 256])
+def test_what_a_page_held_before(hd, cross, page):
+    """Keys and values in a sequence's last page beyond its last token are none of its own, whatever is there."""
+    from rllm_b200.kernels import sm100
+    nh, nkv, lens = 4, 2, ((257, 300), (129, 129), (150, 641))
+    cu, cud, kvl, _, _, table, pages = batch(lens, page, hd, 1)
+    q = rnd(cu[-1], nh * hd, seed=3).bfloat16()
+    kc, vc = rnd(pages, nkv, page, hd, seed=4).bfloat16(), rnd(pages, nkv, page, hd, seed=5).bfloat16()
+    got = []
+    for left in (0.0, float("inf"), float("nan")):
+        for s, (_, n) in enumerate(lens):
+            if n % page:
+                last = int(table[s, n // page])
+                kc[last, :, n % page:] = left
+                vc[last, :, n % page:] = left
+        kw = dict(cross=torch.empty((cu[-1], nh, nkv, hd), device=DEV)) if cross else {}
+        got.append(sm100.attention_prefill_tc(q, kc, vc, cud, kvl, table, 257, nh, hd ** -0.5, None, **kw).clone())
+    sm100.check_error(torch.device(DEV))
+    assert bool(got[0].isfinite().all()) and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
