@@ -144,6 +144,35 @@ __device__ __forceinline__ void tile_product(float (&acc)[4][4 * NT], const floa
   }
 }
 
+// The same for the lower triangle of a [64][64] A, the warp's rows its upper (half 0) or lower 32: what lies right of the
+// diagonal is left out, not multiplied as zero. A token's sum then holds nothing of the tokens after it, which zero times an
+// infinity or NaN of theirs would bring in.
+__device__ __forceinline__ void triangle_product(float (&acc)[4][4], const float* A, int lda, const float* B, int ldb, int half, int row) {
+  if (half) tile_product<1>(acc, A, lda, B, ldb, C / 2);
+  A += half * (C / 2);
+  B += half * (C / 2) * ldb;
+#pragma unroll
+  for (int k = 0; k < C / 2; k += 4) {
+    float4 x[4];
+#pragma unroll
+    for (int i = k / 8; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(A + 8 * i * lda + k);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 y = *reinterpret_cast<const float4*>(B + (k + e) * ldb);
+#pragma unroll
+      for (int i = k / 8; i < 4; ++i) {
+        const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+        if (i > k / 8 || k % 8 + e <= row) {
+          acc[i][0] = fmaf(xv, y.x, acc[i][0]);
+          acc[i][1] = fmaf(xv, y.y, acc[i][1]);
+          acc[i][2] = fmaf(xv, y.z, acc[i][2]);
+          acc[i][3] = fmaf(xv, y.w, acc[i][3]);
+        }
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
   return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
 }
@@ -191,7 +220,8 @@ __device__ __forceinline__ void unit_lower_inverse(const float* L, float* X, flo
       const int I = J + d;
       float x = 0.f;
 #pragma unroll
-      for (int m = 0; m < SB; ++m) x = fmaf(X[(I * SB + t) * LC + I * SB + m], tmp[(J * SB + m) * (SB + 1) + j], x);
+      for (int m = 0; m < SB; ++m)
+        if (m <= t) x = fmaf(X[(I * SB + t) * LC + I * SB + m], tmp[(J * SB + m) * (SB + 1) + j], x);
       X[(I * SB + t) * LC + J * SB + j] = -x;
     }
     __syncthreads();
@@ -469,10 +499,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_kernel(Args a) {
     unit_lower_inverse(G2, G1, tmp);
     // W = X (beta P k), then X (beta v), D value columns at a time in Q's place
     const int rl = (warp & 1) * 32 + (lane >> 2), cl = (warp >> 1) * 16 + 4 * (lane & 3);
-    const int kk = (warp & 1) ? C : C / 2;                 // the upper rows meet the first half only
     for (int c = 0; c < D; c += 64) {
       float acc[4][4] = {};
-      tile_product<1>(acc, G1 + rl * LC, LC, K + c + cl, LDD, kk);
+      triangle_product(acc, G1 + rl * LC, LC, K + c + cl, LDD, warp & 1, lane >> 2);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         *reinterpret_cast<float4*>(to.w + (rl + 8 * i) * LDD + c + cl) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
@@ -490,7 +519,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_kernel(Args a) {
       __syncthreads();
       for (int c = 0; c + (warp >> 1) * 16 < nv; c += 64) {
         float acc[4][4] = {};
-        tile_product<1>(acc, G1 + rl * LC, LC, Q + c + cl, LDD, kk);
+        triangle_product(acc, G1 + rl * LC, LC, Q + c + cl, LDD, warp & 1, lane >> 2);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           *reinterpret_cast<float4*>(to.u + ((v0 + c + cl) / 16 * C + rl + 8 * i) * 16 + cl % 16) =
@@ -657,7 +686,7 @@ __global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
 
 // O of a chunk: M U, then (P q) S on top, 64 value columns a CTA; the first product's operands (the smaller ones) land first.
 template <typename TI, int D, bool DELTA>
-__global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Args a) {
+__global__ void __launch_bounds__(THREADS, D == 64 ? 3 : 2) chunk_out_kernel(Args a) {
   pdl_launch();
   pdl_wait();
   constexpr int LDD = D + 4;
@@ -690,7 +719,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Args a) {
   float acc[4][4] = {};
   const bool ok0 = landed(&full[0], 0, &abort_flag, a.err, 42);
   if (ok0 && tile < tiles)
-    tile_product<1>(acc, M + r * LC, LC, U + tile * C * 16 + c, 16, (warp & 1) ? C : C / 2);       // M is zero right of the diagonal
+    triangle_product(acc, M + r * LC, LC, U + tile * C * 16 + c, 16, warp & 1, lane >> 2);
   if (!landed(&full[1], 0, &abort_flag, a.err, 43) || !ok0 || tile >= tiles) return;
   tile_product<1>(acc, Q + r * LDD, LDD, S + tile * D * 16 + c, 16, D);
   const float skip = a.skip ? a.skip[h] : 0.f;

@@ -128,3 +128,36 @@ def test_gated_linear_attention_in_chunks(lens, dim, vdim, H, bonus):
     if min(lens) < 64:
         s = min(range(S), key=lambda i: lens[i])
         assert torch.equal(got["chunks"][0][cu[s]: cu[s + 1]], got["rows"][0][cu[s]: cu[s + 1]])
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta"])
+@pytest.mark.parametrize("kind", ["channel", "head", "gla"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_a_token_that_is_not_finite(what, kind, bad):
+    """What a token brings is felt from it on, or (a query) by it alone: the tokens before it in its chunk are as they were."""
+    from rllm_b200.kernels import hybrid, mix
+    if what == "beta" and kind == "gla":
+        pytest.skip("gated linear attention has none")
+    H, dim, vdim, at = 2, 64, 64, 64 + 37
+    cu, cud = layout((150, 70))
+    T, slots = cu[-1], torch.arange(2, dtype=torch.int32, device=DEV)
+    x = {"q": rnd(T, H * dim, seed=1), "k": torch.nn.functional.normalize(rnd(T, H, dim, seed=2), dim=-1).view(T, -1),
+         "v": rnd(T, H * vdim, seed=3), "decay": decays(T, H * (1 if kind == "head" else dim), seed=4), "beta": rnd(T, H, seed=5)}
+
+    def scan():
+        state = torch.zeros(2, H, dim, vdim, device=DEV)
+        if kind == "gla":
+            proj = torch.cat([x["q"], x["k"], x["v"]], 1).bfloat16()
+            return mix.gla_scan(proj, 0, H * dim, 2 * H * dim, x["decay"], 1.0, H, dim, vdim, cud, 2, slots, state, long_from=64,
+                                any_short=False, err=ERR())
+        return hybrid.state_scan(x["q"], H, x["k"], H, x["v"], x["decay"], H, dim, vdim, cud, 2, slots, state, beta=x["beta"],
+                                 long_from=64, any_short=False, err=ERR())
+    want = scan()
+    x[what][at] = bad
+    got = scan()
+    mine = slice(at, at + 1) if what == "q" else slice(at, 150)
+    if what != "beta" or bad != bad:                     # the sigmoid of an infinity is one
+        assert not bool(got[mine].isfinite().all())
+    same = torch.ones(T, dtype=torch.bool, device=DEV)
+    same[mine] = False
+    assert bool(want.isfinite().all()) and torch.equal(got[same], want[same])
