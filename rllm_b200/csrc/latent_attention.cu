@@ -685,23 +685,24 @@ RLLM_API int rllm_latent_prepare(int dt, const void* proj, long long ld, int q_o
 // [row tiles, splits, rows, rank], pml: float [row tiles, splits, rows, 2], rows = 64 a tile, or 16 with `few`
 // (the shape for steps of a token or two per sequence; taken when rank is a multiple of 128), row tiles =
 // ceil(T * H / rows) + num_seqs. skip_from > 0: sequences of at least so many rows may be left out (their outputs are then not
-// written), where the tensor-core kernel runs.
+// written), where the tensor-core kernel runs; the others have `live` rows together, which then stand for T in the row tiles.
 RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache, void* out, const int* token_seq,
                                    const int* positions, const int* block_table, int bt_stride, int T, int H, int rank,
                                    int dk, int page_size, float scale, int window, const int* cu_q, int num_seqs,
-                                   int tc, int splits, int few, int skip_from, float* pacc, float* pml, void* stream) {
+                                   int tc, int splits, int few, int skip_from, int live, float* pacc, float* pml, void* stream) {
   if (T <= 0) return 0;
   if (H <= 0 || rank <= 0 || rank > MAX_RANK || dk < rank || page_size <= 0) return ERR_BAD_SIZE;
   if (tc && dt == DT_BF16 && cu_q && num_seqs > 0 && dk % 8 == 0 && rank % 16 == 0 && rank <= 512 &&
       !((uintptr_t)qfull & 15) && !((uintptr_t)cache & 15) && !((uintptr_t)out & 3)) {
-    if (splits < 1 || splits > 32 || (splits > 1 && (!pacc || !pml))) return ERR_BAD_SIZE;
+    if (splits < 1 || splits > 32 || (splits > 1 && (!pacc || !pml)) || live < 0) return ERR_BAD_SIZE;
+    if (skip_from <= 0) live = T;
     cudaStream_t s = (cudaStream_t)stream;
     if (few && rank % 128 == 0) {
       // 16 rows a CTA: steps of a token or two per sequence
       const int nw = rank / 64;
       const int ld = mma_row_pad(dk, nw * 4);                        // 8 warps x nw tiles of 8 columns = rank
       const int smem = (FROWS + 2 * FKT) * ld * 2 + FROWS * (FKT + 1) * 4;
-      const long long blocks = ((long long)T * H + FROWS - 1) / FROWS + num_seqs;
+      const long long blocks = ((long long)live * H + FROWS - 1) / FROWS + num_seqs;
       if (smem <= 220 * 1024 && blocks <= 2147483647LL) {
 #define GO(NW)                                                                                                          \
   do {                                                                                                                  \
@@ -724,7 +725,7 @@ RLLM_API int rllm_latent_attention(int dt, const void* qfull, const void* cache,
     const int nh = rank <= 64 ? 4 : rank <= 128 ? 8 : rank <= 256 ? 16 : 32;
     const int ld = mma_row_pad(dk, nh);
     const int smem = (QROWS + 2 * KT) * ld * 2 + QROWS * (KT + 1) * 4;
-    const long long blocks = ((long long)T * H + QROWS - 1) / QROWS + num_seqs;
+    const long long blocks = ((long long)live * H + QROWS - 1) / QROWS + num_seqs;
     if (smem <= 220 * 1024 && blocks <= 2147483647LL) {
 #define GO(NH)                                                                                                          \
   do {                                                                                                                  \

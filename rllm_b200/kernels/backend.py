@@ -408,7 +408,7 @@ class Backend:
 
     def latent_expanded(self, ctx, q, gate, gate_cols, heads, dim, rot, vdim, rank, window, scale):
         """Portions whose latent attention runs over expanded keys and values: (rows a portion has at least, their cached
-        positions, whether there are shorter portions beside them), or None. A pair of query and key costs 0.26 ns less then
+        positions, (rows, sequences) of the step up to the last shorter portion), or None. A pair of query and key costs 0.26 ns less then
         (16 heads, measured: 590 us against 39 for 2,048 tokens) and a cached position 4.6 ns for its expansion, hence from 32
         visible queries a key on it pays with a margin; the expansion may take 2 GB. Steps whose longest portion has fewer
         than 256 rows wait for their launches and stay as they are, and so do queries and gates whose rows the attention
@@ -421,7 +421,9 @@ class Backend:
         rows = sum(n for _, n in long)
         if rows * heads * (dim + vdim) * 2 > 2 << 30 or 32 * rows > sum(q * min(n, window or n) for q, n in long):
             return None
-        return LATENT_FROM, rows, len(long) < ctx.num_seqs
+        # the scheduler puts decoded tokens in front, so that the rows up to the last shorter portion are theirs alone
+        seqs = max((s + 1 for s, q in enumerate(ctx.q_lens_host) if q < LATENT_FROM), default=0)
+        return LATENT_FROM, rows, (sum(ctx.q_lens_host[:seqs]), seqs)
 
     def latent_expand(self, cache, ctx, w_ukv, rank, long):
         """The cached rows of the long portions' sequences, and every head's keys and values from them (`w_ukv`: W_uk over
@@ -441,24 +443,26 @@ class Backend:
             q, dim + rot, qfull[:, :, rank:] if rot else None, kv, 0, heads * dim, c[:, rank:] if rot else None, ctx.cu_q,
             ctx.kv_lens, ctx.max_q_len, heads, scale, window, out, long_from, gate, gate_cols)
 
-    def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0):
+    def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0, num_seqs=None):
+        """qfull: the rows of the step's first `num_seqs` sequences (None: all); those with at least `skip_from` rows may be left out."""
         # Steps of few rows (decoding) have fewer row tiles than the GPU has SMs: the keys of a tile are then
         # dealt out to several CTAs, at least four key tiles (128 keys) each; steps of a token or two per
         # sequence take the kernel shape with 16 rows a CTA. Everything this depends on is known when a decode
         # graph is captured (rows, sequences, the longest portion, the bound of the key count).
         T, H = qfull.shape[0], qfull.shape[1]
-        longest = max((n for n in ctx.q_lens_host if n < skip_from), default=0) if skip_from else ctx.max_q_len
-        few = longest <= 2 and rank % 128 == 0
+        num_seqs = ctx.num_seqs if num_seqs is None else num_seqs
+        mine = [q for q in ctx.q_lens_host[:num_seqs] if q < skip_from] if skip_from else None
+        few = (max(mine, default=0) if skip_from else ctx.max_q_len) <= 2 and rank % 128 == 0
         rows = 16 if few else 64
         if skip_from:
-            T = sum(q for q in ctx.q_lens_host if q < skip_from)
+            T = sum(mine)
         tiles = max(1, T * H // rows)               # row tiles the step has at least
         keys = min(window, ctx.max_kv_len) if window else ctx.max_kv_len
         splits = max(1, min(16, self.sm_count // tiles, keys // 128))
         return self._mix.latent_attention(qfull, cache.tensors["kv"], ctx.token_seq, ctx.positions,
-                                          cache.block_table, rank, scale, window, cu_q=ctx.cu_q, num_seqs=ctx.num_seqs,
+                                          cache.block_table, rank, scale, window, cu_q=ctx.cu_q, num_seqs=num_seqs,
                                           tensor_cores=self.fast and os.environ.get("RLLM_B200_NO_TC_ATTENTION") != "1",
-                                          splits=splits, few=few, skip_from=skip_from)
+                                          splits=splits, few=few, skip_from=skip_from, rows=T)
 
     def gla_decay(self, z, bias, tau):
         return self._mix.gla_decay(z, bias, tau)

@@ -38,7 +38,7 @@ ops.register_signatures("mix", {
     "rllm_latent_prepare": [c_int, _P, _LL, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, _P,
                             _P, _P, _P, c_int, c_int, _P, _P, _P],
     "rllm_latent_attention": [c_int, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
-                              c_int, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, _P],
+                              c_int, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P, _P],
     "rllm_latent_gather": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "rllm_gla_decay": [_P, _P, c_int, c_int, c_float, _P],
     "rllm_gla_scan": [c_int, _P, _LL, c_int, c_int, c_int, _P, c_float, c_int, c_int, c_int, c_int, c_int, _P, _P, _P,
@@ -319,13 +319,14 @@ def latent_prepare(proj: torch.Tensor, q_off: int, dkv_off: int, heads: int, dim
 def latent_attention(qfull: torch.Tensor, cache: torch.Tensor, token_seq: torch.Tensor, positions: torch.Tensor,
                      block_table: torch.Tensor, rank: int, scale: float, window: int | None,
                      cu_q: torch.Tensor | None = None, num_seqs: int = 0, tensor_cores: bool = True,
-                     splits: int = 1, few: bool = False, skip_from: int = 0) -> torch.Tensor:
+                     splits: int = 1, few: bool = False, skip_from: int = 0, rows: int | None = None) -> torch.Tensor:
     """qfull [T, heads, dk]; cache [pages, page, dk] -> [T, heads, rank] of qfull's dtype. With `cu_q`
     (int32 [num_seqs + 1], the row range of each sequence) bfloat16 problems of fitting sizes run on the
     tensor cores (`tensor_cores` False: never); `splits` > 1 there deals a row tile's keys out to that many
     CTAs and merges their parts (steps of few rows); `few` asks for the kernel shape with 16 rows a CTA (a
     token or two per sequence; taken where the rank is a multiple of 128). `skip_from` > 0: the outputs of sequences of
-    at least so many rows may stay unwritten (they are another kernel's)."""
+    at least so many rows may stay unwritten (they are another kernel's), and `rows` is how many rows the others have: what grid
+    and scratch are sized for (a portion of 2,048 rows beside 8 tokens would ask for 1 GB)."""
     _cuda(qfull, "qfull"); _cuda(cache, "cache")
     T, H, dk = qfull.shape
     if not qfull.is_contiguous() or not cache.is_contiguous() or cache.dtype != qfull.dtype or cache.dim() != 3 \
@@ -341,18 +342,19 @@ def latent_attention(qfull: torch.Tensor, cache: torch.Tensor, token_seq: torch.
     pacc = pml = None
     splits = max(1, min(int(splits), 32))
     few = bool(few) and rank % 128 == 0
+    rows = T if rows is None or not skip_from else int(rows)
     if splits > 1 and cu_q is not None:
-        rows = 16 if few else 64
-        tiles = (T * H + rows - 1) // rows + num_seqs
-        pacc = torch.empty((tiles, splits, rows, rank), dtype=torch.float32, device=qfull.device)
-        pml = torch.empty((tiles, splits, rows, 2), dtype=torch.float32, device=qfull.device)
+        each = 16 if few else 64
+        tiles = (rows * H + each - 1) // each + num_seqs
+        pacc = torch.empty((tiles, splits, each, rank), dtype=torch.float32, device=qfull.device)
+        pml = torch.empty((tiles, splits, each, 2), dtype=torch.float32, device=qfull.device)
     else:
         splits = 1
     _check(_fn("mix", "rllm_latent_attention")(
         _dt(qfull, "qfull"), qfull.data_ptr(), cache.data_ptr(), out.data_ptr(), token_seq.data_ptr(),
         positions.data_ptr(), block_table.data_ptr(), block_table.stride(0), T, H, rank, dk, cache.shape[1],
         float(scale), int(window or 0), _ptr(cu_q), int(num_seqs), int(bool(tensor_cores)), splits, int(few),
-        int(skip_from), _ptr(pacc), _ptr(pml), _stream()), "latent_attention", 2 if splits > 1 else 1)
+        int(skip_from), rows, _ptr(pacc), _ptr(pml), _stream()), "latent_attention", 2 if splits > 1 else 1)
     return out
 
 

@@ -244,7 +244,7 @@ class OpProfile:
         return self._timed("latent_attention", long[1] * (rank + rot) * 2 + _nbytes(q), 2 * heads * (dim + rot + 128) * pairs,
                            self._be.latent_attention_expanded, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, *a)
 
-    def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0):
+    def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0, num_seqs=None):
         T, H, dk = qfull.shape
         lens, qs = ctx.kv_lens_host, ctx.q_lens_host
         if lens is None:
@@ -253,7 +253,7 @@ class OpProfile:
         pairs = sum(q * (s - q) + q * (q + 1) // 2 for s, q in zip(seen, qs))
         nbytes = sum(seen) * dk * qfull.element_size() + _nbytes(qfull) + T * H * rank * qfull.element_size()
         return self._timed("latent_attention", nbytes, 2 * H * (dk + rank) * pairs, self._be.latent_attention,
-                           qfull, cache, ctx, rank, scale, window, skip_from)
+                           qfull, cache, ctx, rank, scale, window, skip_from, num_seqs)
 
     def gla_decay(self, z, bias, tau):
         return self._timed("gla_decay", 2 * _nbytes(z), 0, self._be.gla_decay, z, bias, tau)

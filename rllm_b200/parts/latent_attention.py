@@ -115,10 +115,12 @@ class LatentAttention(Part):
         expanded = None
         if long is not None and (expanded := be.latent_expand(cache, ctx, self._ukv, self.kv_rank, long)) is None:
             long = None                                              # no memory for the expansion
-        if long is None or long[2]:
-            be.linear_heads(q, self.dim + self.rot_dim, self._uk_t, qfull.view(T, H * dk), dk)
-            o = be.latent_attention(qfull, cache, ctx, self.kv_rank, self.scale, self.window, skip_from=long[0] if long else 0)
-            be.linear_heads(o.view(T, H * self.kv_rank), self.kv_rank, self._uv, att, self.vdim, gate=gate, gate_cols=gate_cols)
+        n, seqs, skip_from = (T, None, 0) if long is None else (*long[2], long[0])
+        if n:
+            be.linear_heads(q[:n], self.dim + self.rot_dim, self._uk_t, qfull[:n].view(n, H * dk), dk)
+            o = be.latent_attention(qfull[:n], cache, ctx, self.kv_rank, self.scale, self.window, skip_from, seqs)
+            be.linear_heads(o.view(n, H * self.kv_rank), self.kv_rank, self._uv, att[:n], self.vdim,
+                            gate=None if gate is None else gate[:n], gate_cols=gate_cols)
         if long is not None:
             be.latent_attention_expanded(q, qfull, expanded, ctx, H, self.dim, self.rot_dim, self.kv_rank, self.scale, self.window,
                                          long, att, gate, gate_cols)

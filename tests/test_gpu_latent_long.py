@@ -86,3 +86,27 @@ def test_a_request_beside_one_that_is_not_finite(order, rot):
     got, _, _ = steps(part, w, plan, src)
     assert expanded == 1 and not bool(got["b"].isfinite().any())
     assert bool(want["a"].isfinite().all()) and torch.equal(got["a"], want["a"])
+
+
+def test_single_tokens_beside_a_long_portion():
+    """The short portions' part is sized by their rows: against the same step with every row over the latents, and its memory."""
+    part, w, _ = built(8, 64, 512)
+    order = "abcdefghp"
+    src = {k: rnd(3000 if k == "p" else 21 + 7 * i, W, seed=i).bfloat16().to(DEV) for i, k in enumerate(order)}
+    first = {k: 1100 if k == "p" else len(src[k]) - 1 for k in order}
+    bind(part, w, "bfloat16", "x.")
+    got = []
+    for expanded in (True, False):
+        hs = Harness("bfloat16", [part.cache_spec()], page_size=16, pages=240, slots=9)
+        if not expanded:
+            hs.backend.latent_expanded = lambda *a: None
+        run = lambda step, rows: hs.run(list(step.items()), lambda ctx, cache: part.forward(rows, ctx, cache))
+        run(first, torch.cat([src[k][: first[k]] for k in order]))
+        rows = torch.cat([src[k][first[k]:] for k in order])
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        got.append(run({k: len(src[k]) - first[k] for k in order}, rows))
+        if expanded:
+            assert torch.cuda.max_memory_allocated() - before < 200 << 20
+        hs.engine.check()
+    assert rel(got[0], got[1]) < 2e-2 and bool(got[0].isfinite().all())
