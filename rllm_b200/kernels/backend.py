@@ -19,6 +19,8 @@ from . import ops
 # Rows that a step's longest portion has where attention over latents runs over expanded keys and values, and rows from which
 # a portion beside it does too; rows of a portion from which attention with mixed heads runs in the tcgen05 kernel
 LATENT_LONG, LATENT_FROM, TALK_LONG = 256, 32, 128
+# us that the expansion has to save: its launches and, beside shorter portions, those of the form over the latents (`latent_expanded`)
+LATENT_GAIN, LATENT_GAIN_MIXED = 35.0, 120.0
 TALK_PAIRS = 384 * 384       # pairs of query and key that mixed heads have at least there (`talk_attention` says why)
 
 
@@ -408,18 +410,22 @@ class Backend:
 
     def latent_expanded(self, ctx, q, gate, gate_cols, heads, dim, rot, vdim, rank, window, scale):
         """Portions whose latent attention runs over expanded keys and values: (rows a portion has at least, their cached
-        positions, (rows, sequences) of the step up to the last shorter portion), or None. A pair of query and key costs 0.26 ns less then
-        (16 heads, measured: 590 us against 39 for 2,048 tokens) and a cached position 4.6 ns for its expansion, hence from 32
-        visible queries a key on it pays with a margin; the expansion may take 2 GB. Steps whose longest portion has fewer
-        than 256 rows wait for their launches and stay as they are, and so do queries and gates whose rows the attention
-        kernel cannot copy in pieces of 16 bytes."""
+        positions, (rows, sequences) of the step up to the last shorter portion), or None. Measured for 16 heads: a pair of query
+        and key costs 0.06 + 0.00043 rank ns over the latents (rank 512: 590 us for 2,048 tokens) and 0.03 expanded, a cached
+        position 4.6 ns for its expansion. What that saves has to outweigh the launches. One forward of the part, over the latents
+        against expanded, us: 16 heads of rank 512, 512 tokens 143 / 148, 2,048 tokens 689 / 149, 256 over 2,000 cached ones 270 / 148;
+        64 heads, 256 tokens 170 / 132; beside 16 single tokens, 512 tokens, 16 heads 173 / 194, 64 heads 349 / 348, 128 heads
+        617 / 352. The expansion may take 2 GB. Steps whose longest portion has fewer than 256 rows stay as they are, and so do
+        queries and gates whose rows the attention kernel cannot copy in pieces of 16 bytes."""
         if not self.fast or ctx.graph_safe or ctx.max_q_len < LATENT_LONG or dim != 128 or vdim != 128 or rot not in (0, 64) \
                 or rank % 64 or scale <= 0 or not self._sm100.prefill_dense_supported(q, gate, gate_cols) \
                 or os.environ.get("RLLM_B200_NO_TC_ATTENTION") == "1":
             return None
         long = [(q, n) for q, n in zip(ctx.q_lens_host, ctx.kv_lens_host) if q >= LATENT_FROM]
         rows = sum(n for _, n in long)
-        if rows * heads * (dim + vdim) * 2 > 2 << 30 or 32 * rows > sum(q * min(n, window or n) for q, n in long):
+        pairs = sum(q * min(n - q // 2, window or n) for q, n in long)
+        gain = heads / 16 * ((0.03 + 0.00043 * rank) * pairs - 4.6 * rows) / 1000
+        if rows * heads * (dim + vdim) * 2 > 2 << 30 or gain < (LATENT_GAIN if len(long) == ctx.num_seqs else LATENT_GAIN_MIXED):
             return None
         # the scheduler puts decoded tokens in front, so that the rows up to the last shorter portion are theirs alone
         seqs = max((s + 1 for s, q in enumerate(ctx.q_lens_host) if q < LATENT_FROM), default=0)

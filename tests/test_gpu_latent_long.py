@@ -15,6 +15,14 @@ pytestmark = pytest.mark.gpu
 W, EPS, ROWS = 64, 1e-6, 300
 
 
+@pytest.fixture(autouse=True)
+def expand_small_steps(monkeypatch):
+    """The sizes below show what there is to see and are not worth their launches."""
+    from rllm_b200.kernels import backend
+    monkeypatch.setattr(backend, "LATENT_GAIN", -1e9)
+    monkeypatch.setattr(backend, "LATENT_GAIN_MIXED", -1e9)
+
+
 def built(heads, rot, rank, window=None, q_rank=None):
     """(part, weights, plain implementation) of a layer with a gate a head, or (q_rank) a query latent and a gate an output."""
     from rllm_b200.parts import InterleavedRotary, LatentAttention

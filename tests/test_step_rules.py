@@ -1,0 +1,37 @@
+"""Which form of an operation a step takes, by the sizes of its portions alone: the rules that the backend asks on the host, at
+sizes where both forms were measured."""
+from types import SimpleNamespace
+
+import pytest
+
+
+def step(lens):
+    """A step of [(rows, keys)], as the rules see it."""
+    q, n = [r for r, _ in lens], [k for _, k in lens]
+    return SimpleNamespace(graph_safe=False, q_lens_host=q, kv_lens_host=n, max_q_len=max(q), max_kv_len=max(n), num_seqs=len(lens),
+                           num_tokens=sum(q), per_forward={})
+
+
+@pytest.mark.parametrize("heads,rank,window,lens,expanded", [
+    (16, 512, None, [(512, 512)], False),                       # us over the latents / expanded: 143 / 148
+    (16, 512, None, [(2048, 2048)], True),                      # 689 / 149
+    (16, 512, None, [(256, 2256)], True),                       # 270 / 148
+    (64, 512, None, [(256, 256)], True),                        # 170 / 132
+    (16, 64, None, [(512, 512)], False),                        # 112 / 120
+    (16, 64, None, [(2048, 2048)], True),                       # 317 / 152
+    (16, 512, 128, [(2048, 2048)], True),                       # 203 / 147
+    (16, 512, 128, [(512, 512)], False),                        # 113 / 119
+    (16, 512, None, [(1, 1001)] * 16 + [(512, 512)], False),    # 173 / 194
+    (128, 512, None, [(1, 1001)] * 16 + [(512, 512)], True),    # 617 / 352
+    (128, 512, None, [(1, 1001)] * 63 + [(256, 256)], False),   # 470 / 573
+    (16, 512, None, [(1, 4001)] * 8 + [(2048, 4048)], True),    # 1,665 / 332
+])
+def test_latents_are_expanded_where_it_pays(monkeypatch, heads, rank, window, lens, expanded):
+    from rllm_b200.kernels.backend import Backend
+    monkeypatch.delenv("RLLM_B200_NO_TC_ATTENTION", raising=False)
+    be = SimpleNamespace(fast=True, _sm100=SimpleNamespace(prefill_dense_supported=lambda *a: True))
+    got = Backend.latent_expanded(be, step(lens), None, None, False, heads, 128, 64, 128, rank, window, 0.1)
+    assert (got is not None) == expanded
+    if expanded:
+        short = [r for r, _ in lens if r < 32]
+        assert got[1:] == (sum(n for r, n in lens if r >= 32), (sum(short), len(short)))
