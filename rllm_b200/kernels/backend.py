@@ -20,7 +20,7 @@ from . import ops
 # a portion beside it does too; rows of a portion from which attention with mixed heads runs in the tcgen05 kernel
 LATENT_LONG, LATENT_FROM, TALK_LONG = 256, 32, 128
 # us that the expansion has to save: its launches and, beside shorter portions, those of the form over the latents (`latent_expanded`)
-LATENT_GAIN, LATENT_GAIN_MIXED = 35.0, 120.0
+LATENT_GAIN, LATENT_GAIN_MIXED = 55.0, 220.0
 TALK_PAIRS = 384 * 384       # pairs of query and key that mixed heads have at least there (`talk_attention` says why)
 
 
@@ -411,8 +411,8 @@ class Backend:
     def latent_expanded(self, ctx, q, gate, gate_cols, heads, dim, rot, vdim, rank, window, scale):
         """Portions whose latent attention runs over expanded keys and values: (rows a portion has at least, their cached
         positions, (rows, sequences) of the step up to the last shorter portion), or None. Measured for 16 heads: a pair of query
-        and key costs 0.06 + 0.00043 rank ns over the latents (rank 512: 590 us for 2,048 tokens) and 0.03 expanded, a cached
-        position 4.6 ns for its expansion. What that saves has to outweigh the launches. One forward of the part, over the latents
+        and key costs 0.06 + 0.00043 rank ns over the latents (rank 512: 590 us for 2,048 tokens) and 0.03 expanded, a row
+        41 ns for its products per head, a cached position 4.6 ns for its expansion. What that saves has to outweigh the launches. One forward of the part, over the latents
         against expanded, us: 16 heads of rank 512, 512 tokens 143 / 148, 2,048 tokens 689 / 149, 256 over 2,000 cached ones 270 / 148;
         64 heads, 256 tokens 170 / 132; beside 16 single tokens, 512 tokens, 16 heads 173 / 194, 64 heads 349 / 348, 128 heads
         617 / 352. The expansion may take 2 GB. Steps whose longest portion has fewer than 256 rows stay as they are, and so do
@@ -424,7 +424,7 @@ class Backend:
         long = [(q, n) for q, n in zip(ctx.q_lens_host, ctx.kv_lens_host) if q >= LATENT_FROM]
         rows = sum(n for _, n in long)
         pairs = sum(q * min(n - q // 2, window or n) for q, n in long)
-        gain = heads / 16 * ((0.03 + 0.00043 * rank) * pairs - 4.6 * rows) / 1000
+        gain = heads / 16 * ((0.03 + 0.00043 * rank) * pairs + 41 * sum(q for q, _ in long) - 4.6 * rows) / 1000
         if rows * heads * (dim + vdim) * 2 > 2 << 30 or gain < (LATENT_GAIN if len(long) == ctx.num_seqs else LATENT_GAIN_MIXED):
             return None
         # the scheduler puts decoded tokens in front, so that the rows up to the last shorter portion are theirs alone
