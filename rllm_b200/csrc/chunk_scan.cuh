@@ -545,12 +545,15 @@ __global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
   __shared__ int abort_flag;
   float* S = sm + 2 * STAGE;                             // [NT][D][16]
   float* part = S + D * NC;                              // [4][NT][C][16] sums of U, or [JG - 1][NT][D][16] of S
-  const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * NC, H = a.H, V = a.vdim;
+  const int h = blockIdx.y, v0 = blockIdx.z * NC, H = a.H, V = a.vdim;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n = a.cu_q[seq + 1] - a.cu_q[seq], chunks = chunks_of(n, a.long_from);
-  if (chunks == 0) return;
-  int base = 0;
-  for (int s = 0; s < seq; ++s) base += chunks_of(a.cu_q[s + 1] - a.cu_q[s], a.long_from);
+  int seq = 0, base = 0, chunks = 0;                     // the long sequence of this number, its first chunk, how many it has
+  for (int before = 0; seq < a.num_seqs; ++seq) {
+    chunks = chunks_of(a.cu_q[seq + 1] - a.cu_q[seq], a.long_from);
+    if (chunks > 0 && before++ == (int)blockIdx.x) break;
+    base += chunks;
+  }
+  if (seq == a.num_seqs) return;
   const int slot = a.state_slots ? a.state_slots[seq] : -1;
   float* sp = a.state + ((long long)(slot < 0 ? 0 : slot) * H + h) * D * V + v0;
   if (tid == 0) {
@@ -747,19 +750,25 @@ inline bool takes(const Args& a, int dim) {
          !((uintptr_t)a.scratch & 15) && a.H <= 65535 && a.vdim / 16 <= 65535;
 }
 
-inline long long scratch_floats(int T, int S, int H, int dim, int vdim, bool delta) {
-  return (long long)(T / C + S) * H * (dim == 64 ? Place<64>::floats(vdim, delta) : Place<128>::floats(vdim, delta));
+// Floats of scratch a (chunk, head).
+inline long long scratch_floats(int dim, int vdim, bool delta) {
+  return dim == 64 ? Place<64>::floats(vdim, delta) : Place<128>::floats(vdim, delta);
 }
 
 template <typename TI, int D, bool PERCH, bool DELTA, bool BONUS>
-int launch(const Args& a, int T, cudaStream_t s) {
+int launch(const Args& a, int longs, int chunks, cudaStream_t s) {   // long sequences and their chunks, at most
+  if (longs <= 0 || chunks <= 0) return 0;
   constexpr int LDD = D + 4;
   constexpr int INV = 3 * SB * (SB + 1), MATS = DELTA ? 2 * C * LC + INV : PERCH ? 0 : C * LC + 2 * C;    // from A on
   constexpr int OWN = PERCH ? C * LDD + 4 * D : 0;                                                        // A and blk
   constexpr size_t prep = sizeof(float) * (2 * C + 2 * C * LDD + (MATS > OWN ? MATS : OWN));
   constexpr size_t outs = sizeof(float) * (C * LC + C * LDD + 4 * C * 16 + 4 * D * 16);
   static bool ok_prep[64], ok_out[64], ok_16[64], ok_32[64];
-  const unsigned chunks = (unsigned)(T / C + a.num_seqs);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return -5;
+  }
   auto prep_k = chunk_prep_kernel<TI, D, PERCH, DELTA, BONUS>;
   int rc = allow_dynamic_smem(prep_k, (int)prep, ok_prep);
   if (rc) return rc;
@@ -771,11 +780,11 @@ int launch(const Args& a, int T, cudaStream_t s) {
     const size_t part = (size_t)nc * (DELTA && 4 * C > (JG - 1) * D ? 4 * C : (JG - 1) * D);
     const size_t bytes = sizeof(float) * (2 * stage + D * nc + part);
     const int rc2 = allow_dynamic_smem(kernel, (int)bytes, ok);
-    return rc2 ? rc2 : launch_ex(kernel, dim3(a.num_seqs, a.H, a.vdim / nc), dim3(THREADS), bytes, s, 1, a);
+    return rc2 ? rc2 : launch_ex(kernel, dim3(longs, a.H, a.vdim / nc), dim3(THREADS), bytes, s, 1, a);
   };
   // 16 columns a CTA put twice as many CTAs on the walk; 32 read the rows of W and k half as often. The line is the number
   // of SMs: with more CTAs than that a walk of 16 columns is two waves long.
-  if (a.vdim % 32 == 0 && (long long)a.num_seqs * a.H * (a.vdim / 16) > 148)
+  if (a.vdim % 32 == 0 && (long long)longs * a.H * (a.vdim / 16) > sms)
     rc = carry(chunk_carry_kernel<D, 32, DELTA>, 32, ok_32);
   else
     rc = carry(chunk_carry_kernel<D, 16, DELTA>, 16, ok_16);

@@ -305,7 +305,8 @@ RLLM_API int rllm_gla_decay(float* z, const float* bias, int T, int n, float tau
 RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, int k_off, int v_off, const float* alpha,
                            float qscale, int T, int S, int H, int dim, int vdim, const int* cu_q,
                            const int* state_slots, float* state, float* out, int chunk, float* chunk_state,
-                           float* chunk_decay, const float* bonus, int long_from, int any_short, float* scratch, int* err, void* stream) {
+                           float* chunk_decay, const float* bonus, int longs, int chunks, int long_from, int any_short, float* scratch, int* err,
+                           void* stream) {
   if (S <= 0 || T <= 0) return 0;
   if (H <= 0 || dim <= 0 || dim > MAX_DIM || vdim <= 0) return ERR_BAD_SIZE;
   if (H > 65535 || (vdim + 31) / 32 > 65535) return ERR_TOO_LARGE;
@@ -319,8 +320,8 @@ RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, in
     c.qscale = qscale; c.decay = alpha; c.bonus = bonus; c.H = H; c.vdim = vdim; c.cu_q = cu_q; c.num_seqs = S;
     c.state_slots = state_slots; c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch; c.err = err;
     if (chunked::takes<bf16>(c, dim)) {
-      const int rc = dim == 64 ? (bonus ? chunked::launch<bf16, 64, true, false, true>(c, T, s) : chunked::launch<bf16, 64, true, false, false>(c, T, s))
-                               : (bonus ? chunked::launch<bf16, 128, true, false, true>(c, T, s) : chunked::launch<bf16, 128, true, false, false>(c, T, s));
+      const int rc = dim == 64 ? (bonus ? chunked::launch<bf16, 64, true, false, true>(c, longs, chunks, s) : chunked::launch<bf16, 64, true, false, false>(c, longs, chunks, s))
+                               : (bonus ? chunked::launch<bf16, 128, true, false, true>(c, longs, chunks, s) : chunked::launch<bf16, 128, true, false, false>(c, longs, chunks, s));
       if (rc || !any_short) return rc;
       chunk = 0;                                                       // the short sequences, row by row
     } else {
@@ -338,14 +339,14 @@ RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, in
 #define SCAN(MODE, GRID) (bonus ? SCAN_B(MODE, true, GRID) : SCAN_B(MODE, false, GRID))
   if (chunk <= 0) return SCAN(WHOLE, dim3(S, H, vb));
   if (!chunk_state || !chunk_decay) return ERR_BAD_SIZE;
-  const int chunks = T / chunk + S;                                  // at least as many as the sequences have
-  int rc = SCAN_B(LOCAL, false, dim3(chunks, H, vb));               // what a chunk builds does not depend on the bonus
+  const int pieces = T / chunk + S;                                  // at least as many as the sequences have
+  int rc = SCAN_B(LOCAL, false, dim3(pieces, H, vb));               // what a chunk builds does not depend on the bonus
   if (rc) return rc;
   const int per = dim * vdim;
   rc = launch_ex(gla_carry_kernel, dim3(S, H, (per + 255) / 256), dim3(256), 0, s, 1, cu_q, state_slots, state,
                  chunk_state, (const float*)chunk_decay, chunk, H, dim, vdim);
   if (rc) return rc;
-  return SCAN(FINAL, dim3(chunks, H, vb));
+  return SCAN(FINAL, dim3(pieces, H, vb));
 #undef SCAN
 #undef SCAN_B
 }
@@ -354,7 +355,7 @@ RLLM_API int rllm_gla_scan(int dt, const void* proj, long long ld, int q_off, in
 // for by `scratch` and `long_from`: sequences of at least so many rows run in it, the others (any_short) row by row. 0: not taken.
 RLLM_API int rllm_gla_chunk_floats(int dim, int vdim) {
   if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % 16) return 0;
-  const long long n = chunked::scratch_floats(0, 1, 1, dim, vdim, false);
+  const long long n = chunked::scratch_floats(dim, vdim, false);
   return n < 2147483647LL ? (int)n : 0;
 }
 

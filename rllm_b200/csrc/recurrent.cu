@@ -602,13 +602,13 @@ RLLM_API int rllm_softplus_decay(int dt, const void* z, long long ld, int col0, 
 // Floats of scratch that a (chunk of 64 rows, head) of the chunked form takes; 0: these sizes do not run in chunks.
 RLLM_API int rllm_state_scan_chunk_floats(int dim, int vdim, int delta) {
   if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % 16) return 0;
-  const long long n = chunked::scratch_floats(0, 1, 1, dim, vdim, delta != 0);
+  const long long n = chunked::scratch_floats(dim, vdim, delta != 0);
   return n < 2147483647LL ? (int)n : 0;
 }
 
-static int launch_chunked(const chunked::Args& c, int dim, bool perch, bool delta, int T, cudaStream_t s) {
+static int launch_chunked(const chunked::Args& c, int dim, bool perch, bool delta, int longs, int chunks, cudaStream_t s) {
 #define RLLM_CH(D, P, DL) \
-  if (dim == D && perch == P && delta == DL) return chunked::launch<float, D, P, DL, false>(c, T, s)
+  if (dim == D && perch == P && delta == DL) return chunked::launch<float, D, P, DL, false>(c, longs, chunks, s)
   RLLM_CH(64, false, false); RLLM_CH(64, false, true); RLLM_CH(64, true, false); RLLM_CH(64, true, true);
   RLLM_CH(128, false, false); RLLM_CH(128, false, true); RLLM_CH(128, true, false); RLLM_CH(128, true, true);
 #undef RLLM_CH
@@ -636,7 +636,7 @@ RLLM_API int rllm_state_scan(int beta_dt, const float* q, long long q_ld, int q_
                              int k_heads, const float* v, long long v_ld, const float* decay, int decay_per_channel,
                              const void* beta, long long beta_ld, const float* vscale, const float* skip, int S, int H,
                              int dim, int vdim, const int* cu_q, const int* state_slots, float* state, float* out,
-                             int channels, int T, int long_from, int any_short, float* scratch, int* err, void* stream) {
+                             int channels, int longs, int chunks, int long_from, int any_short, float* scratch, int* err, void* stream) {
   if (S <= 0) return 0;
   if (H <= 0 || dim <= 0 || dim > 1024 || vdim <= 0 || q_heads <= 0 || k_heads <= 0 || H % q_heads || H % k_heads)
     return ERR_BAD_SIZE;
@@ -657,7 +657,7 @@ RLLM_API int rllm_state_scan(int beta_dt, const float* q, long long q_ld, int q_
     c.skip = skip; c.H = H; c.vdim = vdim; c.cu_q = cu_q; c.num_seqs = S; c.state_slots = state_slots;
     c.long_from = long_from; c.state = state; c.out = out; c.scratch = scratch; c.err = err;
     if (chunked::takes<float>(c, dim)) {
-      const int rc = launch_chunked(c, dim, decay_per_channel != 0, beta != nullptr, T, s);
+      const int rc = launch_chunked(c, dim, decay_per_channel != 0, beta != nullptr, longs, chunks, s);
       if (rc || !any_short) return rc;
       a.long_from = long_from;
     }

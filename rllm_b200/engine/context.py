@@ -62,7 +62,10 @@ class StepContext:
 
     def long_rows(self) -> dict:
         """What a recurrence's scan is told about a step with a long portion: from how many rows on a sequence runs in
-        chunks as products of matrices, and whether there are shorter ones beside it."""
+        chunks as products of matrices, whether there are shorter ones beside it, and how many such sequences and chunks of 64
+        there are."""
         if self.graph_safe or self.max_q_len < LONG_FROM:
             return {}
-        return {"long_from": CHUNK_FROM, "any_short": min(self.q_lens_host) < CHUNK_FROM}
+        long = [n for n in self.q_lens_host if n >= CHUNK_FROM]
+        return {"long_from": CHUNK_FROM, "any_short": len(long) < self.num_seqs, "longs": len(long),
+                "chunks": sum((n + 63) // 64 for n in long)}

@@ -21,7 +21,7 @@ ops.register_signatures("recurrent", {
     "rllm_softplus_decay": [c_int, _P, _LL, c_int, _P, _P, c_int, c_int, c_int, _P, _P, _P],
     "rllm_state_scan_split": [c_int],
     "rllm_state_scan": [c_int, _P, _LL, c_int, _P, _LL, c_int, _P, _LL, _P, c_int, _P, _LL, _P, _P, c_int, c_int, c_int,
-                        c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P],
+                        c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, _P],
     "rllm_state_scan_chunk_floats": [c_int, c_int, c_int],
     "rllm_gated_norm": [_P, _P, c_int, _LL, _P, c_int, c_float, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P],
 })
@@ -300,14 +300,16 @@ def softplus_decay(z, col0, n, bias, a_log, want_step=False):
 
 
 def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seqs, state_slots, state, beta=None, vscale=None,
-               skip=None, channels: int = 0, long_from: int = 0, any_short: bool = True, err=None) -> torch.Tensor:
+               skip=None, channels: int = 0, long_from: int = 0, any_short: bool = True, err=None, longs: int | None = None,
+               chunks: int | None = None) -> torch.Tensor:
     """See csrc/recurrent.cu. q [T, q_heads * dim], k [T, k_heads * dim], v [T, heads * vdim]: float32 views with unit
     inner stride; decay float32 [T, heads * dim] (per channel) or [T, heads]; beta: logits [T, heads] of the
     projection's type (delta rule) or None (plain); vscale float32 [T, heads]; skip float32 [heads].
-    -> float32 [T, heads, vdim]; `state` float32 [slots, heads, dim, vdim] is updated. `channels` (32, 16 or 8): key
+    -> float32 [T, heads, vdim]; `state` float32 [slots, heads, dim, vdim] is updated. `channels` (32, 16 or 8): key channels
     a thread where the kernel with compiled sizes runs, for measurements; 0: chosen from the sizes. `long_from` > 0: sequences
     of at least so many rows run in chunks (csrc/chunk_scan.cuh) where the sizes allow; `any_short`: there are others; `err`:
-    the device's error word, without which nothing runs in chunks."""
+    the device's error word, without which nothing runs in chunks; `longs`, `chunks`: how many such sequences, and chunks of 64
+    rows of theirs, there are at most (None: as many as T rows can have)."""
     T = q.shape[0]
     for t, n, c in ((q, "q", q_heads * dim), (k, "k", k_heads * dim), (v, "v", heads * vdim)):
         _rows(t, n, c)
@@ -331,13 +333,14 @@ def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seq
         _f32(skip, "skip", (heads,))
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
     scratch = None
+    longs, chunks = num_seqs if longs is None else longs, T // 64 + num_seqs if chunks is None else chunks
     if long_from > 0 and err is not None and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
-        scratch = _scratch((T // 64 + num_seqs) * heads * per, q.device)
+        scratch = _scratch(chunks * heads * per, q.device)
     _check(_fn("recurrent", "rllm_state_scan")(
         _dt(beta, "beta") if beta is not None else 0, q.data_ptr(), q.stride(0), int(q_heads), k.data_ptr(), k.stride(0),
         int(k_heads), v.data_ptr(), v.stride(0), decay.data_ptr(), int(per_channel), _ptr(beta),
         beta.stride(0) if beta is not None else 0, _ptr(vscale), _ptr(skip), int(num_seqs), int(heads), int(dim), int(vdim),
-        cu_q.data_ptr(), _ptr(state_slots), state.data_ptr(), out.data_ptr(), int(channels), T, int(long_from), int(any_short),
+        cu_q.data_ptr(), _ptr(state_slots), state.data_ptr(), out.data_ptr(), int(channels), int(longs), int(chunks), int(long_from), int(any_short),
         _ptr(scratch), _ptr(err), _stream()), "state_scan", 1 if scratch is None else 3 + int(any_short))
     return out
 

@@ -42,7 +42,7 @@ ops.register_signatures("mix", {
     "rllm_latent_gather": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "rllm_gla_decay": [_P, _P, c_int, c_int, c_float, _P],
     "rllm_gla_scan": [c_int, _P, _LL, c_int, c_int, c_int, _P, c_float, c_int, c_int, c_int, c_int, c_int, _P, _P, _P,
-                      _P, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P],
+                      _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P],
     "rllm_gla_chunk_floats": [c_int, c_int],
     "rllm_shift_mix": [c_int, _P, _P, c_float, _P, c_float, _P, c_int, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, _P],
     "rllm_lowrank_decay": [c_int, _P, _LL, c_int, _P, _P, _P, c_int, c_int, _P],
@@ -387,12 +387,13 @@ def gla_decay(z: torch.Tensor, bias: torch.Tensor, tau: float) -> torch.Tensor:
 def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torch.Tensor, qscale: float, heads: int,
              dim: int, vdim: int, cu_q: torch.Tensor, num_seqs: int, state_slots: torch.Tensor | None,
              state: torch.Tensor, chunk: int = 0, bonus: torch.Tensor | None = None, long_from: int = 0,
-             any_short: bool = True, err=None) -> torch.Tensor:
+             any_short: bool = True, err=None, longs: int | None = None, chunks: int | None = None) -> torch.Tensor:
     """See csrc/gla.cu. -> float32 [T, heads, vdim]; `state` float32 [slots, heads, dim, vdim] is updated.
     `bonus` float32 [heads, dim]: a token reads the state before it and its own product times the bonus.
     `chunk` > 0: sequences are cut into chunks of that many tokens that run side by side (long portions).
     `long_from` > 0: bfloat16 sequences of at least so many rows run as products of matrices (csrc/chunk_scan.cuh) where the
-    sizes allow, in place of `chunk`; `any_short`: there are others; `err`: the device's error word, without which nothing does."""
+    sizes allow, in place of `chunk`; `any_short`: there are others; `err`: the device's error word, without which nothing does;
+    `longs`, `chunks`: how many such sequences, and chunks of 64 rows of theirs, there are at most (None: as many as T rows can have)."""
     T = proj.shape[0]
     _rows(proj, "proj", max(q_off + heads * dim, k_off + heads * dim, v_off + heads * vdim))
     _f32(alpha, "decays", (T, heads * dim))
@@ -406,8 +407,9 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torc
         _f32(bonus, "bonus", (heads, dim))
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=proj.device)
     cs = cd = scratch = None
+    longs, chunks = num_seqs if longs is None else longs, T // 64 + num_seqs if chunks is None else chunks
     if long_from > 0 and err is not None and proj.dtype == torch.bfloat16 and (per := _fn("mix", "rllm_gla_chunk_floats")(int(dim), int(vdim))):
-        scratch = _scratch((T // 64 + num_seqs) * heads * per, proj.device)
+        scratch = _scratch(chunks * heads * per, proj.device)
     if chunk > 0 and scratch is None:
         n = T // chunk + num_seqs
         cs = torch.empty((n, heads, dim, vdim), dtype=torch.float32, device=proj.device)
@@ -415,7 +417,8 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torc
     _check(_fn("mix", "rllm_gla_scan")(
         _dt(proj, "proj"), proj.data_ptr(), proj.stride(0), q_off, k_off, v_off, alpha.data_ptr(), float(qscale), T,
         num_seqs, heads, dim, vdim, cu_q.data_ptr(), _ptr(state_slots), state.data_ptr(), out.data_ptr(), int(chunk),
-        _ptr(cs), _ptr(cd), _ptr(bonus), int(long_from), int(any_short), _ptr(scratch), _ptr(err), _stream()), "gla_scan",
+        _ptr(cs), _ptr(cd), _ptr(bonus), int(longs), int(chunks), int(long_from), int(any_short), _ptr(scratch), _ptr(err), _stream()),
+        "gla_scan",
         3 + int(any_short) if scratch is not None else 3 if chunk > 0 else 1)
     return out
 

@@ -161,3 +161,24 @@ def test_a_token_that_is_not_finite(what, kind, bad):
     same = torch.ones(T, dtype=torch.bool, device=DEV)
     same[mine] = False
     assert bool(want.isfinite().all()) and torch.equal(got[same], want[same])
+
+
+def test_the_step_says_how_many_chunks_there_are():
+    """Grids and scratch of the long sequences alone, in any order among short ones: the same bits as with the bounds."""
+    from types import SimpleNamespace
+    from rllm_b200.engine.context import StepContext
+    from rllm_b200.kernels import hybrid, mix
+    lens, H, dim = (1, 300, 63, 64, 1, 65) + (1,) * 40, 2, 64
+    cu, cud = layout(lens)
+    T, S = cu[-1], len(lens)
+    long = StepContext.long_rows(SimpleNamespace(graph_safe=False, max_q_len=300, q_lens_host=list(lens), num_seqs=S))
+    assert long == dict(long_from=64, any_short=True, longs=3, chunks=5 + 1 + 2)
+    q, k, v = rnd(T, H * dim, seed=1), torch.nn.functional.normalize(rnd(T, H, dim, seed=2), dim=-1).view(T, -1), rnd(T, H * dim, seed=3)
+    a, beta, slots = decays(T, H * dim, seed=4), rnd(T, H, seed=5), torch.arange(S, dtype=torch.int32, device=DEV)
+    got = []
+    for kw in (dict(long_from=64, any_short=True), long):
+        state = [rnd(S, H, dim, dim, seed=6) for _ in range(2)]
+        got.append((hybrid.state_scan(q, H, k, H, v, a, H, dim, dim, cud, S, slots, state[0], beta=beta, err=ERR(), **kw),
+                    mix.gla_scan(torch.cat([q, k, v], 1).bfloat16(), 0, H * dim, 2 * H * dim, a, 1.0, H, dim, dim, cud, S, slots,
+                                 state[1], err=ERR(), **kw), *state))
+    assert all(torch.equal(x, y) for x, y in zip(*got)) and all(bool(x.isfinite().all()) for x in got[0])
