@@ -23,6 +23,13 @@ class GroupView:
 # rows, 109 / 57 at 256; state space with 32 heads 49 / 37 and 95 / 44. Four portions of 128 rows with 32 heads are level. Below 256
 # rows a step waits for its launches, of which chunks take three.
 LONG_FROM, CHUNK_FROM = 256, 64
+# A walk row by row takes as long as its longest portion while there is room beside it; once heads and portions fill the GPU, chunks
+# take about as many FMAs and more traffic. `pairs` = heads x (rows of the portions in chunks / the longest), us row by row / in
+# chunks, portions of 256: delta rule with a decay per head, 128 x 128: 64 pairs 193 / 117, 128 207 / 235, 256 375 / 430; decays per
+# channel 64 244 / 135, 128 274 / 269, 256 487 / 488; state space, 128 x 64: 128 175 / 100, 256 189 / 200; heads of 64 x 64: 64 89 / 55,
+# 128 111 / 105, 140 116 / 142, 256 159 / 197; gated linear attention of 128 64 153 / 92, 128 166 / 183. Its three passes over chunks,
+# from 384 rows on, are the slower form at any number (128 x 128, 256 pairs of 512 rows 1,403 / 601; heads of 64 level at 64).
+CHUNK_PAIRS, CHUNK_COLUMNS = 128, 96 * 128     # pairs, and value columns of all pairs, up to which a step's portions run in chunks
 
 
 @dataclass
@@ -60,12 +67,15 @@ class StepContext:
     def all_decode(self) -> bool:
         return self.max_q_len == 1
 
-    def long_rows(self) -> dict:
+    def long_rows(self, heads: int, vdim: int, walked: bool = True) -> dict:
         """What a recurrence's scan is told about a step with a long portion: from how many rows on a sequence runs in
         chunks as products of matrices, whether there are shorter ones beside it, and how many such sequences and chunks of 64
-        there are."""
+        there are. Empty where chunks do not pay; `walked`: the other form goes row by row."""
         if self.graph_safe or self.max_q_len < LONG_FROM:
             return {}
         long = [n for n in self.q_lens_host if n >= CHUNK_FROM]
+        pairs = heads * sum(long) / self.max_q_len
+        if walked and (pairs > CHUNK_PAIRS or pairs * vdim > CHUNK_COLUMNS):
+            return {}
         return {"long_from": CHUNK_FROM, "any_short": len(long) < self.num_seqs, "longs": len(long),
                 "chunks": sum((n + 63) // 64 for n in long)}

@@ -583,7 +583,7 @@ class Backend:
 
     def state_scan(self, q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx, state, beta=None, vscale=None, skip=None):
         # the 32-bit run's results are the same bits however a sequence is cut into steps: row by row
-        long = ctx.long_rows() if self.fast else {}
+        long = ctx.long_rows(heads, vdim) if self.fast else {}
         if long:
             long["err"] = self._err
         return self._hy.state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx.cu_q, ctx.num_seqs,

@@ -70,8 +70,9 @@ class GatedLinearAttention(Part):
         proj = be.linear(x, self.w_in)                                   # [T, q | k | v | gate | a1]
         z = be.linear_f32(proj[:, self._a1_off:], self.w_a2)             # float decay logits [T, H * dim]
         alpha = be.gla_decay(z, self._b_f32, self.tau)                   # in place
+        chunk = scan_chunk(ctx, self.chunk)
         o = be.gla_scan(proj, 0, H * d, 2 * H * d, alpha, d ** -0.5, H, d, v, ctx.cu_q, ctx.num_seqs,
-                        ctx.state_slots, cache.state["S"], scan_chunk(ctx, self.chunk), **ctx.long_rows())
+                        ctx.state_slots, cache.state["S"], chunk, **ctx.long_rows(H, v, walked=not chunk))
         att = be.gla_finish(o, self._norm_f32, self.eps, proj, 2 * H * d + H * v)
         if residual is None:
             return be.linear_f32(att, self.w_o)
@@ -119,8 +120,9 @@ class TimeMixing(Part):
         x, n2 = be.shift_mix(h, norm.weight_f32(), norm.eps, self._mu, ctx, cache.state["prev"], second)    # [T, 5, W]
         proj = be.linear_mixes(x, self.w_in, C, tag="in")                # [T, r | k | v | g | w1]
         decay = be.lowrank_decay(proj[:, 4 * C:], self._w2_t, self._w0)   # float [T, C]
+        chunk = scan_chunk(ctx, self.chunk)
         o = be.gla_scan(proj, 0, C, 2 * C, decay, 1.0, H, d, d, ctx.cu_q, ctx.num_seqs, ctx.state_slots, cache.state["S"],
-                        scan_chunk(ctx, self.chunk), bonus=self._u, **ctx.long_rows())
+                        chunk, bonus=self._u, **ctx.long_rows(H, d, walked=not chunk))
         return be.linear_f32(be.gla_finish(o, self._norm_f32, self.eps, proj, 3 * C), self.w_o, tag="o"), n2
 
 

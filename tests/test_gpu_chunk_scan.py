@@ -171,7 +171,7 @@ def test_the_step_says_how_many_chunks_there_are():
     lens, H, dim = (1, 300, 63, 64, 1, 65) + (1,) * 40, 2, 64
     cu, cud = layout(lens)
     T, S = cu[-1], len(lens)
-    long = StepContext.long_rows(SimpleNamespace(graph_safe=False, max_q_len=300, q_lens_host=list(lens), num_seqs=S))
+    long = StepContext.long_rows(SimpleNamespace(graph_safe=False, max_q_len=300, q_lens_host=list(lens), num_seqs=S), H, dim)
     assert long == dict(long_from=64, any_short=True, longs=3, chunks=5 + 1 + 2)
     q, k, v = rnd(T, H * dim, seed=1), torch.nn.functional.normalize(rnd(T, H, dim, seed=2), dim=-1).view(T, -1), rnd(T, H * dim, seed=3)
     a, beta, slots = decays(T, H * dim, seed=4), rnd(T, H, seed=5), torch.arange(S, dtype=torch.int32, device=DEV)

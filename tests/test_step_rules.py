@@ -35,3 +35,23 @@ def test_latents_are_expanded_where_it_pays(monkeypatch, heads, rank, window, le
     if expanded:
         short = [r for r, _ in lens if r < 32]
         assert got[1:] == (sum(n for r, n in lens if r >= 32), (sum(short), len(short)))
+
+
+@pytest.mark.parametrize("heads,vdim,rows,walked,chunks", [
+    (16, 128, [256], True, 4),                      # us row by row / in chunks: 107 / 56
+    (64, 128, [256], True, 4),                      # 193 / 117
+    (128, 128, [256], True, None),                  # 207 / 235
+    (8, 128, [256] * 16, True, None),               # 207 / 238
+    (16, 128, [256] * 4, True, 16),                 # 193 / 118
+    (32, 64, [256] * 4, True, 16),                  # 175 / 100
+    (16, 64, [256] * 16, True, None),               # 159 / 197
+    (64, 128, [1] * 63 + [256], True, 4),           # 310 / 278
+    (32, 128, [512] * 8, False, 64),                # against three passes: 1,403 / 601
+    (16, 128, [255] * 4, True, None),
+])
+def test_recurrences_run_in_chunks_where_it_pays(heads, vdim, rows, walked, chunks):
+    from rllm_b200.engine.context import StepContext
+    got = StepContext.long_rows(step([(n, n) for n in rows]), heads, vdim, walked)
+    assert got.get("chunks") == chunks
+    if got:
+        assert got["longs"] == sum(n >= 64 for n in rows) and got["any_short"] == (min(rows) < 64)
