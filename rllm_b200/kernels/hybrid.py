@@ -11,7 +11,7 @@ from ctypes import c_float, c_int, c_longlong
 import torch
 
 from . import ops
-from .ops import KernelError, _check, _cuda, _dt, _fn, _ptr, _scratch, _stream
+from .ops import KernelError, _check, _chunk_rows, _cuda, _dt, _fn, _ptr, _scratch, _stream
 
 _P, _LL = ops._P, c_longlong
 
@@ -334,7 +334,7 @@ def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seq
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
     scratch = None
     longs, chunks = num_seqs if longs is None else longs, T // 64 + num_seqs if chunks is None else chunks
-    if long_from > 0 and err is not None and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
+    if long_from > 0 and err is not None and _chunk_rows((q, 0), (k, 0), (v, 0)) and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
         scratch = _scratch(chunks * heads * per, q.device)
     _check(_fn("recurrent", "rllm_state_scan")(
         _dt(beta, "beta") if beta is not None else 0, q.data_ptr(), q.stride(0), int(q_heads), k.data_ptr(), k.stride(0),

@@ -13,7 +13,7 @@ from ctypes import c_float, c_int, c_longlong
 import torch
 
 from . import ops
-from .ops import KernelError, _check, _cuda, _dt, _fn, _ptr, _scratch, _stream
+from .ops import KernelError, _check, _chunk_rows, _cuda, _dt, _fn, _ptr, _scratch, _stream
 
 _P, _LL = ops._P, c_longlong
 GEPI_STORE, GEPI_STORE_F32, GEPI_RELU2, GEPI_SILU_GATED = 0, 1, 2, 3
@@ -408,7 +408,7 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torc
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=proj.device)
     cs = cd = scratch = None
     longs, chunks = num_seqs if longs is None else longs, T // 64 + num_seqs if chunks is None else chunks
-    if long_from > 0 and err is not None and proj.dtype == torch.bfloat16 and (per := _fn("mix", "rllm_gla_chunk_floats")(int(dim), int(vdim))):
+    if long_from > 0 and err is not None and proj.dtype == torch.bfloat16 and _chunk_rows((proj, q_off), (proj, k_off), (proj, v_off)) and (per := _fn("mix", "rllm_gla_chunk_floats")(int(dim), int(vdim))):
         scratch = _scratch(chunks * heads * per, proj.device)
     if chunk > 0 and scratch is None:
         n = T // chunk + num_seqs

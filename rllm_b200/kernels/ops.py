@@ -109,6 +109,11 @@ def _dt(t: torch.Tensor, name: str) -> int:
         raise KernelError(f"{name}: dtype {t.dtype} is not supported (float32 or bfloat16)") from None
 
 
+def _chunk_rows(*views) -> bool:
+    """Can the chunked recurrences read these rows, four neighbouring numbers at a time? (view, column offset) each."""
+    return all(t.stride(0) % 4 == 0 and (t.data_ptr() // t.element_size() + off) % 4 == 0 for t, off in views)
+
+
 def _scratch(n: int, device) -> torch.Tensor | None:
     """Float scratch of a faster form of a kernel, or None where the memory left does not hold it: the other form runs then."""
     try:

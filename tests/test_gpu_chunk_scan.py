@@ -182,3 +182,21 @@ def test_the_step_says_how_many_chunks_there_are():
                     mix.gla_scan(torch.cat([q, k, v], 1).bfloat16(), 0, H * dim, 2 * H * dim, a, 1.0, H, dim, dim, cud, S, slots,
                                  state[1], err=ERR(), **kw), *state))
     assert all(torch.equal(x, y) for x, y in zip(*got)) and all(bool(x.isfinite().all()) for x in got[0])
+
+
+@pytest.mark.parametrize("pad,off", [(2, 0), (0, 2), (4, 0)])
+def test_rows_that_the_chunks_cannot_read(pad, off):
+    """A projection whose rows, or their parts, do not start on four numbers keeps the passes over chunks that it had."""
+    from rllm_b200.kernels import mix
+    H, dim, T = 2, 64, 400
+    cu, cud = layout((T,))
+    proj = rnd(T, off + H * 3 * dim + pad, seed=1).bfloat16()
+    a = torch.exp(-0.01 * rnd(T, H * dim, seed=2).abs())          # slow, so that how the sums are grouped shows
+    args = (proj, off, off + H * dim, off + 2 * H * dim, a, 1.0, H, dim, dim, cud, 1, torch.zeros(1, dtype=torch.int32, device=DEV))
+    state = [rnd(1, H, dim, dim, seed=3) for _ in range(3)]
+    passes = mix.gla_scan(*args, state[0], 128)
+    got = mix.gla_scan(*args, state[1], 128, long_from=64, any_short=False, err=ERR())
+    rows = mix.gla_scan(*args, state[2])
+    same = (torch.equal(got, passes), torch.equal(got, rows))
+    assert same == ((False, False) if pad % 4 == off % 4 == 0 else (True, False)) and torch.equal(state[0], state[1]) == same[0]
+    assert rel(got, rows.double()) < 2e-6
