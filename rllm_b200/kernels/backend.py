@@ -17,11 +17,28 @@ from . import ops
 
 
 # Rows that a step's longest portion has where attention over latents runs over expanded keys and values, and rows from which
-# a portion beside it does too; rows of a portion from which attention with mixed heads runs in the tcgen05 kernel
+# a portion beside it does too; rows of a portion from which attention with mixed heads may run in the tcgen05 kernel
 LATENT_LONG, LATENT_FROM, TALK_LONG = 256, 32, 128
 # us that the expansion has to save: its launches and, beside shorter portions, those of the form over the latents (`latent_expanded`)
 LATENT_GAIN, LATENT_GAIN_MIXED = 55.0, 220.0
-TALK_PAIRS = 384 * 384       # pairs of query and key that mixed heads have at least there (`talk_attention` says why)
+
+
+def talk_on_tcgen05(ctx, nh, nkv, hd, window=None, chunk=None) -> bool:
+    """Do the step's portions of at least TALK_LONG rows run their mixed heads in the tcgen05 kernel? Its launches take some 40 us
+    whatever the size. The mma.sync kernel has a CTA a tile of 64 rows and pair of kv heads that walks its key tiles of 64 at
+    3.2 us each (heads of 64: 2.2) until the CTAs fill the SMs, 0.0142 (0.0075) us a CTA from there. Shorter portions beside stay
+    there and are waited for then. Measured, mma.sync against tcgen05, us: 16 heads of 128 over 4 kv heads 256 x 256 28 / 41, 384 x 384
+    39 / 41, 512 x 512 56 / 40, 128 x 1,200 76 / 43, 2,048 x 2,048 476 / 134; 4 heads over 1 512 x 512 31 / 44, 1,024 x 1,024 51 / 40,
+    512 x 900 beside 17 single tokens 54 / 61; 32 over 4 384 x 384 66 / 43; heads of 64, 16 over 4 512 x 512 33 / 41, 1,024 x 1,024 85 / 41,
+    512 x 900 beside 17 single tokens 77 / 87."""
+    if ctx.graph_safe or ctx.max_q_len < TALK_LONG:
+        return False
+    step, each = (3.2, 0.0142) if hd > 64 else (2.2, 0.0075)
+    seen = lambda k: -(-min(k, window + 64 if window else k, chunk + 64 if chunk else k) // 64)
+    long = [(n, seen(k)) for n, k in zip(ctx.q_lens_host, ctx.kv_lens_host) if n >= TALK_LONG]
+    ctas = sum(-(-n * (nh // nkv) // 64) for n, _ in long) * nkv * nkv
+    beside = max((seen(k) for n, k in zip(ctx.q_lens_host, ctx.kv_lens_host) if n < TALK_LONG), default=0)
+    return max(t for _, t in long) * max(step, each * ctas) >= 42 + step * beside
 
 
 class Normed:
@@ -603,14 +620,10 @@ class Backend:
         kd, vd = cache.k.shape[3], cache.v.shape[3]
         if self.fast and os.environ.get("RLLM_B200_NO_TC_ATTENTION") != "1" \
                 and hy.talk_mma_supported(q.dtype, nh, kd, vd, cache.page_size):
-            # Every head over every kv head's values is ordinary attention: portions of 128 rows and more go to the tcgen05
-            # kernel of prompt portions where they have pairs enough to outweigh its start. Measured at 16 heads of 128 over
-            # 4 kv heads, mma.sync against tcgen05, us: 256 rows x 256 keys 25 / 37, 384 x 384 39 / 39, 512 x 512 55 / 38,
-            # 128 x 1,500 92 / 47, 2,048 x 2,048 515 / 127.
+            # every head over every kv head's values is ordinary attention: long portions go to the tcgen05 kernel of prompt portions
             page = cache.page_size
-            pairs = 0 if ctx.graph_safe else sum(n * k for n, k in zip(ctx.q_lens_host, ctx.kv_lens_host) if n >= TALK_LONG)
-            if pairs >= TALK_PAIRS and kd == vd and page >= 8 and page & (page - 1) == 0 and scale > 0 \
-                    and self._sm100.prefill_tc_supported(q, cache.k):
+            if kd == vd and page >= 8 and page & (page - 1) == 0 and scale > 0 and self._sm100.prefill_tc_supported(q, cache.k) \
+                    and talk_on_tcgen05(ctx, nh, cache.k.shape[1], kd, window, chunk):
                 parts = torch.empty((q.shape[0], nh, cache.k.shape[1], vd), dtype=torch.float32, device=q.device)
                 self._sm100.attention_prefill_tc(q, cache.k, cache.v, ctx.cu_q, ctx.kv_lens, cache.block_table, ctx.max_q_len, nh,
                                                  scale, window, chunk=chunk, sinks=sinks, long_from=TALK_LONG, cross=parts)

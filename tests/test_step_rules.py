@@ -55,3 +55,25 @@ def test_recurrences_run_in_chunks_where_it_pays(heads, vdim, rows, walked, chun
     assert got.get("chunks") == chunks
     if got:
         assert got["longs"] == sum(n >= 64 for n in rows) and got["any_short"] == (min(rows) < 64)
+
+
+@pytest.mark.parametrize("hd,nh,nkv,lens,tcgen05", [
+    (128, 16, 4, [(384, 384)], False),                          # us mma.sync / tcgen05: 39 / 41
+    (128, 16, 4, [(512, 512)], True),                           # 56 / 40
+    (128, 16, 4, [(128, 1200)], True),                          # 76 / 43
+    (128, 16, 4, [(256, 256)] * 4, True),                       # 58 / 42
+    (128, 16, 4, [(1, 800)] * 17 + [(512, 900)], True),         # 144 / 121
+    (128, 4, 1, [(512, 512)], False),                           # 31 / 44
+    (128, 4, 1, [(1024, 1024)], True),                          # 51 / 40
+    (128, 4, 1, [(256, 256)] * 4, False),                       # 25 / 40
+    (128, 4, 1, [(1, 800)] * 17 + [(512, 900)], False),         # 54 / 61
+    (128, 32, 4, [(384, 384)], True),                           # 66 / 43
+    (64, 16, 4, [(512, 512)], False),                           # 33 / 41
+    (64, 16, 4, [(1024, 1024)], True),                          # 85 / 41
+    (64, 16, 4, [(1, 800)] * 17 + [(512, 900)], False),         # 77 / 87
+    (64, 64, 8, [(384, 384)], True),                            # 112 / 96
+    (128, 16, 4, [(127, 4000)], False),
+])
+def test_mixed_heads_on_tcgen05_where_it_pays(hd, nh, nkv, lens, tcgen05):
+    from rllm_b200.kernels.backend import talk_on_tcgen05
+    assert talk_on_tcgen05(step(lens), nh, nkv, hd) == tcgen05
