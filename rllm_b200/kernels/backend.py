@@ -71,10 +71,26 @@ class Backend:
         self.fast = dtype == torch.bfloat16 and os.environ.get("RLLM_B200_GENERIC_ONLY") != "1"
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self._sm100 = self._err = None
+        self._no_room = 1 << 62             # bytes of scratch that the memory left did not hold once
         if self.fast:
             from . import sm100          # builds/loads the tcgen05 library, or raises
             self._sm100 = sm100
             self._err = sm100.init(self.device).err      # the device's error word
+
+    # ---- scratch of the forms that take more memory than the others
+    def scratch(self, n, device):
+        """n floats, or None where the memory left does not hold them. What did not fit once is not asked for again: a failing
+        allocation makes torch's allocator give back all it holds and ask the driver anew, in every layer of every step."""
+        return self._or_none(4 * n, lambda: torch.empty(n, dtype=torch.float32, device=device))
+
+    def _or_none(self, nbytes, make):
+        if nbytes >= self._no_room:
+            return None
+        try:
+            return make()
+        except torch.OutOfMemoryError:
+            self._no_room = nbytes
+            return None
 
     # ---- element-wise / row-wise
     def embed(self, ids, table, err=None, scale=1.0):
@@ -452,12 +468,12 @@ class Backend:
         """The cached rows of the long portions' sequences, and every head's keys and values from them (`w_ukv`: W_uk over
         W_uv); None where the memory left does not hold them."""
         long_from, rows, _ = long
-        try:
+
+        def make():
             c = self._mix.latent_gather(cache.tensors["kv"], cache.block_table, ctx.cu_q, ctx.kv_lens, ctx.num_seqs, long_from,
                                         rows, ctx.max_kv_len)
             return c, self.linear(c[:, :rank], w_ukv)
-        except torch.OutOfMemoryError:
-            return None
+        return self._or_none(2 * rows * (cache.tensors["kv"].shape[2] + w_ukv.shape[0]), make)
 
     def latent_attention_expanded(self, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, out, gate, gate_cols):
         """The long portions' rows of `out` [T, heads * 128]: attention over the expanded keys and values, the gate."""
@@ -491,7 +507,7 @@ class Backend:
         return self._mix.gla_decay(z, bias, tau)
 
     def gla_scan(self, *a, **k):
-        return self._mix.gla_scan(*a, err=self._err, **k)
+        return self._mix.gla_scan(*a, err=self._err, alloc=self.scratch, **k)
 
     def gla_finish(self, *a, **k):
         return self._mix.gla_finish(*a, **k)
@@ -602,7 +618,7 @@ class Backend:
         # the 32-bit run's results are the same bits however a sequence is cut into steps: row by row
         long = ctx.long_rows(heads, vdim) if self.fast else {}
         if long:
-            long["err"] = self._err
+            long |= {"err": self._err, "alloc": self.scratch}
         return self._hy.state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, ctx.cu_q, ctx.num_seqs,
                                    ctx.state_slots, state, beta, vscale, skip, **long)
 

@@ -301,7 +301,7 @@ def softplus_decay(z, col0, n, bias, a_log, want_step=False):
 
 def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seqs, state_slots, state, beta=None, vscale=None,
                skip=None, channels: int = 0, long_from: int = 0, any_short: bool = True, err=None, longs: int | None = None,
-               chunks: int | None = None) -> torch.Tensor:
+               chunks: int | None = None, alloc=_scratch) -> torch.Tensor:
     """See csrc/recurrent.cu. q [T, q_heads * dim], k [T, k_heads * dim], v [T, heads * vdim]: float32 views with unit
     inner stride; decay float32 [T, heads * dim] (per channel) or [T, heads]; beta: logits [T, heads] of the
     projection's type (delta rule) or None (plain); vscale float32 [T, heads]; skip float32 [heads].
@@ -309,7 +309,7 @@ def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seq
     a thread where the kernel with compiled sizes runs, for measurements; 0: chosen from the sizes. `long_from` > 0: sequences
     of at least so many rows run in chunks (csrc/chunk_scan.cuh) where the sizes allow; `any_short`: there are others; `err`:
     the device's error word, without which nothing runs in chunks; `longs`, `chunks`: how many such sequences, and chunks of 64
-    rows of theirs, there are at most (None: as many as T rows can have)."""
+    rows of theirs, there are at most (None: as many as T rows can have); `alloc`: where their scratch comes from, or None."""
     T = q.shape[0]
     for t, n, c in ((q, "q", q_heads * dim), (k, "k", k_heads * dim), (v, "v", heads * vdim)):
         _rows(t, n, c)
@@ -335,7 +335,7 @@ def state_scan(q, q_heads, k, k_heads, v, decay, heads, dim, vdim, cu_q, num_seq
     scratch = None
     longs, chunks = num_seqs if longs is None else longs, T // 64 + num_seqs if chunks is None else chunks
     if long_from > 0 and err is not None and _chunk_rows((q, 0), (k, 0), (v, 0)) and (per := _fn("recurrent", "rllm_state_scan_chunk_floats")(int(dim), int(vdim), int(beta is not None))):
-        scratch = _scratch(chunks * heads * per, q.device)
+        scratch = alloc(chunks * heads * per, q.device)
     _check(_fn("recurrent", "rllm_state_scan")(
         _dt(beta, "beta") if beta is not None else 0, q.data_ptr(), q.stride(0), int(q_heads), k.data_ptr(), k.stride(0),
         int(k_heads), v.data_ptr(), v.stride(0), decay.data_ptr(), int(per_channel), _ptr(beta),

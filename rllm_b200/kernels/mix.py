@@ -387,13 +387,14 @@ def gla_decay(z: torch.Tensor, bias: torch.Tensor, tau: float) -> torch.Tensor:
 def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torch.Tensor, qscale: float, heads: int,
              dim: int, vdim: int, cu_q: torch.Tensor, num_seqs: int, state_slots: torch.Tensor | None,
              state: torch.Tensor, chunk: int = 0, bonus: torch.Tensor | None = None, long_from: int = 0,
-             any_short: bool = True, err=None, longs: int | None = None, chunks: int | None = None) -> torch.Tensor:
+             any_short: bool = True, err=None, longs: int | None = None, chunks: int | None = None,
+             alloc=_scratch) -> torch.Tensor:
     """See csrc/gla.cu. -> float32 [T, heads, vdim]; `state` float32 [slots, heads, dim, vdim] is updated.
     `bonus` float32 [heads, dim]: a token reads the state before it and its own product times the bonus.
     `chunk` > 0: sequences are cut into chunks of that many tokens that run side by side (long portions).
     `long_from` > 0: bfloat16 sequences of at least so many rows run as products of matrices (csrc/chunk_scan.cuh) where the
     sizes allow, in place of `chunk`; `any_short`: there are others; `err`: the device's error word, without which nothing does;
-    `longs`, `chunks`: how many such sequences, and chunks of 64 rows of theirs, there are at most (None: as many as T rows can have)."""
+    `longs`, `chunks`: how many such sequences, and chunks of 64 rows of theirs, there are at most (None: as many as T rows can have); `alloc`: where their scratch comes from, or None."""
     T = proj.shape[0]
     _rows(proj, "proj", max(q_off + heads * dim, k_off + heads * dim, v_off + heads * vdim))
     _f32(alpha, "decays", (T, heads * dim))
@@ -409,7 +410,7 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: torc
     cs = cd = scratch = None
     longs, chunks = num_seqs if longs is None else longs, T // 64 + num_seqs if chunks is None else chunks
     if long_from > 0 and err is not None and proj.dtype == torch.bfloat16 and _chunk_rows((proj, q_off), (proj, k_off), (proj, v_off)) and (per := _fn("mix", "rllm_gla_chunk_floats")(int(dim), int(vdim))):
-        scratch = _scratch(chunks * heads * per, proj.device)
+        scratch = alloc(chunks * heads * per, proj.device)
     if chunk > 0 and scratch is None:
         n = T // chunk + num_seqs
         cs = torch.empty((n, heads, dim, vdim), dtype=torch.float32, device=proj.device)

@@ -115,7 +115,8 @@ def _chunk_rows(*views) -> bool:
 
 
 def _scratch(n: int, device) -> torch.Tensor | None:
-    """Float scratch of a faster form of a kernel, or None where the memory left does not hold it: the other form runs then."""
+    """Float scratch of a faster form of a kernel, or None where the memory left does not hold it: the other form runs then.
+    (A backend's calls come with its `scratch` instead, which asks once.)"""
     try:
         return torch.empty(n, dtype=torch.float32, device=device)
     except torch.OutOfMemoryError:

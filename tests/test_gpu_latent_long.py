@@ -118,3 +118,27 @@ def test_single_tokens_beside_a_long_portion():
             assert torch.cuda.max_memory_allocated() - before < 200 << 20
         hs.engine.check()
     assert rel(got[0], got[1]) < 2e-2 and bool(got[0].isfinite().all())
+
+
+def test_no_room_for_the_forms_that_take_scratch():
+    """An engine whose memory does not hold the expansion or the chunks: the step runs in the forms without them."""
+    from rllm_b200.kernels import hybrid
+    part, w, plain = built(8, 64, 64)
+    src = {k: rnd(ROWS + 1, W, seed=i).bfloat16() for i, k in enumerate("ab")}
+    bind(part, w, "bfloat16", "x.")
+    hs = Harness("bfloat16", [part.cache_spec()], page_size=16, pages=60, slots=2)
+    hs.backend._no_room = 0
+    rows = torch.cat([src["a"], src["b"]]).to(DEV)
+    got = hs.run([("a", ROWS + 1), ("b", ROWS + 1)], lambda ctx, cache: part.forward(rows, ctx, cache)).split(ROWS + 1)
+    for y, x in zip(got, src.values()):
+        assert rel(y, plain(x.double(), as_stored(w, "bfloat16"))) < 4e-2
+
+    def scan(ctx, cache):
+        T, H, d = 300, 2, 64
+        x = [rnd(T, H * d, seed=i).to(DEV) for i in range(4)]
+        state = [torch.zeros(2, H, d, d, device=DEV) for _ in range(2)]
+        a = hs.backend.state_scan(x[0], H, x[1], H, x[2], torch.sigmoid(x[3]), H, d, d, ctx, state[0])
+        return torch.equal(a, hybrid.state_scan(x[0], H, x[1], H, x[2], torch.sigmoid(x[3]), H, d, d, ctx.cu_q, 1, ctx.state_slots,
+                                                state[1])) and torch.equal(*state)
+    hs.engine.end(["a", "b"])
+    assert hs.run([("c", 300)], scan)

@@ -77,3 +77,20 @@ def test_recurrences_run_in_chunks_where_it_pays(heads, vdim, rows, walked, chun
 def test_mixed_heads_on_tcgen05_where_it_pays(hd, nh, nkv, lens, tcgen05):
     from rllm_b200.kernels.backend import talk_on_tcgen05
     assert talk_on_tcgen05(step(lens), nh, nkv, hd) == tcgen05
+
+
+def test_scratch_that_did_not_fit_is_not_asked_for_again(monkeypatch):
+    import torch
+    from rllm_b200.kernels.backend import Backend
+    asked = []
+
+    def empty(n, **k):
+        asked.append(n)
+        if n > 100:
+            raise torch.OutOfMemoryError("no")
+        return n
+    monkeypatch.setattr(torch, "empty", empty)
+    be = SimpleNamespace(_no_room=1 << 62)
+    be._or_none = lambda *a: Backend._or_none(be, *a)
+    got = [Backend.scratch(be, n, "cpu") for n in (50, 400, 500, 400, 200, 300, 100, 200)]
+    assert got == [50, None, None, None, None, None, 100, None] and asked == [50, 400, 200, 100]
