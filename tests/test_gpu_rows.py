@@ -94,3 +94,20 @@ def test_gate_with_gelu_in_the_product(T, F, K):
         assert rel(got, torch.nn.functional.gelu(g, approximate="tanh") * u) < 1e-2   # the normed operand is rounded too
     with pytest.raises(ops.KernelError):
         sm100.gemm(x, w, ops.EPI_STORE, gelu_gate=True)
+
+
+@pytest.mark.parametrize("rows", [8, 16, 64, 256])
+def test_gate_with_gelu_as_in_a_pass_of_its_own(rows):
+    """Products that are exact (small whole numbers, 32nds), so that only the activation can differ: no further from the 64-bit
+    values' roundings than the kernel that activates floats."""
+    from rllm_b200.kernels import hybrid, ops, sm100
+    T, K, F = 256, 64, 1024
+    g = torch.Generator().manual_seed(0)
+    x = torch.randint(-4, 5, (T, K), generator=g).to(DEV).bfloat16()
+    w = (torch.randint(-4, 5, (2 * F, K), generator=g).float() / 32).to(DEV).bfloat16()
+    p = x.double() @ w.double().T
+    a, u = p[:, :F], p[:, F:]
+    want = (0.5 * a * (1 + torch.tanh((2 / torch.pi) ** 0.5 * (a + 0.044715 * a ** 3))) * u).float().bfloat16()
+    apart = hybrid.glu_act(p.float(), torch.bfloat16, "gelu_tanh", 0.0, 1.0)
+    got = torch.cat([sm100.gemm(x[i: i + rows], w, ops.EPI_SWIGLU, gelu_gate=True) for i in range(0, T, rows)])
+    assert float(a.abs().max()) > 6 and int((got != want).sum()) <= int((apart != want).sum())
