@@ -23,10 +23,12 @@
 // than token by token), no longer a chain; a product's operands come in tiles of 32 x 16 a warp, 64 FMAs for 8 loads of 16
 // bytes (8 x 8 outputs a thread, half the loads: level, and 85 us against 59 where a CTA's sum is short).
 // 2,048 tokens, bfloat16 runs, us (token by token before): delta rule with decays per channel, 16 heads of 128 x 128
-// 275 (1,061); with a decay per head, 32 heads 430 (1,050); state space, 32 heads of 128 x 64 200 (745); gated linear attention,
-// 16 heads 215 (405 in three passes over chunks).
+// 272 (1,061); with a decay per head, 32 heads 422 (1,050); state space, 32 heads of 128 x 64 214 (745); gated linear attention,
+// 16 heads 212 (405 in three passes over chunks).
 // 64 tokens: with 32 the walk over the chunks has twice the barriers for the same FMAs, with 128 the triangles cost more than
-// the rest. Sums are grouped differently than token by token, within float rounding.
+// the rest. Sums are grouped differently than token by token, by fours and sixteens, so that no chain is long: outputs' distance from
+// 64 bits (2-norm, 1,024 tokens) 2.1e-7 where decays are slow (row by row 3.0e-7), 1.1e-7 (1.0e-7) where half the state is gone with
+// every token; as chains of 64 and 128 they were at 3.3e-7 and 1.9 to 2.5e-7. The loads hide the additions.
 #pragma once
 #include "common.cuh"
 #include "sm100.cuh"
@@ -115,32 +117,40 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// acc[i][4 n + c] += sum_k A[row + 8 i][k] B[k][col + 16 n + c]: a warp's tile of 32 x 16 NT, `row` = first row + lane / 4,
-// `col` = first column + 4 (lane % 4). K a multiple of 4; A's rows 16 bytes apart in bank phase (stride 4 mod 32).
-template <int NT>
-__device__ __forceinline__ void tile_product(float (&acc)[4][4 * NT], const float* A, int lda, const float* B, int ldb, int K) {
-#pragma unroll 2
-  for (int k = 0; k < K; k += 4) {
-    float4 x[4];
+// acc[i][c] += sum_k A[row + 8 i][k] B[k][col + c]: a warp's tile of 32 x 16, `row` = first row + lane / 4, `col` = first column +
+// 4 (lane % 4). K a multiple of 16; A's rows 16 bytes apart in bank phase (stride 4 mod 32). Four products are added up, then four such
+// sums, then those (no chain longer than K / 16): 0.4 of the error that one chain leaves, and as fast, since the loads bound it.
+__device__ __forceinline__ void add16(float (&acc)[4][4], const float (&s)[4][4]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(A + 8 * i * lda + k);
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float4 y[NT];
+    for (int c = 0; c < 4; ++c) acc[i][c] += s[i][c];
+}
+__device__ __forceinline__ void tile_product(float (&acc)[4][4], const float* A, int lda, const float* B, int ldb, int K) {
+#pragma unroll 1
+  for (int k0 = 0; k0 < K; k0 += 16) {
+    float part[4][4] = {};
 #pragma unroll
-      for (int n = 0; n < NT; ++n) y[n] = *reinterpret_cast<const float4*>(B + (k + e) * ldb + 16 * n);
+    for (int k = k0; k < k0 + 16; k += 4) {
+      float4 x[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+      for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(A + 8 * i * lda + k);
+      float sum[4][4] = {};
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          acc[i][4 * n] = fmaf(xv, y[n].x, acc[i][4 * n]);
-          acc[i][4 * n + 1] = fmaf(xv, y[n].y, acc[i][4 * n + 1]);
-          acc[i][4 * n + 2] = fmaf(xv, y[n].z, acc[i][4 * n + 2]);
-          acc[i][4 * n + 3] = fmaf(xv, y[n].w, acc[i][4 * n + 3]);
+      for (int e = 0; e < 4; ++e) {
+        const float4 y = *reinterpret_cast<const float4*>(B + (k + e) * ldb);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+          sum[i][0] = fmaf(xv, y.x, sum[i][0]);
+          sum[i][1] = fmaf(xv, y.y, sum[i][1]);
+          sum[i][2] = fmaf(xv, y.z, sum[i][2]);
+          sum[i][3] = fmaf(xv, y.w, sum[i][3]);
         }
       }
+      add16(part, sum);
     }
+    add16(acc, part);
   }
 }
 
@@ -148,33 +158,38 @@ __device__ __forceinline__ void tile_product(float (&acc)[4][4 * NT], const floa
 // diagonal is left out, not multiplied as zero. A token's sum then holds nothing of the tokens after it, which zero times an
 // infinity or NaN of theirs would bring in.
 __device__ __forceinline__ void triangle_product(float (&acc)[4][4], const float* A, int lda, const float* B, int ldb, int half, int row) {
-  if (half) tile_product<1>(acc, A, lda, B, ldb, C / 2);
+  if (half) tile_product(acc, A, lda, B, ldb, C / 2);
   A += half * (C / 2);
   B += half * (C / 2) * ldb;
 #pragma unroll
-  for (int k = 0; k < C / 2; k += 4) {
-    float4 x[4];
+  for (int k0 = 0; k0 < C / 2; k0 += 8) {
+    float sum[4][4] = {};
 #pragma unroll
-    for (int i = k / 8; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(A + 8 * i * lda + k);
+    for (int k = k0; k < k0 + 8; k += 4) {
+      float4 x[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float4 y = *reinterpret_cast<const float4*>(B + (k + e) * ldb);
+      for (int i = k / 8; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(A + 8 * i * lda + k);
 #pragma unroll
-      for (int i = k / 8; i < 4; ++i) {
-        const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
-        if (i > k / 8 || k % 8 + e <= row) {
-          acc[i][0] = fmaf(xv, y.x, acc[i][0]);
-          acc[i][1] = fmaf(xv, y.y, acc[i][1]);
-          acc[i][2] = fmaf(xv, y.z, acc[i][2]);
-          acc[i][3] = fmaf(xv, y.w, acc[i][3]);
+      for (int e = 0; e < 4; ++e) {
+        const float4 y = *reinterpret_cast<const float4*>(B + (k + e) * ldb);
+#pragma unroll
+        for (int i = k / 8; i < 4; ++i) {
+          const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+          if (i > k / 8 || k % 8 + e <= row) {
+            sum[i][0] = fmaf(xv, y.x, sum[i][0]);
+            sum[i][1] = fmaf(xv, y.y, sum[i][1]);
+            sum[i][2] = fmaf(xv, y.z, sum[i][2]);
+            sum[i][3] = fmaf(xv, y.w, sum[i][3]);
+          }
         }
       }
     }
+    add16(acc, sum);
   }
 }
 
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
-  return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
+  return c + fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));     // a chain of sums of four
 }
 
 // X (lower triangular, [64][LC]) = (I + L)^-1, L strictly lower [64][LC]; tmp: 3 x 16 x 17 floats. Blocks of 16 on the diagonal
@@ -210,7 +225,7 @@ __device__ __forceinline__ void unit_lower_inverse(const float* L, float* X, flo
       for (int m = 0; m < SB * d; m += 4) {
         const float4 l = *reinterpret_cast<const float4*>(L + (I * SB + t) * LC + J * SB + m);
         const float* xc = X + (J * SB + m) * LC + J * SB + j;
-        y = fmaf(l.x, xc[0], y); y = fmaf(l.y, xc[LC], y); y = fmaf(l.z, xc[2 * LC], y); y = fmaf(l.w, xc[3 * LC], y);
+        y += fmaf(l.x, xc[0], fmaf(l.y, xc[LC], fmaf(l.z, xc[2 * LC], l.w * xc[3 * LC])));
       }
       tmp[(J * SB + t) * (SB + 1) + j] = y;
     }
@@ -316,21 +331,28 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_kernel(Args a) {
     const int r0 = (warp >> 1) * 16 + (lane >> 3), c0 = (warp & 1) * 32 + (lane & 7);
     float m[4][4] = {}, l[4][4] = {};
     if ((warp & 1) * 32 < (warp >> 1) * 16 + 16) {      // else wholly above the diagonal
-      for (int c = 0; c < D; c += 4) {
-        float4 q[4], k[4], kc[4];
+#pragma unroll 1
+      for (int cc = 0; cc < D; cc += 16) {
+        float mp[4][4] = {}, lp[4][4] = {};
+#pragma unroll 1
+        for (int c = cc; c < cc + 16; c += 4) {
+          float4 q[4], k[4], kc[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          q[i] = *reinterpret_cast<const float4*>(Q + (r0 + 4 * i) * LDD + c);
-          if (DELTA) k[i] = *reinterpret_cast<const float4*>(K + (r0 + 4 * i) * LDD + c);
-          kc[i] = *reinterpret_cast<const float4*>(K + (c0 + 8 * i) * LDD + c);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            m[i][j] = dot4(q[i], kc[j], m[i][j]);
-            if (DELTA) l[i][j] = dot4(k[i], kc[j], l[i][j]);
+          for (int i = 0; i < 4; ++i) {
+            q[i] = *reinterpret_cast<const float4*>(Q + (r0 + 4 * i) * LDD + c);
+            if (DELTA) k[i] = *reinterpret_cast<const float4*>(K + (r0 + 4 * i) * LDD + c);
+            kc[i] = *reinterpret_cast<const float4*>(K + (c0 + 8 * i) * LDD + c);
           }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              mp[i][j] = dot4(q[i], kc[j], mp[i][j]);
+              if (DELTA) lp[i][j] = dot4(k[i], kc[j], lp[i][j]);
+            }
+        }
+        add16(m, mp);
+        if (DELTA) add16(l, lp);
       }
     }
 #pragma unroll
@@ -438,16 +460,22 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_kernel(Args a) {
 #pragma unroll
     for (int I = 1; I < C / SB; ++I) {
       float m[C / SB - 1] = {}, l[C / SB - 1] = {};
-      for (int c = 0; c < D; c += 4) {
-        const float4 q = *reinterpret_cast<const float4*>(Q + (I * SB + t) * LDD + c);
-        float4 k;
-        if (DELTA) k = *reinterpret_cast<const float4*>(K + (I * SB + t) * LDD + c);
+      for (int c0 = 0; c0 < D; c0 += 16) {
+        float mp[C / SB - 1] = {}, lp[C / SB - 1] = {};
 #pragma unroll
-        for (int J = 0; J < I; ++J) {
-          const float4 x = *reinterpret_cast<const float4*>(A + (J * SB + j) * LDD + c);
-          m[J] = dot4(q, x, m[J]);
-          if (DELTA) l[J] = dot4(k, x, l[J]);
+        for (int c = c0; c < c0 + 16; c += 4) {
+          const float4 q = *reinterpret_cast<const float4*>(Q + (I * SB + t) * LDD + c);
+          float4 k;
+          if (DELTA) k = *reinterpret_cast<const float4*>(K + (I * SB + t) * LDD + c);
+#pragma unroll
+          for (int J = 0; J < I; ++J) {
+            const float4 x = *reinterpret_cast<const float4*>(A + (J * SB + j) * LDD + c);
+            mp[J] = dot4(q, x, mp[J]);
+            if (DELTA) lp[J] = dot4(k, x, lp[J]);
+          }
         }
+#pragma unroll
+        for (int J = 0; J < I; ++J) { m[J] += mp[J]; if (DELTA) l[J] += lp[J]; }
       }
 #pragma unroll
       for (int J = 0; J < I; ++J) {
@@ -724,7 +752,9 @@ __global__ void __launch_bounds__(THREADS, D == 64 ? 3 : 2) chunk_out_kernel(Arg
   if (ok0 && tile < tiles)
     triangle_product(acc, M + r * LC, LC, U + tile * C * 16 + c, 16, warp & 1, lane >> 2);
   if (!landed(&full[1], 0, &abort_flag, a.err, 43) || !ok0 || tile >= tiles) return;
-  tile_product<1>(acc, Q + r * LDD, LDD, S + tile * D * 16 + c, 16, D);
+  float from[4][4] = {};                                 // apart from M U: where the state is small its parts would each round the whole sum
+  tile_product(from, Q + r * LDD, LDD, S + tile * D * 16 + c, 16, D);
+  add16(acc, from);
   const float skip = a.skip ? a.skip[h] : 0.f;
   const TI* vg = reinterpret_cast<const TI*>(a.v) + (long long)h * V + v0 + tile * 16 + c;
 #pragma unroll

@@ -200,3 +200,31 @@ def test_rows_that_the_chunks_cannot_read(pad, off):
     same = (torch.equal(got, passes), torch.equal(got, rows))
     assert same == ((False, False) if pad % 4 == off % 4 == 0 else (True, False)) and torch.equal(state[0], state[1]) == same[0]
     assert rel(got, rows.double()) < 2e-6
+
+
+@pytest.mark.parametrize("kind", ["channel", "head", "plain", "gla"])
+@pytest.mark.parametrize("slow", [True, False])
+def test_no_further_from_64_bits_than_row_by_row(kind, slow):
+    """Roundings at random add up like the root of the links of a chain; both forms' chains have some 16 to 20 links."""
+    from rllm_b200.kernels import hybrid, mix
+    H, dim, T = 4, 128, 1024
+    cu, cud = layout((T,))
+    slots = torch.zeros(1, dtype=torch.int32, device=DEV)
+    unit = lambda seed: torch.nn.functional.normalize(rnd(T, H, dim, seed=seed), dim=-1)
+    q, k, v = (x.view(T, H * dim) for x in (unit(1), unit(2), rnd(T, H, dim, seed=3)))
+    u = torch.rand(T, H, dim if kind in ("channel", "gla") else 1, generator=torch.Generator().manual_seed(4)).to(DEV)
+    a = torch.exp(-0.01 * u) if slow else u
+    beta = rnd(T, H, seed=5) if kind in ("channel", "head") else None
+    if kind == "gla":
+        proj = torch.cat([q, k, v], 1).bfloat16()
+        q, k, v = (x.contiguous() for x in proj.float().split(H * dim, 1))
+        run = lambda kw: mix.gla_scan(proj, 0, H * dim, 2 * H * dim, a.view(T, -1), 1.0, H, dim, dim, cud, 1, slots,
+                                      torch.zeros(1, H, dim, dim, device=DEV), **kw)
+    else:
+        run = lambda kw: hybrid.state_scan(q, H, k, H, v, a.view(T, -1), H, dim, dim, cud, 1, slots,
+                                           torch.zeros(1, H, dim, dim, device=DEV), beta=beta, **kw)
+    d = lambda x: x.double().view(T, H, -1)
+    want, _ = recurrence(d(q), d(k), d(v), a.double(), torch.zeros(H, dim, dim, dtype=torch.float64, device=DEV),
+                         torch.sigmoid(beta.double()) if beta is not None else None)
+    rows, chunks = rel(run({}), want), rel(run(dict(long_from=64, any_short=False, err=ERR())), want)
+    assert chunks < 1.2 * rows, (chunks, rows)
