@@ -43,6 +43,14 @@ def _nbytes(*tensors) -> int:
     return sum(t.numel() * t.element_size() for t in tensors if isinstance(t, torch.Tensor))
 
 
+def _visible(q: int, n: int, window: int | None) -> int:
+    """Pairs of a query and a key it sees: the last q of n positions, each with itself and the window - 1 before it (None: all)."""
+    if not window or window >= n:
+        return q * (n - q) + q * (q + 1) // 2
+    short = max(0, min(q, window - (n - q)))          # rows that see every position up to their own, fewer than a window
+    return short * (n - q) + short * (short + 1) // 2 + (q - short) * window
+
+
 class OpProfile:
     """Wraps a `Backend`: the same methods, each timed under a class name."""
 
@@ -238,20 +246,28 @@ class OpProfile:
     def latent_prepare(self, proj, *a, **k):
         return self._timed("latent_prepare", 2 * _nbytes(proj), 0, self._be.latent_prepare, proj, *a, **k)
 
+    def latent_expand(self, cache, ctx, w_ukv, rank, long):
+        rows, row = long[1], 2 * cache.tensors["kv"].shape[2]
+        # gathered (read, written), read by the product; the weights; what comes out
+        return self._timed("latent_expand", rows * (2 * row + 2 * rank + 2 * w_ukv.shape[0]) + _nbytes(w_ukv), 2 * rows * w_ukv.numel(),
+                           self._be.latent_expand, cache, ctx, w_ukv, rank, long)
+
     def latent_attention_expanded(self, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, *a):
         lens = [(n, L) for n, L in zip(ctx.q_lens_host, ctx.kv_lens_host) if n >= long[0]]
-        pairs = sum(n * ((min(L, window + n - 1) if window else L) - n) + n * (n + 1) // 2 for n, L in lens)
-        return self._timed("latent_attention", long[1] * (rank + rot) * 2 + _nbytes(q), 2 * heads * (dim + rot + 128) * pairs,
+        pairs = sum(_visible(n, L, window) for n, L in lens)
+        nbytes = sum(_nbytes(t) for t in expanded) + sum(n for n, _ in lens) * heads * (dim + rot + 128) * 2
+        return self._timed("latent_attention", nbytes, 2 * heads * (dim + rot + 128) * pairs,
                            self._be.latent_attention_expanded, q, qfull, expanded, ctx, heads, dim, rot, rank, scale, window, long, *a)
 
     def latent_attention(self, qfull, cache, ctx, rank, scale, window, skip_from=0, num_seqs=None):
-        T, H, dk = qfull.shape
+        _, H, dk = qfull.shape
         lens, qs = ctx.kv_lens_host, ctx.q_lens_host
         if lens is None:
             lens, qs = [ctx.max_kv_len] * ctx.num_seqs, [1] * ctx.num_seqs
-        seen = [min(L, window + q - 1) if window else L for L, q in zip(lens, qs)]
-        pairs = sum(q * (s - q) + q * (q + 1) // 2 for s, q in zip(seen, qs))
-        nbytes = sum(seen) * dk * qfull.element_size() + _nbytes(qfull) + T * H * rank * qfull.element_size()
+        mine = [(L, q) for L, q in list(zip(lens, qs))[:num_seqs] if not skip_from or q < skip_from]      # the others are left out
+        pairs = sum(_visible(q, L, window) for L, q in mine)
+        seen = sum(min(L, window + q - 1) if window else L for L, q in mine)
+        nbytes = (seen * dk + sum(q for _, q in mine) * H * (dk + rank)) * qfull.element_size()
         return self._timed("latent_attention", nbytes, 2 * H * (dk + rank) * pairs, self._be.latent_attention,
                            qfull, cache, ctx, rank, scale, window, skip_from, num_seqs)
 

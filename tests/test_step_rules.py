@@ -94,3 +94,27 @@ def test_scratch_that_did_not_fit_is_not_asked_for_again(monkeypatch):
     be._or_none = lambda *a: Backend._or_none(be, *a)
     got = [Backend.scratch(be, n, "cpu") for n in (50, 400, 500, 400, 200, 300, 100, 200)]
     assert got == [50, None, None, None, None, None, 100, None] and asked == [50, 400, 200, 100]
+
+
+def test_profile_counts_a_portion_once():
+    """Rows over the latents, expansion and attention over what it made: every pair of query and key in one line."""
+    import torch
+    from rllm_b200.kernels import profile
+    lens, window, heads, rank, rot = [(1, 500), (300, 700), (3, 40), (64, 64)], 100, 4, 64, 64
+    for q, n in lens:
+        for w in (None, 1, 30, 100, 500, 5000):
+            assert profile._visible(q, n, w) == sum(min(p + 1, w or p + 1) for p in range(n - q, n))
+    ctx, lines = step(lens), []
+    prof = profile.OpProfile.__new__(profile.OpProfile)
+    prof._be = SimpleNamespace(latent_attention=None, latent_attention_expanded=None, latent_expand=None)
+    prof._timed = lambda cls, nbytes, flops, fn, *a, **k: lines.append((cls, nbytes, flops))
+    bf = lambda *s: torch.empty(s, dtype=torch.bfloat16)
+    pairs = {s: profile._visible(*lens[s], window) for s in range(4)}
+    long, rows = (32, 764, (304, 3)), 764
+    prof.latent_expand(SimpleNamespace(tensors={"kv": bf(9, 16, rank + rot)}), ctx, bf(heads * 256, rank), rank, long)
+    prof.latent_attention(bf(304, heads, rank + rot), None, ctx, rank, 0.1, window, 32, 3)
+    prof.latent_attention_expanded(None, None, (bf(rows, rank + rot), bf(rows, heads * 256)), ctx, heads, 128, rot, rank, 0.1, window, long)
+    assert [f for _, _, f in lines] == [2 * rows * heads * 256 * rank, 2 * heads * (2 * rank + rot) * (pairs[0] + pairs[2]),
+                                        2 * heads * (128 + rot + 128) * (pairs[1] + pairs[3])]
+    assert lines[1][1] == 2 * ((100 + 40) * (rank + rot) + 4 * heads * (2 * rank + rot))
+    assert lines[2][1] == 2 * (rows * (rank + rot + heads * 256) + 364 * heads * (128 + rot + 128))
