@@ -78,10 +78,15 @@ class LatentAttention(Part):
 
     def finalize(self, device, dtype):
         H = self.heads
+        # every head's keys and values out of a latent, where long portions may want them (`Backend.latent_expanded`): the two
+        # weights under each other, of which they are views from then on
+        self._ukv = None
+        if dtype == torch.bfloat16 and self.dim == self.vdim == 128 and self.rot_dim in (0, 64) and self.kv_rank % 64 == 0:
+            self._ukv = torch.cat([self.w_uk, self.w_uv], 0)
+            self.w_uk, self.w_uv = self._ukv.split([H * self.dim, H * self.vdim], 0)
         # per head: [kv_rank, dim] so that the fold is a product with K = dim; [vdim, kv_rank] as stored
         self._uk_t = self.w_uk.view(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
         self._uv = self.w_uv.view(H, self.vdim, self.kv_rank)
-        self._ukv = torch.cat([self.w_uk, self.w_uv], 0)          # every head's keys and values out of a latent
         self._norm_f32 = self.w_latent_norm.float().contiguous()
         self._q_norm_f32 = None if self.w_q_norm is None else self.w_q_norm.float().contiguous()
 

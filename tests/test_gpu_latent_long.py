@@ -142,3 +142,18 @@ def test_no_room_for_the_forms_that_take_scratch():
                                                 state[1])) and torch.equal(*state)
     hs.engine.end(["a", "b"])
     assert hs.run([("c", 300)], scan)
+
+
+@pytest.mark.parametrize("dtype,heads,vdim,kept", [("bfloat16", 4, 128, True), ("bfloat16", 4, 64, False), ("float32", 4, 128, False)])
+def test_weights_are_kept_once(dtype, heads, vdim, kept):
+    """Keys' and values' weights under each other are the weights themselves, and are not made where nothing reads them."""
+    from rllm_b200.parts import InterleavedRotary, LatentAttention
+    m = ZK.latent(heads, 128, 64, vdim, 64, 0.1, 10000.0, 64, None)
+    part = LatentAttention(W, heads, 128, 64, vdim, 64, 0.1, InterleavedRotary(64, 10000.0, 64))
+    w = latent_weights(W, m, seed=3)
+    bind(part, w, dtype, "x.")
+    assert (part._ukv is not None) == kept
+    for got, name in ((part.w_uk, "x.uk"), (part.w_uv, "x.uv")):
+        assert torch.equal(got.cpu(), w[name].to(DT[dtype])) and got.is_contiguous()
+        assert not kept or got.untyped_storage().data_ptr() == part._ukv.untyped_storage().data_ptr()
+    assert part._uv.data_ptr() == part.w_uv.data_ptr()
