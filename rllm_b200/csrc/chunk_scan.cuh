@@ -96,16 +96,21 @@ __device__ __forceinline__ void bulk(float* smem, const float* gmem, int n, uint
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm100::smem_u32(smem)),
                "l"(gmem), "r"(4 * n), "r"(sm100::smem_u32(bar)) : "memory");
 }
-// All threads wait for a barrier's phase. A wait that runs out leaves its mark, waits once more (a copy may still be on its way
-// into this CTA's memory) and ends the CTA's work.
-__device__ __forceinline__ bool landed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err, int role) {
-  bool ok = sm100::mbar_wait(bar, parity, abort_flag);
-  if (!ok) {
-    *abort_flag = 1;
-    sm100::record_failure(err, role);
-    volatile int none = 0;
-    sm100::mbar_wait(bar, parity, &none);
-  }
+// A wait has run out: it leaves its mark and waits once more for the copies that may still be on their way into this CTA's memory,
+// this one and the one after (null: none). Out of line, so that the walk's code is not arranged around it.
+__device__ __noinline__ void give_up(uint64_t* bar, uint32_t parity, uint64_t* next, uint32_t next_parity, volatile int* abort_flag,
+                                     int* err, int role) {
+  *abort_flag = 1;
+  sm100::record_failure(err, role);
+  volatile int none = 0;
+  sm100::mbar_wait(bar, parity, &none);
+  if (next) sm100::mbar_wait(next, next_parity, &none);
+}
+// All threads wait for a barrier's phase; false: some wait ran out, and the CTA's work ends.
+__device__ __forceinline__ bool landed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err, int role,
+                                       uint64_t* next = nullptr, uint32_t next_parity = 0) {
+  const bool ok = sm100::mbar_wait(bar, parity, abort_flag);
+  if (!ok) give_up(bar, parity, next, next_parity, abort_flag, err, role);
   return __syncthreads_and(ok);
 }
 
@@ -620,7 +625,8 @@ __global__ void __launch_bounds__(THREADS) chunk_carry_kernel(Args a) {
     const float* ps = us + C * NC;
     for (int x = tid; x < D * (NC / 4); x += THREADS)    // the state that the chunk meets
       *reinterpret_cast<float4*>(in.s + (long long)(v0 / 16) * D * 16 + 4 * x) = *reinterpret_cast<const float4*>(S + 4 * x);
-    if (!landed(&full[ci & 1], (uint32_t)(ci >> 1) & 1u, &abort_flag, a.err, 41)) return;
+    if (!landed(&full[ci & 1], (uint32_t)(ci >> 1) & 1u, &abort_flag, a.err, 41, ci + 1 < chunks ? &full[(ci + 1) & 1] : nullptr,
+                (uint32_t)((ci + 1) >> 1) & 1u)) return;
     if (DELTA) {
       const int r = (warp & 1) * 32 + (lane >> 2), k0 = (warp >> 1) * (D / 4);
       float acc[NT][4][4] = {};
