@@ -591,7 +591,6 @@ latent_attention_few_kernel(const bf16* __restrict__ qfull, const bf16* __restri
   }
 }
 
-// The splits' parts of every row, merged in split order: out = sum_s e^(m_s - M) acc_s / sum_s e^(m_s - M) l_s.
 // A warp a cached position of the sequences of at least `long_from` rows: their rows one after the other, sequence by sequence
 // in order (pages given back: zeros). Pieces of 16 bytes; grid.x covers the longest sequence, grid.y the sequences.
 __global__ void __launch_bounds__(256)
@@ -612,6 +611,7 @@ latent_gather_kernel(const uint4* __restrict__ cache, const int* __restrict__ bl
   for (int i = lane; i < pieces; i += 32) dst[i] = page < 0 ? make_uint4(0, 0, 0, 0) : src[i];
 }
 
+// The splits' parts of every row, merged in split order: out = sum_s e^(m_s - M) acc_s / sum_s e^(m_s - M) l_s.
 // grid.x: the row tiles (of `qrows` rows) as in the kernel that left the parts; grid.y: blocks of 32 columns; a
 // warp takes rows, its lanes the columns, all splits' values asked for at once.
 __global__ void __launch_bounds__(256)

@@ -16,8 +16,10 @@
 //   A thread owns a value column and every `split`-th key channel (`split` neighbouring lanes share a column and
 //   join their sums by shuffles); it keeps its share of S in registers while it walks the sequence's tokens, a few
 //   at a time through shared memory. The order of every sum depends on the sizes only, so a position's result is
-//   the same bits however its tokens were cut into steps. Queries and keys may be shared by groups of heads.
-//   Where the caller says so (`long_from`), sequences of at least that many rows run in chunks instead (chunk_scan.cuh).
+//   the same bits however its tokens were cut into steps (the 32-bit run). Queries and keys may be shared by groups of heads.
+//   Where the caller says so (`long_from`, bfloat16 runs), sequences of at least that many rows run in chunks instead
+//   (chunk_scan.cuh), with sums in another order: a position's bits then depend on the cut, and on the portions of other
+//   requests in the step, by whose lengths and number the caller decides.
 // gated_norm: per (token, group of columns) y / sqrt(mean(y^2) + eps) * w, with a gate act(g) applied to y before
 //   the norm or to the result after it; act silu or sigmoid.
 #include "common.cuh"
