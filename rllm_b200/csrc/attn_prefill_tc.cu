@@ -417,7 +417,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     } else if (warp == 2) {
       // (Q comes from the softmax warps, each thread its own row: one warp fetching a row tile spent 5 us
       // of every item on the addresses of its 1,024 copies)
-      if (lane == 0 && n_steps > 0) {
+      if (elect_one() && n_steps > 0) {
         // ... and warp 2 then issues the S products, as far ahead as accumulators are free
         bool ok = true;
         if (!mbar_wait(&q_full, 0u, &abort_flag)) { abort_flag = 1; record_failure(p.err, 27, 0); ok = false; }
@@ -476,7 +476,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------ the PV products (one thread); without
     // TMA the loaders are all busy and this thread issues S as well, three steps ahead
-    if (lane == 0 && n_tiles > 0) {
+    if (elect_one() && n_tiles > 0) {
       bool ok = true;
       if (!TMA)
         for (int k = 0; k < SB && k < n_steps && ok; ++k) issue_s(k, ok);

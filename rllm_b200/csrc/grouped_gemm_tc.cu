@@ -79,7 +79,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   const uint32_t tmem_base = tmem_base_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int i = 0; i < n_kb; ++i) {
         const int s = i % STAGES;
@@ -100,7 +100,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(TM, TN);
       const uint64_t d0 = umma_desc_sw128(smem_u32(smem));
       bool ok = true;

@@ -13,6 +13,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// One thread of a converged warp, the same one every time. A role that issues tensor copies, MMAs or commits is guarded by this and
+// not by `lane == 0`: the compiler then knows that one thread runs, where it otherwise makes these instructions, which take
+// their operands from uniform registers, ready for any number of threads. A block of four MMAs and a commit cost its
+// thread 540 cycles behind `lane == 0` and 295 behind this (products on pairs of CTAs, stamps in a copy of the kernel).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -41,11 +51,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Waits for the phase with the given parity, at most ~`limit_cycles` clock cycles, and gives
 // up early when `*abort_flag` (shared memory) is set by another role of the same CTA.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           long long limit_cycles = 4000000000LL) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_test_wait(bar, parity)) return true;       // 13 cycles where the phase is complete, try_wait 55
   const long long t0 = clock64();
   int spins = 0;
   while (!mbar_try_wait(bar, parity)) {

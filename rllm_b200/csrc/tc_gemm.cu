@@ -68,9 +68,8 @@ enum : int { EPI_STORE = 0, EPI_STORE_F32 = 1, EPI_ACCUM_F32 = 2, EPI_SWIGLU = 3
 constexpr int BM = 128;        // weight rows per tile (MMA M)
 constexpr int BK = 64;         // K per stage: 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 192;   // warp 0 TMA, warp 1 MMA + TMEM, warps 2..5 epilogue
-constexpr int THREADS_SMALL = 224;   // the small-tile kernel has a second MMA warp (6)
-constexpr int THREADS_MANY = 320;    // the persistent kernel has eight epilogue warps (2..9), two on each quarter of the rows
+constexpr int THREADS_SMALL = 224;   // warp 0 TMA, warp 1 MMA + TMEM, warps 2..5 epilogue, warp 6 a second MMA warp
+constexpr int THREADS_MANY = 320;    // the persistent kernels have eight epilogue warps (2..9), two on each quarter of the rows
 constexpr int MAX_CLUSTER = 8;
 // shared memory of a small-tile CTA in KB: 84 + 138 (gate/up pair) = 222 KB, so that any two
 // small-tile kernels of a layer fit one SM together (measured: worth 20 % of a step of 9 to 64 tokens)
@@ -312,7 +311,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol_w = policy_evict_first();   // weights are read once per step
       const uint64_t pol_x = policy_evict_last();    // the token tile is shared by every weight tile
       const int x0 = p.x_rows ? n0 / p.x_rows * p.x_gs : 0;
@@ -357,7 +356,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     // tile of 16 or 32 needs five of them (nine with a gate/up pair) for every K block: one thread
     // would hold the weight stream at about 60 GB/s per SM. With an even number of stages two
     // threads (warps 1 and 6) take the K blocks in turn; the epilogue adds their accumulator sets.
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
       constexpr int STEP = C::TWO ? 2 : 1;
       const int w = warp == 1 ? 0 : 1;
@@ -731,6 +730,217 @@ template <int BN, bool DUAL, int WR = BM> struct PCfg {
   static_assert(2 * ACC_COLS <= 512, "two accumulator sets must fit in TMEM");
 };
 
+// One tile's accumulator set, from TMEM to the output, by eight warps (2..9): `taddr` is this warp's quarter of the set. A warp
+// reads the TMEM lanes of its quarter (warp % 4); the two warps of a quarter take half of the token columns each. One warp on
+// a scheduler waits out every instruction's latency alone, so an epilogue's time goes with the instructions per warp, and
+// the last tile's epilogue is not hidden by a mainloop. xch, tok_off: see the rotary epilogue.
+constexpr int XS = BM + 4;
+template <int BN, int EPI, bool SWAP, int WR>
+__device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t taddr, int bn, int t0, int n0, int warp, int lane,
+                                              float* xch, long long* tok_off) {
+  constexpr bool DUAL = (EPI == EPI_SWIGLU);
+  constexpr bool ROPE = (EPI == EPI_QKV_ROPE);
+  const int row = (warp & 3) * 32 + lane;
+  const int grp = (warp - 2) >> 2;
+  const int n = n0 + row;
+  if (SWAP) {
+    // this thread's row is a token; its gate values are columns 0..WR-1, its up values WR..2 WR-1. The
+    // first warp of a quarter takes the lower half of the features, the second the upper, 32 at a
+    // time, and writes them as 16-byte pieces of the token's output row.
+    const int t = t0 + row;
+    bf16* crow = (bf16*)p.C + (size_t)t * p.ldc + n0;
+#pragma unroll 1
+    for (int c0 = grp * (WR / 2); c0 < grp * (WR / 2) + WR / 2; c0 += 32) {
+      if (n0 + c0 >= p.N) break;
+      uint32_t g[32], u[32];
+      tmem_ld32(taddr + c0, g);
+      tmem_ld32(taddr + WR + c0, u);
+      tmem_ld_wait();
+      if (t < p.T) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (n0 + c0 + 8 * q >= p.N) break;
+          float h[8];                                         // float, rounded once to bfloat16
+          if (p.act == 2) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float gv = __uint_as_float(g[8 * q + e]);
+              h[e] = gelu_gate(gv) * __uint_as_float(u[8 * q + e]);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float gv = __uint_as_float(g[8 * q + e]);
+              h[e] = __fdividef(gv, 1.f + __expf(-gv)) * __uint_as_float(u[8 * q + e]);
+            }
+          }
+          uint4 pk;
+          pk.x = pack_bf16x2(h[0], h[1]); pk.y = pack_bf16x2(h[2], h[3]);
+          pk.z = pack_bf16x2(h[4], h[5]); pk.w = pack_bf16x2(h[6], h[7]);
+          *reinterpret_cast<uint4*>(crow + c0 + 8 * q) = pk;
+        }
+      }
+    }
+  } else if (ROPE) {
+    // Rotation needs a row's pair partner, which lies half a head away in another warp's TMEM lanes, and
+    // with one warp on each scheduler an epilogue is bound by the instructions it issues. So 32 token
+    // columns at a time go through shared memory ([token][row], rows padded by 4 against bank
+    // conflicts), and from there each of the 256 threads takes, for one token, two groups of 8
+    // neighbouring rows: values, partners and angles as 16-byte loads, the rotated result as one
+    // 16-byte store into C and one into the cache.
+    // (a row's place in the buffer has bit 2 flipped in the upper half of each 64 rows, so that the
+    // eight threads of a 16-byte read, 8 rows apart, meet 32 different banks)
+    auto xrow = [](int r_) { return r_ ^ (((r_ >> 5) & 1) << 2); };
+    const RopeArgs& r = p.rope;
+    const int et = (warp - 2) * 32 + lane, tt = et >> 3, q8 = (et & 7) * 8;
+    const int half = r.rot_dim >> 1;
+    bool g_turn[2], g_low[2], g_live[2];
+    int g_fi[2], g_part[2];
+    bf16* g_cache[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int rb = q8 + 64 * k, nn = n0 + rb;
+      const int head = nn / r.hd, d = nn - head * r.hd;
+      g_live[k] = nn < p.N;
+      g_turn[k] = g_live[k] && head < r.nh + r.nkv && d < r.rot_dim;
+      g_low[k] = d < half;
+      g_fi[k] = g_low[k] ? d : d - half;
+      g_part[k] = g_turn[k] ? (g_low[k] ? rb + half : rb - half) : rb;
+      const bool is_k = head < r.nh + r.nkv;
+      g_cache[k] = (g_live[k] && head >= r.nh && r.slots != nullptr)
+          ? (is_k ? r.kcache : r.vcache) + (size_t)(head - r.nh - (is_k ? 0 : r.nkv)) * r.page_size * r.hd + d : nullptr;
+    }
+    // where each token of the tile starts in a cache (elements; -1: not written), once for all rows
+    if (r.slots != nullptr) {
+      for (int c = et; c < bn; c += 256) {
+        const int t = t0 + c;
+        const int slot = t < p.T ? r.slots[t] : -1;
+        tok_off[c] = slot >= 0 ? ((long long)(slot / r.page_size) * r.nkv * r.page_size + slot % r.page_size) * r.hd : -1ll;
+      }
+    }
+    // This thread's angles are asked for one chunk ahead, all at once: they come from L2, which is
+    // busy with the operands, and a chunk that waited for its own would wait about as long again
+    // as it works.
+    float4 ang[2][4], ang_next[2][4];
+    auto ask_angles = [&](int c0, float4 (&a)[2][4]) {
+      if (r.cos_sin == nullptr || t0 + c0 >= p.T) return;
+      const float2* trow = r.cos_sin + (size_t)min(t0 + c0 + tt, p.T - 1) * half;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (g_turn[k]) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[k][i] = __ldg(reinterpret_cast<const float4*>(trow + g_fi[k]) + i);
+        }
+      }
+    };
+    ask_angles(0, ang_next);
+#pragma unroll 1
+    for (int c0 = 0; c0 < bn; c0 += 32) {
+      if (t0 + c0 >= p.T) break;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ang[k][i] = ang_next[k][i];
+      if (c0 + 32 < bn) ask_angles(c0 + 32, ang_next);
+      {
+        uint32_t g[16];                               // 16 of the 32 columns from each warp of a quarter
+        tmem_ld16(taddr + c0 + 16 * grp, g);
+        tmem_ld_wait();
+#pragma unroll
+        for (int jj = 0; jj < 16; ++jj) xch[(16 * grp + jj) * XS + xrow(row)] = __uint_as_float(g[jj]);
+      }
+      epilogue8_sync();
+      const int t = t0 + c0 + tt;
+      if (t < p.T && c0 + tt < bn) {
+        const float* xr = xch + tt * XS;
+        const long long coff = r.slots != nullptr ? tok_off[c0 + tt] : -1ll;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (!g_live[k]) continue;
+          const float4 v0 = *reinterpret_cast<const float4*>(xr + xrow(q8 + 64 * k));
+          const float4 v1 = *reinterpret_cast<const float4*>(xr + xrow(q8 + 64 * k + 4));
+          float o[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+          if (g_turn[k]) {
+            const float4 w0 = *reinterpret_cast<const float4*>(xr + xrow(g_part[k]));
+            const float4 w1 = *reinterpret_cast<const float4*>(xr + xrow(g_part[k] + 4));
+            const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            float cs[8], sn[8];
+            if (r.cos_sin != nullptr) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float4 a = ang[k][i];
+                cs[2 * i] = a.x; sn[2 * i] = a.y; cs[2 * i + 1] = a.z; sn[2 * i + 1] = a.w;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) { const float2 a = angle_of(r, t, g_fi[k] + i); cs[i] = a.x; sn[i] = a.y; }   // no table given
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = g_low[k] ? o[i] * cs[i] - w[i] * sn[i] : w[i] * sn[i] + o[i] * cs[i];
+          }
+          uint4 pk;
+          pk.x = pack_bf16x2(o[0], o[1]); pk.y = pack_bf16x2(o[2], o[3]);
+          pk.z = pack_bf16x2(o[4], o[5]); pk.w = pack_bf16x2(o[6], o[7]);
+          *reinterpret_cast<uint4*>((bf16*)p.C + (size_t)t * p.ldc + n0 + q8 + 64 * k) = pk;
+          if (g_cache[k] != nullptr && coff >= 0) *reinterpret_cast<uint4*>(g_cache[k] + coff) = pk;
+        }
+      }
+      epilogue8_sync();                               // all have read before the next 32 columns come in
+    }
+  } else {
+    // The tile leaves TMEM 64 token columns at a time (32 of each half of a gate/up pair): a load from
+    // TMEM and the wait for it are a round trip of their own, and sixteen of them for a tile of 256
+    // columns were most of what the epilogue took. The residual values of the same columns are
+    // fetched while the accumulator values are on their way.
+    // (with ten warps a thread has 168 registers: the residual's 64 beside the accumulator's 64 would spill)
+    constexpr int CW = (DUAL || BN < 128 || EPI == EPI_ACCUM_F32) ? 32 : 64;
+    float* cbase = (float*)p.C + (size_t)t0 * p.ldc + n;
+    // the first warp of a quarter takes the columns up to `mid` (a multiple of 32), the second the rest;
+    // `lim`: columns of this warp that are tokens of the tile and of the step
+    const int mid = ((bn / 2 + 31) / 32) * 32;
+    const int c_begin = grp == 0 ? 0 : mid;
+    const int lim = min(grp == 0 ? mid : bn, p.T - t0);
+#pragma unroll 1
+    for (int c0 = c_begin; c0 < lim; c0 += CW) {
+      uint32_t g[CW], u[DUAL ? CW : 1];
+      float r[EPI == EPI_ACCUM_F32 ? CW : 1];
+      if (DUAL) {
+        tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
+        tmem_ld32(taddr + BN + c0, reinterpret_cast<uint32_t(&)[32]>(u));
+      } else if (CW == 32) {
+        tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
+      } else {
+        tmem_ld64(taddr + c0, reinterpret_cast<uint32_t(&)[64]>(g));
+      }
+      if (EPI == EPI_ACCUM_F32 && n < p.N) {
+        const float* cp = cbase + (size_t)c0 * p.ldc;
+#pragma unroll
+        for (int jj = 0; jj < CW; ++jj) r[jj] = (c0 + jj < lim) ? __ldcg(cp + (size_t)jj * p.ldc) : 0.f;
+      }
+      tmem_ld_wait();
+      if (n < p.N) {
+        if (EPI == EPI_ACCUM_F32) {
+          float* cp = cbase + (size_t)c0 * p.ldc;
+#pragma unroll
+          for (int jj = 0; jj < CW; ++jj)
+            if (c0 + jj < lim) cp[(size_t)jj * p.ldc] = r[jj] + __uint_as_float(g[jj]);
+        } else if (EPI == EPI_STORE) {
+          bf16* cp = (bf16*)p.C + (size_t)(t0 + c0) * p.ldc + n;
+          store_act_all(p, g);
+#pragma unroll
+          for (int jj = 0; jj < CW; ++jj, cp += p.ldc)
+            if (c0 + jj < lim) *cp = __float2bfloat16_rn(__uint_as_float(g[jj]));
+        } else {
+#pragma unroll
+          for (int jj = 0; jj < CW; ++jj) {
+            if (c0 + jj < lim) emit<EPI>(p, t0 + c0 + jj, n, __uint_as_float(g[jj]), DUAL ? __uint_as_float(u[jj]) : 0.f);
+          }
+        }
+      }
+    }
+  }
+}
+
 template <int BN, int EPI, bool SWAP, int WR = BM>
 __global__ void __launch_bounds__(THREADS_MANY, 1)
 tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -750,7 +960,6 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
   __shared__ int never_flag;
   // rotary epilogue: a row's pair partner lies 16+ rows away, in another warp's TMEM lanes; the
   // epilogue warps pass 32 columns at a time through this buffer
-  constexpr int XS = BM + 4;
   __shared__ __align__(16) float xch[ROPE ? 32 * XS : 4];
   __shared__ long long tok_off[ROPE ? BN : 1];
   __shared__ int epi_fail;
@@ -780,7 +989,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol_x = policy_evict_last();    // the token tiles are read by every weight tile
       pdl_wait();                                    // activations come from the kernel before
       int it = 0, issued = 0;
@@ -810,7 +1019,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // SWAP: the 128 tokens are the rows and the tile's 128 (64) gate and 128 (64) up weight rows, which
       // lie one after the other in a stage, the 256 (128) columns of one product
       const uint32_t idesc = SWAP ? umma_idesc_bf16(BM, 2 * WR) : umma_idesc_bf16(BM, bn);
@@ -849,18 +1058,12 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue warps (2..9): a warp reads the
-    // TMEM lanes of its quarter (warp % 4); the two warps of a quarter take half of the token columns
-    // each. One warp on a scheduler waits out every instruction's latency alone, so an epilogue's time
-    // goes with the instructions per warp, and the last tile's epilogue is not hidden by a mainloop.
-    const int row = (warp & 3) * 32 + lane;
-    const int grp = (warp - 2) >> 2;
+    // ------------------------------------------------------------ epilogue warps (2..9)
     pdl_wait();
     int ti = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++ti) {
       const int t0 = (tile % t_tiles) * bn, n0 = (tile / t_tiles) * WR;
-      const int n = n0 + row;
       const int buf = ti & 1, use = ti >> 1;
       ok = mbar_wait(&acc_full[buf], (uint32_t)use & 1u, &abort_flag);
       if (!ok) { abort_flag = 1; record_failure(p.err, 3); }
@@ -873,202 +1076,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(buf * C::ACC_COLS);
-      if (SWAP) {
-        // this thread's row is a token; its gate values are columns 0..WR-1, its up values WR..2 WR-1. The
-        // first warp of a quarter takes the lower half of the features, the second the upper, 32 at a
-        // time, and writes them as 16-byte pieces of the token's output row.
-        const int t = t0 + row;
-        bf16* crow = (bf16*)p.C + (size_t)t * p.ldc + n0;
-#pragma unroll 1
-        for (int c0 = grp * (WR / 2); c0 < grp * (WR / 2) + WR / 2; c0 += 32) {
-          if (n0 + c0 >= p.N) break;
-          uint32_t g[32], u[32];
-          tmem_ld32(taddr + c0, g);
-          tmem_ld32(taddr + WR + c0, u);
-          tmem_ld_wait();
-          if (t < p.T) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if (n0 + c0 + 8 * q >= p.N) break;
-              float h[8];                                         // float, rounded once to bfloat16
-              if (p.act == 2) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  const float gv = __uint_as_float(g[8 * q + e]);
-                  h[e] = gelu_gate(gv) * __uint_as_float(u[8 * q + e]);
-                }
-              } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  const float gv = __uint_as_float(g[8 * q + e]);
-                  h[e] = __fdividef(gv, 1.f + __expf(-gv)) * __uint_as_float(u[8 * q + e]);
-                }
-              }
-              uint4 pk;
-              pk.x = pack_bf16x2(h[0], h[1]); pk.y = pack_bf16x2(h[2], h[3]);
-              pk.z = pack_bf16x2(h[4], h[5]); pk.w = pack_bf16x2(h[6], h[7]);
-              *reinterpret_cast<uint4*>(crow + c0 + 8 * q) = pk;
-            }
-          }
-        }
-      } else if (ROPE) {
-        // Rotation needs a row's pair partner, which lies half a head away in another warp's TMEM lanes, and
-        // with one warp on each scheduler an epilogue is bound by the instructions it issues. So 32 token
-        // columns at a time go through shared memory ([token][row], rows padded by 4 against bank
-        // conflicts), and from there each of the 256 threads takes, for one token, two groups of 8
-        // neighbouring rows: values, partners and angles as 16-byte loads, the rotated result as one
-        // 16-byte store into C and one into the cache.
-        // (a row's place in the buffer has bit 2 flipped in the upper half of each 64 rows, so that the
-        // eight threads of a 16-byte read, 8 rows apart, meet 32 different banks)
-        auto xrow = [](int r_) { return r_ ^ (((r_ >> 5) & 1) << 2); };
-        const RopeArgs& r = p.rope;
-        const int et = (warp - 2) * 32 + lane, tt = et >> 3, q8 = (et & 7) * 8;
-        const int half = r.rot_dim >> 1;
-        bool g_turn[2], g_low[2], g_live[2];
-        int g_fi[2], g_part[2];
-        bf16* g_cache[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const int rb = q8 + 64 * k, nn = n0 + rb;
-          const int head = nn / r.hd, d = nn - head * r.hd;
-          g_live[k] = nn < p.N;
-          g_turn[k] = g_live[k] && head < r.nh + r.nkv && d < r.rot_dim;
-          g_low[k] = d < half;
-          g_fi[k] = g_low[k] ? d : d - half;
-          g_part[k] = g_turn[k] ? (g_low[k] ? rb + half : rb - half) : rb;
-          const bool is_k = head < r.nh + r.nkv;
-          g_cache[k] = (g_live[k] && head >= r.nh && r.slots != nullptr)
-              ? (is_k ? r.kcache : r.vcache) + (size_t)(head - r.nh - (is_k ? 0 : r.nkv)) * r.page_size * r.hd + d : nullptr;
-        }
-        // where each token of the tile starts in a cache (elements; -1: not written), once for all rows
-        if (r.slots != nullptr) {
-          for (int c = et; c < bn; c += 256) {
-            const int t = t0 + c;
-            const int slot = t < p.T ? r.slots[t] : -1;
-            tok_off[c] = slot >= 0 ? ((long long)(slot / r.page_size) * r.nkv * r.page_size + slot % r.page_size) * r.hd : -1ll;
-          }
-        }
-        // This thread's angles are asked for one chunk ahead, all at once: they come from L2, which is
-        // busy with the operands, and a chunk that waited for its own would wait about as long again
-        // as it works.
-        float4 ang[2][4], ang_next[2][4];
-        auto ask_angles = [&](int c0, float4 (&a)[2][4]) {
-          if (r.cos_sin == nullptr || t0 + c0 >= p.T) return;
-          const float2* trow = r.cos_sin + (size_t)min(t0 + c0 + tt, p.T - 1) * half;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            if (g_turn[k]) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) a[k][i] = __ldg(reinterpret_cast<const float4*>(trow + g_fi[k]) + i);
-            }
-          }
-        };
-        ask_angles(0, ang_next);
-#pragma unroll 1
-        for (int c0 = 0; c0 < bn; c0 += 32) {
-          if (t0 + c0 >= p.T) break;
-#pragma unroll
-          for (int k = 0; k < 2; ++k)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ang[k][i] = ang_next[k][i];
-          if (c0 + 32 < bn) ask_angles(c0 + 32, ang_next);
-          {
-            uint32_t g[16];                               // 16 of the 32 columns from each warp of a quarter
-            tmem_ld16(taddr + c0 + 16 * grp, g);
-            tmem_ld_wait();
-#pragma unroll
-            for (int jj = 0; jj < 16; ++jj) xch[(16 * grp + jj) * XS + xrow(row)] = __uint_as_float(g[jj]);
-          }
-          epilogue8_sync();
-          const int t = t0 + c0 + tt;
-          if (t < p.T && c0 + tt < bn) {
-            const float* xr = xch + tt * XS;
-            const long long coff = r.slots != nullptr ? tok_off[c0 + tt] : -1ll;
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              if (!g_live[k]) continue;
-              const float4 v0 = *reinterpret_cast<const float4*>(xr + xrow(q8 + 64 * k));
-              const float4 v1 = *reinterpret_cast<const float4*>(xr + xrow(q8 + 64 * k + 4));
-              float o[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-              if (g_turn[k]) {
-                const float4 w0 = *reinterpret_cast<const float4*>(xr + xrow(g_part[k]));
-                const float4 w1 = *reinterpret_cast<const float4*>(xr + xrow(g_part[k] + 4));
-                const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-                float cs[8], sn[8];
-                if (r.cos_sin != nullptr) {
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) {
-                    const float4 a = ang[k][i];
-                    cs[2 * i] = a.x; sn[2 * i] = a.y; cs[2 * i + 1] = a.z; sn[2 * i + 1] = a.w;
-                  }
-                } else {
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) { const float2 a = angle_of(r, t, g_fi[k] + i); cs[i] = a.x; sn[i] = a.y; }   // no table given
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = g_low[k] ? o[i] * cs[i] - w[i] * sn[i] : w[i] * sn[i] + o[i] * cs[i];
-              }
-              uint4 pk;
-              pk.x = pack_bf16x2(o[0], o[1]); pk.y = pack_bf16x2(o[2], o[3]);
-              pk.z = pack_bf16x2(o[4], o[5]); pk.w = pack_bf16x2(o[6], o[7]);
-              *reinterpret_cast<uint4*>((bf16*)p.C + (size_t)t * p.ldc + n0 + q8 + 64 * k) = pk;
-              if (g_cache[k] != nullptr && coff >= 0) *reinterpret_cast<uint4*>(g_cache[k] + coff) = pk;
-            }
-          }
-          epilogue8_sync();                               // all have read before the next 32 columns come in
-        }
-      } else {
-        // The tile leaves TMEM 64 token columns at a time (32 of each half of a gate/up pair): a load from
-        // TMEM and the wait for it are a round trip of their own, and sixteen of them for a tile of 256
-        // columns were most of what the epilogue took. The residual values of the same columns are
-        // fetched while the accumulator values are on their way.
-        // (with ten warps a thread has 168 registers: the residual's 64 beside the accumulator's 64 would spill)
-        constexpr int CW = (DUAL || BN < 128 || EPI == EPI_ACCUM_F32) ? 32 : 64;
-        float* cbase = (float*)p.C + (size_t)t0 * p.ldc + n;
-        // the first warp of a quarter takes the columns up to `mid` (a multiple of 32), the second the rest;
-        // `lim`: columns of this warp that are tokens of the tile and of the step
-        const int mid = ((bn / 2 + 31) / 32) * 32;
-        const int c_begin = grp == 0 ? 0 : mid;
-        const int lim = min(grp == 0 ? mid : bn, p.T - t0);
-#pragma unroll 1
-        for (int c0 = c_begin; c0 < lim; c0 += CW) {
-          uint32_t g[CW], u[DUAL ? CW : 1];
-          float r[EPI == EPI_ACCUM_F32 ? CW : 1];
-          if (DUAL) {
-            tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
-            tmem_ld32(taddr + BN + c0, reinterpret_cast<uint32_t(&)[32]>(u));
-          } else if (CW == 32) {
-            tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
-          } else {
-            tmem_ld64(taddr + c0, reinterpret_cast<uint32_t(&)[64]>(g));
-          }
-          if (EPI == EPI_ACCUM_F32 && n < p.N) {
-            const float* cp = cbase + (size_t)c0 * p.ldc;
-#pragma unroll
-            for (int jj = 0; jj < CW; ++jj) r[jj] = (c0 + jj < lim) ? __ldcg(cp + (size_t)jj * p.ldc) : 0.f;
-          }
-          tmem_ld_wait();
-          if (n < p.N) {
-            if (EPI == EPI_ACCUM_F32) {
-              float* cp = cbase + (size_t)c0 * p.ldc;
-#pragma unroll
-              for (int jj = 0; jj < CW; ++jj)
-                if (c0 + jj < lim) cp[(size_t)jj * p.ldc] = r[jj] + __uint_as_float(g[jj]);
-            } else if (EPI == EPI_STORE) {
-              bf16* cp = (bf16*)p.C + (size_t)(t0 + c0) * p.ldc + n;
-              store_act_all(p, g);
-#pragma unroll
-              for (int jj = 0; jj < CW; ++jj, cp += p.ldc)
-                if (c0 + jj < lim) *cp = __float2bfloat16_rn(__uint_as_float(g[jj]));
-            } else {
-#pragma unroll
-              for (int jj = 0; jj < CW; ++jj) {
-                if (c0 + jj < lim) emit<EPI>(p, t0 + c0 + jj, n, __uint_as_float(g[jj]), DUAL ? __uint_as_float(u[jj]) : 0.f);
-              }
-            }
-          }
-        }
-      }
+      tile_epilogue<BN, EPI, SWAP, WR>(p, taddr, bn, t0, n0, warp, lane, xch, tok_off);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);      // this warp's quarter of the set is read out
@@ -1080,38 +1088,36 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 }
 
 // ---------------------------------------------------------------------------- many tokens, two SMs a tile
-// The same persistent scheme on pairs of CTAs (a cluster of two, `tcgen05.mma.cta_group::2`): a tile is
-// 256 weight rows x BN tokens; each CTA of the pair loads its own 128 weight rows and its own half of
-// the token tile into its own shared memory (plain TMA loads, no multicast) and keeps its 128
-// accumulator rows in its own TMEM; the even CTA issues the MMAs, which read both CTAs' shared
-// memory. Per FLOP an SM takes in a third fewer operand bytes than alone (32 KB instead of 48 KB per
-// 64 of K at BN = 256), and operand bytes into the SM are what bounds the one-SM kernel above.
+// The same persistent scheme on pairs of CTAs (a cluster of two, `tcgen05.mma.cta_group::2`): a tile is 256 weight rows x
+// any number of tokens in steps of 32 up to 256; each CTA of the pair loads its own 128 weight rows and its own half of the
+// token tile into its own shared memory (plain TMA loads, no multicast) and keeps its 128 accumulator rows in its own TMEM; the
+// even CTA issues the MMAs, which read both CTAs' shared memory. Gate/up pairs put 256 tokens on the rows, 128 in each CTA; the
+// tile's 128 gate rows lie in the even CTA, its 128 up rows in the odd one, so that each CTA holds both values of its tokens.
+// Per FLOP an SM takes in and reads out a third fewer operand bytes than alone (32 KB instead of 48 KB per 64 of K), and
+// shared memory's 128 bytes a cycle are what bounds the one-SM kernel above: XXXPAIR
 // Hand-overs: a stage's bytes from both CTAs are counted by the even CTA's `full` barrier (the odd
 // CTA's loads name it by its cluster address); the even CTA's MMA thread commits to both CTAs' `empty`
 // and `acc_full` barriers; both CTAs' epilogue warps arrive at the even CTA's `acc_empty`. Both CTAs
 // allocate and free TMEM, and meet at a cluster barrier before they free it and leave, so that no
 // signal or MMA ever addresses a CTA that is gone. Every wait is bounded.
-template <int BN, bool DUAL> struct PairCfg {
-  static constexpr int A_TILES = DUAL ? 2 : 1;
-  static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = (BN / 2) * BK * 2;              // this CTA's half of the token tile
-  static constexpr int W_BYTES = A_TILES * A_BYTES;
-  static constexpr int STAGE_BYTES = W_BYTES + B_BYTES;
-  static constexpr int STAGES_RAW = 208 * 1024 / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
+// The weights' copies of the first stages are issued before the wait for the kernel in front.
+struct PairCfg {
+  static constexpr int A_BYTES = BM * BK * 2;                    // this CTA's 128 rows
+  static constexpr int B_BYTES = BM * BK * 2;                    // its half of the columns' operand, up to 128 rows
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = 6;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES;
-  static constexpr int ACC_COLS = A_TILES * BN;
-  static constexpr int TMEM_COLS = 2 * ACC_COLS <= 64 ? 64 : 2 * ACC_COLS <= 128 ? 128 : 2 * ACC_COLS <= 256 ? 256 : 512;
-  static_assert(2 * ACC_COLS <= 512, "two accumulator sets must fit in TMEM");
+  static constexpr int ACC_COLS = 256, TMEM_COLS = 512;          // two accumulator sets
 };
 constexpr long long PAIR_WAIT_CYCLES = 1000000000LL;             // about half a second
 
-template <int BN, int EPI>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int EPI>
+__global__ void __launch_bounds__(THREADS_MANY, 1)
 tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                     const Params p) {
-  constexpr bool DUAL = (EPI == EPI_SWIGLU);
-  typedef PairCfg<BN, DUAL> C;
+  constexpr bool SWAP = (EPI == EPI_SWIGLU);                // tokens on the rows
+  constexpr bool ROPE = (EPI == EPI_QKV_ROPE);
+  typedef PairCfg C;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::STAGES];     // used in the even CTA: both CTAs' bytes of a stage
   __shared__ __align__(8) uint64_t empty_bar[C::STAGES];    // in each CTA: the pair's MMAs have read the stage
@@ -1120,21 +1126,27 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ int never_flag;
+  __shared__ __align__(16) float xch[ROPE ? 32 * XS : 4];   // rotary epilogue, as in the kernel above
+  __shared__ long long tok_off[ROPE ? 256 : 1];
+  __shared__ int epi_fail;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   const int pair_id = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int t_tiles = (p.T + BN - 1) / BN, n_tiles = (p.N + 2 * BM - 1) / (2 * BM);
+  const int bn = p.bn;                                      // tokens per tile (256 on the rows)
+  constexpr int NT = SWAP ? BM : 2 * BM;                    // output features per tile
+  const int t_tiles = (p.T + bn - 1) / bn, n_tiles = (p.N + NT - 1) / NT;
   const int tiles = t_tiles * n_tiles;
   const int n_kb = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
     abort_flag = 0;
     never_flag = 0;
+    epi_fail = 0;
     fence_barrier_init();
   }
   if (warp == 0 && lane == 0) { prefetch_tensormap(&tmap_w); prefetch_tensormap(&tmap_x); }
@@ -1148,35 +1160,48 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (in both CTAs)
-    if (lane == 0) {
-      pdl_wait();
-      int it = 0, issued = 0;
-      bool ok = true;
-      for (int tile = pair_id; tile < tiles && ok; tile += n_pairs) {
-        const int t0 = (tile % t_tiles) * BN + (int)rank * (BN / 2);
-        const int n0 = (tile / t_tiles) * (2 * BM) + (int)rank * BM;
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-          if (it >= C::STAGES && !mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag, PAIR_WAIT_CYCLES)) {
-            abort_flag = 1; record_failure(p.err, 5, (int)rank); ok = false; break;
-          }
-          uint8_t* st = smem + (size_t)s * C::STAGE_BYTES;
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
-          const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);
-          const int k = kb * BK;
-          tma_load_2d_pair(st, &tmap_w, bar, k, n0);
-          if (DUAL) tma_load_2d_pair(st + C::A_BYTES, &tmap_w, bar, k, p.up_row0 + n0);
-          tma_load_2d_pair(st + C::W_BYTES, &tmap_x, bar, k, t0);
-          issued = it + 1;
-        }
+    if (elect_one()) {
+      const uint32_t stage_bytes = 2u * (uint32_t)(C::A_BYTES + (SWAP ? C::B_BYTES : bn * BK));     // of both CTAs
+      const int mine = (tiles - pair_id + n_pairs - 1) / n_pairs * n_kb;       // blocks of K of all this pair's tiles
+      const int pre = mine < C::STAGES ? mine : C::STAGES;
+      // this CTA's first row of either operand in a tile
+      auto w_row = [&](int tile) { const int n0 = tile / t_tiles * NT; return SWAP ? (rank == 0 ? n0 : p.up_row0 + n0) : n0 + (int)rank * BM; };
+      auto x_row = [&](int tile) { return tile % t_tiles * bn + (int)rank * (SWAP ? BM : bn / 2); };
+      auto copy = [&](bool weights, int s, int k, int y) {
+        uint8_t* st = smem + (size_t)s * C::STAGE_BYTES + (weights != SWAP ? 0 : C::A_BYTES);
+        tma_load_2d_pair(st, weights ? &tmap_w : &tmap_x, map_to_rank(smem_u32(&full_bar[s]), 0), k, y);
+      };
+      // the first stages' weights do not depend on the kernel before this one
+      for (int i = 0; i < pre; ++i) {
+        if (leader) mbar_expect_tx(&full_bar[i], stage_bytes);
+        copy(true, i, i % n_kb * BK, w_row(pair_id + i / n_kb * n_pairs));
       }
-      (void)issued;
+      pdl_wait();
+      for (int i = 0; i < pre; ++i) copy(false, i, i % n_kb * BK, x_row(pair_id + i / n_kb * n_pairs));
+      int it = pre, tile = pair_id + pre / n_kb * n_pairs, kb = pre % n_kb;
+      int wy = w_row(tile), xy = x_row(tile);
+      for (; it < mine; ++it) {
+        const int s = it % C::STAGES;
+        const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
+        if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag, PAIR_WAIT_CYCLES)) {
+          abort_flag = 1; record_failure(p.err, 5, (int)rank); break;
+        }
+        if (leader) mbar_expect_tx(&full_bar[s], stage_bytes);
+        copy(true, s, kb * BK, wy);
+        copy(false, s, kb * BK, xy);
+        if (++kb == n_kb) { kb = 0; tile += n_pairs; wy = w_row(tile); xy = x_row(tile); }
+      }
+      if (abort_flag && leader) {
+        // let copies already issued land before the CTAs' shared memory is given back
+        for (int i = max(0, it - C::STAGES); i < it; ++i)
+          mbar_wait(&full_bar[i % C::STAGES], (uint32_t)(i / C::STAGES) & 1u, &never_flag, 200000000LL);
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA only)
-    if (lane == 0 && leader) {
-      constexpr uint32_t idesc = umma_idesc_bf16(2 * BM, BN);
+    if (elect_one() && leader) {
+      const uint32_t idesc = umma_idesc_bf16(2 * BM, SWAP ? 256 : bn);
+      const uint64_t d0 = umma_desc_sw128(smem_u32(smem));
       int it = 0, ti = 0;
       bool ok = true;
       for (int tile = pair_id; tile < tiles && ok; tile += n_pairs, ++ti) {
@@ -1191,79 +1216,40 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
           if (!mbar_wait(&full_bar[s], ph, &abort_flag, PAIR_WAIT_CYCLES)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + (size_t)s * C::STAGE_BYTES);
-          const uint64_t da = umma_desc_sw128(a_addr);
-          const uint64_t db = umma_desc_sw128(a_addr + C::W_BYTES);
+          const uint64_t da = d0 + (uint64_t)(s * (C::STAGE_BYTES >> 4)), db = da + (uint64_t)(C::A_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-            const uint64_t koff = (uint64_t)(k * UMMA_K * 2 / 16);
-            umma_bf16_pair(acc_addr, da + koff, db + koff, idesc, acc);
-            if (DUAL) umma_bf16_pair(acc_addr + BN, umma_desc_sw128(a_addr + C::A_BYTES) + koff, db + koff, idesc, acc);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_pair(acc_addr, da + (uint64_t)(k * UMMA_K * 2 / 16), db + (uint64_t)(k * UMMA_K * 2 / 16), idesc, kb > 0 || k > 0);
           umma_commit_pair_both(&empty_bar[s]);      // the stage is free, in both CTAs
         }
-        if (ok) {
-          umma_commit_pair_both(&acc_full[buf]);
-        }
+        if (ok) umma_commit_pair_both(&acc_full[buf]);
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue warps (2..5), in both CTAs
-    const int row = (warp & 3) * 32 + lane;
+    // ------------------------------------------------------------ epilogue warps (2..9), in both CTAs
     const uint32_t drained = map_to_rank(smem_u32(&acc_empty[0]), 0);        // the even CTA's acc_empty[0]
     pdl_wait();
     int ti = 0;
     bool ok = true;
     for (int tile = pair_id; tile < tiles && ok; tile += n_pairs, ++ti) {
-      const int t0 = (tile % t_tiles) * BN, n0 = (tile / t_tiles) * (2 * BM) + (int)rank * BM;
-      const int n = n0 + row;
+      const int t0 = (tile % t_tiles) * bn + (SWAP ? (int)rank * BM : 0);
+      const int n0 = (tile / t_tiles) * NT + (SWAP ? 0 : (int)rank * BM);
       const int buf = ti & 1, use = ti >> 1;
       ok = mbar_wait(&acc_full[buf], (uint32_t)use & 1u, &abort_flag, PAIR_WAIT_CYCLES);
       if (!ok) { abort_flag = 1; record_failure(p.err, 3, (int)rank); }
       ok = __all_sync(0xffffffffu, ok);
+      if (ROPE) {                                        // the eight warps leave together or not at all
+        if (!ok) epi_fail = 1;
+        epilogue8_sync();
+        ok = epi_fail == 0;
+      }
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(buf * C::ACC_COLS);
-      // 64 token columns at a time, the residual values fetched while the accumulator's are on their way
-      // (as in tc_gemm_persistent_kernel)
-      constexpr int CW = DUAL ? 32 : 64;
-      float* cbase = (float*)p.C + (size_t)t0 * p.ldc + n;
-#pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += CW) {
-        if (t0 + c0 >= p.T) break;
-        uint32_t g[CW], u[DUAL ? CW : 1];
-        float r[EPI == EPI_ACCUM_F32 ? CW : 1];
-        if (DUAL) {
-          tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
-          tmem_ld32(taddr + BN + c0, reinterpret_cast<uint32_t(&)[32]>(u));
-        } else {
-          tmem_ld64(taddr + c0, reinterpret_cast<uint32_t(&)[64]>(g));
-        }
-        if (EPI == EPI_ACCUM_F32 && n < p.N) {
-          const float* cp = cbase + (size_t)c0 * p.ldc;
-#pragma unroll
-          for (int jj = 0; jj < CW; ++jj) r[jj] = (t0 + c0 + jj < p.T) ? __ldcg(cp + (size_t)jj * p.ldc) : 0.f;
-        }
-        tmem_ld_wait();
-        if (n < p.N) {
-          if (EPI == EPI_ACCUM_F32) {
-            float* cp = cbase + (size_t)c0 * p.ldc;
-#pragma unroll
-            for (int jj = 0; jj < CW; ++jj)
-              if (t0 + c0 + jj < p.T) cp[(size_t)jj * p.ldc] = r[jj] + __uint_as_float(g[jj]);
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < CW; ++jj) {
-              const int t = t0 + c0 + jj;
-              if (t < p.T) emit<EPI>(p, t, n, __uint_as_float(g[jj]), DUAL ? __uint_as_float(u[jj]) : 0.f);
-            }
-          }
-        }
-      }
+      tile_epilogue<256, EPI, SWAP, BM>(p, taddr, bn, t0, n0, warp, lane, xch, tok_off);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(drained + (uint32_t)(buf * 8));   // this warp's quarter of this CTA's half is read out
+      if (lane == 0) mbar_arrive_cluster(drained + (uint32_t)(buf * 8));   // this warp's part of this CTA's half is read out
     }
   }
   tc_fence_before();
@@ -1350,17 +1336,18 @@ int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const Params
   return launch_ex(tc_gemm_persistent_kernel<BN, EPI, SWAP, WR>, dim3(ctas), dim3(THREADS_MANY), C::SMEM_BYTES, s, 1, mw, mx, p);
 }
 
-template <int BN, int EPI>
+template <int EPI>
 int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int sm_count, cudaStream_t s) {
-  typedef PairCfg<BN, EPI == EPI_SWIGLU> C;
+  typedef PairCfg C;
   static bool configured[64] = {};
-  if (allow_dynamic_smem(tc_gemm_pair_kernel<BN, EPI>, C::SMEM_BYTES, configured)) return -5;
-  const int tiles = ((p.T + BN - 1) / BN) * ((p.N + 2 * BM - 1) / (2 * BM));
+  if (allow_dynamic_smem(tc_gemm_pair_kernel<EPI>, C::SMEM_BYTES, configured)) return -5;
+  const int nt = EPI == EPI_SWIGLU ? BM : 2 * BM;
+  const int tiles = ((p.T + p.bn - 1) / p.bn) * ((p.N + nt - 1) / nt);
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   // the two CTAs of a pair are neighbours along x: blocks 2i and 2i + 1
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(THREADS_MANY);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = s;
   cudaLaunchAttribute attrs[2];
@@ -1375,16 +1362,14 @@ int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, i
   }
   cfg.attrs = attrs;
   cfg.numAttrs = n;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_gemm_pair_kernel<BN, EPI>, mw, mx, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_gemm_pair_kernel<EPI>, mw, mx, p);
   if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
   return 0;
 }
 
-// Whether pairs of CTAs take the products of long prompt portions (rllm_tc_gemm_set_pairs). Off unless asked
-// for: measured on a B200 (2,048 tokens, Llama 3.2 1B shapes) the pair kernel gives the same bits and is
-// level with the one-SM kernel on the q/k/v product and 4 to 12 % behind on the others; its MMA thread
-// waits for operands 40 to 70 % of the time although an SM takes in a third fewer bytes.
-bool g_pairs = false;
+// Which products run on pairs of CTAs (rllm_tc_gemm_set_pairs): 0 the rule below, 1 all that pairs take, 32 to 256 those
+// with that many tokens a tile, -1 none.
+int g_pairs = 0;
 
 template <int EPI>
 int launch_many(int bn, const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int sm_count, cudaStream_t s) {
@@ -1483,6 +1468,13 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
   if (few_out) *few_out = few;
 }
 
+// Tokens per tile of the kernel on pairs of CTAs, or 0 where the one-CTA kernels take the product.
+int plan_pairs(int epi, int T, int N, int K, int sm_count) {
+  if (g_pairs >= 32) return epi == EPI_SWIGLU ? 256 : g_pairs;
+  if (g_pairs != 1) return 0;
+  return 256;
+}
+
 // X null: the fused-norm variants (norm must be given, T <= NORM_MAX_T).
 int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void* W, void* Cout, long long ldc,
         int T, int N, int K, int allow_split, int* err, int sm_count, const RopeArgs* rope, void* stream, int x_rows = 0,
@@ -1505,13 +1497,21 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   const bool many = !few;            // the persistent kernel (no ranges of K, no norm in front)
   if (many && norm) return ERR_BAD_SIZE;
   const bool dual = epi == EPI_SWIGLU;
+  if (many && rope) {
+    // the rotary epilogue of long portions moves groups of 8 neighbouring features as 16 bytes
+    if (rope->hd % 16 || rope->rot_dim % 16 || ldc % 8) return ERR_BAD_SIZE;
+    if (((uintptr_t)Cout | (uintptr_t)rope->kcache | (uintptr_t)rope->vcache | (uintptr_t)rope->cos_sin) & 15) return ERR_BAD_ALIGN;
+  }
   CUtensorMap mw, mx;
   if ((rc = cached_map(&mw, W, dual ? 2LL * N : N, K, K, BM))) return rc;
-  // long portions: a tile of 256 weight rows x bn tokens on a pair of CTAs, each loading half of the token tile
-  const bool pair = g_pairs && !norm && !x_rows && epi != EPI_QKV_ROPE && sm_count >= 2 && many && T >= (dual ? 128 : 256);
-  if (pair) bn = dual ? 128 : 256;                                   // the pair kernel's tile is fixed
+  // long portions on pairs of CTAs
+  const bool pairs_take = g_pairs >= 0 && !norm && !x_rows && sm_count >= 2 && many &&
+      (!dual || (N % 8 == 0 && ldc % 8 == 0 && !((uintptr_t)Cout & 15)));
+  const int pair_bn = pairs_take ? plan_pairs(epi, T, N, K, sm_count) : 0;
+  const bool pair = pair_bn > 0;
+  if (pair) bn = pair_bn;
   if (norm) mx = mw;                                                 // not used by the kernel
-  else if ((rc = make_map(&mx, X, T, x_rows ? (long long)((N - 1) / x_rows) * x_gs + K : K, ldx, pair ? bn / 2 : bn))) return rc;
+  else if ((rc = make_map(&mx, X, T, x_rows ? (long long)((N - 1) / x_rows) * x_gs + K : K, ldx, pair ? (dual ? BM : bn / 2) : bn))) return rc;
   Params p;
   p.C = Cout; p.ldc = (int)ldc; p.T = T; p.N = N; p.K = K; p.up_row0 = N; p.splits = splits; p.err = err; p.bn = bn;
   p.act = epi == EPI_STORE || epi == EPI_SWIGLU ? t_store_act : 0;
@@ -1524,16 +1524,12 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   const bool nm = norm != nullptr;
   if (pair) {
     switch (epi) {
-      case EPI_STORE: return launch_pair<256, EPI_STORE>(mw, mx, p, sm_count, s);
-      case EPI_STORE_F32: return launch_pair<256, EPI_STORE_F32>(mw, mx, p, sm_count, s);
-      case EPI_ACCUM_F32: return launch_pair<256, EPI_ACCUM_F32>(mw, mx, p, sm_count, s);
-      case EPI_SWIGLU: return launch_pair<128, EPI_SWIGLU>(mw, mx, p, sm_count, s);
+      case EPI_STORE: return launch_pair<EPI_STORE>(mw, mx, p, sm_count, s);
+      case EPI_STORE_F32: return launch_pair<EPI_STORE_F32>(mw, mx, p, sm_count, s);
+      case EPI_ACCUM_F32: return launch_pair<EPI_ACCUM_F32>(mw, mx, p, sm_count, s);
+      case EPI_SWIGLU: return launch_pair<EPI_SWIGLU>(mw, mx, p, sm_count, s);
+      case EPI_QKV_ROPE: return launch_pair<EPI_QKV_ROPE>(mw, mx, p, sm_count, s);
     }
-  }
-  if (many && rope) {
-    // the persistent kernel's rotary epilogue moves groups of 8 neighbouring features as 16 bytes
-    if (rope->hd % 16 || rope->rot_dim % 16 || ldc % 8) return ERR_BAD_SIZE;
-    if (((uintptr_t)Cout | (uintptr_t)rope->kcache | (uintptr_t)rope->vcache | (uintptr_t)rope->cos_sin) & 15) return ERR_BAD_ALIGN;
   }
   if (many && dual && g_token_rows && N % 8 == 0 && ldc % 8 == 0 && !((uintptr_t)Cout & 15)) {
     // tiles of 64 gate and 64 up rows where tiles of 128 would leave half of the SMs without one
@@ -1574,7 +1570,7 @@ RLLM_API int rllm_tc_gemm_plan(int epi, int T, int N, int K, int sm_count, int a
   return 0;
 }
 
-RLLM_API int rllm_tc_gemm_set_pairs(int on) { g_pairs = on != 0; return 0; }
+RLLM_API int rllm_tc_gemm_set_pairs(int on) { g_pairs = on > 1 ? (on < 32 ? 32 : on > 256 ? 256 : on & ~31) : on; return 0; }
 RLLM_API int rllm_tc_gemm_set_token_rows(int on) { g_token_rows = on != 0; return 0; }
 
 // The store epilogue (0) may carry an activation in the bits above the epilogue's number: epi = 0 | 1 << 8 stores
