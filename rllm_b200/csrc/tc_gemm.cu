@@ -735,15 +735,17 @@ template <int BN, bool DUAL, int WR = BM> struct PCfg {
 // a scheduler waits out every instruction's latency alone, so an epilogue's time goes with the instructions per warp, and
 // the last tile's epilogue is not hidden by a mainloop. xch, tok_off: see the rotary epilogue.
 constexpr int XS = BM + 4;
-template <int BN, int EPI, bool SWAP, int WR>
-__device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t taddr, int bn, int t0, int n0, int warp, int lane,
-                                              float* xch, long long* tok_off) {
+// `ready` waits for the set to be complete (false: it will not be); the first angles are asked for before.
+template <int BN, int EPI, bool SWAP, int WR, class Ready>
+__device__ __forceinline__ bool tile_epilogue(const Params& p, uint32_t taddr, int bn, int t0, int n0, int warp, int lane,
+                                              float* xch, long long* tok_off, Ready ready) {
   constexpr bool DUAL = (EPI == EPI_SWIGLU);
   constexpr bool ROPE = (EPI == EPI_QKV_ROPE);
   const int row = (warp & 3) * 32 + lane;
   const int grp = (warp - 2) >> 2;
   const int n = n0 + row;
   if (SWAP) {
+    if (!ready()) return false;
     // this thread's row is a token; its gate values are columns 0..WR-1, its up values WR..2 WR-1. The
     // first warp of a quarter takes the lower half of the features, the second the upper, 32 at a
     // time, and writes them as 16-byte pieces of the token's output row.
@@ -834,6 +836,7 @@ __device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t taddr, i
       }
     };
     ask_angles(0, ang_next);
+    if (!ready()) return false;
 #pragma unroll 1
     for (int c0 = 0; c0 < bn; c0 += 32) {
       if (t0 + c0 >= p.T) break;
@@ -890,55 +893,63 @@ __device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t taddr, i
   } else {
     // The tile leaves TMEM 64 token columns at a time (32 of each half of a gate/up pair): a load from
     // TMEM and the wait for it are a round trip of their own, and sixteen of them for a tile of 256
-    // columns were most of what the epilogue took. The residual values of the same columns are
-    // fetched while the accumulator values are on their way.
-    // (with ten warps a thread has 168 registers: the residual's 64 beside the accumulator's 64 would spill)
+    // columns were most of what the epilogue took.
     constexpr int CW = (DUAL || BN < 128 || EPI == EPI_ACCUM_F32) ? 32 : 64;
-    float* cbase = (float*)p.C + (size_t)t0 * p.ldc + n;
     // the first warp of a quarter takes the columns up to `mid` (a multiple of 32), the second the rest;
     // `lim`: columns of this warp that are tokens of the tile and of the step
     const int mid = ((bn / 2 + 31) / 32) * 32;
     const int c_begin = grp == 0 ? 0 : mid;
     const int lim = min(grp == 0 ? mid : bn, p.T - t0);
+    if constexpr (EPI == EPI_ACCUM_F32) {
+      // One addition per value in the memory's own units, rounded as an addition here would be (below 1.2e-38 it gives zero):
+      // half of the traffic, and no round trip to L2 for the residual per 32 columns. 2,048 tokens x 2,048: K 2,048 21.1 -> 17.4 us,
+      // K 8,192 59.7 -> 55.3 (pairs of CTAs 55.0 -> 51.5); residual values asked for 32 columns ahead instead 20.0, 58.4 and 54.2.
+      if (!ready()) return false;
+      float* cbase = (float*)p.C + (size_t)t0 * p.ldc + n;
 #pragma unroll 1
-    for (int c0 = c_begin; c0 < lim; c0 += CW) {
-      uint32_t g[CW], u[DUAL ? CW : 1];
-      float r[EPI == EPI_ACCUM_F32 ? CW : 1];
-      if (DUAL) {
+      for (int c0 = c_begin; c0 < lim; c0 += CW) {
+        uint32_t g[CW];
         tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
-        tmem_ld32(taddr + BN + c0, reinterpret_cast<uint32_t(&)[32]>(u));
-      } else if (CW == 32) {
-        tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
-      } else {
-        tmem_ld64(taddr + c0, reinterpret_cast<uint32_t(&)[64]>(g));
-      }
-      if (EPI == EPI_ACCUM_F32 && n < p.N) {
-        const float* cp = cbase + (size_t)c0 * p.ldc;
-#pragma unroll
-        for (int jj = 0; jj < CW; ++jj) r[jj] = (c0 + jj < lim) ? __ldcg(cp + (size_t)jj * p.ldc) : 0.f;
-      }
-      tmem_ld_wait();
-      if (n < p.N) {
-        if (EPI == EPI_ACCUM_F32) {
+        tmem_ld_wait();
+        if (n < p.N) {
           float* cp = cbase + (size_t)c0 * p.ldc;
 #pragma unroll
           for (int jj = 0; jj < CW; ++jj)
-            if (c0 + jj < lim) cp[(size_t)jj * p.ldc] = r[jj] + __uint_as_float(g[jj]);
-        } else if (EPI == EPI_STORE) {
-          bf16* cp = (bf16*)p.C + (size_t)(t0 + c0) * p.ldc + n;
-          store_act_all(p, g);
-#pragma unroll
-          for (int jj = 0; jj < CW; ++jj, cp += p.ldc)
-            if (c0 + jj < lim) *cp = __float2bfloat16_rn(__uint_as_float(g[jj]));
+            if (c0 + jj < lim) atomicAdd(cp + (size_t)jj * p.ldc, __uint_as_float(g[jj]));
+        }
+      }
+    } else {
+      if (!ready()) return false;
+#pragma unroll 1
+      for (int c0 = c_begin; c0 < lim; c0 += CW) {
+        uint32_t g[CW], u[DUAL ? CW : 1];
+        if (DUAL) {
+          tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
+          tmem_ld32(taddr + BN + c0, reinterpret_cast<uint32_t(&)[32]>(u));
+        } else if (CW == 32) {
+          tmem_ld32(taddr + c0, reinterpret_cast<uint32_t(&)[32]>(g));
         } else {
+          tmem_ld64(taddr + c0, reinterpret_cast<uint32_t(&)[64]>(g));
+        }
+        tmem_ld_wait();
+        if (n < p.N) {
+          if (EPI == EPI_STORE) {
+            bf16* cp = (bf16*)p.C + (size_t)(t0 + c0) * p.ldc + n;
+            store_act_all(p, g);
 #pragma unroll
-          for (int jj = 0; jj < CW; ++jj) {
-            if (c0 + jj < lim) emit<EPI>(p, t0 + c0 + jj, n, __uint_as_float(g[jj]), DUAL ? __uint_as_float(u[jj]) : 0.f);
+            for (int jj = 0; jj < CW; ++jj, cp += p.ldc)
+              if (c0 + jj < lim) *cp = __float2bfloat16_rn(__uint_as_float(g[jj]));
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < CW; ++jj) {
+              if (c0 + jj < lim) emit<EPI>(p, t0 + c0 + jj, n, __uint_as_float(g[jj]), DUAL ? __uint_as_float(u[jj]) : 0.f);
+            }
           }
         }
       }
     }
   }
+  return true;
 }
 
 template <int BN, int EPI, bool SWAP, int WR = BM>
@@ -1065,18 +1076,21 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++ti) {
       const int t0 = (tile % t_tiles) * bn, n0 = (tile / t_tiles) * WR;
       const int buf = ti & 1, use = ti >> 1;
-      ok = mbar_wait(&acc_full[buf], (uint32_t)use & 1u, &abort_flag);
-      if (!ok) { abort_flag = 1; record_failure(p.err, 3); }
-      ok = __all_sync(0xffffffffu, ok);
-      if (ROPE) {                                        // the eight warps leave together or not at all
-        if (!ok) epi_fail = 1;
-        epilogue8_sync();
-        ok = epi_fail == 0;
-      }
-      if (!ok) break;
-      tc_fence_after();
+      auto ready = [&]() {
+        bool got = mbar_wait(&acc_full[buf], (uint32_t)use & 1u, &abort_flag);
+        if (!got) { abort_flag = 1; record_failure(p.err, 3); }
+        got = __all_sync(0xffffffffu, got);
+        if (ROPE) {                                      // the eight warps leave together or not at all
+          if (!got) epi_fail = 1;
+          epilogue8_sync();
+          got = epi_fail == 0;
+        }
+        tc_fence_after();
+        return got;
+      };
       const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(buf * C::ACC_COLS);
-      tile_epilogue<BN, EPI, SWAP, WR>(p, taddr, bn, t0, n0, warp, lane, xch, tok_off);
+      ok = tile_epilogue<BN, EPI, SWAP, WR>(p, taddr, bn, t0, n0, warp, lane, xch, tok_off, ready);
+      if (!ok) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);      // this warp's quarter of the set is read out
@@ -1094,7 +1108,8 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 // even CTA issues the MMAs, which read both CTAs' shared memory. Gate/up pairs put 256 tokens on the rows, 128 in each CTA; the
 // tile's 128 gate rows lie in the even CTA, its 128 up rows in the odd one, so that each CTA holds both values of its tokens.
 // Per FLOP an SM takes in and reads out a third fewer operand bytes than alone (32 KB instead of 48 KB per 64 of K), and
-// shared memory's 128 bytes a cycle are what bounds the one-SM kernel above: XXXPAIR
+// shared memory's 128 bytes a cycle are what bounds the one-SM kernel above: 2,048 x 2,048 x 8,192 takes 315 ns a 64 of K and tile
+// of 256 x 256, where one SM takes 390 for 128 x 240.
 // Hand-overs: a stage's bytes from both CTAs are counted by the even CTA's `full` barrier (the odd
 // CTA's loads name it by its cluster address); the even CTA's MMA thread commits to both CTAs' `empty`
 // and `acc_full` barriers; both CTAs' epilogue warps arrive at the even CTA's `acc_empty`. Both CTAs
@@ -1235,18 +1250,21 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const int t0 = (tile % t_tiles) * bn + (SWAP ? (int)rank * BM : 0);
       const int n0 = (tile / t_tiles) * NT + (SWAP ? 0 : (int)rank * BM);
       const int buf = ti & 1, use = ti >> 1;
-      ok = mbar_wait(&acc_full[buf], (uint32_t)use & 1u, &abort_flag, PAIR_WAIT_CYCLES);
-      if (!ok) { abort_flag = 1; record_failure(p.err, 3, (int)rank); }
-      ok = __all_sync(0xffffffffu, ok);
-      if (ROPE) {                                        // the eight warps leave together or not at all
-        if (!ok) epi_fail = 1;
-        epilogue8_sync();
-        ok = epi_fail == 0;
-      }
-      if (!ok) break;
-      tc_fence_after();
+      auto ready = [&]() {
+        bool got = mbar_wait(&acc_full[buf], (uint32_t)use & 1u, &abort_flag, PAIR_WAIT_CYCLES);
+        if (!got) { abort_flag = 1; record_failure(p.err, 3, (int)rank); }
+        got = __all_sync(0xffffffffu, got);
+        if (ROPE) {                                      // the eight warps leave together or not at all
+          if (!got) epi_fail = 1;
+          epilogue8_sync();
+          got = epi_fail == 0;
+        }
+        tc_fence_after();
+        return got;
+      };
       const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(buf * C::ACC_COLS);
-      tile_epilogue<256, EPI, SWAP, BM>(p, taddr, bn, t0, n0, warp, lane, xch, tok_off);
+      ok = tile_epilogue<256, EPI, SWAP, BM>(p, taddr, bn, t0, n0, warp, lane, xch, tok_off, ready);
+      if (!ok) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(drained + (uint32_t)(buf * 8));   // this warp's part of this CTA's half is read out
@@ -1469,10 +1487,9 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
 }
 
 // Tokens per tile of the kernel on pairs of CTAs, or 0 where the one-CTA kernels take the product.
-int plan_pairs(int epi, int T, int N, int K, int sm_count) {
+int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
   if (g_pairs >= 32) return epi == EPI_SWIGLU ? 256 : g_pairs;
-  if (g_pairs != 1) return 0;
-  return 256;
+  return g_pairs == 1 ? 256 : 0;
 }
 
 // X null: the fused-norm variants (norm must be given, T <= NORM_MAX_T).
@@ -1507,7 +1524,7 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   // long portions on pairs of CTAs
   const bool pairs_take = g_pairs >= 0 && !norm && !x_rows && sm_count >= 2 && many &&
       (!dual || (N % 8 == 0 && ldc % 8 == 0 && !((uintptr_t)Cout & 15)));
-  const int pair_bn = pairs_take ? plan_pairs(epi, T, N, K, sm_count) : 0;
+  const int pair_bn = pairs_take ? plan_pairs(epi, T, N, K, bn, sm_count) : 0;
   const bool pair = pair_bn > 0;
   if (pair) bn = pair_bn;
   if (norm) mx = mw;                                                 // not used by the kernel
