@@ -1486,10 +1486,33 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
   if (few_out) *few_out = few;
 }
 
-// Tokens per tile of the kernel on pairs of CTAs, or 0 where the one-CTA kernels take the product.
+// Tokens per tile of the kernel on pairs of CTAs, or 0 where the one-CTA kernel (tiles of `bn` tokens) takes the product. Both
+// times are modelled: waves of tiles x blocks of K x a block's time, which goes with the tile's tokens down to what issuing a
+// block takes, + the start and the last epilogue. Fitted to measurements (ns):
+// a block takes a CTA max(165, 1.63 a token), a pair max(200, 1.3 a token), with gate/up 400 and 310; one-CTA kernel / pairs by this
+// rule, us: 2,048 tokens, 3,072 x 2,048 26.2 / 23.0 (192 tokens a tile), 2 x 8,192 x 2,048 98.0 / 89.2, 16,384 x 4,096 188 / 171; 1,905 tokens,
+// 2,048 x 8,192 53.2 / 47.3 (224); 2,834 tokens 88.7 / 70.6 (160); 643 tokens, 2 x 8,192 x 2,048 42.0 / 36.8. Where the rule leaves the
+// product to single CTAs, us single / best width on pairs: 643 tokens, 2,048 x 2,048 11.4 / 12.8, 2,048 x 8,192 29.2 / 31.2; 256 tokens 25.6 / 29.7.
+// Up to 128 tokens a pair has half a tile to work on.
 int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
-  if (g_pairs >= 32) return epi == EPI_SWIGLU ? 256 : g_pairs;
-  return g_pairs == 1 ? 256 : 0;
+  const bool dual = epi == EPI_SWIGLU;
+  if (g_pairs >= 32) return dual ? 256 : g_pairs;
+  if (g_pairs == 1) return 256;
+  if (T <= 128) return 0;
+  const long long kb = (K + BK - 1) / BK;
+  auto waves = [&](int tokens, int rows, int places) {
+    const long long tiles = (long long)((T + tokens - 1) / tokens) * ((N + rows - 1) / rows);
+    return (tiles + places - 1) / places;
+  };
+  const long long one = waves(bn, BM, sm_count) * kb * (dual ? 400 : bn > 101 ? bn * 163 / 100 : 165) + 4000 + 14 * bn;
+  long long best = one - one / 50;
+  int best_bn = 0;
+  for (int cand = 256; cand >= (dual ? 256 : 64); cand -= 32) {
+    const long long t = waves(cand, dual ? BM : 2 * BM, sm_count / 2) * kb * (dual ? 310 : cand > 153 ? cand * 13 / 10 : 200) +
+                        (dual ? 7500 : 4500 + 18 * cand);
+    if (t < best) { best = t; best_bn = cand; }
+  }
+  return best_bn;
 }
 
 // X null: the fused-norm variants (norm must be given, T <= NORM_MAX_T).

@@ -101,9 +101,9 @@ def stream_supported(epilogue: int, norm: bool, T: int, N: int, K: int, hd: int 
     return ok
 
 
-def set_pairs(on: bool) -> None:
-    """Products of long prompt portions on pairs of CTAs (`tcgen05.mma.cta_group::2`) or on single CTAs
-    (the default: measured level or faster)."""
+def set_pairs(on: bool | int) -> None:
+    """Products of more than 64 tokens on pairs of CTAs (`tcgen05.mma.cta_group::2`): True all that pairs take, False (the
+    default) those that are faster there by the launcher's rule, -1 none; 32 to 256: all, with that many tokens a tile."""
     ops._fn("sm100", "rllm_tc_gemm_set_pairs")(int(on))
 
 
