@@ -1,5 +1,5 @@
 """ctypes face of the native host runtime (library "host", csrc/host_runtime.cpp): page pools,
-the tables of what every live request holds, and the writer of a decode step's metadata."""
+the tables of what every live request holds, and the writers of a step's metadata."""
 from __future__ import annotations
 
 from ctypes import POINTER, c_int, c_longlong, c_void_p
@@ -21,6 +21,7 @@ _SIGS = {
     "rllm_cache_check": (_I, [_P]), "rllm_rows_new": (_P, [_I, _I]), "rllm_rows_delete": (None, [_P]),
     "rllm_rows_forget": (None, [_P, _I]),
     "rllm_fill_decode": (_I, [_P, _P, _I, _P, _P, _I, _P, _P]),
+    "rllm_fill_step": (_I, [_P, _I, _P, _P, _I, _P, _P]),
 }
 
 

@@ -349,3 +349,37 @@ RLLM_API int rllm_fill_decode(void* cv, void* rv, int S, const int* handles, con
   }
   return dirty;
 }
+
+// The metadata of any step besides its token ids and wanted rows: S holdings that bring q_lens[s] tokens each, T together, into `host`
+// (int32, preset to -1): offs[1] positions [T] | offs[2] which sequence [T] | offs[3] first row [S + 1] | offs[4] key counts [S] |
+//   offs[5] state slots [S] | per group g: offs[7 + 2g] cache slots [T], offs[8 + 2g] block table [S, P].
+// Returns 0, or < 0 on a bad handle, a token without a page or a table wider than P.
+RLLM_API int rllm_fill_step(void* cv, int S, const int* handles, const int* q_lens, int P, int* host, const long long* offs) {
+  Cache* c = static_cast<Cache*>(cv);
+  const int G = (int)c->pools.size(), ps = c->page_size;
+  int q0 = 0;
+  host[offs[3]] = 0;
+  for (int s = 0; s < S; ++s) {
+    Holding* h = holding(c, handles[s]);
+    if (!h) return -9;
+    const int q = q_lens[s], start = h->num_tokens;
+    for (int i = 0; i < q; ++i) { host[offs[1] + q0 + i] = start + i; host[offs[2] + q0 + i] = s; }
+    host[offs[3] + s + 1] = q0 + q;
+    host[offs[4] + s] = start + q;
+    host[offs[5] + s] = handles[s];
+    for (int g = 0; g < G; ++g) {
+      const std::vector<int>& pages = h->pages[(size_t)g];
+      const int held = (int)pages.size();
+      if (held > P) return -4;
+      if (q > 0 && (start + q - 1) / ps >= held) return -2;       // a new token has no page
+      if (held) std::memcpy(host + offs[8 + 2 * g] + (long long)s * P, pages.data(), (size_t)held * sizeof(int));
+      int* slots = host + offs[7 + 2 * g] + q0;
+      for (int i = 0, p = start / ps, off = start % ps; i < q; ++i) {
+        slots[i] = pages[(size_t)p] * ps + off;
+        if (++off == ps) { off = 0; ++p; }
+      }
+    }
+    q0 += q;
+  }
+  return 0;
+}

@@ -176,32 +176,22 @@ class Engine:
 
     def fill_meta(self, host: np.ndarray, lay: MetaLayout, entries: list[Entry], rcs) -> None:
         """Write the step's metadata into `host` (int32, `lay.total` long, preset to -1)."""
-        ps = self.cache.page_size
-        T, S, P, G = lay.T, lay.S, lay.P, lay.G
-        ids, pos, tseq = lay.view(host, 0, T), lay.view(host, 1, T), lay.view(host, 2, T)
-        cu, kvl, sslot = lay.view(host, 3, S + 1), lay.view(host, 4, S), lay.view(host, 5, S)
-        rows = lay.view(host, 6, max(lay.n_rows, 1))
+        ids, rows = lay.view(host, 0, lay.T), lay.view(host, 6, max(lay.n_rows, 1))
+        counts = np.empty((2, lay.S), dtype=np.int32)
+        counts[0] = [rc.handle for rc in rcs]
+        counts[1] = q_lens = [len(e.tokens) for e in entries]
+        # positions, ranges, slots and tables by the native writer: row by row in Python they took 130 us of a step with 26 requests
+        cache = self.cache
+        code = cache._L.fill_step(cache._ptr, lay.S, counts[0].ctypes.data, counts[1].ctypes.data, lay.P, host.ctypes.data,
+                                  lay.offs.ctypes.data)
+        if code < 0:
+            raise StepError(f"step metadata could not be written (code {code})")
         r = q0 = 0
-        cu[0] = 0
-        for s, (e, rc) in enumerate(zip(entries, rcs)):
-            q = len(e.tokens)
-            start = rc.num_tokens
+        for e, q in zip(entries, q_lens):
             ids[q0:q0 + q] = e.tokens
-            pos[q0:q0 + q] = np.arange(start, start + q, dtype=np.int32)
-            tseq[q0:q0 + q] = s
-            cu[s + 1] = q0 + q
-            kvl[s] = start + q
-            sslot[s] = rc.state_slot
             for w in e.want:
                 rows[r] = q0 + w
                 r += 1
-            for g in range(G):
-                pages = rc.pages_array(g)
-                o = int(lay.offs[8 + 2 * g]) + s * P
-                host[o: o + len(pages)] = pages
-                p = pos[q0:q0 + q]
-                o = int(lay.offs[7 + 2 * g]) + q0
-                host[o: o + q] = pages[p // ps] * ps + p % ps
             q0 += q
         if lay.n_rows == 0:
             rows[0] = 0

@@ -111,9 +111,12 @@ class Backend:
         wider weight (the output head) gets the norm from its own kernel, once. So does a gate/up
         pair from 33 tokens on: its faster kernel there (tokens on the accumulator's rows, no ranges
         of K to merge) takes no norm in front (64 tokens: 14.8 us + the norm's 2 against 19.4)."""
-        if gate_up and isinstance(x, Normed) and x.shape[0] > 32:
+        if not isinstance(x, Normed):
             return False
-        if not (isinstance(x, Normed) and x._tensor is None and self._sm100 is not None and w.shape[0] % 4 == 0
+        T = x.shape[0]
+        if T > self._sm100.norm_max_tokens() or (gate_up and T > 32):        # a Normed exists on the serving path only
+            return False
+        if not (x._tensor is None and self._sm100 is not None and w.shape[0] % 4 == 0
                 and os.environ.get("RLLM_B200_NO_NORM_FUSION") != "1"
                 and self._sm100.norm_supported(x.h, x.weight, w, x.rows)):
             return False
@@ -153,7 +156,7 @@ class Backend:
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w):
             # a bias is added after the product (a small kernel): the product stays on the tensor cores
-            y = self._sm100.gemm(x, w, ops.EPI_STORE)
+            y = self._sm100.product(x, w, ops.EPI_STORE)
             return y if bias is None else ops.add_bias(y, bias)
         return ops.gemm_simt(x, w, ops.EPI_STORE, bias=bias)
 
@@ -164,14 +167,14 @@ class Backend:
             return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE_F32, rows=x.rows)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w):
-            return self._sm100.gemm(x, w, ops.EPI_STORE_F32)
+            return self._sm100.product(x, w, ops.EPI_STORE_F32)
         return ops.gemm_simt(x, w, ops.EPI_STORE_F32)
 
     def linear_residual(self, x, w, residual):
         """residual (float32, in place) += x W^T"""
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w):
-            return self._sm100.gemm(x, w, ops.EPI_ACCUM_F32, out=residual)
+            return self._sm100.product(x, w, ops.EPI_ACCUM_F32, out=residual)
         return ops.gemm_simt(x, w, ops.EPI_ACCUM_F32, out=residual)
 
     def linear_swiglu(self, x, w_gate_up):
@@ -180,7 +183,7 @@ class Backend:
             return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w_gate_up):
-            return self._sm100.gemm(x, w_gate_up, ops.EPI_SWIGLU)
+            return self._sm100.product(x, w_gate_up, ops.EPI_SWIGLU)
         return ops.gemm_simt(x, w_gate_up, ops.EPI_SWIGLU)
 
     # ---- position encoding + cache write, attention
@@ -215,7 +218,7 @@ class Backend:
             writes = cache.writes
             return self._sm100.gemm_qkv_rope(x, w_qkv, positions, inv_freq, cache.slots if writes else None,
                                              cache.k if writes else None, cache.v if writes else None,
-                                             nh, nkv, hd, cache.page_size, rot_dim, table=table)
+                                             nh, nkv, hd, cache.page_size, rot_dim, table=table, asked=True)
         qkv = self.linear(x, w_qkv, bias=bias)
         self.rope_cache_write(qkv, positions, inv_freq, cache, nh, nkv, hd, rot_dim, ctx=ctx, key=key)
         return qkv
@@ -375,7 +378,7 @@ class Backend:
             return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE, rows=x.rows, act=act)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w) and fuse:
-            return self._sm100.gemm(x, w, ops.EPI_STORE, act=act)            # in the product's store epilogue
+            return self._sm100.product(x, w, ops.EPI_STORE, act=act)         # in the product's store epilogue
         if act == "gelu_erf":
             return ops.gemm_simt(x, w, ops.EPI_GELU_ERF)
         if act == "gelu_tanh":
@@ -568,7 +571,7 @@ class Backend:
                 return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows, gelu_gate=True)
             x = x.tensor() if isinstance(x, Normed) else x
             if self._tc(x, w_gate_up):
-                return self._sm100.gemm(x, w_gate_up, ops.EPI_SWIGLU, gelu_gate=True)
+                return self._sm100.product(x, w_gate_up, ops.EPI_SWIGLU, gelu_gate=True)
         return self._hy.glu_act(self.linear_f32(x, w_gate_up, tag="gate_up"), self.dtype, act, limit, alpha)
 
     def experts_glu_up(self, x, w_gate_up, plan, act, limit=0.0, alpha=1.0, block=None):

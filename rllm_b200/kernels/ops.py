@@ -88,12 +88,14 @@ def _check(rc: int, what: str, launches: int = 1) -> None:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
-    """The current stream's handle (asked once per launch: the short way, where torch has it)."""
+    """The current stream's handle (asked once per launch: the short way, where torch has it; the device too, since
+    `torch.cuda.current_device` first asks whether CUDA is set up, which whoever holds a tensor there knows)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
 
 

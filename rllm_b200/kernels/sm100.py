@@ -53,6 +53,10 @@ _states: dict[int, _State] = {}
 
 
 def init(device) -> _State:
+    if type(device) is torch.device:
+        st = _states.get(device.index)             # every launch asks
+        if st is not None:
+            return st
     device = torch.device(device)
     idx = device.index if device.index is not None else torch.cuda.current_device()
     st = _states.get(idx)
@@ -113,10 +117,13 @@ def set_token_rows(on: bool) -> None:
 
 
 def gemm_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
-    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.dim() == 2 and w.dim() == 2
-            and x.stride(1) == 1 and w.is_contiguous() and x.shape[1] == w.shape[1]
-            and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
-            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.shape[0] > 0)
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        return False
+    xs, ws = x.shape, w.shape
+    if len(xs) != 2 or len(ws) != 2 or xs[1] != ws[1] or xs[1] % 8 or xs[0] <= 0:
+        return False
+    ld, one = x.stride()
+    return one == 1 and ld % 8 == 0 and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
 
 
 def out_supported(out: torch.Tensor) -> bool:
@@ -154,6 +161,16 @@ def gemm(x: torch.Tensor, w: torch.Tensor, epilogue: int, out: torch.Tensor | No
     code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0)
     if not gemm_supported(x, w):
         raise ops.KernelError("tc gemm: operands must be bfloat16, K a multiple of 8, 16-byte aligned")
+    return _product(x, w, epilogue, code, out, split)
+
+
+def product(x: torch.Tensor, w: torch.Tensor, epilogue: int, out: torch.Tensor | None = None, act: str | None = None,
+            gelu_gate: bool = False) -> torch.Tensor:
+    """`gemm` for a caller that has just asked `gemm_supported` about these operands (asking takes the host 4 us)."""
+    return _product(x, w, epilogue, epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0), out, True)
+
+
+def _product(x, w, epilogue, code, out, split):
     st = init(x.device)
     T, K = x.shape
     N = w.shape[0] // 2 if epilogue == ops.EPI_SWIGLU else w.shape[0]
@@ -269,11 +286,12 @@ def qkv_rope_supported(x: torch.Tensor, w: torch.Tensor, kcache, hd: int, rot_di
 def gemm_qkv_rope(x: torch.Tensor | None, w_qkv: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tensor,
                   slots: torch.Tensor | None, kcache: torch.Tensor | None, vcache: torch.Tensor | None,
                   nh: int, nkv: int, hd: int, page_size: int, rot_dim: int, split: bool = True,
-                  norm: tuple | None = None, table: torch.Tensor | None = None) -> torch.Tensor:
+                  norm: tuple | None = None, table: torch.Tensor | None = None, asked: bool = False) -> torch.Tensor:
     """qkv = x w_qkv^T with q and k rotated by position and k, v written to the paged cache at
     `slots` (None: no write), all in the product's epilogue. Returns qkv [T, (nh + 2 nkv) * hd].
     `norm` = (h, g, eps) instead of x: RMSNorm of the float rows h in front, in the same kernel.
-    `table`: `ops.rope_table` of these positions ([T, rot_dim / 2, 2]); else the angles are computed here."""
+    `table`: `ops.rope_table` of these positions ([T, rot_dim / 2, 2]); else the angles are computed here. `asked`: the caller
+    has just asked `qkv_rope_supported` about x, w_qkv and kcache."""
     T, K = norm[0].shape if norm is not None else x.shape
     # steps of at most 8 tokens: the weight-streaming kernel (any head size that is a multiple of 32)
     streamed = split and rot_dim == hd and stream_supported(EPI_QKV_ROPE, norm is not None, T, (nh + 2 * nkv) * hd, K, hd)
@@ -284,7 +302,7 @@ def gemm_qkv_rope(x: torch.Tensor | None, w_qkv: torch.Tensor, positions: torch.
             raise ops.KernelError("tc gemm with norm and rotary epilogue: sizes not supported")
         dev = h.device
     else:
-        if not (gemm_supported(x, w_qkv) and (128 % hd == 0 or streamed)
+        if not asked and not (gemm_supported(x, w_qkv) and (128 % hd == 0 or streamed)
                 and (kcache is None or kcache.dtype == torch.bfloat16)):
             raise ops.KernelError("tc gemm with rotary epilogue: bfloat16 operands and a head size dividing 128")
         dev = x.device
@@ -515,6 +533,22 @@ def attention_decode(q, kcache, vcache, kv_lens, block_table, nh, scale, window,
     return out
 
 
+def _mixed_step(ctx):
+    """Of a step whose first D sequences bring one token each (the scheduler puts decoding first) and the others more: (D, longest
+    portion of the others, most keys of the D, kv_lens of the D, cu_q and kv_lens of the others); else None. Worked out once a
+    forward pass."""
+    shared = getattr(ctx, "per_forward", {})
+    if "mixed" not in shared:
+        lens, keys = ctx.q_lens_host, ctx.kv_lens_host
+        D = 0
+        if lens is not None and keys is not None:
+            while D < len(lens) and lens[D] == 1:
+                D += 1
+        shared["mixed"] = (D, max(lens[D:]), max(keys[:D]), ctx.kv_lens[:D], ctx.cu_q[D:], ctx.kv_lens[D:]) \
+            if D and D < len(lens) else None
+    return shared["mixed"]
+
+
 def attention(q, cache, ctx, nh, scale, window):
     """The backend's hook: None when this kernel does not take the sizes at hand."""
     if not attention_supported(q, cache.k):
@@ -529,20 +563,15 @@ def attention(q, cache, ctx, nh, scale, window):
         # long portions over long contexts: tiles of 128 (token, head) rows x 128 keys on the tcgen05
         # tensor cores (measured against the mma.sync kernel, head size 64: level at 512 keys, 1.4 x at
         # 1,024, 2.3 x at 2,048; head size 128: 1.2 x at 512, 2 x at 1,024, 3.2 x at 2,048; behind at 256)
-        lens = ctx.q_lens_host
-        D = 0                    # sequences in front that bring one token each (the scheduler puts decoding first)
-        if lens is not None and ctx.kv_lens_host is not None and decode_supported(q, cache.k, nh):
-            while D < len(lens) and lens[D] == 1:
-                D += 1
-        if 0 < D < len(lens) and max(lens[D:]) * G >= 128:
+        mixed = _mixed_step(ctx)
+        if mixed is not None and mixed[1] * G >= 128 and decode_supported(q, cache.k, nh):
             # a mixed step: the decode kernel for the single tokens (a row tile of the other kernel
             # would hold one token's heads and nothing else), the portions after them on tcgen05
+            D, longest, most_keys, kv_single, cu_rest, kv_rest = mixed
             hd = cache.k.shape[3]
             out = torch.empty((q.shape[0], nh * hd), dtype=torch.bfloat16, device=q.device)
-            attention_decode(q[:D], cache.k, cache.v, ctx.kv_lens[:D], cache.block_table[:D], nh, scale, window,
-                             max(ctx.kv_lens_host[:D]), out=out[:D])
-            attention_prefill_tc(q, cache.k, cache.v, ctx.cu_q[D:], ctx.kv_lens[D:], cache.block_table[D:],
-                                 max(lens[D:]), nh, scale, window, out=out)
+            attention_decode(q[:D], cache.k, cache.v, kv_single, cache.block_table[:D], nh, scale, window, most_keys, out=out[:D])
+            attention_prefill_tc(q, cache.k, cache.v, cu_rest, kv_rest, cache.block_table[D:], longest, nh, scale, window, out=out)
             return out
         return attention_prefill_tc(q, cache.k, cache.v, ctx.cu_q, ctx.kv_lens, cache.block_table, ctx.max_q_len,
                                     nh, scale, window)
