@@ -253,6 +253,12 @@ __device__ __forceinline__ void epilogue8_sync() {            // the persistent 
   asm volatile("bar.sync 1, 256;" ::: "memory");
 }
 
+// A place in a ring of STAGES stages: the next one, and the phase's parity.
+template <int STAGES, int STEP = 1> struct RingPos {
+  uint32_t s, ph;
+  __device__ __forceinline__ void next() { s += STEP; if (s >= STAGES) { s -= STAGES; ph ^= 1u; } }
+};
+
 template <int BN, int EPI, bool NORM>
 __global__ void __launch_bounds__(THREADS_SMALL, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -315,33 +321,30 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       const uint64_t pol_w = policy_evict_first();   // weights are read once per step
       const uint64_t pol_x = policy_evict_last();    // the token tile is shared by every weight tile
       const int x0 = p.x_rows ? n0 / p.x_rows * p.x_gs : 0;
+      const uint32_t st0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
       // weights of the first stages do not depend on the kernel before this one
       const int pre = n_kb < C::STAGES ? n_kb : C::STAGES;
-      for (int i = 0; i < pre; ++i) {
-        uint8_t* st = smem + (size_t)i * C::STAGE_BYTES;
-        mbar_expect_tx(&full_bar[i], NORM ? W_BYTES : C::STAGE_BYTES);
-        const int k = (kb_begin + i) * BK;
-        tma_load_2d_hint(st, &tmap_w, &full_bar[i], k, n0, pol_w);
-        if (DUAL) tma_load_2d_hint(st + C::A_BYTES, &tmap_w, &full_bar[i], k, p.up_row0 + n0, pol_w);
+      int k = kb_begin * BK;
+      for (int i = 0; i < pre; ++i, k += BK) {
+        const uint32_t st = st0 + (uint32_t)(i * C::STAGE_BYTES), full = full0 + (uint32_t)(8 * i);
+        mbar_expect_tx(full, NORM ? W_BYTES : C::STAGE_BYTES);
+        tma_load_2d_hint(st, &tmap_w, full, k, n0, pol_w);
+        if (DUAL) tma_load_2d_hint(st + C::A_BYTES, &tmap_w, full, k, p.up_row0 + n0, pol_w);
       }
       if (!NORM) {
         pdl_wait();                                  // activations come from the kernel before
-        for (int i = 0; i < pre; ++i) {
-          uint8_t* st = smem + (size_t)i * C::STAGE_BYTES;
-          tma_load_2d_hint(st + W_BYTES, &tmap_x, &full_bar[i], x0 + (kb_begin + i) * BK, t0, pol_x);
-        }
+        for (int i = 0; i < pre; ++i)
+          tma_load_2d_hint(st0 + (uint32_t)(i * C::STAGE_BYTES) + W_BYTES, &tmap_x, full0 + (uint32_t)(8 * i), x0 + (kb_begin + i) * BK, t0, pol_x);
       }
       int issued = pre;
-      for (int i = pre; i < n_kb; ++i) {
-        const int s = i % C::STAGES;
-        const uint32_t ph = (uint32_t)(i / C::STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag)) { abort_flag = 1; record_failure(p.err, 1); break; }
-        uint8_t* st = smem + (size_t)s * C::STAGE_BYTES;
-        mbar_expect_tx(&full_bar[s], NORM ? W_BYTES : C::STAGE_BYTES);
-        const int k = (kb_begin + i) * BK;
-        tma_load_2d_hint(st, &tmap_w, &full_bar[s], k, n0, pol_w);
-        if (DUAL) tma_load_2d_hint(st + C::A_BYTES, &tmap_w, &full_bar[s], k, p.up_row0 + n0, pol_w);
-        if (!NORM) tma_load_2d_hint(st + W_BYTES, &tmap_x, &full_bar[s], x0 + k, t0, pol_x);
+      RingPos<C::STAGES> at{0u, 0u};
+      for (int i = pre; i < n_kb; ++i, k += BK, at.next()) {
+        if (!mbar_wait(empty0 + 8 * at.s, at.ph, &abort_flag)) { abort_flag = 1; record_failure(p.err, 1); break; }
+        const uint32_t st = st0 + at.s * C::STAGE_BYTES, full = full0 + 8 * at.s;
+        mbar_expect_tx(full, NORM ? W_BYTES : C::STAGE_BYTES);
+        tma_load_2d_hint(st, &tmap_w, full, k, n0, pol_w);
+        if (DUAL) tma_load_2d_hint(st + C::A_BYTES, &tmap_w, full, k, p.up_row0 + n0, pol_w);
+        if (!NORM) tma_load_2d_hint(st + W_BYTES, &tmap_x, full, x0 + k, t0, pol_x);
         issued = i + 1;
       }
       if (abort_flag) {
@@ -364,12 +367,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       // a descriptor moves with its address (16 bytes a unit): one is built, the rest are sums
       const uint64_t d0 = umma_desc_sw128(smem_u32(smem));
       bool ok = true;
-      for (int i = w; i < n_kb && ok; i += STEP) {
-        const int s = i % C::STAGES;
-        const uint32_t ph = (uint32_t)(i / C::STAGES) & 1u;
-        if (!mbar_wait(&full_bar[s], ph, &abort_flag)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      RingPos<C::STAGES, STEP> at{(uint32_t)w, 0u};
+      for (int i = w; i < n_kb; i += STEP, at.next()) {
+        if (!mbar_wait(full0 + 8 * at.s, at.ph, &abort_flag)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
         tc_fence_after();
-        const uint64_t da = d0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
+        const uint64_t da = d0 + at.s * (uint32_t)(C::STAGE_BYTES >> 4);
         const uint64_t db = da + (uint64_t)(W_BYTES >> 4);
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k) {
@@ -378,7 +381,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           umma_bf16(acc_addr, da + koff, db + koff, idesc, acc);
           if (DUAL) umma_bf16(acc_addr + BN, da + (uint64_t)(C::A_BYTES >> 4) + koff, db + koff, idesc, acc);
         }
-        umma_commit(&empty_bar[s]);      // the stage is free once these MMAs have read it
+        umma_commit(empty0 + 8 * at.s);      // the stage is free once these MMAs have read it
       }
       if (ok && n_kb > w) umma_commit(&acc_bar);      // this thread's accumulator set is complete
     }
@@ -1003,24 +1006,24 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     if (elect_one()) {
       const uint64_t pol_x = policy_evict_last();    // the token tiles are read by every weight tile
       pdl_wait();                                    // activations come from the kernel before
-      int it = 0, issued = 0;
+      const uint32_t st0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint32_t bytes = (uint32_t)(C::W_BYTES + bn * BK * 2);
+      int issued = 0;
       bool ok = true;
+      RingPos<C::STAGES> at{0u, 1u};                 // a stage's first filling waits for nothing: the parity of the phase before the first
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const int t0 = (tile % t_tiles) * bn, n0 = (tile / t_tiles) * WR;
         const int x0 = p.x_rows ? n0 / p.x_rows * p.x_gs : 0;
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-          if (it >= C::STAGES && !mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag)) {
+        for (int k = 0; k < n_kb * BK; k += BK, at.next()) {
+          if (!mbar_wait(empty0 + 8 * at.s, at.ph, &abort_flag)) {
             abort_flag = 1; record_failure(p.err, 5); ok = false; break;
           }
-          uint8_t* st = smem + (size_t)s * C::STAGE_BYTES;
-          mbar_expect_tx(&full_bar[s], (uint32_t)(C::W_BYTES + bn * BK * 2));
-          const int k = kb * BK;
-          tma_load_2d(st, &tmap_w, &full_bar[s], k, n0);
-          if (DUAL) tma_load_2d(st + C::A_BYTES, &tmap_w, &full_bar[s], k, p.up_row0 + n0);
-          tma_load_2d_hint(st + C::W_BYTES, &tmap_x, &full_bar[s], x0 + k, t0, pol_x);
-          issued = it + 1;
+          const uint32_t st = st0 + at.s * C::STAGE_BYTES, full = full0 + 8 * at.s;
+          mbar_expect_tx(full, bytes);
+          tma_load_2d(st, &tmap_w, full, k, n0);
+          if (DUAL) tma_load_2d(st + C::A_BYTES, &tmap_w, full, k, p.up_row0 + n0);
+          tma_load_2d_hint(st + C::W_BYTES, &tmap_x, full, x0 + k, t0, pol_x);
+          ++issued;
         }
       }
       if (abort_flag) {
@@ -1034,8 +1037,11 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
       // SWAP: the 128 tokens are the rows and the tile's 128 (64) gate and 128 (64) up weight rows, which
       // lie one after the other in a stage, the 256 (128) columns of one product
       const uint32_t idesc = SWAP ? umma_idesc_bf16(BM, 2 * WR) : umma_idesc_bf16(BM, bn);
-      int it = 0, ti = 0;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint64_t d0 = umma_desc_sw128(smem_u32(smem));     // a descriptor moves with its address, 16 bytes a unit
+      int ti = 0;
       bool ok = true;
+      RingPos<C::STAGES> at{0u, 0u};
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++ti) {
         const int buf = ti & 1, use = ti >> 1;
         if (use > 0 && !mbar_wait(&acc_empty[buf], (uint32_t)(use - 1) & 1u, &abort_flag)) {
@@ -1043,27 +1049,20 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         }
         tc_fence_after();
         const uint32_t acc_addr = tmem_base + (uint32_t)(buf * C::ACC_COLS);
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-          if (!mbar_wait(&full_bar[s], ph, &abort_flag)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
+        for (int kb = 0; kb < n_kb; ++kb, at.next()) {
+          if (!mbar_wait(full0 + 8 * at.s, at.ph, &abort_flag)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + (size_t)s * C::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + C::W_BYTES;
-          const uint64_t da = umma_desc_sw128(a_addr);
-          const uint64_t db = umma_desc_sw128(b_addr);
+          const uint64_t da = d0 + at.s * (uint32_t)(C::STAGE_BYTES >> 4);
+          const uint64_t db = da + (uint64_t)(C::W_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
             const uint64_t koff = (uint64_t)(k * UMMA_K * 2 / 16);
             if (SWAP) { umma_bf16(acc_addr, db + koff, da + koff, idesc, acc); continue; }
             umma_bf16(acc_addr, da + koff, db + koff, idesc, acc);
-            if (DUAL) {
-              const uint64_t du = umma_desc_sw128(a_addr + C::A_BYTES);
-              umma_bf16(acc_addr + BN, du + koff, db + koff, idesc, acc);
-            }
+            if (DUAL) umma_bf16(acc_addr + BN, da + (uint64_t)(C::A_BYTES >> 4) + koff, db + koff, idesc, acc);
           }
-          umma_commit(&empty_bar[s]);
+          umma_commit(empty0 + 8 * at.s);
         }
         if (ok) umma_commit(&acc_full[buf]);
       }
@@ -1182,9 +1181,10 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       // this CTA's first row of either operand in a tile
       auto w_row = [&](int tile) { const int n0 = tile / t_tiles * NT; return SWAP ? (rank == 0 ? n0 : p.up_row0 + n0) : n0 + (int)rank * BM; };
       auto x_row = [&](int tile) { return tile % t_tiles * bn + (int)rank * (SWAP ? BM : bn / 2); };
+      const uint32_t st0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), even0 = map_to_rank(full0, 0);
       auto copy = [&](bool weights, int s, int k, int y) {
-        uint8_t* st = smem + (size_t)s * C::STAGE_BYTES + (weights != SWAP ? 0 : C::A_BYTES);
-        tma_load_2d_pair(st, weights ? &tmap_w : &tmap_x, map_to_rank(smem_u32(&full_bar[s]), 0), k, y);
+        tma_load_2d_pair(st0 + (uint32_t)s * C::STAGE_BYTES + (weights != SWAP ? 0u : (uint32_t)C::A_BYTES), weights ? &tmap_w : &tmap_x,
+                         even0 + 8u * (uint32_t)s, k, y);
       };
       // the first stages' weights do not depend on the kernel before this one
       for (int i = 0; i < pre; ++i) {
@@ -1195,15 +1195,14 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       for (int i = 0; i < pre; ++i) copy(false, i, i % n_kb * BK, x_row(pair_id + i / n_kb * n_pairs));
       int it = pre, tile = pair_id + pre / n_kb * n_pairs, kb = pre % n_kb;
       int wy = w_row(tile), xy = x_row(tile);
-      for (; it < mine; ++it) {
-        const int s = it % C::STAGES;
-        const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag, PAIR_WAIT_CYCLES)) {
+      RingPos<C::STAGES> at{0u, 0u};                          // (this loop only runs where the first round has filled every stage)
+      for (; it < mine; ++it, at.next()) {
+        if (!mbar_wait(empty0 + 8 * at.s, at.ph, &abort_flag, PAIR_WAIT_CYCLES)) {
           abort_flag = 1; record_failure(p.err, 5, (int)rank); break;
         }
-        if (leader) mbar_expect_tx(&full_bar[s], stage_bytes);
-        copy(true, s, kb * BK, wy);
-        copy(false, s, kb * BK, xy);
+        if (leader) mbar_expect_tx(full0 + 8 * at.s, stage_bytes);
+        copy(true, (int)at.s, kb * BK, wy);
+        copy(false, (int)at.s, kb * BK, xy);
         if (++kb == n_kb) { kb = 0; tile += n_pairs; wy = w_row(tile); xy = x_row(tile); }
       }
       if (abort_flag && leader) {
@@ -1217,8 +1216,10 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (elect_one() && leader) {
       const uint32_t idesc = umma_idesc_bf16(2 * BM, SWAP ? 256 : bn);
       const uint64_t d0 = umma_desc_sw128(smem_u32(smem));
-      int it = 0, ti = 0;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      int ti = 0;
       bool ok = true;
+      RingPos<C::STAGES> at{0u, 0u};
       for (int tile = pair_id; tile < tiles && ok; tile += n_pairs, ++ti) {
         const int buf = ti & 1, use = ti >> 1;
         if (use > 0 && !mbar_wait(&acc_empty[buf], (uint32_t)(use - 1) & 1u, &abort_flag, PAIR_WAIT_CYCLES)) {
@@ -1226,18 +1227,16 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         tc_fence_after();
         const uint32_t acc_addr = tmem_base + (uint32_t)(buf * C::ACC_COLS);
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-          if (!mbar_wait(&full_bar[s], ph, &abort_flag, PAIR_WAIT_CYCLES)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
+        for (int kb = 0; kb < n_kb; ++kb, at.next()) {
+          if (!mbar_wait(full0 + 8 * at.s, at.ph, &abort_flag, PAIR_WAIT_CYCLES)) { abort_flag = 1; record_failure(p.err, 2); ok = false; break; }
           tc_fence_after();
-          const uint64_t da = d0 + (uint64_t)(s * (C::STAGE_BYTES >> 4)), db = da + (uint64_t)(C::A_BYTES >> 4);
+          const uint64_t da = d0 + at.s * (uint32_t)(C::STAGE_BYTES >> 4), db = da + (uint64_t)(C::A_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma_bf16_pair(acc_addr, da + (uint64_t)(k * UMMA_K * 2 / 16), db + (uint64_t)(k * UMMA_K * 2 / 16), idesc, kb > 0 || k > 0);
-          umma_commit_pair_both(&empty_bar[s]);      // the stage is free, in both CTAs
+          umma_commit_pair_both(empty0 + 8 * at.s);      // the stage is free, in both CTAs
         }
-        if (ok) umma_commit_pair_both(&acc_full[buf]);
+        if (ok) umma_commit_pair_both(smem_u32(&acc_full[buf]));
       }
     }
   } else {
