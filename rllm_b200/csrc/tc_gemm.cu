@@ -95,9 +95,9 @@ template <int BN, bool DUAL> struct Cfg {
   static constexpr int A_BYTES = BM * BK * 2;                  // 16 KB per weight tile
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_TILES * A_BYTES + B_BYTES;
-  // token tiles up to 64 (decode, small mixed steps) stay under half an SM's shared memory so
-  // that two kernels' CTAs are resident side by side; large tiles take what one CTA can have
-  static constexpr bool SMALL = BN <= 64;
+  // token tiles up to 32 (decode, small mixed steps) stay under half an SM's shared memory so
+  // that two kernels' CTAs are resident side by side; larger tiles take what one CTA can have
+  static constexpr bool SMALL = BN <= 32;
   // a landing area of its own only where it leaves an even number of stages (see TWO): tiles of 16 of
   // a single weight tile; the others land in the (by then idle) stage ring
   static constexpr bool DEDICATED = BN <= 16 && !DUAL;
@@ -1413,6 +1413,10 @@ int launch_bn(int bn, bool norm, const CUtensorMap& mw, const CUtensorMap& mx, c
     case 16: return launch<16, EPI, false>(mw, mx, p, grid, s);
     case 32: return launch<32, EPI, false>(mw, mx, p, grid, s);
   }
+  if constexpr (EPI != EPI_SWIGLU && EPI != EPI_QKV_ROPE) {            // see plan_ranges
+    if (bn == 64) return launch<64, EPI, false>(mw, mx, p, grid, s);
+    if (bn == 128) return launch<128, EPI, false>(mw, mx, p, grid, s);
+  }
   return ERR_BAD_SIZE;
 }
 
@@ -1514,6 +1518,25 @@ int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
   return best_bn;
 }
 
+// Ranges of K for token tiles of 64 (up to 128 tokens) and 128 (up to 256): how many of 2 or 4 CTAs of a cluster share an output tile,
+// or 0 where the other plans stand. A CTA takes in some 160 GB/s whatever it computes, so that a narrow weight on few CTAs waits
+// for its copies; merging the parts costs some 6 us with 64 tokens a tile and 10 with 128. So: the CTAs fit on the SMs at
+// once and fill three quarters of them, and the blocks of K that a CTA is spared (165 ns each) pay for the merge. Before / with
+// ranges, us: 2,048 x 8,192, 100 tokens 21.9 / 14.4, 192 25.6 / 19.6; 2,048 x 2,048, 100 tokens 13.9 / 9.7; 4,096 x 16,384, 64 tokens
+// 30.1 / 26.4, 100 46.9 / 32.0, 256 47.9 / 40.6; 4,096 x 4,096, 100 tokens 19.2 / 16.5, 64 tokens 15.0 / 14.3. Where the line leaves them: 2,048 x
+// 8,192, 64 tokens 12.7 / 14.2, 384 26.9 / 30.2; 4,096 x 4,096, 192 tokens 17.8 / 19.3; 2,048 x 2,048, 192 tokens 10.2 / 13.2.
+int plan_ranges(int epi, int T, int N, int K, int sm_count) {
+  if (T <= 32 || T > 256 || epi == EPI_SWIGLU || epi == EPI_QKV_ROPE) return 0;
+  const int bn = T <= 128 ? 64 : 128, kb = (K + BK - 1) / BK;
+  const long long tiles = (long long)((T + bn - 1) / bn) * ((N + BM - 1) / BM);
+  for (int ranges = 4; ranges >= 2; ranges >>= 1) {
+    const long long ctas = tiles * ranges;
+    if (ctas > sm_count || ctas * 4 < sm_count * 3LL || kb < 8 * ranges) continue;
+    return T <= 128 || (long long)(kb - kb / ranges) * 165 >= 12000 ? ranges : 0;
+  }
+  return 0;
+}
+
 // X null: the fused-norm variants (norm must be given, T <= NORM_MAX_T).
 int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void* W, void* Cout, long long ldc,
         int T, int N, int K, int allow_split, int* err, int sm_count, const RopeArgs* rope, void* stream, int x_rows = 0,
@@ -1533,6 +1556,8 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   int bn, splits;
   bool few;
   plan(epi, T, N, K, sm_count, allow_split, &bn, &splits, &few, norm != nullptr);
+  const int ranges = !norm && !x_rows && allow_split == 1 ? plan_ranges(epi, T, N, K, sm_count) : 0;
+  if (ranges) { few = true; bn = T <= 128 ? 64 : 128; splits = ranges; }
   const bool many = !few;            // the persistent kernel (no ranges of K, no norm in front)
   if (many && norm) return ERR_BAD_SIZE;
   const bool dual = epi == EPI_SWIGLU;
