@@ -48,10 +48,19 @@ __global__ void postnorm_kernel(float* __restrict__ h, const float* __restrict__
   }
 }
 
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
 // The same for rows of 4 * VPT * blockDim numbers at most: every thread keeps VPT float4 of the row in registers,
-// all of a row's loads are in flight together (a step of single tokens is a handful of rows: latency is all).
-template <typename TO, int VPT, bool OUT>
-__global__ void __launch_bounds__(1024) postnorm_vec_kernel(float* __restrict__ h, const float* __restrict__ y, int parts,
+// all of a row's loads are in flight together (a step of single tokens is a handful of rows: latency is all). Bound by its bytes
+// where rows are many: a CTA a row with up to four float4 a thread, so that several rows share an SM and one waits for its sum
+// while others load (2,047 rows of 4,096 with a copy 31.9 -> 25.6 us, 2,048 of 2,048 13.1 -> 11.2 against one
+// float4 a thread and a copy by 2 bytes).
+template <typename TO, int VPT, bool OUT, int MAXT>
+__global__ void __launch_bounds__(MAXT) postnorm_vec_kernel(float* __restrict__ h, const float* __restrict__ y, int parts,
                                                            const float* __restrict__ y2, const float* __restrict__ zg,
                                                            int zg_ld, float alpha, const float* __restrict__ w, int H,
                                                            float eps, TO* __restrict__ copy) {
@@ -64,11 +73,14 @@ __global__ void __launch_bounds__(1024) postnorm_vec_kernel(float* __restrict__ 
   const float4* yr = y ? reinterpret_cast<const float4*>(y + t * parts * H) : nullptr;
   const float4* y2r = y2 ? reinterpret_cast<const float4*>(y2 + t * H) : nullptr;
   float4 v[VPT], e[VPT], x[OUT ? VPT : 1];
+  constexpr bool AHEAD = MAXT <= 256;                // a CTA of 1,024 has no registers for the weights beside the row
+  float4 ww[AHEAD ? VPT : 1];
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     v[k] = i < n4 ? hr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     e[k] = (y2r && i < n4) ? y2r[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (AHEAD) ww[AHEAD ? k : 0] = i < n4 ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float g2 = (y2 && zg) ? 1.f / (1.f + expf(-zg[t * zg_ld])) : 1.f;
 #pragma unroll
@@ -97,17 +109,14 @@ __global__ void __launch_bounds__(1024) postnorm_vec_kernel(float* __restrict__ 
   for (int k = 0; k < VPT; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i < n4) {
-      const float4 ww = reinterpret_cast<const float4*>(w)[i];
-      float4 o = make_float4(v[k].x * r * ww.x, v[k].y * r * ww.y, v[k].z * r * ww.z, v[k].w * r * ww.w);
+      const float4 wk = AHEAD ? ww[AHEAD ? k : 0] : reinterpret_cast<const float4*>(w)[i];
+      float4 o = make_float4(v[k].x * r * wk.x, v[k].y * r * wk.y, v[k].z * r * wk.z, v[k].w * r * wk.w);
       if (OUT) {
         const float4 b = x[OUT ? k : 0];
         o = make_float4(fmaf(alpha, o.x, b.x), fmaf(alpha, o.y, b.y), fmaf(alpha, o.z, b.z), fmaf(alpha, o.w, b.w));
       }
       hr[i] = o;
-      if (copy) {
-        TO* c = copy + t * H + 4 * (size_t)i;
-        c[0] = from_f32<TO>(o.x); c[1] = from_f32<TO>(o.y); c[2] = from_f32<TO>(o.z); c[3] = from_f32<TO>(o.w);
-      }
+      if (copy) store4(copy + t * H + 4 * (size_t)i, o);
     }
   }
 }
@@ -115,15 +124,18 @@ __global__ void __launch_bounds__(1024) postnorm_vec_kernel(float* __restrict__ 
 template <typename TO, bool OUT>
 int launch_postnorm(float* h, const float* y, int parts, const float* y2, const float* zg, int zg_ld, float alpha,
                     const float* w, int T, int H, float eps, TO* copy, cudaStream_t s) {
-  const bool vec = H % 4 == 0 && !((uintptr_t)h & 15) && !((uintptr_t)y & 15) && !((uintptr_t)y2 & 15) && !((uintptr_t)w & 15);
+  const bool vec = H % 4 == 0 && !((uintptr_t)h & 15) && !((uintptr_t)y & 15) && !((uintptr_t)y2 & 15) && !((uintptr_t)w & 15) &&
+                   !((uintptr_t)copy & 15);
   if (vec && H <= 4 * 1024 * 4) {
     const int n4 = H / 4;
-    if (n4 <= 1024) {
-      const int threads = (n4 + 31) / 32 * 32;
-      return launch_ex(postnorm_vec_kernel<TO, 1, OUT>, dim3(T), dim3(threads), 0, s, 1, h, y, parts, y2, zg, zg_ld, alpha, w, H, eps, copy);
-    }
-    const int threads = ((n4 + 3) / 4 + 31) / 32 * 32;
-    return launch_ex(postnorm_vec_kernel<TO, 4, OUT>, dim3(T), dim3(threads), 0, s, 1, h, y, parts, y2, zg, zg_ld, alpha, w, H, eps, copy);
+    // by the row's length alone, so that a row's sum has the same order in every step
+#define RLLM_PN(VPT, MAXT) launch_ex(postnorm_vec_kernel<TO, VPT, OUT, MAXT>, dim3(T), dim3(((n4 + VPT - 1) / VPT + 31) / 32 * 32), 0, s, 1, h, y, parts, y2, zg, \
+                               zg_ld, alpha, w, H, eps, copy)
+    if (n4 <= 256) return RLLM_PN(1, 256);
+    if (n4 <= 512) return RLLM_PN(2, 256);
+    if (n4 <= 1024) return RLLM_PN(4, 256);
+    return RLLM_PN(4, 1024);
+#undef RLLM_PN
   }
   static bool done[64] = {};
   const int smem = H * (int)sizeof(float);
