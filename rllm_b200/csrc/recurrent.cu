@@ -71,7 +71,9 @@ __global__ void short_conv_kernel(const TI* __restrict__ x, long long ld, int co
 // Four taps (what every configuration here has), four neighbouring channels a thread, RUN tokens one after the other with
 // the last three inputs in registers: an input is read 1 + 3 / RUN times instead of four, in pieces of 8 or 16 bytes. The sums'
 // order is the kernel's above, so the bits are too. Bound by its bytes (2 or 4 in, 4 out a value): 2,048 tokens x 6,144 channels
-// of bfloat16 70.7 us with a token and a channel a thread.
+// of bfloat16 70.7 us with a token and a channel a thread. A run whose inputs all lie in its portion, which is nearly every one,
+// has them on their way together and asks nothing more about its tokens: 22.1 -> 20.3 us (8,192 channels 40.8 -> 36.0); what is left
+// beside the bytes is the silu.
 template <typename TI, int RUN>
 __global__ void __launch_bounds__(128) short_conv4_kernel(const TI* __restrict__ x, long long ld, int col0, int C,
                                                           const float* __restrict__ w, const float* __restrict__ bias,
@@ -92,6 +94,29 @@ __global__ void __launch_bounds__(128) short_conv4_kernel(const TI* __restrict__
   }
   const TI* xc = x + col0 + c;
   auto row = [&](int r) { return chunked::load4(xc + (long long)r * ld); };
+  if (RUN > 1 && t1 - t0 == RUN) {
+    const int s0 = token_seq[t0];
+    if (token_seq[t1 - 1] == s0 && t0 - 3 >= cu_q[s0]) {
+      float4 v[RUN + 3];
+#pragma unroll
+      for (int i = 0; i < RUN + 3; ++i) v[i] = row(t0 - 3 + i);
+#pragma unroll
+      for (int i = 0; i < RUN; ++i) {
+        float a[4] = {b[0], b[1], b[2], b[3]};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a[0] = fmaf(wt[0][j], v[i + j].x, a[0]); a[1] = fmaf(wt[1][j], v[i + j].y, a[1]);
+          a[2] = fmaf(wt[2][j], v[i + j].z, a[2]); a[3] = fmaf(wt[3][j], v[i + j].w, a[3]);
+        }
+        if (silu) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = a[e] / (1.f + expf(-a[e]));
+        }
+        *reinterpret_cast<float4*>(out + (long long)(t0 + i) * C + c) = make_float4(a[0], a[1], a[2], a[3]);
+      }
+      return;
+    }
+  }
   float4 in[4];                                           // inputs of rows t - 3 .. t
   in[0] = t0 >= 3 ? row(t0 - 3) : make_float4(0.f, 0.f, 0.f, 0.f);
   in[1] = t0 >= 2 ? row(t0 - 2) : make_float4(0.f, 0.f, 0.f, 0.f);
