@@ -353,26 +353,39 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
 
 // One CTA per token, a thread per (kv head c, four value columns): it reads A[g, c] of every head g once and adds it into
 // the outputs of the heads that use kv head c, HB of them at a time, each sum in the order of the heads. Bound by the parts'
-// bytes (2,048 tokens x 16 heads x 512: 29 us with a column a thread).
+// bytes (2,048 tokens x 16 heads x 512: 29 us with a column a thread). Single tokens over SPLITS ranges of keys are a few CTAs, whose
+// time is their chain of loads: with the ranges counted at compile time those of several heads are on their way together
+// (8 tokens, 16 heads
+// of 128 over 4 kv heads, three ranges: the decode step of two such layers and two others 359 -> 323 us).
 constexpr int HB = 4;
+template <int SPLITS>
 __global__ void __launch_bounds__(128) talk_mix_kernel(const float* __restrict__ parts, const float* __restrict__ mix,
-                                                       bf16* __restrict__ out, int nh, int nkv, int vd, int splits, int n_tokens,
+                                                       bf16* __restrict__ out, int nh, int nkv, int vd, int n_splits, int n_tokens,
                                                        const float* __restrict__ ml) {
+  const int splits = SPLITS > 0 ? SPLITS : n_splits;       // 0: more than eight ranges
+  constexpr int HELD = SPLITS > 0 ? SPLITS : 1;
   pdl_launch();
   pdl_wait();
   extern __shared__ float msm[];                    // [nh][nh], with ranges of keys their factors [splits][nh] behind
   for (int i = threadIdx.x; i < nh * nh; i += blockDim.x) msm[i] = mix[i];
   const int t = blockIdx.x, rep = nh / nkv;
   float* fac = msm + nh * nh;
-  if (splits > 1)
+  if constexpr (SPLITS != 1)
     for (int g = threadIdx.x; g < nh; g += blockDim.x) {
+      auto of = [&](int s) { return *reinterpret_cast<const float2*>(ml + (((size_t)s * n_tokens + t) * nh + g) * 2); };
+      float2 x[HELD];
+      if (SPLITS > 0)
+#pragma unroll
+        for (int s = 0; s < HELD; ++s) x[s] = of(s);
       float M = -INFINITY, L = 0.f;
-      for (int s = 0; s < splits; ++s) M = fmaxf(M, ml[(((size_t)s * n_tokens + t) * nh + g) * 2]);
+#pragma unroll
+      for (int s = 0; s < splits; ++s) M = fmaxf(M, SPLITS > 0 ? x[SPLITS > 0 ? s : 0].x : of(s).x);
+#pragma unroll
       for (int s = 0; s < splits; ++s) {
-        const float2 x = *reinterpret_cast<const float2*>(ml + (((size_t)s * n_tokens + t) * nh + g) * 2);
-        const float f = x.x == -INFINITY ? 0.f : fast_exp2(x.x - M);
+        const float2 y = SPLITS > 0 ? x[SPLITS > 0 ? s : 0] : of(s);
+        const float f = y.x == -INFINITY ? 0.f : fast_exp2(y.x - M);
         fac[s * nh + g] = f;
-        L = fmaf(x.y, f, L);
+        L = fmaf(y.y, f, L);
       }
       for (int s = 0; s < splits; ++s) fac[s * nh + g] *= L > 0.f ? 1.f / L : 0.f;
     }
@@ -385,16 +398,21 @@ __global__ void __launch_bounds__(128) talk_mix_kernel(const float* __restrict__
       float4 acc[HB];
 #pragma unroll
       for (int i = 0; i < HB; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
+#pragma unroll(SPLITS == 1 ? 8 : 4)
       for (int g = 0; g < nh; ++g) {
-        float4 a = *reinterpret_cast<const float4*>(A + ((size_t)g * nkv + c) * vd + d);
-        if (splits > 1) {
+        auto part = [&](int s) { return *reinterpret_cast<const float4*>(A + (((size_t)s * n_tokens * nh + g) * nkv + c) * vd + d); };
+        float4 x[HELD];
+#pragma unroll
+        for (int s = 0; s < HELD; ++s) x[s] = part(s);
+        float4 a = x[0];
+        if constexpr (SPLITS != 1) {
           const float f0 = fac[g];
           a = make_float4(a.x * f0, a.y * f0, a.z * f0, a.w * f0);
+#pragma unroll
           for (int s = 1; s < splits; ++s) {
             const float f = fac[s * nh + g];
-            const float4 x = *reinterpret_cast<const float4*>(A + (((size_t)s * n_tokens * nh + g) * nkv + c) * vd + d);
-            a.x = fmaf(x.x, f, a.x); a.y = fmaf(x.y, f, a.y); a.z = fmaf(x.z, f, a.z); a.w = fmaf(x.w, f, a.w);
+            const float4 y = SPLITS > 0 ? x[SPLITS > 0 ? s : 0] : part(s);
+            a.x = fmaf(y.x, f, a.x); a.y = fmaf(y.y, f, a.y); a.z = fmaf(y.z, f, a.z); a.w = fmaf(y.w, f, a.w);
           }
         }
 #pragma unroll
@@ -461,6 +479,19 @@ RLLM_API int rllm_talk_attention_mma(const void* q, long long q_stride, const vo
   else { if (few) GO(128, true) else GO(128, false) }
 #undef GO
   if (rc) return rc;
-  return launch_ex(talk_mix_kernel, dim3((unsigned)n_tokens), dim3(128), sizeof(float) * (nh * nh + (a.splits > 1 ? a.splits * nh : 0)), s, 1,
-                   (const float*)parts, mix, (bf16*)out, nh, nkv, vd, a.splits, n_tokens, (const float*)ml);
+  auto mixed = [&](auto kernel) {
+    return launch_ex(kernel, dim3((unsigned)n_tokens), dim3(128), sizeof(float) * (nh * nh + (a.splits > 1 ? a.splits * nh : 0)), s, 1,
+                     (const float*)parts, mix, (bf16*)out, nh, nkv, vd, a.splits, n_tokens, (const float*)ml);
+  };
+  switch (a.splits) {
+    case 1: return mixed(talk_mix_kernel<1>);
+    case 2: return mixed(talk_mix_kernel<2>);
+    case 3: return mixed(talk_mix_kernel<3>);
+    case 4: return mixed(talk_mix_kernel<4>);
+    case 5: return mixed(talk_mix_kernel<5>);
+    case 6: return mixed(talk_mix_kernel<6>);
+    case 7: return mixed(talk_mix_kernel<7>);
+    case 8: return mixed(talk_mix_kernel<8>);
+    default: return mixed(talk_mix_kernel<0>);
+  }
 }
