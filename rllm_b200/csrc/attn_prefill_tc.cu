@@ -70,7 +70,6 @@ static_assert(SOFTMAX_WARP0 * 32 * REGS_LOW + 4 * RT * 32 * REGS_HIGH <= 168 * T
                                  // are used: loader warp w always fills stage w (tiles w, w + 3, ...), so its waits
                                  // on that stage's barriers follow one another phase by phase; a warp that moved
                                  // between stages could be two phases ahead, which a parity cannot tell
-constexpr int SB = 3;            // S accumulators: one per row tile in its softmax, one being computed ahead
 constexpr int TMEM_COLS = 512;
 
 // Sizes that follow from the head sizes: keys of KD and values of VD numbers, 64 / 64, 128 / 128 or 192 / 128. Operands lie in
@@ -87,7 +86,13 @@ template <int KD, int VD> struct Shape {
   static constexpr int K_BYTES = HA * ATOM_KEYS, V_BYTES = VA * ATOM_KEYS;     // one tile
   static constexpr int Q_BYTES = HA * ATOM_ROWS;     // one row tile of Q
   static constexpr int SMEM_BYTES = 1024 + RT * Q_BYTES + KVS * (K_BYTES + V_BYTES);   // Q[2], K[KVS], V[KVS]
-  static constexpr int S_COL = 0, O_COL = SB * PN;   // TMEM: three S accumulators (P of a step in S's place), then the output of both row tiles
+  // TMEM: the S accumulators and P, then the output of both row tiles. Heads of 64: three accumulators that the steps take in turn, P of a
+  // step in S's place. Keys of 128 and more (BESIDE): an accumulator a row tile and P beside it, so that a row tile's next S is computed as
+  // soon as its scores are in registers, and not when the PV of the step three before is complete. 8,192 tokens: heads of 128
+  // 555 -> 497 us (2,048: 45.7 -> 42.3), heads of 64 410 -> 484.
+  static constexpr bool BESIDE = KD > 64;
+  static constexpr int SB = BESIDE ? RT : 3;
+  static constexpr int S_COL = 0, P_COL = BESIDE ? RT * PN : 0, O_COL = BESIDE ? RT * PN + RT * PN / 2 : SB * PN;
   static_assert(O_COL + RT * VD <= TMEM_COLS, "S and the outputs must fit in TMEM");
 };
 
@@ -200,7 +205,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   constexpr bool DENSE = MODE == DENSE_ROWS;
   static_assert(TMA || MODE == PLAIN, "the other forms come by tensor copies");
   typedef Shape<KD, VD> C;
-  constexpr int KVS = C::KVS;
+  constexpr int KVS = C::KVS, SB = C::SB;
+  constexpr bool BESIDE = C::BESIDE;
   extern __shared__ uint8_t pf_smem_raw[];
   __shared__ __align__(8) uint64_t kv_full[KVS], kv_empty[KVS], s_full[SB], s_free[SB], p_full[RT], pv_full[RT], q_full;
   __shared__ uint32_t tmem_base_slot;
@@ -255,7 +261,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   __syncthreads();                                      // everybody has left the item before
   if (threadIdx.x == 0) {
     for (int i = 0; i < KVS; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
-    for (int i = 0; i < SB; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 1); }
+    for (int i = 0; i < SB; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], BESIDE ? 4 : 1); }
     for (int i = 0; i < RT; ++i) { mbar_init(&p_full[i], 4); mbar_init(&pv_full[i], 1); }
     mbar_init(&q_full, TMA ? 4 * RT : RT);             // TMA: one arrival per softmax warp, which brings its own rows of Q
     fence_barrier_init();
@@ -307,21 +313,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   };
 
   if constexpr (!SOFTMAX) {
-  // ---- the products. Step k is (row tile g, K tile t); its S lands in accumulator k % 3.
+  // ---- the products. Step k is (row tile g, K tile t); its S lands in accumulator acc_of(k, g), used for the turn_of(k, t)-th time.
   constexpr uint32_t id_s = idesc(PM, PN, false);
   constexpr uint32_t id_pv = idesc(PM, 64, true);       // 64 output values at a time
   auto step = [&](int k, int& g, int& t) {
     if (k < 2 * n_both) { g = k & 1; t = k >> 1; } else { g = g_long; t = n_both + (k - 2 * n_both); }
   };
+  auto acc_of = [&](int k, int g) { return BESIDE ? g : k % SB; };
+  auto turn_of = [&](int k, int t) { return BESIDE ? t : k / SB; };
   // descriptors move with the address: 16 bytes are one unit of the start-address field
   const uint64_t dq0 = umma_desc_sw128(q_s), dk0 = umma_desc_sw128(k_s), dv0 = umma_desc_sw128(v_s);
   auto issue_s = [&](int k, bool& ok) {                 // S = Q K^T of step k (one thread)
     int g, t;
     step(k, g, t);
     const int ks = t % NST;
-    if (k >= SB) {
-      // the PV product of step k - 3 is complete: its P lay in the accumulator's place
-      if (!mbar_wait(&s_free[k % SB], (uint32_t)(k / SB - 1) & 1u, &abort_flag)) {
+    if (BESIDE ? t > 0 : k >= SB) {
+      // BESIDE: the row tile's threads have its scores before in their registers; else the PV product of step k - 3 is complete, whose P
+      // lay in the accumulator's place
+      if (!mbar_wait(&s_free[acc_of(k, g)], (uint32_t)(turn_of(k, t) - 1) & 1u, &abort_flag)) {
         abort_flag = 1; record_failure(p.err, 28, k); ok = false; return;
       }
     }
@@ -330,12 +339,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     }
     tc_fence_after();
     const uint64_t dq = dq0 + (uint64_t)(g * (C::Q_BYTES >> 4)), dk = dk0 + (uint64_t)(ks * (C::K_BYTES >> 4));
-    const uint32_t acc = tmem_base + C::S_COL + (uint32_t)(k % SB) * PN;
+    const uint32_t acc = tmem_base + C::S_COL + (uint32_t)acc_of(k, g) * PN;
 #pragma unroll
     for (int kk = 0; kk < KD / 16; ++kk)                // 16 values a product: atom kk / 4, 32 bytes on within it
       umma_bf16(acc, dq + (uint64_t)((kk >> 2) * (C::ATOM_ROWS >> 4) + (kk & 3) * 2),
                 dk + (uint64_t)((kk >> 2) * (C::ATOM_KEYS >> 4) + (kk & 3) * 2), id_s, kk > 0);
-    umma_commit(&s_full[k % SB]);
+    umma_commit(&s_full[acc_of(k, g)]);
   };
   auto issue_pv = [&](int k, bool& ok) {                // PV of step k, added to the row tile's output (one thread)
     int g, t;
@@ -346,7 +355,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     }
     tc_fence_after();
     const uint64_t dv = dv0 + (uint64_t)((t % NST) * (C::V_BYTES >> 4));
-    const uint32_t acc = tmem_base + C::O_COL + (uint32_t)g * VD, pa = tmem_base + C::S_COL + (uint32_t)(k % SB) * PN;
+    const uint32_t acc = tmem_base + C::O_COL + (uint32_t)g * VD, pa = tmem_base + (BESIDE ? C::P_COL + (uint32_t)g * (PN / 2) : C::S_COL + (uint32_t)(k % SB) * PN);
 #pragma unroll
     for (int a = 0; a < C::VA; ++a)                     // 64 output values = one atom of V
 #pragma unroll
@@ -355,7 +364,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         umma_bf16_ts(acc + (uint32_t)(a * 64), pa + (uint32_t)(ks * 8), dv + (uint64_t)(a * (C::ATOM_KEYS >> 4) + ks * (2048 >> 4)),
                      id_pv, t > 0 || ks > 0);
     umma_commit(&pv_full[g]);
-    umma_commit(&s_free[k % SB]);
+    if (!BESIDE) umma_commit(&s_free[k % SB]);
     if (g == 1 || t >= n_both) umma_commit(&kv_empty[t % NST]);     // the last reader of this K and V stage
   };
   if (warp < LOADERS && TMA) {
@@ -475,17 +484,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     }
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------ the PV products (one thread); without
-    // TMA the loaders are all busy and this thread issues S as well, three steps ahead
+    // TMA the loaders are all busy and this thread issues S as well
     if (elect_one() && n_tiles > 0) {
       bool ok = true;
+      const int ahead = BESIDE ? (n_both > 0 ? 2 : 1) : SB;       // without TMA: steps that S is ahead of PV
       if (!TMA)
-        for (int k = 0; k < SB && k < n_steps && ok; ++k) issue_s(k, ok);
+        for (int k = 0; k < ahead && k < n_steps && ok; ++k) issue_s(k, ok);
       for (int k = 0; k < n_steps && ok; ++k) {
-        issue_pv(k, ok);
-        if (!TMA && ok && k + SB < n_steps) issue_s(k + SB, ok);
+        if (!TMA && BESIDE && k + ahead < n_steps) issue_s(k + ahead, ok);
+        if (ok) issue_pv(k, ok);
+        if (!TMA && !BESIDE && ok && k + ahead < n_steps) issue_s(k + ahead, ok);
       }
-      // nothing of this item may still be on its way to a barrier when the next item sets them up again
-      for (int k = max(0, n_steps - SB); k < n_steps && ok; ++k)
+      // nothing of this item may still be on its way to a barrier when the next item sets them up again (BESIDE: S and the last PV have been
+      // waited for by the softmax warps)
+      for (int k = max(0, n_steps - SB); !BESIDE && k < n_steps && ok; ++k)
         if (!mbar_wait(&s_free[k % SB], (uint32_t)(k / SB) & 1u, &abort_flag)) {
           abort_flag = 1; record_failure(p.err, 29, k); ok = false;
         }
@@ -547,14 +559,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     for (int t = 0; t < n_mine; ++t) {
       const int j0 = tile_first(t);
       const int k = t < n_both ? 2 * t + g : 2 * n_both + (t - n_both);
-      const uint32_t s_addr = lane_addr + C::S_COL + (uint32_t)(k % SB) * PN;   // this step's S accumulator
-      if (!wait_on(&s_full[k % SB], (uint32_t)(k / SB) & 1u, 24, t)) { ok = false; break; }
+      const int sa = BESIDE ? g : k % SB;
+      const uint32_t s_addr = lane_addr + C::S_COL + (uint32_t)sa * PN;          // this step's S accumulator
+      const uint32_t p_addr = BESIDE ? lane_addr + C::P_COL + (uint32_t)g * (PN / 2) : s_addr;
+      if (!wait_on(&s_full[sa], (uint32_t)(BESIDE ? t : k / SB) & 1u, 24, t)) { ok = false; break; }
       tc_fence_after();
       // ---- the row's PN scores, the hidden ones -inf, and their maximum
       uint32_t v[NC][32];
 #pragma unroll
       for (int c = 0; c < NC; ++c) tmem_ld32(s_addr + 32 * c, v[c]);
       tmem_ld_wait();
+      if (BESIDE) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[g]);           // the row tile's next S may be computed
+      }
       if (CAP) {
         float far[NC];
 #pragma unroll
@@ -619,12 +638,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       const bool move = !sig && cand > m + 8.f;           // also the first visible key (m = -inf)
       float corr = 1.f;
       if (move) { corr = fast_exp2(m - cand); m = cand; l *= corr; }      // exp2(-inf) = 0
-      // PV of the tile before has to be complete only where the output is touched; else the wait comes behind the
-      // exponentials (a phase is never skipped, so that a parity says which one it is)
+      // PV of the tile before has to be complete where the output is touched, or (BESIDE) where its P lies in this one's place; else the
+      // wait comes behind the exponentials (a phase is never skipped, so that a parity says which one it is)
       auto pv_before = [&]() { return t == 0 || wait_on(&pv_full[g], (uint32_t)(t - 1) & 1u, 25, t); };
       const bool moves = __any_sync(0xffffffffu, move);
-      if (moves) {
+      if (BESIDE || moves) {
         if (!pv_before()) { ok = false; break; }
+      }
+      if (moves) {
         if (t > 0) {
           tc_fence_after();
 #pragma unroll
@@ -666,10 +687,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
             pk[i] = pack_bf16(e0, e1);
           }
         }
-        tmem_st16(s_addr + 16 * c, pk);
+        tmem_st16(p_addr + 16 * c, pk);
       }
       tmem_st_wait();
-      if (!moves && !pv_before()) { ok = false; break; }
+      if (!BESIDE && !moves && !pv_before()) { ok = false; break; }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[g]);
