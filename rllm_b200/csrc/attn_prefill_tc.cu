@@ -24,17 +24,21 @@
 //               heads of 64) against 431, 58 against 49 at 2,048; heads of 128 688 against 626, 60 against 55.
 //               What bounds a step is what its two warps a scheduler issue and wait for, not the
 //               exponentials' unit: a quarter of them on the FMA pipe (a polynomial) cost 441 and 689 us,
-//               an S accumulator a row tile with P beside it and the wait behind the packed results 471 and 646.
+//               an S accumulator a row tile with P beside it was slower too, but is faster at heads of 128 since one elected thread issues (Shape).
 //               The row's output stays in TMEM, where PV of tile after tile is added up. The
 //               exponentials are taken against a maximum that is moved only when the true one
 //               has grown by more than 2^8 since (P then stays below 2^8, which bf16 holds as
 //               well as values below 1); when it moves, the thread scales its row of the output
 //               in TMEM (tcgen05.ld / st) before the next PV is added.
 // The (row tile, K tile) steps are numbered k = 0, 1, ... in the order A0 B0 A1 B1 ...; S of step k
-// lands in accumulator k % 3 once PV of step k - 3, whose P lay there, is complete, so while both row tiles are in their softmax the scores of the step
+// lands in accumulator k % 3 (heads of 128: see Shape) once PV of step k - 3, whose P lay there, is complete, so while both row tiles are in their softmax the scores of the step
 // after are computed already, and a row tile that has written its P goes on at once: the four warp
 // schedulers always have a warp with work (two warps each, one of either tile).
 // TMEM: three S accumulators and PV of both tiles, 512 columns.
+// Where a work item's two row tiles lie: next to each other, or (`fold`) as far from one end of the sequence's rows as from the other. Items of
+// neighbours are as long as the keys they see, which balances where every CTA gets several; where the items are no more than the
+// SMs, the longest is the launch, and folded ones are all alike. 16 / 4 heads of 128 over
+// 2,048 tokens 42.3 -> 38.8 us, 512 over 512 with 32 / 8 heads of 64 15.0 -> 13.6; 16 heads of 192 / 128 over 2,048 62 -> 39.5 with both changes.
 // A key j is visible when j <= position of the row and j > position - window, or when j <= position and j <
 // keep_first (kept first keys): the tiles of the kept keys that the window's walk does not reach are walked first, then
 // the window's, as one list. With `sigmoid` a visible key's weight is sigmoid(score + bias[head]) in place of the
@@ -113,6 +117,7 @@ struct PfParams {
   float cap_z;           // scale / cap
   int box_rows;          // TMA variant: keys per copy = min(page size, 128)
   int row_pairs, num_seqs, sm_count;
+  int fold;              // an item's row tiles are the i-th from either end of the sequence's (no window, no blocks)
   int long_from;         // CROSS, DENSE: sequences with fewer rows are left out (another kernel's)
   float* cross;          // not null: every query head meets every kv head's values, and the output is the floats
                          // [token][query head][kv head of the values][VD] here
@@ -252,11 +257,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   for (int round = 0;; ++round) {
   const int item = round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
   if (item >= items) break;
-  const int tile0 = (p.row_pairs - 1 - item / (p.nkv * vheads * p.num_seqs)) * RT;      // first of the item's row tiles
+  const int place = item / (p.nkv * vheads * p.num_seqs);
   const int kvh = item % p.nkv, seq = (item / (p.nkv * vheads)) % p.num_seqs;
   const int vh = MODE == CROSS ? item / p.nkv % p.nkv : kvh;                         // the kv head of the values
-  // an item beyond its sequence's rows (a short portion beside long ones) is skipped by all threads alike
-  if (tile0 * PM >= (p.cu_q[seq + 1] - p.cu_q[seq]) * G) continue;
+  // the item's row tiles, the second at least as late as the first. An item beyond its sequence's rows (a short portion beside long
+  // ones) is skipped by all threads alike
+  const int n_rows = ((p.cu_q[seq + 1] - p.cu_q[seq]) * G + PM - 1) / PM;              // row tiles that the sequence has
+  int tile[RT];
+  if (p.fold) { tile[1] = n_rows - 1 - place; tile[0] = place < tile[1] ? place : n_rows; }
+  else { tile[0] = (p.row_pairs - 1 - place) * RT; tile[1] = tile[0] + 1; }
+  if (p.fold ? place > tile[1] : tile[0] >= n_rows) continue;
   if (MODE != PLAIN && p.cu_q[seq + 1] - p.cu_q[seq] < p.long_from) continue;
   __syncthreads();                                      // everybody has left the item before
   if (threadIdx.x == 0) {
@@ -279,15 +289,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   // before the window's first tile; a kept key inside the window's tiles is seen there).
   int kv_begin = 0, n_kept = 0, n_t[RT];
   {
-    const int p_min = kv_len - q_len + (tile0 * PM) / G;
+    const int p_min = kv_len - q_len + (min(tile[0], tile[1]) * PM) / G;
     int first = (p.window > 0 && p_min - p.window + 1 > 0) ? p_min - p.window + 1 : 0;
     if (p.chunk > 0) first = max(first, p_min / p.chunk * p.chunk);
     kv_begin = first / PN * PN;
     n_kept = min((min(p.keep_first, first) + PN - 1) / PN, kv_begin / PN);
 #pragma unroll
     for (int g = 0; g < RT; ++g) {
-      const bool active = (tile0 + g) * PM < rows_total;         // uniform: a row tile beyond the sequence's rows is empty
-      const int p_max = kv_len - q_len + min(q_len - 1, ((tile0 + g) * PM + PM - 1) / G);
+      const bool active = tile[g] < n_rows;                      // uniform: a row tile beyond the sequence's rows is empty
+      const int p_max = kv_len - q_len + min(q_len - 1, (tile[g] * PM + PM - 1) / G);
       n_t[g] = active ? n_kept + (p_max + 1 - kv_begin + PN - 1) / PN : 0;
     }
   }
@@ -302,7 +312,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
 #pragma unroll 4
     for (int i = 0; i < n / 4; ++i) {
       const int r = r0 + rbase + 4 * i;                  // row of the item: row tile r / 128, row r % 128 of it
-      const int row = tile0 * PM + r;
+      const int row = tile[r / PM] * PM + r % PM;
       const bool valid = row < rows_total;
       const int tok = valid ? row / G : 0, head = kvh * G + (valid ? row % G : 0);
       const bf16* src = p.q + (size_t)(q0 + tok) * p.q_stride + (size_t)head * KD + ch * 8;
@@ -514,7 +524,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     const int n_mine = n_t[g];
     const int quad = warp & 3;                            // the TMEM lanes this warp may read: 32 quad ...
     const int r = quad * 32 + lane;
-    const int row = (tile0 + g) * PM + r;
+    const int row = tile[g] * PM + r;
     const bool valid = row < rows_total;
     const int tok = valid ? row / G : 0, head = kvh * G + (valid ? row % G : 0);
     const int pos = valid ? kv_len - q_len + tok : kv_len - 1;      // a row beyond the sequence: zeros that look on like the last one's
@@ -901,6 +911,7 @@ RLLM_API int rllm_attention_prefill_tc(const void* q, int q_stride, const void* 
   if (items > 2147483647LL) return ERR_TOO_LARGE;
   int sms;
   if (int rc = multiprocessors(sm_count, sms)) return rc;
+  p.fold = p.window <= 0 && p.chunk <= 0 && p.row_pairs > 1 && items <= sms;
   const int ctas = items < sms ? (int)items : sms;
   // pages of a power of two from 8 keys up (whole 1 KB swizzle atoms) come by tensor copies
   const bool tma = p.page_shift >= 3 && (long long)num_pages * nkv <= 2147483647LL;
@@ -947,6 +958,7 @@ RLLM_API int rllm_attention_prefill_dense(const void* q, int q_stride, int q_hea
   if (items > 2147483647LL) return ERR_TOO_LARGE;
   int sms;
   if (int rc = multiprocessors(sm_count, sms)) return rc;
+  p.fold = p.window <= 0 && p.chunk <= 0 && p.row_pairs > 1 && items <= sms;
   const int ctas = items < sms ? (int)items : sms;
   CUtensorMap mk, mv, mr;
   int rc;
