@@ -481,11 +481,16 @@ def decode_supported(q: torch.Tensor, kcache: torch.Tensor, nh: int) -> bool:
     return attention_supported(q, kcache) and nh // nkv <= 16 and kcache.data_ptr() % 16 == 0
 
 
-def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int) -> int:
+def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: int = 64) -> int:
     """Ranges the keys of a sequence are cut into (= CTAs per cluster). Measured on a B200: a CTA
-    costs about as much as 1,150 keys before its first key and a range 30 more at the merge, two CTAs
-    fit an SM, and CTAs beyond that wait for a free place; the number of ranges with the least
-    (rounds of CTAs over the places) x (1,150 + keys per range) + 30 x ranges is taken. Up to 8
+    costs about as much as 1,150 keys before its first key and a range 65 more at the merge, two CTAs
+    fit an SM, and CTAs beyond that wait for a free place; a cluster's start and merge cost a decode step what 350 keys of heads of 64 do
+    with one sequence and 430 with four and more. The number of ranges with the least (rounds of CTAs over the places) x (1,150 + keys
+    per range) + 65 x ranges + a cluster's cost is taken. Decode steps of 16 layers with 8 kv heads, us, one range / the best number:
+    contexts of 300 1 sequence 554 / 565 (4), 8 sequences 604 / 639 (4); of 1,000 625 / 571 and 670 / 659; of 4,000 949 / 626 (8) and 1,012 / 742 (4).
+    Clusters of more than four CTAs need their places inside one GPC and start late where they come to more than four fifths of all
+    places (contexts of 1,000: 4 sequences 629 with 6 ranges, 670 with 8; 6 sequences 647 with 5, 704 with 6; 7 sequences 657 with 4, 712 with 5),
+    and threes beyond two thirds (10 sequences 841 with 2, 879 with 3); at heads of 128, whose ranges take longer, they do not show. Up to 8
     ranges any number; 12 and 16 (clusters beyond the portable size, for one or two long sequences:
     16,384 keys of one sequence 13.3 us against 18.3 with 8) only from 16,384 keys on and while the CTAs
     leave a quarter of the places free: a large cluster needs its places inside one GPC (9 ranges of 4
@@ -494,13 +499,16 @@ def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int) -> in
     alone, but the step at batch 1 0.621 ms against 0.615, at batch 2 0.692 against 0.642)."""
     base = max(1, num_seqs * nkv)
     places = 2 * sm_count
+    cluster = min(430, 320 + 4 * base) * 64 / hd
     best, best_cost = 1, None
     for s in (1, 2, 3, 4, 5, 6, 7, 8, 12, 16):
         if s > 1 and max_kv_len // s < 64:
             break
         if s > 8 and (base * s * 4 > places * 3 or max_kv_len < 16384):
             break
-        cost = -(-base * s // places) * (1150 + max_kv_len / s) + 30 * s
+        if hd == 64 and ((4 < s <= 8 and base * s * 16 > places * 13) or (s == 3 and base * s * 3 > places * 2)):
+            continue
+        cost = -(-base * s // places) * (1150 + max_kv_len / s) + 65 * s + (cluster if s > 1 else 0)
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
@@ -521,7 +529,7 @@ def attention_decode(q, kcache, vcache, kv_lens, block_table, nh, scale, window,
             or not vcache.is_contiguous() or block_table.dtype != torch.int32 or kv_lens.dtype != torch.int32:
         raise ops.KernelError("attention_decode: caches must be contiguous and alike, tables int32")
     if splits is None:
-        splits = decode_splits(S, nkv, max_kv_len, st.sm_count)
+        splits = decode_splits(S, nkv, max_kv_len, st.sm_count, hd)
     if out is None:
         out = torch.empty((S, nh * hd), dtype=torch.bfloat16, device=q.device)
     rc = ops._fn("sm100", "rllm_attention_decode")(
@@ -554,8 +562,9 @@ def attention(q, cache, ctx, nh, scale, window):
     if not attention_supported(q, cache.k):
         return None
     if ctx.max_q_len == 1 and decode_supported(q, cache.k, nh):
-        return attention_decode(q, cache.k, cache.v, ctx.kv_lens, cache.block_table, nh, scale, window,
-                                ctx.max_kv_len)
+        # a captured step serves contexts from half of its bound up to it: the number of ranges is chosen for those between
+        keys = ctx.max_kv_len * 3 // 4 if ctx.graph_safe and ctx.max_kv_len < 16384 else ctx.max_kv_len
+        return attention_decode(q, cache.k, cache.v, ctx.kv_lens, cache.block_table, nh, scale, window, keys)
     nkv = cache.k.shape[1]
     G = nh // nkv
     if ctx.max_q_len * G >= 128 and ctx.max_kv_len >= TC_ATTENTION_MIN_KEYS \
