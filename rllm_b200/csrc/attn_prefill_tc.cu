@@ -79,7 +79,7 @@ constexpr int TMEM_COLS = 512;
 // Sizes that follow from the head sizes: keys of KD and values of VD numbers, 64 / 64, 128 / 128 or 192 / 128. Operands lie in
 // shared memory as "atoms" of 128-byte rows (64 values), swizzled: a tile wider than 64 values is several atoms one after
 // the other. With keys of 192 the queries leave room for three stages.
-template <int KD, int VD> struct Shape {
+template <int KD, int VD, bool CAP = false> struct Shape {
   static_assert((KD == 64 && VD == 64) || (KD == 128 && VD == 128) || (KD == 192 && VD == 128), "head sizes");
   static constexpr int PN = KD == 64 ? 128 : 64;     // keys per tile (a V tile is 16 KB either way)
   static constexpr int KVS = KD == 192 ? 3 : 4;      // K/V stages
@@ -91,10 +91,10 @@ template <int KD, int VD> struct Shape {
   static constexpr int Q_BYTES = HA * ATOM_ROWS;     // one row tile of Q
   static constexpr int SMEM_BYTES = 1024 + RT * Q_BYTES + KVS * (K_BYTES + V_BYTES);   // Q[2], K[KVS], V[KVS]
   // TMEM: the S accumulators and P, then the output of both row tiles. Heads of 64: three accumulators that the steps take in turn, P of a
-  // step in S's place. Keys of 128 and more (BESIDE): an accumulator a row tile and P beside it, so that a row tile's next S is computed as
+  // step in S's place. Keys of 128 and more, unbounded (BESIDE): an accumulator a row tile and P beside it, so that a row tile's next S is computed as
   // soon as its scores are in registers, and not when the PV of the step three before is complete. 8,192 tokens: heads of 128
-  // 555 -> 497 us (2,048: 45.7 -> 42.3), heads of 64 410 -> 484.
-  static constexpr bool BESIDE = KD > 64;
+  // 555 -> 497 us (2,048: 45.7 -> 42.3), heads of 64 410 -> 484; bounded scores (CAP), heads of 128, 741 -> 853.
+  static constexpr bool BESIDE = KD > 64 && !CAP;
   static constexpr int SB = BESIDE ? RT : 3;
   static constexpr int S_COL = 0, P_COL = BESIDE ? RT * PN : 0, O_COL = BESIDE ? RT * PN + RT * PN / 2 : SB * PN;
   static_assert(O_COL + RT * VD <= TMEM_COLS, "S and the outputs must fit in TMEM");
@@ -209,7 +209,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
                        const __grid_constant__ CUtensorMap tmap_r, const PfParams p) {
   constexpr bool DENSE = MODE == DENSE_ROWS;
   static_assert(TMA || MODE == PLAIN, "the other forms come by tensor copies");
-  typedef Shape<KD, VD> C;
+  typedef Shape<KD, VD, CAP> C;
   constexpr int KVS = C::KVS, SB = C::SB;
   constexpr bool BESIDE = C::BESIDE;
   extern __shared__ uint8_t pf_smem_raw[];
@@ -833,7 +833,7 @@ int cache_map(CUtensorMap* out, const void* ptr, long long planes, int page_size
 template <int KD, int VD, bool TMA, bool CAP, int MODE>
 int launch_pf_c(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, const PfParams& p, int ctas, cudaStream_t s) {
   static bool configured[64] = {};
-  constexpr int smem = Shape<KD, VD>::SMEM_BYTES;
+  constexpr int smem = Shape<KD, VD, CAP>::SMEM_BYTES;
   if (allow_dynamic_smem(attn_prefill_tc_kernel<KD, VD, TMA, CAP, MODE>, smem, configured)) return -5;
   return launch_ex(attn_prefill_tc_kernel<KD, VD, TMA, CAP, MODE>, dim3(ctas), dim3(THREADS), smem, s, 1, mk, mv, mr, p);
 }
