@@ -1,19 +1,20 @@
-// Weight-streaming matrix product for steps of at most 8 tokens (decoding at small batch):
-//     C[T, N] = X[T, K] * W[N, K]^T,  T <= 8
+// Weight-streaming matrix product for steps of at most 8 tokens, some products of up to 16 (decoding at small batch):
+//     C[T, N] = X[T, K] * W[N, K]^T,  T <= 16
 //
 // At these sizes the product is a read of W and nothing else, so the kernel is built around the
 // read. A job is a slab of 16 weight rows (or a pair of slabs whose results meet in the epilogue:
 // gate and up rows for SwiGLU, a rotary pair d / d + hd/2 of a head for the q/k/v projection).
 // The 16 warps of a CTA split K between them; every warp copies its own pieces of the slab
 // (16 rows x 128 values of K = 4 KB a chunk) with cp.async into a ring of its own and multiplies with
-// mma.sync m16n8k16: weights are the A operand (16 rows), the tokens the B operand (n = 8). A lane's
+// mma.sync m16n8k16: weights are the A operand (16 rows), the tokens the B operand (n = 8; of 9 to 16 tokens two
+// groups, both multiplied with each fragment of weights as it is read). A lane's
 // 16-byte fragment read holds 8 consecutive values of K of one row; the contraction index is permuted
 // the same way on both operands, so no shuffle or ldmatrix is needed. The warps' partial sums meet in
 // shared memory, are added in warp order, and the epilogue runs one thread per output. There are no
 // thread-block clusters, no tensor memory and no barriers other than two __syncthreads a batch of
 // jobs: what a 16 KB tcgen05 tile costs in fixed work (allocation, mbarrier hand-overs, 50 ns an
 // issued MMA, the push to the column's owner) is what a step of 8 tokens spent its time on. The
-// tcgen05 kernels of tc_gemm.cu take over from 9 tokens.
+// tcgen05 kernels of tc_gemm.cu take over from 9 or 17 tokens (`streams_16`).
 //
 // The token operand is small and the same for every job, so a warp builds its fragments once,
 // after the predecessor has finished, and keeps them in registers (K up to 8,192), or fetches them
@@ -48,9 +49,9 @@ struct Cfg {
   static constexpr int WARPS = 16;
   static constexpr int THREADS = WARPS * 32;
   static constexpr int RING = 3;                 // chunks in flight per warp
-  static constexpr int BATCH = 2;                // jobs whose partial sums lie in shared memory together
+  static constexpr int SUMS = 4;                 // slabs' partial sums, of 8 tokens each, that lie in shared memory together
   static constexpr int RING_BYTES = WARPS * RING * CHUNK_BYTES;
-  static constexpr int RED_FLOATS = BATCH * 2 * WARPS * 16 * NT;
+  static constexpr int RED_FLOATS = SUMS * WARPS * 16 * NT;
   static constexpr int SMEM_BYTES = RING_BYTES + RED_FLOATS * 4;
 };
 
@@ -167,16 +168,18 @@ __device__ __forceinline__ void load_frag(const Params& p, int k0, int g, int t,
 // warp = two rows x four units) meet no bank twice. A lane reads what other lanes copied: every lane
 // waits for its own copies, then the warp meets (__syncwarp) before the reads and again before the
 // slot is refilled.
-template <int EPI, bool NORM, int NCH>
+template <int EPI, bool NORM, int NCH, int G>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 stream_gemm_kernel(const Params p) {
   typedef Cfg C;
-  constexpr int WARPS = C::WARPS, RING = C::RING, BATCH = C::BATCH, THREADS = C::THREADS;
+  constexpr int WARPS = C::WARPS, RING = C::RING, THREADS = C::THREADS;
   constexpr int TILES = (EPI == EPI_SWIGLU || EPI == EPI_QKV_ROPE) ? 2 : 1;
+  constexpr int BATCH = G == 1 ? 2 : C::SUMS / (TILES * G);       // jobs between two meetings of the warps
+  static_assert(BATCH >= 1 && BATCH * TILES * G <= C::SUMS);
   static_assert(!(NORM && NCH == 0), "norm in front needs resident fragments");
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float ss_red[WARPS][NT];
-  float* red = reinterpret_cast<float*>(smem + C::RING_BYTES);    // [job of batch][tile][warp][row][token]
+  __shared__ float ss_red[WARPS][NT * G];
+  float* red = reinterpret_cast<float*>(smem + C::RING_BYTES);    // [job of batch][tile][group][warp][row][token]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem) + warp * (RING * CHUNK_BYTES);
   const int nchw = NCH ? NCH : p.nchw;
@@ -208,22 +211,25 @@ stream_gemm_kernel(const Params p) {
   pdl_wait();                                    // the token operand does, and nothing is written before
 
   // ---- the token fragments
-  uint4 bres[NCH ? NCH : 1][4];
-  float ss = 0.f;
+  uint4 bres[NCH ? NCH : 1][G][4];
   if (NCH) {
 #pragma unroll
-    for (int ci = 0; ci < (NCH ? NCH : 1); ++ci) load_frag<NORM>(p, (warp * nchw + ci) * CK, g, t, bres[ci], ss);
-    if (NORM) {
-      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-      if (t == 0) ss_red[warp][g] = ss;
+    for (int q = 0; q < G; ++q) {
+      float ss = 0.f;
+#pragma unroll
+      for (int ci = 0; ci < (NCH ? NCH : 1); ++ci) load_frag<NORM>(p, (warp * nchw + ci) * CK, NT * q + g, t, bres[ci][q], ss);
+      if (NORM) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (t == 0) ss_red[warp][NT * q + g] = ss;
+      }
     }
   }
 
   int cslot = 0;
   // rows g and g + 8 have the parity of g: one key for both
   const uint32_t frag_off = (uint32_t)(g * 256), frag_key = (uint32_t)((g & 1) << 2);
-  auto consume = [&](float (&acc)[4], const uint4 (&b)[4]) {
+  auto consume = [&](float (&acc)[G][4], const uint4 (&b)[G][4]) {
     cp_wait<RING - 1>();
     __syncwarp();
     const uint32_t src = ring + cslot * CHUNK_BYTES + frag_off;
@@ -233,8 +239,11 @@ stream_gemm_kernel(const Params p) {
       uint4 lo, hi;
       asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "r"(a));
       asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "r"(a + 8 * 256));
-      mma16816(acc, lo.x, hi.x, lo.y, hi.y, b[kb].x, b[kb].y);
-      mma16816(acc, lo.z, hi.z, lo.w, hi.w, b[kb].z, b[kb].w);
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        mma16816(acc[q], lo.x, hi.x, lo.y, hi.y, b[q][kb].x, b[q][kb].y);
+        mma16816(acc[q], lo.z, hi.z, lo.w, hi.w, b[q][kb].z, b[q][kb].w);
+      }
     }
     cslot = cslot + 1 == RING ? 0 : cslot + 1;
     __syncwarp();                                // every lane has read the slot that is refilled now
@@ -244,51 +253,58 @@ stream_gemm_kernel(const Params p) {
   auto x_offset = [&](int j) -> long long {
     return p.x_rows ? (long long)((blockIdx.x + j * gridDim.x) * 16 / p.x_rows) * p.x_gs : 0;
   };
-  uint4 bcur[4], bnext[4];                       // NCH 0 only
-  if (!NCH && my_jobs > 0) {
+  uint4 bcur[G][4], bnext[G][4];                 // NCH 0 only
+  auto fetch = [&](int ci, long long xoff, uint4 (&b)[G][4]) {
     float unused = 0.f;
-    load_frag<false>(p, (warp * nchw) * CK, g, t, bcur, unused, x_offset(0));
-  }
+#pragma unroll
+    for (int q = 0; q < G; ++q) load_frag<false>(p, (warp * nchw + ci) * CK, NT * q + g, t, b[q], unused, xoff);
+  };
+  if (!NCH && my_jobs > 0) fetch(0, x_offset(0), bcur);
   for (int batch0 = 0; batch0 < my_jobs; batch0 += BATCH) {
     const int nb = min(BATCH, my_jobs - batch0);
     for (int jb = 0; jb < nb; ++jb) {
 #pragma unroll
       for (int tile = 0; tile < TILES; ++tile) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        float acc[G][4] = {};
         if (NCH) {
 #pragma unroll
           for (int ci = 0; ci < (NCH ? NCH : 1); ++ci) consume(acc, bres[ci]);
         } else {
-          float unused = 0.f;
           for (int ci = 0; ci < nchw; ++ci) {
             // the next chunk's fragments, one chunk ahead also across tiles and jobs
             const bool more = ci + 1 < nchw || tile + 1 < TILES || batch0 + jb + 1 < my_jobs;
             if (more) {
               const int nj = ci + 1 < nchw || tile + 1 < TILES ? batch0 + jb : batch0 + jb + 1;
-              load_frag<false>(p, (warp * nchw + (ci + 1 < nchw ? ci + 1 : 0)) * CK, g, t, bnext, unused, x_offset(nj));
+              fetch(ci + 1 < nchw ? ci + 1 : 0, x_offset(nj), bnext);
             }
             consume(acc, bcur);
 #pragma unroll
-            for (int kb = 0; kb < 4; ++kb) bcur[kb] = bnext[kb];
+            for (int q = 0; q < G; ++q)
+#pragma unroll
+              for (int kb = 0; kb < 4; ++kb) bcur[q][kb] = bnext[q][kb];
           }
         }
         // (a row's 8 token columns are stored with their index flipped by the row's group of four, red_col:
         // the epilogue's threads, 16 rows of one token side by side, then meet 16 different banks)
-        float* r = red + ((size_t)((jb * 2 + tile) * WARPS + warp)) * (16 * NT);
-        *reinterpret_cast<float2*>(r + g * NT + red_col(g, 2 * t)) = make_float2(acc[0], acc[1]);
-        *reinterpret_cast<float2*>(r + (g + 8) * NT + red_col(g + 8, 2 * t)) = make_float2(acc[2], acc[3]);
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+          float* r = red + ((size_t)(((jb * TILES + tile) * G + q) * WARPS + warp)) * (16 * NT);
+          *reinterpret_cast<float2*>(r + g * NT + red_col(g, 2 * t)) = make_float2(acc[q][0], acc[q][1]);
+          *reinterpret_cast<float2*>(r + (g + 8) * NT + red_col(g + 8, 2 * t)) = make_float2(acc[q][2], acc[q][3]);
+        }
       }
     }
     __syncthreads();
     // ---- the warps' parts in warp order, then the epilogue: thread = (job of batch, token, row of slab)
-    for (int e = threadIdx.x; e < nb * 128; e += THREADS) {
-      const int jb = e >> 7, tok = (e >> 4) & 7, r = e & 15;
+    for (int e = threadIdx.x; e < nb * (16 * NT * G); e += THREADS) {
+      const int jb = e / (16 * NT * G), tok = (e >> 4) & (NT * G - 1), r = e & 15;
       if (tok >= p.T) continue;
       float s0 = 0.f, s1 = 0.f;
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) {
-        s0 += red[(size_t)((jb * 2) * WARPS + w) * (16 * NT) + r * NT + red_col(r, tok)];
-        if (TILES == 2) s1 += red[(size_t)((jb * 2 + 1) * WARPS + w) * (16 * NT) + r * NT + red_col(r, tok)];
+        const float* part = red + (size_t)((jb * TILES * G + tok / NT) * WARPS + w) * (16 * NT) + r * NT + red_col(r, tok % NT);
+        s0 += part[0];
+        if (TILES == 2) s1 += part[G * WARPS * 16 * NT];
       }
       if (NORM) {
         float sq = 0.f;
@@ -345,23 +361,55 @@ stream_gemm_kernel(const Params p) {
 }
 
 // ------------------------------------------------------------------------------------ host side
-template <int EPI, bool NORM, int NCH>
+template <int EPI, bool NORM, int NCH, int G>
 int launch(const Params& p, int ctas, cudaStream_t s) {
   typedef Cfg C;
   static bool configured[64] = {};
-  if (allow_dynamic_smem(stream_gemm_kernel<EPI, NORM, NCH>, C::SMEM_BYTES, configured)) return -5;
-  return launch_ex(stream_gemm_kernel<EPI, NORM, NCH>, dim3(ctas), dim3(C::THREADS), C::SMEM_BYTES, s, 1, p);
+  if (allow_dynamic_smem(stream_gemm_kernel<EPI, NORM, NCH, G>, C::SMEM_BYTES, configured)) return -5;
+  return launch_ex(stream_gemm_kernel<EPI, NORM, NCH, G>, dim3(ctas), dim3(C::THREADS), C::SMEM_BYTES, s, 1, p);
+}
+
+// Which products of 9 to 16 tokens come here (microseconds a call at 16 tokens, calls back to back on weights out of L2;
+// here | the tcgen05 kernel). The weights' stream costs what it costs at 8 tokens; what grows is what a CTA has to
+// read of the tokens, once where its fragments stay in registers, with every job where they do not:
+//   into the residual, K up to 4,096 (two chunks of two groups resident): 2,048 x 2,048 3.7 | 4.7, 3,072 x 3,072 5.9 | 6.8,
+//     4,096 x 4,096 7.8 | 9.0; K up to 8,192 where a CTA has one job: 2,048 x 8,192 9.7 | 10.4, 2,048 x 5,440 7.3 | 8.0, but
+//     not beyond (2,048 x 14,336 16.0 | 14.6, 3,072 x 8,192 16.1 | 12.1);
+//   gate/up with the norm in front, K 2,048: 8,192 wide 12.9 | 16.6, 5,440 10.4 | 11.9, 1,024 5.6 | 5.7. Wider pairs have a tcgen05
+//     tile for each SM and more (16,384 wide: 24.8 | 23.7), and with two chunks the float rows are too much to read
+//     (10,880 x 4,096 35.6 | 34.0);
+//   gate/up without it: 8,192 x 2,048 10.8 | 15.3, 8,192 x 3,072 17.4 | 19.7, 14,336 x 4,096 36.3 | 39.4;
+//   q/k/v with rotation, 3,072 x 2,048: 6.5 | 7.5.
+// In a step of Llama 1B's shapes (all four): 9 requests at 300 874 -> 703 us, 12 at 1,300 905 -> 780, 16 at 2,000 950 -> 868.
+// The other stores stay where they were: with the norm in front they are level (2,048 x 2,048 5.5 | 5.3, 8,192 wide
+// 9.7 | 9.3), as is the head (80.8 | 81.5). At 9 tokens the lines lie at the same places.
+// Four groups (17 to 32 tokens, K 2,048) lose with the norm in front: a CTA then reads as many bytes of float rows as of
+// weights (gate/up 19.7 | 17.8 at 32 tokens, q/k/v 10.1 | 9.4; a step of 24 requests 1,065 us | 997).
+constexpr int SMS = 148;                         // of the one GPU that this is built for
+constexpr bool has_16(int epi) { return epi == EPI_ACCUM_F32 || epi == EPI_SWIGLU || epi == EPI_QKV_ROPE; }
+bool streams_16(int epi, bool norm, int N, int nchw, int hd) {
+  if (!has_16(epi) || (epi == EPI_QKV_ROPE && 128 % hd)) return false;    // heads that the tcgen05 kernel takes as well
+  if (nchw > (norm ? 1 : 2)) return epi == EPI_ACCUM_F32 && N / 16 <= SMS && nchw <= MAX_RESIDENT;
+  return !(norm && epi == EPI_SWIGLU) || N <= 64 * SMS;
 }
 
 template <int EPI, bool NORM>
 int launch_nch(const Params& p, int ctas, cudaStream_t s) {
-  switch (p.x_rows ? 0 : p.nchw) {               // operand columns that change from job to job: fragments chunk by chunk
-    case 1: return launch<EPI, NORM, 1>(p, ctas, s);
-    case 2: return launch<EPI, NORM, 2>(p, ctas, s);
-    case 3: return launch<EPI, NORM, 3>(p, ctas, s);
-    case 4: return launch<EPI, NORM, 4>(p, ctas, s);
+  if (p.T > NT) {                                // streams_16
+    if constexpr (has_16(EPI)) {
+      if (p.nchw == 1) return launch<EPI, NORM, 1, 2>(p, ctas, s);
+      if constexpr (!NORM) if (p.nchw == 2) return launch<EPI, false, 2, 2>(p, ctas, s);
+      if constexpr (EPI == EPI_ACCUM_F32 && !NORM) return launch<EPI, false, 0, 2>(p, ctas, s);
+    }
+    return ERR_BAD_SIZE;
   }
-  if constexpr (!NORM) return launch<EPI, false, 0>(p, ctas, s);
+  switch (p.x_rows ? 0 : p.nchw) {               // operand columns that change from job to job: fragments chunk by chunk
+    case 1: return launch<EPI, NORM, 1, 1>(p, ctas, s);
+    case 2: return launch<EPI, NORM, 2, 1>(p, ctas, s);
+    case 3: return launch<EPI, NORM, 3, 1>(p, ctas, s);
+    case 4: return launch<EPI, NORM, 4, 1>(p, ctas, s);
+  }
+  if constexpr (!NORM) return launch<EPI, false, 0, 1>(p, ctas, s);
   return ERR_BAD_SIZE;
 }
 
@@ -369,11 +417,11 @@ int chunks_per_warp(int K) { return ((K + CK - 1) / CK + Cfg::WARPS - 1) / Cfg::
 
 // Can the kernel take this problem? The rules the launchers below enforce.
 int supported(int epi, bool norm, int T, int N, int K, int hd) {
-  if (T < 1 || T > NT || N < 16 || N % 16 || K < 32 || K % 32) return 0;
+  if (T < 1 || T > 2 * NT || N < 16 || N % 16 || K < 32 || K % 32) return 0;
   if (epi < 0 || epi > EPI_QKV_ROPE) return 0;
   if (norm && (epi == EPI_ACCUM_F32 || chunks_per_warp(K) > MAX_RESIDENT)) return 0;
   if (epi == EPI_QKV_ROPE && (hd < 32 || hd % 32 || N % hd)) return 0;
-  return 1;
+  return T <= NT || streams_16(epi, norm, N, chunks_per_warp(K), hd);
 }
 
 int run(int epi, bool norm, Params& p, int sm_count, cudaStream_t s) {
@@ -416,7 +464,7 @@ RLLM_API int rllm_stream_gemm_supported(int epi, int norm, int T, int N, int K, 
   return supported(epi, norm != 0, T, N, K, hd);
 }
 
-// C[T, N] = X W^T for T <= 8. X: bf16 [T, K] with row stride ldx, or null: then X = rmsnorm(h[rows]; g, eps)
+// C[T, N] = X W^T for T <= 8, or 16 where `streams_16` says so. X: bf16 [T, K] with row stride ldx, or null: then X = rmsnorm(h[rows]; g, eps)
 // built inside the kernel from float rows h (stride ldh; rows null: row t). W: bf16 [N, K] contiguous
 // ([2N, K] for SwiGLU: gate rows, then up rows). Epilogues 0..3 as in rllm_tc_gemm.
 RLLM_API int rllm_stream_gemm(int epi, const void* X, long long ldx, const float* h, long long ldh, const int* rows,
@@ -445,7 +493,7 @@ RLLM_API int rllm_stream_gemm_mixes(const void* X, long long ldx, int x_rows, lo
   return run(EPI_STORE, false, p, sm_count, (cudaStream_t)stream);
 }
 
-// The q/k/v projection for T <= 8 with the rotation of q and k (pairs d, d + hd/2 of every head, the
+// The q/k/v projection for T <= 8, or 16 where `streams_16` says so, with the rotation of q and k (pairs d, d + hd/2 of every head, the
 // whole head rotated) and the write of k and v into the paged cache in its epilogue; arguments as in
 // rllm_tc_gemm_qkv_rope. Head size a multiple of 32.
 RLLM_API int rllm_stream_gemm_qkv_rope(const void* X, long long ldx, const float* h, long long ldh, const void* g,

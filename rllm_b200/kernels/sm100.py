@@ -94,9 +94,9 @@ _stream_ok: dict[tuple, bool] = {}
 
 
 def stream_supported(epilogue: int, norm: bool, T: int, N: int, K: int, hd: int = 0) -> bool:
-    """Does the weight-streaming kernel for steps of at most 8 tokens take this product? (N: output
-    features, of one half with the SwiGLU epilogue.)"""
-    if not STREAM or T > 8:
+    """Does the weight-streaming kernel for steps of at most 8 tokens, some products of up to 16, take this product? (N:
+    output features, of one half with the SwiGLU epilogue.)"""
+    if not STREAM or T > 16:
         return False
     key = (epilogue, norm, T, N, K, hd)
     ok = _stream_ok.get(key)
@@ -293,7 +293,7 @@ def gemm_qkv_rope(x: torch.Tensor | None, w_qkv: torch.Tensor, positions: torch.
     `table`: `ops.rope_table` of these positions ([T, rot_dim / 2, 2]); else the angles are computed here. `asked`: the caller
     has just asked `qkv_rope_supported` about x, w_qkv and kcache."""
     T, K = norm[0].shape if norm is not None else x.shape
-    # steps of at most 8 tokens: the weight-streaming kernel (any head size that is a multiple of 32)
+    # steps of at most 8 tokens: the weight-streaming kernel (any head size that is a multiple of 32), up to 16 for some K
     streamed = split and rot_dim == hd and stream_supported(EPI_QKV_ROPE, norm is not None, T, (nh + 2 * nkv) * hd, K, hd)
     if norm is not None:
         h, g, eps = norm
