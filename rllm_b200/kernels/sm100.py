@@ -486,10 +486,11 @@ def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: i
     costs about as much as 1,150 keys before its first key and a range 65 more at the merge, two CTAs
     fit an SM, and CTAs beyond that wait for a free place; a cluster's start and merge cost a decode step what 350 keys of heads of 64 do
     with one sequence and 430 with four and more. The number of ranges with the least (rounds of CTAs over the places) x (1,150 + keys
-    per range) + 65 x ranges (six at most: the merge of more
+    per range) + 65 x ranges (seven at most: the merge of more
     runs beside the last keys) + a cluster's cost is taken. Decode steps of 16 layers with 8 kv heads, us, one range / the best number:
     contexts of 300 1 sequence 554 / 565 (4), 8 sequences 604 / 639 (4); of 1,000 625 / 571 and 670 / 659; of 4,000 949 / 626 (8) and 1,012 / 742 (4).
-    One sequence by ranges: of 2,040 keys 602 with 4, 615 with 5, 594 with 6, 598 with 8; of 4,090 658, 639, 630, and 635 with 7, 624 with 8.
+    One sequence by ranges: of 2,040 keys 602 with 4, 615 with 5, 594 with 6, 598 with 8 (of about 1,100 570 with 5, 579 with 8,
+    under the same bound); of 4,090 658, 639, 630, and 635 with 7, 624 with 8.
     Clusters of more than four CTAs need their places inside one GPC and start late where they come to more than four fifths of all
     places (contexts of 1,000: 4 sequences 629 with 6 ranges, 670 with 8; 6 sequences 647 with 5, 704 with 6; 7 sequences 657 with 4, 712 with 5),
     and threes beyond two thirds (10 sequences 841 with 2, 879 with 3); at heads of 128, whose ranges take longer, they do not show. Up to 8
@@ -510,7 +511,7 @@ def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: i
             break
         if hd == 64 and ((4 < s <= 8 and base * s * 16 > places * 13) or (s == 3 and base * s * 3 > places * 2)):
             continue
-        cost = -(-base * s // places) * (1150 + max_kv_len / s) + 65 * min(s, 6) + (cluster if s > 1 else 0)
+        cost = -(-base * s // places) * (1150 + max_kv_len / s) + 65 * min(s, 7) + (cluster if s > 1 else 0)
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
