@@ -1538,6 +1538,24 @@ int plan_ranges(int epi, int T, int N, int K, int sm_count) {
   return 0;
 }
 
+// Which kernel runs a product, and on what tiles: the one place where that is decided, for the launcher and for who asks
+// (rllm_tc_gemm_plan). `norm`: RMSNorm in front; `mixes`: groups of weight rows with input columns of their own; `rows16`: 16-byte
+// pieces of an output row can be stored (what gate/up pairs with tokens on the rows and on pairs of CTAs need).
+struct Choice {
+  int bn, splits;      // tokens a tile, ranges of K
+  bool few, pair;      // the small-tile kernel; the persistent one on pairs of CTAs
+};
+Choice choose(int epi, int T, int N, int K, int sm_count, int allow_split, bool norm, bool mixes, bool rows16) {
+  Choice c{0, 1, false, false};
+  plan(epi, T, N, K, sm_count, allow_split, &c.bn, &c.splits, &c.few, norm);
+  if (const int ranges = !norm && !mixes && allow_split == 1 ? plan_ranges(epi, T, N, K, sm_count) : 0) {
+    c.few = true; c.bn = T <= 128 ? 64 : 128; c.splits = ranges;
+  }
+  if (g_pairs >= 0 && !c.few && !norm && !mixes && sm_count >= 2 && (epi != EPI_SWIGLU || rows16))
+    if (const int bn = plan_pairs(epi, T, N, K, c.bn, sm_count)) { c.bn = bn; c.pair = true; }
+  return c;
+}
+
 // X null: the fused-norm variants (norm must be given, T <= NORM_MAX_T).
 int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void* W, void* Cout, long long ldc,
         int T, int N, int K, int allow_split, int* err, int sm_count, const RopeArgs* rope, void* stream, int x_rows = 0,
@@ -1554,12 +1572,10 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   }
   int rc = get_encoder();
   if (rc) return rc;
-  int bn, splits;
-  bool few;
-  plan(epi, T, N, K, sm_count, allow_split, &bn, &splits, &few, norm != nullptr);
-  const int ranges = !norm && !x_rows && allow_split == 1 ? plan_ranges(epi, T, N, K, sm_count) : 0;
-  if (ranges) { few = true; bn = T <= 128 ? 64 : 128; splits = ranges; }
-  const bool many = !few;            // the persistent kernel (no ranges of K, no norm in front)
+  const bool rows16 = N % 8 == 0 && ldc % 8 == 0 && !((uintptr_t)Cout & 15);
+  const Choice ch = choose(epi, T, N, K, sm_count, allow_split, norm != nullptr, x_rows != 0, rows16);
+  const int bn = ch.bn, splits = ch.splits;
+  const bool many = !ch.few, pair = ch.pair;      // the persistent kernels (no ranges of K, no norm in front), on single CTAs or pairs
   if (many && norm) return ERR_BAD_SIZE;
   const bool dual = epi == EPI_SWIGLU;
   if (many && rope) {
@@ -1569,12 +1585,6 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   }
   CUtensorMap mw, mx;
   if ((rc = cached_map(&mw, W, dual ? 2LL * N : N, K, K, BM))) return rc;
-  // long portions on pairs of CTAs
-  const bool pairs_take = g_pairs >= 0 && !norm && !x_rows && sm_count >= 2 && many &&
-      (!dual || (N % 8 == 0 && ldc % 8 == 0 && !((uintptr_t)Cout & 15)));
-  const int pair_bn = pairs_take ? plan_pairs(epi, T, N, K, bn, sm_count) : 0;
-  const bool pair = pair_bn > 0;
-  if (pair) bn = pair_bn;
   if (norm) mx = mw;                                                 // not used by the kernel
   else if ((rc = make_map(&mx, X, T, x_rows ? (long long)((N - 1) / x_rows) * x_gs + K : K, ldx, pair ? (dual ? BM : bn / 2) : bn))) return rc;
   Params p;
@@ -1596,7 +1606,7 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
       case EPI_QKV_ROPE: return launch_pair<EPI_QKV_ROPE>(mw, mx, p, sm_count, s);
     }
   }
-  if (many && dual && g_token_rows && N % 8 == 0 && ldc % 8 == 0 && !((uintptr_t)Cout & 15)) {
+  if (many && dual && g_token_rows && rows16) {
     // tiles of 64 gate and 64 up rows where tiles of 128 would leave half of the SMs without one
     const long long tiles128 = (long long)((T + bn - 1) / bn) * ((N + BM - 1) / BM);
     if (tiles128 * 2 <= sm_count + sm_count / 8) {
@@ -1628,10 +1638,12 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
 
 }  // namespace
 
-// Token tile and ranges of K (= CTAs per cluster) the launcher would choose.
-RLLM_API int rllm_tc_gemm_plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_out,
-                               int* splits_out) {
-  plan(epi, T, N, K, sm_count, allow_split, bn_out, splits_out);
+// What the launcher runs (`choose`): tokens a tile, ranges of K (= CTAs per cluster), and whether on pairs of CTAs. Output rows are taken to
+// be contiguous and aligned.
+RLLM_API int rllm_tc_gemm_plan(int epi, int T, int N, int K, int sm_count, int allow_split, int norm, int* bn_out, int* splits_out,
+                               int* pair_out) {
+  const Choice c = choose(epi, T, N, K, sm_count, allow_split, norm != 0, false, N % 8 == 0);
+  *bn_out = c.bn; *splits_out = c.splits; *pair_out = c.pair;
   return 0;
 }
 

@@ -98,8 +98,10 @@ def cmd_gemm(a) -> None:
         else:
             x = torch.randn(T, K, device=DEV, dtype=torch.bfloat16)
             fns = [(lambda w=w: sm100.gemm(x, w, epi, out=out, split=split)) for w in ws]
-        bn, sp = sm100.plan(epi, T, N, K, split=split)
-        run(fns, a.plain, f"gemm {epi_name} T={T} N={N} K={K} tile={bn} ranges={sp}" + (" norm" if a.norm else ""),
+        bn, sp, pair = sm100.launch_plan(epi, T, N, K, sm100.init(DEV).sm_count, split, a.norm)
+        streamed = split and sm100.stream_supported(epi, a.norm, T, N, K)
+        how = "streamed" if streamed else f"tile={bn} ranges={sp}" + (" pairs" if pair else "")
+        run(fns, a.plain, f"gemm {epi_name} T={T} N={N} K={K} {how}" + (" norm" if a.norm else ""),
             nbytes=rows * K * 2, flops=2.0 * T * rows * K)
     sm100.check_error(DEV)
 

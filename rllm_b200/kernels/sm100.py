@@ -15,7 +15,7 @@ ops.register_signatures("sm100", {
     "rllm_tc_gemm_mixes": [_P, c_longlong, c_int, c_int, _P, _P, c_longlong, c_int, c_int, c_int, _P, c_int, _P],
     "rllm_tc_gemm_set_pairs": [c_int],
     "rllm_tc_gemm_set_token_rows": [c_int],
-    "rllm_tc_gemm_plan": [c_int, c_int, c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int)],
+    "rllm_tc_gemm_plan": [c_int, c_int, c_int, c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int)],
     "rllm_tc_gemm_norm": [c_int, _P, c_longlong, _P, _P, c_int, c_float, _P, _P, c_longlong, c_int, c_int, c_int,
                           c_int, _P, c_int, _P],
     "rllm_tc_gemm_norm_max_tokens": [],
@@ -131,13 +131,18 @@ def out_supported(out: torch.Tensor) -> bool:
     return out.stride(1) == 1 and out.data_ptr() % 16 == 0 and out.stride(0) * out.element_size() % 16 == 0
 
 
+def launch_plan(epilogue: int, T: int, N: int, K: int, sm_count: int, split: bool | int = True, norm: bool = False) -> tuple[int, int, bool]:
+    """(tokens a tile, ranges of K = CTAs per cluster, on pairs of CTAs?) of what the tcgen05 launcher runs for a product on a GPU
+    of `sm_count` SMs. `split`: False one CTA per tile, True its own choice, a number > 1 that many ranges. (The rotary
+    epilogue's number is `EPI_QKV_ROPE`; products that the streaming kernel takes first are not the launcher's: `stream_supported`.)"""
+    bn, sp, pair = c_int(), c_int(), c_int()
+    ops._fn("sm100", "rllm_tc_gemm_plan")(epilogue, T, N, K, sm_count, int(split), int(norm), byref(bn), byref(sp), byref(pair))
+    return bn.value, sp.value, bool(pair.value)
+
+
 def plan(epilogue: int, T: int, N: int, K: int, device="cuda:0", split: bool | int = True) -> tuple[int, int]:
-    """(token tile, ranges of K = CTAs per cluster) the tcgen05 launcher chooses for a problem.
-    `split`: False one CTA per tile, True its own choice, a number > 1 that many ranges."""
-    st = init(device)
-    bn, sp = c_int(), c_int()
-    ops._fn("sm100", "rllm_tc_gemm_plan")(epilogue, T, N, K, st.sm_count, int(split), byref(bn), byref(sp))
-    return bn.value, sp.value
+    """(tokens a tile, ranges of K) of `launch_plan` on this device."""
+    return launch_plan(epilogue, T, N, K, init(device).sm_count, split)[:2]
 
 
 ACT_RELU2 = 1 << 8          # added to the store epilogue's number: max(value, 0)^2 is stored

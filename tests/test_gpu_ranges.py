@@ -16,11 +16,17 @@ def rel(a, b):
     return float((a.float() - b.float()).abs().max()) / max(float(b.abs().max()), 1e-30)
 
 
+# the sizes below that wide tiles and ranges of K take; the others lie behind the rule's lines
+RANGED = [(65, 2048, 2048), (100, 2048, 8192), (127, 4096, 1096), (33, 4096, 2048), (64, 4096, 4104), (129, 2048, 8192), (192, 2044, 8200),
+          (256, 4096, 16384)]
+
+
 @pytest.mark.parametrize("T,N,K", [(65, 2048, 2048), (100, 2048, 8192), (128, 2048, 1000), (127, 4096, 1096), (33, 4096, 2048), (64, 4096, 4104),
                                    (129, 2048, 8192), (192, 2044, 8200), (256, 4096, 16384), (255, 1924, 5440), (256, 2048, 4096), (257, 2048, 8192),
                                    (32, 4096, 2048), (100, 4740, 2048), (97, 1800, 520), (96, 2048, 448)])
 def test_ranges_of_wide_tiles(T, N, K):
     from rllm_b200.kernels import ops, sm100
+    assert (sm100.plan(ops.EPI_STORE, T, N, K) in ((64, 2), (64, 4), (128, 2), (128, 4))) == ((T, N, K) in RANGED)
     x, w = rnd(T, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
     ref = x.float() @ w.float().t()
     res = torch.randn(T, N, generator=torch.Generator().manual_seed(3)).to(DEV)

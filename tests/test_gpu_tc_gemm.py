@@ -256,14 +256,21 @@ def test_plan_splits_small_batches_only():
     bn, splits = sm100.plan(ops.EPI_STORE, 8, 3072, 2048)
     assert bn == 16 and 2 <= splits <= 8                 # 24 tiles: a cluster of ranges of K per tile
     assert sm100.plan(ops.EPI_ACCUM_F32, 64, 2048, 8192) == (32, 8)      # two tiles of 32 tokens
-    assert sm100.plan(ops.EPI_ACCUM_F32, 128, 2048, 8192) == (32, 8)     # a narrow weight keeps its ranges of K
-    assert sm100.plan(ops.EPI_ACCUM_F32, 129, 2048, 8192) == (64, 1)
+    assert sm100.plan(ops.EPI_ACCUM_F32, 128, 2048, 8192) == (64, 4)     # a narrow weight keeps its ranges of K
+    assert sm100.plan(ops.EPI_ACCUM_F32, 129, 2048, 8192) == (128, 4)
+    assert sm100.plan(ops.EPI_ACCUM_F32, 257, 2048, 8192) == (64, 1)
     assert sm100.plan(ops.EPI_STORE, 128, 3072, 2048) == (64, 1)
     assert sm100.plan(ops.EPI_STORE, 8, 3072, 2048, split=False) == (16, 1)
-    # long portions: the tile width that fills whole waves of 148 CTAs (288 tiles of 176 tokens; 144 of 240)
-    assert sm100.plan(ops.EPI_STORE, 2048, 3072, 2048) == (176, 1)
-    assert sm100.plan(ops.EPI_ACCUM_F32, 2048, 2048, 8192) == (240, 1)
-    assert sm100.plan(ops.EPI_SWIGLU, 2048, 8192, 2048) == (128, 1)
+    # long portions on single CTAs: the tile width that fills whole waves of 148 (288 tiles of 176 tokens; 144 of 240); on pairs a
+    # gate/up tile has 256 tokens
+    sm100.set_pairs(-1)
+    try:
+        assert sm100.plan(ops.EPI_STORE, 2048, 3072, 2048) == (176, 1)
+        assert sm100.plan(ops.EPI_ACCUM_F32, 2048, 2048, 8192) == (240, 1)
+        assert sm100.plan(ops.EPI_SWIGLU, 2048, 8192, 2048) == (128, 1)
+    finally:
+        sm100.set_pairs(False)
+    assert sm100.plan(ops.EPI_SWIGLU, 2048, 8192, 2048) == (256, 1)
     assert sm100.plan(ops.EPI_SWIGLU, 96, 8192, 2048) == (128, 1)        # tokens on the accumulator's rows from 65 on
     assert sm100.plan(ops.EPI_SWIGLU, 64, 8192, 2048) == (128, 1)        # and from 33 on where no norm is in front
     assert sm100.plan(ops.EPI_SWIGLU, 32, 8192, 2048) == (32, 2)

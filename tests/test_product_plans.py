@@ -1,0 +1,35 @@
+"""Which kernel the tcgen05 launcher runs for a product (no GPU: the choice is made on the host), on either side of each of its lines."""
+import pytest
+
+from rllm_b200.kernels import ops, sm100
+
+STORE, F32, ACCUM, SWIGLU, ROPE = ops.EPI_STORE, ops.EPI_STORE_F32, ops.EPI_ACCUM_F32, ops.EPI_SWIGLU, sm100.EPI_QKV_ROPE
+SMS = 148
+
+
+@pytest.mark.parametrize("epi,T,N,K,want", [
+    # ranges of K with tiles of 64 and 128 tokens: a narrow weight of a long K
+    (ACCUM, 64, 2048, 8192, (32, 8, False)), (ACCUM, 100, 2048, 8192, (64, 4, False)), (ACCUM, 128, 2048, 8192, (64, 4, False)),
+    (ACCUM, 129, 2048, 8192, (128, 4, False)), (ACCUM, 256, 2048, 8192, (128, 4, False)), (ACCUM, 257, 2048, 8192, (64, 1, False)),
+    (ACCUM, 100, 4096, 16384, (64, 2, False)), (ACCUM, 256, 4096, 16384, (128, 2, False)), (STORE, 100, 2048, 2048, (64, 4, False)),
+    # ... and not where too few SMs would have a CTA, or the ranges would not pay for their merge
+    (ACCUM, 192, 2048, 2048, (64, 1, False)), (ACCUM, 192, 4096, 4096, (64, 1, False)), (STORE, 128, 3072, 2048, (64, 1, False)),
+    (ROPE, 100, 2048, 8192, (32, 8, False)), (SWIGLU, 64, 2048, 8192, (32, 8, False)),
+    # pairs of CTAs: more than 128 tokens, where the model of both kernels says so
+    (SWIGLU, 128, 8192, 2048, (128, 1, False)), (SWIGLU, 129, 8192, 2048, (256, 1, True)), (SWIGLU, 2048, 8192, 2048, (256, 1, True)),
+    (ACCUM, 643, 2048, 2048, (80, 1, False)), (ACCUM, 643, 2048, 8192, (80, 1, False)), (ACCUM, 1905, 2048, 8192, (224, 1, True)),
+    (ACCUM, 2834, 2048, 8192, (160, 1, True)), (ROPE, 128, 3072, 2048, (64, 1, False)), (SWIGLU, 2048, 8191, 2048, (128, 1, False)),
+])
+def test_the_launchers_choice(epi, T, N, K, want):
+    assert sm100.launch_plan(epi, T, N, K, SMS) == want
+
+
+def test_no_ranges_and_no_pairs_where_they_are_not_asked_for():
+    assert sm100.launch_plan(ACCUM, 128, 2048, 8192, SMS, split=False)[1] == 1
+    assert sm100.launch_plan(STORE, 64, 3072, 2048, SMS, norm=True) == sm100.launch_plan(STORE, 64, 3072, 2048, SMS, split=True)
+    sm100.set_pairs(-1)
+    try:
+        assert sm100.launch_plan(SWIGLU, 2048, 8192, 2048, SMS) == (128, 1, False)
+        assert sm100.launch_plan(STORE, 2048, 3072, 2048, SMS) == (176, 1, False)
+    finally:
+        sm100.set_pairs(False)
