@@ -22,8 +22,8 @@
 // bf16(h * g) built from the float residual stream, the warps add up h^2 on the way and the
 // epilogue multiplies by rsqrt(mean + eps), as the tcgen05 kernel does.
 //
-// Programmatic dependent launch: the kernel lets its successor start at once and copies its first
-// weight chunks (which no kernel writes) before it waits for its predecessor; a successor's CTA takes an
+// Programmatic dependent launch: the kernel lets its successor start at once and copies its first weight chunks before
+// it waits for its predecessor, where the caller says that no earlier launch writes them (`w_fixed`); a successor's CTA takes an
 // SM as soon as this kernel's CTA there has left.
 //
 // Reference counterparts: matvec_bf16 (src/gpu/cuda/shaders/matmul.cu:49-77), fused_gate_up_swiglu
@@ -82,6 +82,7 @@ struct Params {
   long long ldc;
   int T;
   int act;                  // gate/up epilogue: 2 gelu in its tanh form for silu; store epilogue: 1 stores max(value, 0)^2, 2 gelu(value) in its tanh form, 3 in its erf form
+  int w_fixed;              // no launch that may still be running writes W: its copies need not wait for the kernel in front
   int njobs;
   int nchw;                 // chunks per warp and tile
   RopeArgs rope;
@@ -205,8 +206,9 @@ stream_gemm_kernel(const Params p) {
     cp_commit();
     pslot = pslot + 1 == RING ? 0 : pslot + 1;
   };
+  if (!p.w_fixed) pdl_wait();
 #pragma unroll
-  for (int i = 0; i < RING; ++i) produce();      // weights do not depend on the kernel before this one
+  for (int i = 0; i < RING; ++i) produce();      // weights do not depend on the kernel before this one, unless the caller could not say so
 
   pdl_wait();                                    // the token operand does, and nothing is written before
 
@@ -466,11 +468,11 @@ RLLM_API int rllm_stream_gemm_supported(int epi, int norm, int T, int N, int K, 
 
 // C[T, N] = X W^T for T <= 8, or 16 where `streams_16` says so. X: bf16 [T, K] with row stride ldx, or null: then X = rmsnorm(h[rows]; g, eps)
 // built inside the kernel from float rows h (stride ldh; rows null: row t). W: bf16 [N, K] contiguous
-// ([2N, K] for SwiGLU: gate rows, then up rows). Epilogues 0..3 as in rllm_tc_gemm.
+// ([2N, K] for SwiGLU: gate rows, then up rows). Epilogues 0..3, activations and bit 16 (W fixed) as in rllm_tc_gemm.
 RLLM_API int rllm_stream_gemm(int epi, const void* X, long long ldx, const float* h, long long ldh, const int* rows,
                               const void* g, int g_dt, float eps, const void* W, void* Cout, long long ldc,
                               int T, int N, int K, int sm_count, void* stream) {
-  const int act = epi >> 8;                       // as in rllm_tc_gemm: 0 | 1 << 8 stores max(value, 0)^2, 0 | 2 << 8 gelu(value), 0 | 3 << 8 its erf form
+  const int act = (epi >> 8) & 0xff, w_fixed = (epi >> 16) & 1;      // as in rllm_tc_gemm: 0 | 1 << 8 stores max(value, 0)^2, 0 | 2 << 8 gelu(value), 0 | 3 << 8 its erf form
   epi &= 0xff;
   if (epi < 0 || epi > EPI_SWIGLU || act > 3 || (act && epi != EPI_STORE && !(epi == EPI_SWIGLU && act == 2))) return ERR_BAD_SIZE;
   const bool norm = X == nullptr;
@@ -478,18 +480,19 @@ RLLM_API int rllm_stream_gemm(int epi, const void* X, long long ldx, const float
   Params p = {};
   p.W = (const bf16*)W; p.N = N; p.K = K; p.up_row0 = N; p.x = (const bf16*)X; p.ldx = ldx;
   p.h = h; p.ldh = ldh; p.rows = rows; p.g = g; p.g_is_bf16 = g_dt == DT_BF16; p.eps = eps;
-  p.C = Cout; p.ldc = ldc; p.T = T; p.act = act;
+  p.C = Cout; p.ldc = ldc; p.T = T; p.act = act; p.w_fixed = w_fixed;
   return run(epi, norm, p, sm_count, (cudaStream_t)stream);
 }
 
 // C[T, N] = one product per group of weight rows, T <= 8: rows n of W in group n / x_rows multiply X's columns from
-// (n / x_rows) * x_gs on (the last group may be shorter). bf16, store epilogue; x_rows and N multiples of 16, x_gs of 8.
+// (n / x_rows) * x_gs on (the last group may be shorter). bf16, store epilogue; x_rows and N multiples of 16, x_gs of 8. No launch
+// that may still be running writes W.
 RLLM_API int rllm_stream_gemm_mixes(const void* X, long long ldx, int x_rows, long long x_gs, const void* W, void* Cout,
                                     long long ldc, int T, int N, int K, int sm_count, void* stream) {
   if (x_rows <= 0 || x_rows % 16 || x_gs % 8) return ERR_BAD_SIZE;
   Params p = {};
   p.W = (const bf16*)W; p.N = N; p.K = K; p.x = (const bf16*)X; p.ldx = ldx; p.x_rows = x_rows; p.x_gs = x_gs;
-  p.C = Cout; p.ldc = ldc; p.T = T;
+  p.C = Cout; p.ldc = ldc; p.T = T; p.w_fixed = 1;
   return run(EPI_STORE, false, p, sm_count, (cudaStream_t)stream);
 }
 
@@ -500,14 +503,14 @@ RLLM_API int rllm_stream_gemm_qkv_rope(const void* X, long long ldx, const float
                                        int g_dt, float eps, const void* W, void* QKV, long long ldc, int T, int K,
                                        const int* positions, const float* inv_freq, const void* cos_sin,
                                        const int* slots, void* kcache, void* vcache, int nh, int nkv, int hd,
-                                       int page_size, int sm_count, void* stream) {
+                                       int page_size, int w_fixed, int sm_count, void* stream) {
   if (hd <= 0 || nh <= 0 || nkv <= 0 || page_size <= 0) return ERR_BAD_SIZE;
   const bool norm = X == nullptr;
   if (norm && (!h || !g || (g_dt != DT_F32 && g_dt != DT_BF16))) return ERR_BAD_SIZE;
   Params p = {};
   p.W = (const bf16*)W; p.N = (nh + 2 * nkv) * hd; p.K = K; p.x = (const bf16*)X; p.ldx = ldx;
   p.h = h; p.ldh = ldh; p.rows = nullptr; p.g = g; p.g_is_bf16 = g_dt == DT_BF16; p.eps = eps;
-  p.C = QKV; p.ldc = ldc; p.T = T;
+  p.C = QKV; p.ldc = ldc; p.T = T; p.w_fixed = w_fixed;
   p.rope.positions = positions; p.rope.inv_freq = inv_freq; p.rope.cos_sin = (const float2*)cos_sin;
   p.rope.slots = slots; p.rope.kcache = (bf16*)kcache; p.rope.vcache = (bf16*)vcache;
   p.rope.nh = nh; p.rope.nkv = nkv; p.rope.hd = hd; p.rope.page_size = page_size;

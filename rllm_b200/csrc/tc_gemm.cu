@@ -37,8 +37,8 @@
 // lands in the (by then idle) stage ring after one more cluster barrier.
 //
 // Programmatic dependent launch: the kernel lets its successor start at once, and itself
-// fetches its first weight tiles (which no earlier kernel writes) before it waits for its
-// predecessor; activations are read and outputs written only after that wait. Small token
+// fetches its first weight tiles before it waits for its predecessor where the caller says that
+// no earlier launch writes them (`w_fixed`; else it waits first); activations are read and outputs written only after that wait. Small token
 // tiles keep their shared memory under half an SM's, so that the successor's CTAs find room
 // beside them and their weight tiles are already on the way when the predecessor ends.
 //
@@ -156,6 +156,7 @@ struct Params {
   int x_rows, x_gs;   // x_rows > 0: weight rows in groups of that many (a multiple of BM), group g reads X's columns from g * x_gs on
   int act;            // store epilogue: 0 the value as it is, 1 max(value, 0)^2, 2 gelu in its tanh form, 3 gelu in its erf form;
                       // gate/up epilogue: what the gate passes, 0 silu, 2 gelu in its tanh form
+  int w_fixed;        // no launch that may still be running writes W: its copies need not wait for the kernel in front
   RopeArgs rope;
   NormArgs norm;      // NORM variants only
 };
@@ -322,7 +323,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       const uint64_t pol_x = policy_evict_last();    // the token tile is shared by every weight tile
       const int x0 = p.x_rows ? n0 / p.x_rows * p.x_gs : 0;
       const uint32_t st0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
-      // weights of the first stages do not depend on the kernel before this one
+      // weights of the first stages do not depend on the kernel before this one, unless the caller could not say so
+      if (!p.w_fixed) pdl_wait();
       const int pre = n_kb < C::STAGES ? n_kb : C::STAGES;
       int k = kb_begin * BK;
       for (int i = 0; i < pre; ++i, k += BK) {
@@ -1114,7 +1116,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 // and `acc_full` barriers; both CTAs' epilogue warps arrive at the even CTA's `acc_empty`. Both CTAs
 // allocate and free TMEM, and meet at a cluster barrier before they free it and leave, so that no
 // signal or MMA ever addresses a CTA that is gone. Every wait is bounded.
-// The weights' copies of the first stages are issued before the wait for the kernel in front.
+// The weights' copies of the first stages are issued before the wait for the kernel in front (`w_fixed`).
 struct PairCfg {
   static constexpr int A_BYTES = BM * BK * 2;                    // this CTA's 128 rows
   static constexpr int B_BYTES = BM * BK * 2;                    // its half of the columns' operand, up to 128 rows
@@ -1186,7 +1188,8 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         tma_load_2d_pair(st0 + (uint32_t)s * C::STAGE_BYTES + (weights != SWAP ? 0u : (uint32_t)C::A_BYTES), weights ? &tmap_w : &tmap_x,
                          even0 + 8u * (uint32_t)s, k, y);
       };
-      // the first stages' weights do not depend on the kernel before this one
+      // the first stages' weights do not depend on the kernel before this one, unless the caller could not say so
+      if (!p.w_fixed) pdl_wait();
       for (int i = 0; i < pre; ++i) {
         if (leader) mbar_expect_tx(&full_bar[i], stage_bytes);
         copy(true, i, i % n_kb * BK, w_row(pair_id + i / n_kb * n_pairs));
@@ -1558,7 +1561,7 @@ Choice choose(int epi, int T, int N, int K, int sm_count, int allow_split, bool 
 
 // X null: the fused-norm variants (norm must be given, T <= NORM_MAX_T).
 int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void* W, void* Cout, long long ldc,
-        int T, int N, int K, int allow_split, int* err, int sm_count, const RopeArgs* rope, void* stream, int x_rows = 0,
+        int T, int N, int K, int allow_split, int* err, int sm_count, const RopeArgs* rope, void* stream, bool w_fixed, int x_rows = 0,
         int x_gs = 0) {
   if (T <= 0 || N <= 0) return 0;
   if (K <= 0 || K % 8) return ERR_BAD_SIZE;                          // TMA: strides multiple of 16 bytes
@@ -1591,6 +1594,7 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
   p.C = Cout; p.ldc = (int)ldc; p.T = T; p.N = N; p.K = K; p.up_row0 = N; p.splits = splits; p.err = err; p.bn = bn;
   p.act = epi == EPI_STORE || epi == EPI_SWIGLU ? t_store_act : 0;
   p.x_rows = x_rows; p.x_gs = x_gs;
+  p.w_fixed = w_fixed;
   p.rope = rope ? *rope : RopeArgs{};
   p.norm = norm ? *norm : NormArgs{};
   dim3 grid((T + bn - 1) / bn, (N + BM - 1) / BM, splits);
@@ -1652,9 +1656,11 @@ RLLM_API int rllm_tc_gemm_set_token_rows(int on) { g_token_rows = on != 0; retur
 
 // The store epilogue (0) may carry an activation in the bits above the epilogue's number: epi = 0 | 1 << 8 stores
 // max(value, 0)^2, 0 | 2 << 8 gelu(value) in its tanh form, 0 | 3 << 8 in its erf form; the gate/up epilogue (3) gelu in its
-// tanh form for silu, 3 | 2 << 8. The launcher's own state for one call:
+// tanh form for silu, 3 | 2 << 8. Bit 16: no launch that may still be running writes W (`w_fixed`). The launcher's own state for one call:
 struct StoreAct {
-  explicit StoreAct(int& epi) {
+  bool w_fixed;
+  explicit StoreAct(int& epi) : w_fixed((epi >> 16) & 1) {
+    epi &= ~(1 << 16);
     const int act = epi >> 8, e = epi & 0xff;
     const bool fine = act == 0 || (e == EPI_STORE && act <= 3) || (e == EPI_SWIGLU && act == 2);
     t_store_act = fine ? act : 0;
@@ -1666,27 +1672,27 @@ struct StoreAct {
 // X: [T, K] bf16, row stride ldx; W: [N, K] bf16 contiguous ([2N, K] for SwiGLU: gate rows then up
 // rows); C: [T, N] with row stride ldc, bf16 (store, SwiGLU) or float (store-float, accumulate).
 // allow_split 0: one CTA per output tile whatever the size; 1: the launcher's choice of ranges of K;
-// n > 1: n ranges where ranges are allowed. Returns 0, or a negative refusal.
+// n > 1: n ranges where ranges are allowed. Without bit 16 of epi W may come from the launch just before. Returns 0, or a negative refusal.
 RLLM_API int rllm_tc_gemm(int epi, const void* X, long long ldx, const void* W, void* Cout, long long ldc,
                           int T, int N, int K, int allow_split, int* err, int sm_count, void* stream) {
   const StoreAct sa(epi);
   if (epi < 0 || epi > 3 || !X) return ERR_BAD_SIZE;
-  return run(epi, X, ldx, nullptr, W, Cout, ldc, T, N, K, allow_split, err, sm_count, nullptr, stream);
+  return run(epi, X, ldx, nullptr, W, Cout, ldc, T, N, K, allow_split, err, sm_count, nullptr, stream, sa.w_fixed);
 }
 
 // One product per group of weight rows, in one launch: rows n of W in group n / x_rows multiply X's columns from
 // (n / x_rows) * x_gs on (the last group may be shorter). Store epilogue; x_rows a multiple of the 128 rows of a tile, K of
-// the 64 values of a stage (a stage never reaches into the next group's columns), x_gs of 8.
+// the 64 values of a stage (a stage never reaches into the next group's columns), x_gs of 8. No launch that may still be running writes W.
 RLLM_API int rllm_tc_gemm_mixes(const void* X, long long ldx, int x_rows, int x_gs, const void* W, void* Cout, long long ldc,
                                 int T, int N, int K, int* err, int sm_count, void* stream) {
   if (!X || x_rows <= 0 || x_rows % BM || x_gs % 8 || x_gs < K || K % BK) return ERR_BAD_SIZE;
-  return run(EPI_STORE, X, ldx, nullptr, W, Cout, ldc, T, N, K, 1, err, sm_count, nullptr, stream, x_rows, x_gs);
+  return run(EPI_STORE, X, ldx, nullptr, W, Cout, ldc, T, N, K, 1, err, sm_count, nullptr, stream, true, x_rows, x_gs);
 }
 
 // The same product with RMSNorm in front, in one kernel: X[t, :] = h[row(t), :] * rsqrt(mean(h^2) + eps) * g,
 // row(t) = rows[t], or t when rows is null. h float [*, K] with row stride ldh (a multiple of 4); g the norm
 // weight [K], float (g_dt 0) or bfloat16 (g_dt 1). T at most 64 (rllm_tc_gemm_norm_max_tokens); epilogues
-// store, store-float and SwiGLU.
+// store, store-float and SwiGLU. Bit 16 of epi as in rllm_tc_gemm.
 RLLM_API int rllm_tc_gemm_norm(int epi, const float* h, long long ldh, const int* rows, const void* g, int g_dt,
                                float eps, const void* W, void* Cout, long long ldc, int T, int N, int K,
                                int allow_split, int* err, int sm_count, void* stream) {
@@ -1694,7 +1700,7 @@ RLLM_API int rllm_tc_gemm_norm(int epi, const float* h, long long ldh, const int
   if (epi < 0 || epi > 3 || epi == EPI_ACCUM_F32 || !h || !g || (g_dt != DT_F32 && g_dt != DT_BF16)) return ERR_BAD_SIZE;
   NormArgs nm;
   nm.h = h; nm.ldh = ldh; nm.rows = rows; nm.g = g; nm.g_is_bf16 = g_dt == DT_BF16; nm.eps = eps;
-  return run(epi, nullptr, 0, &nm, W, Cout, ldc, T, N, K, allow_split, err, sm_count, nullptr, stream);
+  return run(epi, nullptr, 0, &nm, W, Cout, ldc, T, N, K, allow_split, err, sm_count, nullptr, stream, sa.w_fixed);
 }
 RLLM_API int rllm_tc_gemm_norm_max_tokens() { return NORM_MAX_T; }
 
@@ -1703,12 +1709,12 @@ RLLM_API int rllm_tc_gemm_norm_max_tokens() { return NORM_MAX_T; }
 // positions[t] * inv_freq[i]; rotated k and plain v also go to the paged cache at slots[t]
 // (slots null or < 0: no write). Head size must divide 128 so that no head straddles two tiles.
 // cos_sin: the step's table [T][rot_dim / 2] of (cos, sin), or null to compute them in the epilogue.
-// X null: RMSNorm in front as in rllm_tc_gemm_norm (h, ldh, g, g_dt, eps; T at most 64).
+// X null: RMSNorm in front as in rllm_tc_gemm_norm (h, ldh, g, g_dt, eps; T at most 64). w_fixed: no launch that may still be running writes W.
 RLLM_API int rllm_tc_gemm_qkv_rope(const void* X, long long ldx, const float* h, long long ldh, const void* g,
                                    int g_dt, float eps, const void* W, void* QKV, long long ldc, int T,
                                    int K, const int* positions, const float* inv_freq, const void* cos_sin,
                                    const int* slots, void* kcache, void* vcache, int nh, int nkv, int hd, int page_size,
-                                   int rot_dim, int allow_split, int* err, int sm_count, void* stream) {
+                                   int rot_dim, int allow_split, int w_fixed, int* err, int sm_count, void* stream) {
   if (hd <= 0 || BM % hd || rot_dim % 2 || rot_dim > hd || rot_dim < 0 || nh <= 0 || nkv <= 0 || page_size <= 0)
     return ERR_BAD_SIZE;
   RopeArgs r;
@@ -1721,5 +1727,5 @@ RLLM_API int rllm_tc_gemm_qkv_rope(const void* X, long long ldx, const float* h,
     nm.h = h; nm.ldh = ldh; nm.rows = nullptr; nm.g = g; nm.g_is_bf16 = g_dt == DT_BF16; nm.eps = eps;
   }
   return run(EPI_QKV_ROPE, X, ldx, fused ? &nm : nullptr, W, QKV, ldc, T, (nh + 2 * nkv) * hd, K, allow_split, err,
-             sm_count, &r, stream);
+             sm_count, &r, stream, w_fixed != 0);
 }

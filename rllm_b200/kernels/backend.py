@@ -152,7 +152,7 @@ class Backend:
     def linear(self, x, w, bias=None, tag=None):
         # `tag` names the product for per-operation timing (kernels/profile.py); it changes nothing here
         if bias is None and self._fused_norm(x, w):
-            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE, rows=x.rows)
+            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE, rows=x.rows, w_fixed=True)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w):
             # a bias is added after the product (a small kernel): the product stays on the tensor cores
@@ -164,7 +164,7 @@ class Backend:
         if w.shape[0] <= ops.SKINNY_MAX:         # a gate row, a handful of heads: a warp a token
             return ops.gemm_skinny(x.tensor() if isinstance(x, Normed) else x, w)
         if self._fused_norm(x, w):
-            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE_F32, rows=x.rows)
+            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE_F32, rows=x.rows, w_fixed=True)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w):
             return self._sm100.product(x, w, ops.EPI_STORE_F32)
@@ -180,7 +180,7 @@ class Backend:
     def linear_swiglu(self, x, w_gate_up):
         """silu(x Wg^T) * (x Wu^T) with w_gate_up = [Wg; Wu]"""
         if self._fused_norm(x, w_gate_up, gate_up=True):
-            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows)
+            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows, w_fixed=True)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w_gate_up):
             return self._sm100.product(x, w_gate_up, ops.EPI_SWIGLU)
@@ -211,14 +211,14 @@ class Backend:
             writes = cache.writes
             return self._sm100.gemm_qkv_rope(None, w_qkv, positions, inv_freq, cache.slots if writes else None,
                                              kc, cache.v if writes else None, nh, nkv, hd, cache.page_size,
-                                             rot_dim, norm=(x.h, x.weight, x.eps), table=table)
+                                             rot_dim, norm=(x.h, x.weight, x.eps), table=table, w_fixed=True)
         x = x.tensor() if isinstance(x, Normed) else x
         if bias is None and self._sm100 is not None and \
                 self._sm100.qkv_rope_supported(x, w_qkv, cache.k if cache.writes else None, hd, rot_dim):
             writes = cache.writes
             return self._sm100.gemm_qkv_rope(x, w_qkv, positions, inv_freq, cache.slots if writes else None,
                                              cache.k if writes else None, cache.v if writes else None,
-                                             nh, nkv, hd, cache.page_size, rot_dim, table=table, asked=True)
+                                             nh, nkv, hd, cache.page_size, rot_dim, table=table, asked=True, w_fixed=True)
         qkv = self.linear(x, w_qkv, bias=bias)
         self.rope_cache_write(qkv, positions, inv_freq, cache, nh, nkv, hd, rot_dim, ctx=ctx, key=key)
         return qkv
@@ -277,7 +277,7 @@ class Backend:
         for g in range(G):
             wg, xg, og = w[g * N: (g + 1) * N], x[:, g], out[:, g * N: g * N + N]
             if self._tc(xg, wg) and self._sm100.out_supported(og):
-                self._sm100.gemm(xg, wg, ops.EPI_STORE, out=og)
+                self._sm100.product(xg, wg, ops.EPI_STORE, out=og)
             else:
                 ops.gemm_simt(xg, wg, ops.EPI_STORE, out=og)
         return out
@@ -375,7 +375,7 @@ class Backend:
             raise ops.KernelError(f"activation {act!r} has no kernel")
         fuse = os.environ.get("RLLM_B200_NO_ACT_FUSION") != "1"
         if fuse and self._fused_norm(x, w):                                  # the norm in front, the activation behind
-            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE, rows=x.rows, act=act)
+            return self._sm100.gemm_norm(x.h, x.weight, x.eps, w, ops.EPI_STORE, rows=x.rows, act=act, w_fixed=True)
         x = x.tensor() if isinstance(x, Normed) else x
         if self._tc(x, w) and fuse:
             return self._sm100.product(x, w, ops.EPI_STORE, act=act)         # in the product's store epilogue
@@ -384,7 +384,7 @@ class Backend:
         if act == "gelu_tanh":
             return self._hy.act_rows(self.linear_f32(x, w, tag="up"), self.dtype, act)
         if self._tc(x, w):
-            return self._sink.relu2_(self._sm100.gemm(x, w, ops.EPI_STORE))
+            return self._sink.relu2_(self._sm100.product(x, w, ops.EPI_STORE))
         return ops.gemm_simt(x, w, ops.EPI_RELU2)
 
     def qk_norm_rope_store(self, proj, q_off, k_off, v_off, nh, nkv, kd, vd, rot, wq, wk, eps, table, cache, vfirst=None,
@@ -568,7 +568,7 @@ class Backend:
             return self.linear_swiglu(x, w_gate_up)
         if act == "gelu_tanh":
             if self._fused_norm(x, w_gate_up, gate_up=True):
-                return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows, gelu_gate=True)
+                return self._sm100.gemm_norm(x.h, x.weight, x.eps, w_gate_up, ops.EPI_SWIGLU, rows=x.rows, gelu_gate=True, w_fixed=True)
             x = x.tensor() if isinstance(x, Normed) else x
             if self._tc(x, w_gate_up):
                 return self._sm100.product(x, w_gate_up, ops.EPI_SWIGLU, gelu_gate=True)

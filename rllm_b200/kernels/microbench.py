@@ -94,10 +94,10 @@ def cmd_gemm(a) -> None:
         if a.norm:
             h = torch.randn(T, K, device=DEV)
             g = torch.ones(K, device=DEV)
-            fns = [(lambda w=w: sm100.gemm_norm(h, g, 1e-5, w, epi, split=split)) for w in ws]
+            fns = [(lambda w=w: sm100.gemm_norm(h, g, 1e-5, w, epi, split=split, w_fixed=True)) for w in ws]
         else:
             x = torch.randn(T, K, device=DEV, dtype=torch.bfloat16)
-            fns = [(lambda w=w: sm100.gemm(x, w, epi, out=out, split=split)) for w in ws]
+            fns = [(lambda w=w: sm100.gemm(x, w, epi, out=out, split=split, w_fixed=True)) for w in ws]
         bn, sp, pair = sm100.launch_plan(epi, T, N, K, sm100.init(DEV).sm_count, split, a.norm)
         streamed = split and sm100.stream_supported(epi, a.norm, T, N, K)
         how = "streamed" if streamed else f"tile={bn} ranges={sp}" + (" pairs" if pair else "")
@@ -129,7 +129,7 @@ def cmd_gemm_rope(a, N: int, K: int) -> None:
         else:
             x, norm = torch.randn(T, K, device=DEV, dtype=torch.bfloat16), None
         fns = [(lambda w=w: sm100.gemm_qkv_rope(x, w, pos, inv_freq, slots, kc, vc, nh, nkv, hd, page, hd,
-                                                split=split, table=table, norm=norm)) for w in ws]
+                                                split=split, table=table, norm=norm, w_fixed=True)) for w in ws]
         run(fns, a.plain, f"gemm qkv+rope T={T} N={N} K={K} heads {nh}/{nkv} of {hd}" + (" norm" if a.norm else "")
             + (f" ranges asked {a.ranges}" if a.ranges > 1 else ""), nbytes=N * K * 2, flops=2.0 * T * N * K)
     sm100.check_error(DEV)
@@ -469,9 +469,9 @@ def cmd_gated(a) -> None:
         # gelu in the epilogue of the up product beside relu squared there, and beside the float product with a pass after it
         x, wu = bf(T, W), bf(4 * W, W)
         for act in ("gelu_tanh", "relu2"):
-            run([lambda act=act: sm100.gemm(x, wu, ops.EPI_STORE, act=act)] * 4, 0,
+            run([lambda act=act: sm100.gemm(x, wu, ops.EPI_STORE, act=act, w_fixed=True)] * 4, 0,
                 f"{'  like: ' if act == 'relu2' else ''}up product with {act} in its epilogue T={T} {W} -> {4 * W}", flops=2.0 * T * W * 4 * W)
-        run([lambda: hybrid.act_rows(sm100.gemm(x, wu, ops.EPI_STORE_F32), torch.bfloat16, "gelu_tanh")] * 4, 0,
+        run([lambda: hybrid.act_rows(sm100.gemm(x, wu, ops.EPI_STORE_F32, w_fixed=True), torch.bfloat16, "gelu_tanh")] * 4, 0,
             f"  the float product and a pass for the gelu T={T}", flops=2.0 * T * W * 4 * W)
     for B in a.batch:                                    # B single tokens at context C
         C = a.context
@@ -541,7 +541,7 @@ def cmd_bounded(a) -> None:
             run([lambda: sink.postnorm(h, y, 0.5, w, 1e-6, copy=copy, output=output)] * 4, 0, f"{label} T={T} width={W}", nbytes=T * W * 14)
         x, wu = bf(T, W), bf(4 * W, W)
         for act in ("gelu_erf", "gelu_tanh", "relu2"):
-            run([lambda act=act: sm100.gemm(x, wu, ops.EPI_STORE, act=act)] * 4, 0,
+            run([lambda act=act: sm100.gemm(x, wu, ops.EPI_STORE, act=act, w_fixed=True)] * 4, 0,
                 f"{'' if act == 'gelu_erf' else '  like: '}up product with {act} in its epilogue T={T} {W} -> {4 * W}", flops=2.0 * T * W * 4 * W)
         _delta_pair(hybrid, 1, T, W)
     for B in a.batch:                                    # B single tokens at context C
@@ -600,7 +600,7 @@ def cmd_timemix(a) -> None:
         wt = wz.t().contiguous()
         run([lambda: mix.lowrank_decay(z, wt, b0)] * 4, 0, f"decays {what}, rank {rank}", C * rank * 2 + T * C * 4, 2.0 * T * C * rank)
         zf, bb = torch.randn(T, C, device=DEV), torch.randn(C, device=DEV)
-        run([lambda: (sm100.gemm(z, wz, ops.EPI_STORE_F32, out=zf), mix.gla_decay(zf, bb, 16.0))] * 4, 0,
+        run([lambda: (sm100.gemm(z, wz, ops.EPI_STORE_F32, out=zf, w_fixed=True), mix.gla_decay(zf, bb, 16.0))] * 4, 0,
             f"  like: product and decays of gated linear attention {what}", C * rank * 2 + T * C * 4, 2.0 * T * C * rank)
         from .backend import Backend
         be = Backend(torch.bfloat16)

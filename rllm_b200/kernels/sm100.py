@@ -20,13 +20,13 @@ ops.register_signatures("sm100", {
                           c_int, _P, c_int, _P],
     "rllm_tc_gemm_norm_max_tokens": [],
     "rllm_tc_gemm_qkv_rope": [_P, c_longlong, _P, c_longlong, _P, c_int, c_float, _P, _P, c_longlong, c_int, c_int,
-                              _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P],
+                              _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P],
     "rllm_stream_gemm_supported": [c_int, c_int, c_int, c_int, c_int, c_int],
     "rllm_stream_gemm": [c_int, _P, c_longlong, _P, c_longlong, _P, _P, c_int, c_float, _P, _P, c_longlong, c_int,
                          c_int, c_int, c_int, _P],
     "rllm_stream_gemm_mixes": [_P, c_longlong, c_int, c_longlong, _P, _P, c_longlong, c_int, c_int, c_int, c_int, _P],
     "rllm_stream_gemm_qkv_rope": [_P, c_longlong, _P, c_longlong, _P, c_int, c_float, _P, _P, c_longlong, c_int, c_int,
-                                  _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P],
+                                  _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "rllm_wait_probe": [_P, c_longlong, c_int, _P],
     "rllm_attention_fa": [_P, c_int, _P, _P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
                           c_int, c_int, c_float, c_int, c_int, _P, _P, _P],
@@ -148,22 +148,25 @@ def plan(epilogue: int, T: int, N: int, K: int, device="cuda:0", split: bool | i
 ACT_RELU2 = 1 << 8          # added to the store epilogue's number: max(value, 0)^2 is stored
 ACT_GELU_TANH = 2 << 8      # likewise: gelu(value) in its tanh form
 ACT_GELU_ERF = 3 << 8       # gelu(value) in its erf form
+W_FIXED = 1 << 16           # no launch that may still be running writes the weight: its copies begin before the kernel in front has ended
 STORE_ACTS = {None: 0, "relu2": ACT_RELU2, "gelu_tanh": ACT_GELU_TANH, "gelu_erf": ACT_GELU_ERF}
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, epilogue: int, out: torch.Tensor | None = None,
-         split: bool = True, relu2: bool = False, act: str | None = None, gelu_gate: bool = False) -> torch.Tensor:
+         split: bool = True, relu2: bool = False, act: str | None = None, gelu_gate: bool = False,
+         w_fixed: bool = False) -> torch.Tensor:
     """C = X W^T on the tensor cores. x [T, K] bf16 (unit inner stride); w [N, K] bf16 ([2N, K] with
     the SwiGLU epilogue). `out` is required for the accumulate epilogue (the float residual). `act`
     (store epilogue only; `relu2` True is act "relu2"): the activation of the float result is what is rounded and
     stored: "relu2" max(., 0)^2, "gelu_tanh" gelu in its tanh form, "gelu_erf" in its erf form. `gelu_gate` (SwiGLU epilogue
-    only): the gate passes gelu in its tanh form instead of silu."""
+    only): the gate passes gelu in its tanh form instead of silu. `w_fixed`: w is not written by work that may still be
+    running on this stream (a model's weights are not): it is then read before the kernels in front have ended."""
     if gelu_gate and epilogue != ops.EPI_SWIGLU:
         raise ops.KernelError("tc gemm: gelu_gate goes with the SwiGLU epilogue only")
     act = "relu2" if relu2 else act
     if act is not None and (epilogue != ops.EPI_STORE or act not in STORE_ACTS):
         raise ops.KernelError("tc gemm: an activation (relu2, gelu_tanh, gelu_erf) goes with the store epilogue only")
-    code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0)
+    code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0) | (W_FIXED if w_fixed else 0)
     if not gemm_supported(x, w):
         raise ops.KernelError("tc gemm: operands must be bfloat16, K a multiple of 8, 16-byte aligned")
     return _product(x, w, epilogue, code, out, split)
@@ -171,8 +174,9 @@ def gemm(x: torch.Tensor, w: torch.Tensor, epilogue: int, out: torch.Tensor | No
 
 def product(x: torch.Tensor, w: torch.Tensor, epilogue: int, out: torch.Tensor | None = None, act: str | None = None,
             gelu_gate: bool = False) -> torch.Tensor:
-    """`gemm` for a caller that has just asked `gemm_supported` about these operands (asking takes the host 4 us)."""
-    return _product(x, w, epilogue, epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0), out, True)
+    """`gemm` with a weight that is fixed (`w_fixed`), for a caller that has just asked `gemm_supported` about these operands
+    (asking takes the host 4 us)."""
+    return _product(x, w, epilogue, epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0) | W_FIXED, out, True)
 
 
 def _product(x, w, epilogue, code, out, split):
@@ -201,8 +205,8 @@ def _product(x, w, epilogue, code, out, split):
 
 def gemm_mixes(x: torch.Tensor, w: torch.Tensor, rows_each: int, out: torch.Tensor) -> bool:
     """out[:, n] = x[:, n // rows_each] w[n]^T in one launch: steps of at most 8 tokens on the weight-streaming kernel, longer
-    ones on tcgen05; x [T, G, K] contiguous, w [R, K], out [T, R], bfloat16. False (nothing launched) where neither takes
-    the sizes."""
+    ones on tcgen05; x [T, G, K] contiguous, w [R, K] (fixed, as `w_fixed` of `gemm`), out [T, R], bfloat16. False (nothing
+    launched) where neither takes the sizes."""
     T, G, K = x.shape
     N = w.shape[0]
     if K % 8 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16 or w.data_ptr() % 16 \
@@ -245,9 +249,10 @@ def norm_supported(h: torch.Tensor, g: torch.Tensor, w: torch.Tensor, rows: torc
 
 
 def gemm_norm(h: torch.Tensor, g: torch.Tensor, eps: float, w: torch.Tensor, epilogue: int,
-              rows: torch.Tensor | None = None, split: bool = True, act: str | None = None, gelu_gate: bool = False) -> torch.Tensor:
-    """C = rmsnorm(h[rows]; g, eps) W^T in one kernel (store, store-float or SwiGLU epilogue; `act` and `gelu_gate` as in
-    `gemm`)."""
+              rows: torch.Tensor | None = None, split: bool = True, act: str | None = None, gelu_gate: bool = False,
+              w_fixed: bool = False) -> torch.Tensor:
+    """C = rmsnorm(h[rows]; g, eps) W^T in one kernel (store, store-float or SwiGLU epilogue; `act`, `gelu_gate` and `w_fixed`
+    as in `gemm`)."""
     if gelu_gate and epilogue != ops.EPI_SWIGLU:
         raise ops.KernelError("tc gemm with norm: gelu_gate goes with the SwiGLU epilogue only")
     if act is not None and (epilogue != ops.EPI_STORE or act not in STORE_ACTS):
@@ -257,7 +262,7 @@ def gemm_norm(h: torch.Tensor, g: torch.Tensor, eps: float, w: torch.Tensor, epi
                               f"{norm_max_tokens()} tokens, bfloat16 weights, 16-byte aligned")
     if epilogue not in (ops.EPI_STORE, ops.EPI_STORE_F32, ops.EPI_SWIGLU):
         raise ops.KernelError("tc gemm with norm: epilogue must be store, store-float or SwiGLU")
-    code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0)
+    code = epilogue | STORE_ACTS[act] | (ACT_GELU_TANH if gelu_gate else 0) | (W_FIXED if w_fixed else 0)
     st = init(h.device)
     T = h.shape[0] if rows is None else rows.numel()
     K = h.shape[1]
@@ -291,12 +296,13 @@ def qkv_rope_supported(x: torch.Tensor, w: torch.Tensor, kcache, hd: int, rot_di
 def gemm_qkv_rope(x: torch.Tensor | None, w_qkv: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tensor,
                   slots: torch.Tensor | None, kcache: torch.Tensor | None, vcache: torch.Tensor | None,
                   nh: int, nkv: int, hd: int, page_size: int, rot_dim: int, split: bool = True,
-                  norm: tuple | None = None, table: torch.Tensor | None = None, asked: bool = False) -> torch.Tensor:
+                  norm: tuple | None = None, table: torch.Tensor | None = None, asked: bool = False,
+                  w_fixed: bool = False) -> torch.Tensor:
     """qkv = x w_qkv^T with q and k rotated by position and k, v written to the paged cache at
     `slots` (None: no write), all in the product's epilogue. Returns qkv [T, (nh + 2 nkv) * hd].
     `norm` = (h, g, eps) instead of x: RMSNorm of the float rows h in front, in the same kernel.
     `table`: `ops.rope_table` of these positions ([T, rot_dim / 2, 2]); else the angles are computed here. `asked`: the caller
-    has just asked `qkv_rope_supported` about x, w_qkv and kcache."""
+    has just asked `qkv_rope_supported` about x, w_qkv and kcache. `w_fixed` as in `gemm`."""
     T, K = norm[0].shape if norm is not None else x.shape
     # steps of at most 8 tokens: the weight-streaming kernel (any head size that is a multiple of 32), up to 16 for some K
     streamed = split and rot_dim == hd and stream_supported(EPI_QKV_ROPE, norm is not None, T, (nh + 2 * nkv) * hd, K, hd)
@@ -337,13 +343,13 @@ def gemm_qkv_rope(x: torch.Tensor | None, w_qkv: torch.Tensor, positions: torch.
         rc = ops._fn("sm100", "rllm_stream_gemm_qkv_rope")(
             *xa, w_qkv.data_ptr(), out.data_ptr(), out.stride(0), T, K, positions.data_ptr(),
             inv_freq.data_ptr(), ops._ptr(table), ops._ptr(slots), ops._ptr(kcache) if slots is not None else None,
-            ops._ptr(vcache) if slots is not None else None, nh, nkv, hd, page_size, st.sm_count, ops._stream())
+            ops._ptr(vcache) if slots is not None else None, nh, nkv, hd, page_size, int(w_fixed), st.sm_count, ops._stream())
         ops._check(rc, "stream_gemm_qkv_rope")
         return out
     rc = ops._fn("sm100", "rllm_tc_gemm_qkv_rope")(
         *xa, w_qkv.data_ptr(), out.data_ptr(), out.stride(0), T, K, positions.data_ptr(),
         inv_freq.data_ptr(), ops._ptr(table), ops._ptr(slots), ops._ptr(kcache) if slots is not None else None,
-        ops._ptr(vcache) if slots is not None else None, nh, nkv, hd, page_size, rot_dim, int(split),
+        ops._ptr(vcache) if slots is not None else None, nh, nkv, hd, page_size, rot_dim, int(split), int(w_fixed),
         st.err.data_ptr(), st.sm_count, ops._stream())
     ops._check(rc, "tc_gemm_qkv_rope")
     return out
