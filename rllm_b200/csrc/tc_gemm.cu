@@ -1104,7 +1104,8 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 
 // ---------------------------------------------------------------------------- many tokens, two SMs a tile
 // The same persistent scheme on pairs of CTAs (a cluster of two, `tcgen05.mma.cta_group::2`): a tile is 256 weight rows x
-// any number of tokens in steps of 16 up to 256; each CTA of the pair loads its own 128 weight rows and its own half of the
+// any number of tokens in steps of 32 up to 256 (odd multiples of 16 gave the same bits, but no table of the instruction's shapes over
+// two CTAs that names them is at hand); each CTA of the pair loads its own 128 weight rows and its own half of the
 // token tile into its own shared memory (plain TMA loads, no multicast) and keeps its 128 accumulator rows in its own TMEM; the
 // even CTA issues the MMAs, which read both CTAs' shared memory. Gate/up pairs put 256 tokens on the rows, 128 in each CTA; the
 // tile's 128 gate rows lie in the even CTA, its 128 up rows in the odd one, so that each CTA holds both values of its tokens.
@@ -1497,8 +1498,7 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
 // block takes, + the start and the last epilogue. Fitted to measurements (ns):
 // a block takes a CTA max(165, 1.63 a token), a pair max(200, 1.3 a token), with gate/up 400 and 310; one-CTA kernel / pairs by this
 // rule, us: 2,048 tokens, 3,072 x 2,048 26.2 / 23.0 (192 tokens a tile), 2 x 8,192 x 2,048 98.0 / 89.2, 16,384 x 4,096 188 / 171; 1,905 tokens,
-// 2,048 x 8,192 53.2 / 47.3 (224); 2,834 tokens 88.7 / 70.6 (160); 2,047 tokens, 4,096 x 16,384 206 / 198 (240; in steps of 32 216 with 160,
-// 226 with 256); 643 tokens, 2 x 8,192 x 2,048 42.0 / 36.8. Where the rule leaves the
+// 2,048 x 8,192 53.2 / 47.3 (224); 2,834 tokens 88.7 / 70.6 (160); 643 tokens, 2 x 8,192 x 2,048 42.0 / 36.8. Where the rule leaves the
 // product to single CTAs, us single / best width on pairs: 643 tokens, 2,048 x 2,048 11.4 / 12.8, 2,048 x 8,192 29.2 / 31.2; 256 tokens 25.6 / 29.7.
 // Up to 128 tokens a pair has half a tile to work on.
 int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
@@ -1514,7 +1514,7 @@ int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
   const long long one = waves(bn, BM, sm_count) * kb * (dual ? 400 : bn > 101 ? bn * 163 / 100 : 165) + 4000 + 14 * bn;
   long long best = one - one / 50;
   int best_bn = 0;
-  for (int cand = 256; cand >= (dual ? 256 : 64); cand -= 16) {
+  for (int cand = 256; cand >= (dual ? 256 : 64); cand -= 32) {
     const long long t = waves(cand, dual ? BM : 2 * BM, sm_count / 2) * kb * (dual ? 310 : cand > 153 ? cand * 13 / 10 : 200) +
                         (dual ? 7500 : 4500 + 18 * cand);
     if (t < best) { best = t; best_bn = cand; }
@@ -1651,7 +1651,7 @@ RLLM_API int rllm_tc_gemm_plan(int epi, int T, int N, int K, int sm_count, int a
   return 0;
 }
 
-RLLM_API int rllm_tc_gemm_set_pairs(int on) { g_pairs = on > 1 ? (on < 32 ? 32 : on > 256 ? 256 : on & ~15) : on; return 0; }
+RLLM_API int rllm_tc_gemm_set_pairs(int on) { g_pairs = on > 1 ? (on < 32 ? 32 : on > 256 ? 256 : on & ~31) : on; return 0; }
 RLLM_API int rllm_tc_gemm_set_token_rows(int on) { g_token_rows = on != 0; return 0; }
 
 // The store epilogue (0) may carry an activation in the bits above the epilogue's number: epi = 0 | 1 << 8 stores

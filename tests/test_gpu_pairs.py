@@ -32,8 +32,7 @@ def both(run, pairs):
 
 @pytest.mark.parametrize("T,N,K,width", [(65, 256, 64, 64), (129, 2048, 136, 96), (257, 260, 1000, 128), (300, 520, 72, 160), (1905, 384, 520, 192),
                                          (2047, 1160, 264, 224), (700, 128, 2048, 256), (513, 8192, 128, 256), (161, 4, 64, 64),
-                                         (2834, 2048, 192, 160), (4096, 3072, 128, 192), (2047, 516, 136, 240),
-                                         (300, 260, 264, 112), (1000, 256, 72, 176), (333, 512, 200, 80)])
+                                         (2834, 2048, 192, 160), (4096, 3072, 128, 192)])
 def test_widths_and_edges(T, N, K, width):
     from rllm_b200.kernels import ops, sm100
     x, w = rnd(T, K, seed=1), rnd(2 * N, K, seed=2, scale=K ** -0.5)
@@ -52,8 +51,7 @@ def test_widths_and_edges(T, N, K, width):
 
 
 @pytest.mark.parametrize("T,nh,nkv,hd,rot,width", [(65, 32, 8, 64, 64, 64), (300, 5, 3, 64, 32, 96), (643, 6, 2, 128, 128, 128), (1905, 4, 4, 32, 16, 160),
-                                                   (2048, 12, 4, 128, 64, 192), (257, 3, 1, 16, 16, 256), (2048, 8, 4, 64, 64, 176),
-                                                   (500, 4, 2, 64, 48, 80)])
+                                                   (2048, 12, 4, 128, 64, 192), (257, 3, 1, 16, 16, 256)])
 @pytest.mark.parametrize("table", [True, False])
 def test_rotary_epilogue(T, nh, nkv, hd, rot, width, table):
     from rllm_b200.kernels import ops, sm100

@@ -33,3 +33,18 @@ def test_no_ranges_and_no_pairs_where_they_are_not_asked_for():
         assert sm100.launch_plan(STORE, 2048, 3072, 2048, SMS) == (176, 1, False)
     finally:
         sm100.set_pairs(False)
+
+
+def test_pairs_take_tiles_in_steps_of_32_tokens():
+    """`tcgen05.mma` over two CTAs: 32 to 256 columns in steps of 32 are the shapes the kernel issues, whatever is asked for."""
+    for N, K in ((2048, 2048), (3072, 2048), (2048, 8192), (4096, 16384), (6144, 4096)):
+        for T in range(129, 3000, 61):
+            for epi in (STORE, ACCUM, ROPE):
+                tile, ranges, pairs = sm100.launch_plan(epi, T, N, K, SMS)
+                assert not pairs or (tile % 32 == 0 and ranges == 1)
+    try:
+        for asked, width in ((176, 160), (240, 224), (80, 64), (256, 256), (33, 32)):
+            sm100.set_pairs(asked)
+            assert sm100.launch_plan(STORE, 1000, 2048, 2048, SMS) == (width, 1, True)
+    finally:
+        sm100.set_pairs(False)
