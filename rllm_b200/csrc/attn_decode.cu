@@ -444,6 +444,13 @@ int launch_dec(const DecParams& p, const SoftCap& cap, int num_seqs, cudaStream_
 
 }  // namespace
 
+// CTAs of the kernel that an SM holds at once, at most two (an SM has 228 KB of shared memory and keeps 1 KB of it per CTA).
+RLLM_API int rllm_attention_decode_per_sm(int nh, int nkv, int hd) {
+  if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv || nh / nkv > 16) return 1;
+  const int smem = hd == 64 ? DCfg<64>::smem_bytes(nh / nkv) : DCfg<128>::smem_bytes(nh / nkv);
+  return 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
+}
+
 // q: [S, ...] bf16, one row per sequence, stride q_stride, head h at h*hd; out likewise.
 // kcache / vcache: [num_pages][nkv][page_size][hd] bf16. kv_lens [S]: keys visible to each
 // sequence's token (its own included). splits: ranges of keys per sequence (1..16, one cluster).

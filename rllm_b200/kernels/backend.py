@@ -421,7 +421,8 @@ class Backend:
             sm = self._sm100
             if ctx.max_q_len == 1 and not keep_first and not sigmoid and sm.decode_supported(q, cache.k, nh):
                 return sm.attention_decode(q, cache.k, cache.v, ctx.kv_lens, cache.block_table, nh, scale, window, keys,
-                                           chunk=chunk, sinks=sinks, gate=gate, softcap=softcap)
+                                           chunk=chunk, sinks=sinks, gate=gate, softcap=softcap,
+                                           captured=ctx.graph_safe and keys == ctx.max_kv_len)     # cut by a window or block: no bound that doubles
             lens = ctx.q_lens_host
             if ctx.max_q_len * G >= 128 and ctx.max_kv_len >= sm.TC_ATTENTION_MIN_KEYS and sm.prefill_tc_supported(q, cache.k) \
                     and lens is not None and min(lens) * G >= 128:

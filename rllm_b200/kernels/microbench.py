@@ -155,7 +155,7 @@ def cmd_attn_decode(a) -> None:
     q = torch.randn(a.batch, nh * hd, device=DEV, dtype=torch.bfloat16)
     out = torch.empty_like(q)
     nbytes = a.batch * a.context * nkv * hd * 2 * 2
-    auto = sm100.decode_splits(a.batch, nkv, a.context, sm100.init(DEV).sm_count)
+    auto = sm100.decode_splits(a.batch, nkv, a.context, sm100.init(DEV).sm_count, hd, per_sm=sm100.decode_per_sm(nh, nkv, hd))
     for sp in (a.splits or [auto]):
         fns = [(lambda kc=kc, vc=vc: sm100.attention_decode(q, kc, vc, lens, bt, nh, hd ** -0.5, None, a.context,
                                                             splits=sp, out=out)) for kc, vc in caches]

@@ -34,6 +34,7 @@ ops.register_signatures("sm100", {
                                   c_int, c_int, c_float, c_int, c_int, _P, _P, c_int, c_int, c_int, c_float, c_int, _P, _P, c_int, _P],
     "rllm_attention_prefill_dense": [_P, c_int, c_int, _P, c_longlong, c_int, _P, _P, c_longlong, c_int, c_int, _P, c_int, c_longlong, _P,
                                      c_int, _P, _P, c_int, c_int, c_int, c_float, c_int, _P, c_int, c_int, c_int, _P, c_int, _P],
+    "rllm_attention_decode_per_sm": [c_int, c_int, c_int],
     "rllm_attention_decode": [_P, c_int, _P, _P, c_longlong, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int,
                               c_int, c_float, c_int, c_int, _P, _P, c_int, c_float, c_int, _P, _P],
 })
@@ -492,47 +493,63 @@ def decode_supported(q: torch.Tensor, kcache: torch.Tensor, nh: int) -> bool:
     return attention_supported(q, kcache) and nh // nkv <= 16 and kcache.data_ptr() % 16 == 0
 
 
-def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: int = 64) -> int:
-    """Ranges the keys of a sequence are cut into (= CTAs per cluster). Measured on a B200: a CTA
-    costs about as much as 1,150 keys before its first key and a range 65 more at the merge, two CTAs
-    fit an SM, and CTAs beyond that wait for a free place; a cluster's start and merge cost a decode step what 350 keys of heads of 64 do
-    with one sequence and 430 with four and more. The number of ranges with the least (rounds of CTAs over the places) x (1,150 + keys
-    per range) + 65 x ranges (seven at most: the merge of more
-    runs beside the last keys) + a cluster's cost is taken. Decode steps of 16 layers with 8 kv heads, us, one range / the best number:
-    contexts of 300 1 sequence 554 / 565 (4), 8 sequences 604 / 639 (4); of 1,000 625 / 571 and 670 / 659; of 4,000 949 / 626 (8) and 1,012 / 742 (4).
-    One sequence by ranges: of 2,040 keys 602 with 4, 615 with 5, 594 with 6, 598 with 8 (of about 1,100 570 with 5, 579 with 8,
-    under the same bound); of 4,090 658, 639, 630, and 635 with 7, 624 with 8.
-    Clusters of more than four CTAs need their places inside one GPC and start late where they come to more than four fifths of all
-    places (contexts of 1,000: 4 sequences 629 with 6 ranges, 670 with 8; 6 sequences 647 with 5, 704 with 6; 7 sequences 657 with 4, 712 with 5),
-    and threes beyond two thirds (10 sequences 841 with 2, 879 with 3); at heads of 128, whose ranges take longer, they do not show. Up to 8
-    ranges any number; 12 and 16 (clusters beyond the portable size, for one or two long sequences:
-    16,384 keys of one sequence 13.3 us against 18.3 with 8) only from 16,384 keys on and while the CTAs
-    leave a quarter of the places free: a large cluster needs its places inside one GPC (9 ranges of 4
-    sequences, 288 CTAs on 296 places: 16.7 us against 10.8 with 8), and inside a decode step, behind a
-    kernel whose CTAs fill whole SMs, it starts later than a small one (4,096 keys: 6.3 us against 6.9
+_decode_per_sm: dict[tuple, int] = {}
+
+
+def decode_per_sm(nh: int, nkv: int, hd: int) -> int:
+    """CTAs of the decode kernel that fit an SM (their shared memory goes with the query heads of a kv head)."""
+    key = (nh // nkv, hd)
+    n = _decode_per_sm.get(key)
+    if n is None:
+        n = _decode_per_sm[key] = int(ops._fn("sm100", "rllm_attention_decode_per_sm")(nh, nkv, hd))
+    return n
+
+
+def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: int = 64, captured: bool = False, per_sm: int = 2) -> int:
+    """Ranges the keys of a sequence are cut into (= CTAs per cluster), by one cost for all callers, in units of what a key of heads of 64
+    takes: rounds of CTAs over the places (`per_sm` an SM) x (1,150 before the first key + the keys of a range) + 40 a range for the
+    merge + 200 where there is a cluster at all. `captured`: max_kv_len is a captured step's bound, which serves
+    contexts from half of it up; the cost is then that of three quarters. Clusters of 3 and of 5 to 8 CTAs need their places inside one GPC,
+    which they do not fill evenly: where a round is more than 13/16 full of them (3/4 with one CTA an SM) the last ones start late, and they are not
+    considered.
+
+    Measured on a B200 (captured decode steps, us, 1 range / 2 / 4 / the best number): 16 layers with 32 / 8 heads of 64, 1 sequence of 300 keys 479 /
+    497 / 498 / 479 (1), of 1,000 560 / 517 / 507 / 506 (5), of 2,030 663 / 584 / 528 / 523 (5), of 4,080 887 / 683 / 591 / 561 (8); 8 sequences of
+    300 533 / 566 / 569 / 533 (1), of 1,000 620 / 613 / 592 / 592 (4), of 4,080 997 / 805 / 707 / 707 (4); 8 layers with 32 / 8 heads of 128, 1 sequence of
+    300 707 / 705 / 693 / 692 (7), of 2,030 945 / 821 / 747 / 712 (8). Late clusters: heads of 64, contexts of 1,000, 4 sequences
+    558 with 6 and 7 ranges, 603 with 8 (256 of 296 places); 6 sequences 574 with 4, 582 with 5, 625 with 6; 12 sequences 704 with 2, 773 with 3. Over
+    770 measurements (1 to 64 sequences, 100 to 8,000 keys, heads of 64 and 128 over 4 and 8 kv heads) the choice is 0.2 % from the best number of
+    each on average; the most that it is behind is 4 % up to 4,080 keys, where contexts of one bound want different numbers, and 7 % at one point beyond.
+
+    12 and 16 ranges (clusters beyond the portable size, for one or two long sequences: 16,384 keys of one sequence 13.3 us against 18.3
+    with 8) only from 16,384 keys on and while the CTAs leave a quarter of the places free (9 ranges of 4
+    sequences, 288 CTAs on 296 places: 16.7 us against 10.8 with 8); inside a decode step, behind a
+    kernel whose CTAs fill whole SMs, such a cluster starts later than a small one (4,096 keys: 6.3 us against 6.9
     alone, but the step at batch 1 0.621 ms against 0.615, at batch 2 0.692 against 0.642)."""
     base = max(1, num_seqs * nkv)
-    places = 2 * sm_count
-    cluster = min(430, 320 + 4 * base) * 64 / hd
+    places = per_sm * sm_count
+    keys = max_kv_len * 3 // 4 if captured else max_kv_len
     best, best_cost = 1, None
     for s in (1, 2, 3, 4, 5, 6, 7, 8, 12, 16):
-        if s > 1 and max_kv_len // s < 64:
+        if s > 1 and keys // s < 64:
             break
         if s > 8 and (base * s * 4 > places * 3 or max_kv_len < 16384):
             break
-        if hd == 64 and ((4 < s <= 8 and base * s * 16 > places * 13) or (s == 3 and base * s * 3 > places * 2)):
+        rounds = -(-base * s // places)
+        if s in (3, 5, 6, 7, 8) and base * s * 16 > rounds * places * (13 if per_sm > 1 else 12):
             continue
-        cost = -(-base * s // places) * (1150 + max_kv_len / s) + 65 * min(s, 7) + (cluster if s > 1 else 0)
+        cost = rounds * (1150 + keys * hd / 64 / s) + 40 * s + (200 if s > 1 else 0)
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
 
 
 def attention_decode(q, kcache, vcache, kv_lens, block_table, nh, scale, window, max_kv_len, splits=None,
-                     out=None, chunk=None, sinks=None, gate=None, softcap=None):
+                     out=None, chunk=None, sinks=None, gate=None, softcap=None, captured=False):
     """Attention for a step in which every sequence brings one token: the ranges of a sequence's
     keys are merged inside a thread-block cluster (bf16, head size 64 or 128, any page size). `softcap`: scores bounded,
-    softcap * tanh(score / softcap)."""
+    softcap * tanh(score / softcap). `splits`: that many ranges; None: by `decode_splits` from max_kv_len, the most keys that a
+    token sees, or (`captured`) the bound of a captured step."""
     st = init(q.device)
     num_pages, nkv, page_size, hd = kcache.shape
     S = kv_lens.numel()
@@ -543,7 +560,7 @@ def attention_decode(q, kcache, vcache, kv_lens, block_table, nh, scale, window,
             or not vcache.is_contiguous() or block_table.dtype != torch.int32 or kv_lens.dtype != torch.int32:
         raise ops.KernelError("attention_decode: caches must be contiguous and alike, tables int32")
     if splits is None:
-        splits = decode_splits(S, nkv, max_kv_len, st.sm_count, hd)
+        splits = decode_splits(S, nkv, max_kv_len, st.sm_count, hd, captured, decode_per_sm(nh, nkv, hd))
     if out is None:
         out = torch.empty((S, nh * hd), dtype=torch.bfloat16, device=q.device)
     rc = ops._fn("sm100", "rllm_attention_decode")(
@@ -576,9 +593,8 @@ def attention(q, cache, ctx, nh, scale, window):
     if not attention_supported(q, cache.k):
         return None
     if ctx.max_q_len == 1 and decode_supported(q, cache.k, nh):
-        # a captured step serves contexts from half of its bound up to it: the number of ranges is chosen for those between
-        keys = ctx.max_kv_len * 3 // 4 if ctx.graph_safe and ctx.max_kv_len < 16384 else ctx.max_kv_len
-        return attention_decode(q, cache.k, cache.v, ctx.kv_lens, cache.block_table, nh, scale, window, keys)
+        return attention_decode(q, cache.k, cache.v, ctx.kv_lens, cache.block_table, nh, scale, window, ctx.max_kv_len,
+                                captured=ctx.graph_safe)
     nkv = cache.k.shape[1]
     G = nh // nkv
     if ctx.max_q_len * G >= 128 and ctx.max_kv_len >= TC_ATTENTION_MIN_KEYS \

@@ -46,10 +46,10 @@ def test_decode_at_benchmark_sizes(hd, longest):
     wide = torch.full((S, cap // page), -1, dtype=torch.int32)       # the table as wide as the graph's
     wide[:, : bt.shape[1]] = bt
     st = sm100.init(DEV)
-    chosen = sm100.decode_splits(S, nkv, cap, st.sm_count)
+    chosen = sm100.decode_splits(S, nkv, cap, st.sm_count, hd, captured=True, per_sm=sm100.decode_per_sm(nh, nkv, hd))
     assert chosen >= 2                                               # ranges are in play at these lengths
     out = sm100.attention_decode(q.reshape(S, nh * hd).to(DEV), kc.to(DEV), vc.to(DEV), i32(lens), wide.to(DEV), nh,
-                                 hd ** -0.5, None, cap)              # splits: the kernel's own choice
+                                 hd ** -0.5, None, cap, captured=True)     # splits: the kernel's own choice
     sm100.check_error(DEV)
     for s in range(S):
         ref = P.attention_tail(q[s: s + 1].float(), ks[s].float(), vs[s].float(), hd ** -0.5)[0]
