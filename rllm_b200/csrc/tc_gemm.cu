@@ -1493,13 +1493,20 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
   if (few_out) *few_out = few;
 }
 
+// Gate/up products with the tokens on the rows: tiles of 64 gate and 64 up rows where tiles of 128 would leave half of the SMs without one.
+bool half_rows(int T, int N, int sm_count) {
+  return (long long)((T + BM - 1) / BM) * ((N + BM - 1) / BM) * 2 <= sm_count + sm_count / 8;
+}
+
 // Tokens per tile of the kernel on pairs of CTAs, or 0 where the one-CTA kernel (tiles of `bn` tokens) takes the product. Both
-// times are modelled: waves of tiles x blocks of K x a block's time, which goes with the tile's tokens down to what issuing a
-// block takes, + the start and the last epilogue. Fitted to measurements (ns):
-// a block takes a CTA max(165, 1.63 a token), a pair max(200, 1.3 a token), with gate/up 400 and 310; one-CTA kernel / pairs by this
-// rule, us: 2,048 tokens, 3,072 x 2,048 26.2 / 23.0 (192 tokens a tile), 2 x 8,192 x 2,048 98.0 / 89.2, 16,384 x 4,096 188 / 171; 1,905 tokens,
-// 2,048 x 8,192 53.2 / 47.3 (224); 2,834 tokens 88.7 / 70.6 (160); 643 tokens, 2 x 8,192 x 2,048 42.0 / 36.8. Where the rule leaves the
-// product to single CTAs, us single / best width on pairs: 643 tokens, 2,048 x 2,048 11.4 / 12.8, 2,048 x 8,192 29.2 / 31.2; 256 tokens 25.6 / 29.7.
+// times are modelled: waves of tiles x blocks of K x a block's time + the start and the last epilogue. Fitted (ns) to 1,270 products of 22 weights
+// (640 x 1,024 to 16,384 x 4,096) at 18 counts of 129 to 2,834 tokens, each timed on single CTAs and at every width on pairs: of a
+// single CTA a block takes 1.76 a token of the tile, of a pair max(220, 1.1 a token); gate/up 383 (202 with half of the rows) and 322. The
+// rule's choice is 0.2 % behind the best of those on average, and 6 % at most behind single CTAs (1,500 tokens, 3,072 x 2,048: 16.1 us | 17.1
+// with 256 a tile). Single CTAs | pairs by this rule, us: 2,047 tokens, 3,072 x 2,048 23.4 | 21.4 (192), 2 x 8,192 x 2,048 102 | 90, 16,384 x 4,096
+// 195 | 177, 4,096 x 16,384 217 | 196; 1,905 tokens, 2,048 x 8,192 52.0 | 47.3 (224); 643 tokens, 2 x 8,192 x 2,048 41.6 | 37.4. Where it leaves the
+// product to single CTAs, single | best width on pairs: 384 tokens, 2 x 1,024 x 5,440 19.6 | 28.7 (half of the rows), 300 tokens, 2 x 2,048 x 4,096
+// 16.8 | 23.6, 1,024 tokens, 4,096 x 1,536 13.7 | 14.4, 643 tokens, 2,048 x 8,192 28.1 | 29.2.
 // Up to 128 tokens a pair has half a tile to work on.
 int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
   const bool dual = epi == EPI_SWIGLU;
@@ -1511,12 +1518,16 @@ int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
     const long long tiles = (long long)((T + tokens - 1) / tokens) * ((N + rows - 1) / rows);
     return (tiles + places - 1) / places;
   };
-  const long long one = waves(bn, BM, sm_count) * kb * (dual ? 400 : bn > 101 ? bn * 163 / 100 : 165) + 4000 + 14 * bn;
+  if (dual) {
+    const bool half = g_token_rows && half_rows(T, N, sm_count);
+    const long long one = waves(bn, half ? 64 : BM, sm_count) * kb * (half ? 202 : 383) + 4000;
+    return waves(256, BM, sm_count / 2) * kb * 322 + 5400 < one - one / 50 ? 256 : 0;
+  }
+  const long long one = waves(bn, BM, sm_count) * kb * (bn * 176 / 100) + 7000;
   long long best = one - one / 50;
   int best_bn = 0;
-  for (int cand = 256; cand >= (dual ? 256 : 64); cand -= 32) {
-    const long long t = waves(cand, dual ? BM : 2 * BM, sm_count / 2) * kb * (dual ? 310 : cand > 153 ? cand * 13 / 10 : 200) +
-                        (dual ? 7500 : 4500 + 18 * cand);
+  for (int cand = 256; cand >= 64; cand -= 32) {
+    const long long t = waves(cand, 2 * BM, sm_count / 2) * kb * (cand > 200 ? cand * 11 / 10 : 220) + 3800 + 29 * cand;
     if (t < best) { best = t; best_bn = cand; }
   }
   return best_bn;
@@ -1611,9 +1622,7 @@ int run(int epi, const void* X, long long ldx, const NormArgs* norm, const void*
     }
   }
   if (many && dual && g_token_rows && rows16) {
-    // tiles of 64 gate and 64 up rows where tiles of 128 would leave half of the SMs without one
-    const long long tiles128 = (long long)((T + bn - 1) / bn) * ((N + BM - 1) / BM);
-    if (tiles128 * 2 <= sm_count + sm_count / 8) {
+    if (half_rows(T, N, sm_count)) {
       CUtensorMap mw64;
       if ((rc = cached_map(&mw64, W, 2LL * N, K, K, 64))) return rc;
       return launch_persistent<128, EPI_SWIGLU, true, 64>(mw64, mx, p, sm_count, s);

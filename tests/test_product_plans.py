@@ -18,7 +18,8 @@ SMS = 148
     # pairs of CTAs: more than 128 tokens, where the model of both kernels says so
     (SWIGLU, 128, 8192, 2048, (128, 1, False)), (SWIGLU, 129, 8192, 2048, (256, 1, True)), (SWIGLU, 2048, 8192, 2048, (256, 1, True)),
     (ACCUM, 643, 2048, 2048, (80, 1, False)), (ACCUM, 643, 2048, 8192, (80, 1, False)), (ACCUM, 1905, 2048, 8192, (224, 1, True)),
-    (ACCUM, 2834, 2048, 8192, (160, 1, True)), (ROPE, 128, 3072, 2048, (64, 1, False)), (SWIGLU, 2048, 8191, 2048, (128, 1, False)),
+    (SWIGLU, 384, 1024, 5440, (128, 1, False)), (SWIGLU, 300, 2048, 4096, (128, 1, False)), (STORE, 1024, 4096, 1536, (256, 1, False)),
+    (ACCUM, 2047, 4096, 16384, (256, 1, True)), (ACCUM, 2834, 2048, 8192, (160, 1, True)), (ROPE, 128, 3072, 2048, (64, 1, False)), (SWIGLU, 2048, 8191, 2048, (128, 1, False)),
 ])
 def test_the_launchers_choice(epi, T, N, K, want):
     assert sm100.launch_plan(epi, T, N, K, SMS) == want
