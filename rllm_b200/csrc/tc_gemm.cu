@@ -1534,20 +1534,29 @@ int plan_pairs(int epi, int T, int N, int K, int bn, int sm_count) {
 }
 
 // Ranges of K for token tiles of 64 (up to 128 tokens) and 128 (up to 256): how many of 2 or 4 CTAs of a cluster share an output tile,
-// or 0 where the other plans stand. A CTA takes in some 160 GB/s whatever it computes, so that a narrow weight on few CTAs waits
-// for its copies; merging the parts costs some 6 us with 64 tokens a tile and 10 with 128. So: the CTAs fit on the SMs at
-// once and fill three quarters of them, and the blocks of K that a CTA is spared (165 ns each) pay for the merge. Before / with
-// ranges, us: 2,048 x 8,192, 100 tokens 21.9 / 14.4, 192 25.6 / 19.6; 2,048 x 2,048, 100 tokens 13.9 / 9.7; 4,096 x 16,384, 64 tokens
-// 30.1 / 26.4, 100 46.9 / 32.0, 256 47.9 / 40.6; 4,096 x 4,096, 100 tokens 19.2 / 16.5, 64 tokens 15.0 / 14.3. Where the line leaves them: 2,048 x
-// 8,192, 64 tokens 12.7 / 14.2, 384 26.9 / 30.2; 4,096 x 4,096, 192 tokens 17.8 / 19.3; 2,048 x 2,048, 192 tokens 10.2 / 13.2.
-int plan_ranges(int epi, int T, int N, int K, int sm_count) {
+// or 0 where the other plan stands (`few`: small tiles and their own ranges; else the persistent kernel with `bn_other` tokens a tile). A narrow weight on
+// few CTAs waits for its copies, which a CTA takes in at some 160 GB/s whatever it computes. So: the CTAs fit on the SMs at
+// once and fill three quarters of them (clusters of 4 no more than nine tenths: 36 of them, on 144 of 148 SMs, start late). us with the other plan | with ranges:
+//   up to 64 tokens, against two tiles of 32 with as many ranges, from 48 blocks of K on (64 for 2 ranges into the residual): 64 tokens into the residual, 4,096 x 16,384 30.1 | 26.9,
+//     33 tokens, 4,096 x 3,072 9.4 | 8.7, 8,192 x 8,192 by a tenth; not 8,192 x 2,048 12.3 | 14.0, 4,096 x 2,048 8.5 | 9.0, 4,608 x 4,608 19.0 | 20.8 (36 clusters);
+//   65 to 128 tokens against small tiles with 8 ranges, always: 100 tokens, 2,048 x 2,048 12.7 | 8.5, 2,048 x 8,192 21.2 | 13.1;
+//   against the persistent kernel, whose block of 64 tokens takes 159 ns, where the blocks spared pay for the merge: 100 tokens into the residual,
+//     4,096 x 16,384 43.4 | 34.6; not 4,096 x 4,096 13.7 | 15.2, 4,096 x 2,048 8.7 | 12.5; stored 4,096 x 2,048 8.5 | 9.7 but 4,096 x 4,096 13.6 | 12.5;
+//     192 tokens, 2,048 x 8,192 22.9 | 18.6, not 4,096 x 10,880 30.7 | 35.3 (tiles of 128: 12 us of blocks spared at least).
+int plan_ranges(int epi, int T, int N, int K, int sm_count, bool few, int bn_other) {
   if (T <= 32 || T > 256 || epi == EPI_SWIGLU || epi == EPI_QKV_ROPE) return 0;
-  const int bn = T <= 128 ? 64 : 128, kb = (K + BK - 1) / BK;
-  const long long tiles = (long long)((T + bn - 1) / bn) * ((N + BM - 1) / BM);
+  const int bn = T <= 128 ? 64 : 128, kb = (K + BK - 1) / BK, n_tiles = (N + BM - 1) / BM;
+  const long long tiles = (long long)((T + bn - 1) / bn) * n_tiles;
   for (int ranges = 4; ranges >= 2; ranges >>= 1) {
     const long long ctas = tiles * ranges;
-    if (ctas > sm_count || ctas * 4 < sm_count * 3LL || kb < 8 * ranges) continue;
-    return T <= 128 || (long long)(kb - kb / ranges) * 165 >= 12000 ? ranges : 0;
+    if (ctas > sm_count || ctas * 4 < sm_count * 3LL || kb < 8 * ranges || (ranges == 4 && ctas * 10 > sm_count * 9LL)) continue;
+    if (T <= 64) return kb >= (ranges == 2 && epi == EPI_ACCUM_F32 ? 64 : 48) ? ranges : 0;
+    if (few) return ranges;
+    if (bn == 128 && (kb - kb / ranges) * 165 < 12000) return 0;
+    const long long waves = ((long long)((T + bn_other - 1) / bn_other) * n_tiles + sm_count - 1) / sm_count;
+    const long long other = waves * kb * (bn_other > 90 ? bn_other * 176 / 100 : 159) + 3600;
+    const long long with = (kb + ranges - 1) / ranges * (bn == 64 ? 190 : 268) + (bn == 64 ? 6800 : 7000) + (epi == EPI_ACCUM_F32 ? 2500 : 0);
+    return with < other ? ranges : 0;
   }
   return 0;
 }
@@ -1562,7 +1571,7 @@ struct Choice {
 Choice choose(int epi, int T, int N, int K, int sm_count, int allow_split, bool norm, bool mixes, bool rows16) {
   Choice c{0, 1, false, false};
   plan(epi, T, N, K, sm_count, allow_split, &c.bn, &c.splits, &c.few, norm);
-  if (const int ranges = !norm && !mixes && allow_split == 1 ? plan_ranges(epi, T, N, K, sm_count) : 0) {
+  if (const int ranges = !norm && !mixes && allow_split == 1 ? plan_ranges(epi, T, N, K, sm_count, c.few, c.bn) : 0) {
     c.few = true; c.bn = T <= 128 ? 64 : 128; c.splits = ranges;
   }
   if (g_pairs >= 0 && !c.few && !norm && !mixes && sm_count >= 2 && (epi != EPI_SWIGLU || rows16))

@@ -17,13 +17,13 @@ def rel(a, b):
 
 
 # the sizes below that wide tiles and ranges of K take; the others lie behind the rule's lines
-RANGED = [(65, 2048, 2048), (100, 2048, 8192), (127, 4096, 1096), (33, 4096, 2048), (64, 4096, 4104), (129, 2048, 8192), (192, 2044, 8200),
-          (256, 4096, 16384)]
+RANGED = [(65, 2048, 2048), (100, 2048, 8192), (64, 4096, 4104), (129, 2048, 8192), (192, 2044, 8200), (256, 4096, 16384), (33, 4090, 4104),
+          (127, 4096, 5000)]
 
 
 @pytest.mark.parametrize("T,N,K", [(65, 2048, 2048), (100, 2048, 8192), (128, 2048, 1000), (127, 4096, 1096), (33, 4096, 2048), (64, 4096, 4104),
                                    (129, 2048, 8192), (192, 2044, 8200), (256, 4096, 16384), (255, 1924, 5440), (256, 2048, 4096), (257, 2048, 8192),
-                                   (32, 4096, 2048), (100, 4740, 2048), (97, 1800, 520), (96, 2048, 448)])
+                                   (32, 4096, 2048), (33, 4090, 4104), (127, 4096, 5000), (100, 4740, 2048), (97, 1800, 520), (96, 2048, 448)])
 def test_ranges_of_wide_tiles(T, N, K):
     from rllm_b200.kernels import ops, sm100
     assert (sm100.plan(ops.EPI_STORE, T, N, K) in ((64, 2), (64, 4), (128, 2), (128, 4))) == ((T, N, K) in RANGED)

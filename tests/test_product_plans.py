@@ -11,8 +11,11 @@ SMS = 148
     # ranges of K with tiles of 64 and 128 tokens: a narrow weight of a long K
     (ACCUM, 64, 2048, 8192, (32, 8, False)), (ACCUM, 100, 2048, 8192, (64, 4, False)), (ACCUM, 128, 2048, 8192, (64, 4, False)),
     (ACCUM, 129, 2048, 8192, (128, 4, False)), (ACCUM, 256, 2048, 8192, (128, 4, False)), (ACCUM, 257, 2048, 8192, (64, 1, False)),
+    (STORE, 100, 4096, 4096, (64, 2, False)), (ACCUM, 64, 4096, 4096, (64, 4, False)), (STORE, 33, 4096, 3072, (64, 4, False)),
     (ACCUM, 100, 4096, 16384, (64, 2, False)), (ACCUM, 256, 4096, 16384, (128, 2, False)), (STORE, 100, 2048, 2048, (64, 4, False)),
     # ... and not where too few SMs would have a CTA, or the ranges would not pay for their merge
+    (ACCUM, 100, 4096, 4096, (64, 1, False)), (STORE, 100, 4096, 2048, (64, 1, False)), (ACCUM, 192, 4096, 10880, (64, 1, False)),
+    (ACCUM, 64, 8192, 2048, (32, 2, False)), (STORE, 33, 4096, 2048, (32, 4, False)), (ACCUM, 64, 4608, 4608, (32, 4, False)),
     (ACCUM, 192, 2048, 2048, (64, 1, False)), (ACCUM, 192, 4096, 4096, (64, 1, False)), (STORE, 128, 3072, 2048, (64, 1, False)),
     (ROPE, 100, 2048, 8192, (32, 8, False)), (SWIGLU, 64, 2048, 8192, (32, 8, False)),
     # pairs of CTAs: more than 128 tokens, where the model of both kernels says so
