@@ -507,8 +507,8 @@ def decode_per_sm(nh: int, nkv: int, hd: int) -> int:
 
 def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: int = 64, captured: bool = False, per_sm: int = 2) -> int:
     """Ranges the keys of a sequence are cut into (= CTAs per cluster), by one cost for all callers, in units of what a key of heads of 64
-    takes: rounds of CTAs over the places (`per_sm` an SM) x (1,150 before the first key + the keys of a range) + 40 a range for the
-    merge + 200 where there is a cluster at all. `captured`: max_kv_len is a captured step's bound, which serves
+    takes: rounds of CTAs over the places (`per_sm` an SM) x (1,150 before the first key + the keys of a range) + for the merge of a
+    range's parts 52 (of six warps, heads of 64) or 40 (of four, heads of 128) + 200 where there is a cluster at all. `captured`: max_kv_len is a captured step's bound, which serves
     contexts from half of it up; the cost is then that of three quarters. Clusters of 3 and of 5 to 8 CTAs need their places inside one GPC,
     which they do not fill evenly: where a round is more than 13/16 full of them (3/4 with one CTA an SM) the last ones start late, and they are not
     considered.
@@ -518,8 +518,8 @@ def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: i
     300 533 / 566 / 569 / 533 (1), of 1,000 620 / 613 / 592 / 592 (4), of 4,080 997 / 805 / 707 / 707 (4); 8 layers with 32 / 8 heads of 128, 1 sequence of
     300 707 / 705 / 693 / 692 (7), of 2,030 945 / 821 / 747 / 712 (8). Late clusters: heads of 64, contexts of 1,000, 4 sequences
     558 with 6 and 7 ranges, 603 with 8 (256 of 296 places); 6 sequences 574 with 4, 582 with 5, 625 with 6; 12 sequences 704 with 2, 773 with 3. Over
-    770 measurements (1 to 64 sequences, 100 to 8,000 keys, heads of 64 and 128 over 4 and 8 kv heads) the choice is 0.2 % from the best number of
-    each on average; the most that it is behind is 4 % up to 4,080 keys, where contexts of one bound want different numbers, and 7 % at one point beyond.
+    1,346 measurements (1 to 64 sequences, 200 to 8,000 keys, heads of 64 and 128 over 4 and 8 kv heads) the choice is 0.3 % behind the best number
+    of each on average, and at most 6 % where contexts of 550 and of 1,000 keys, under one bound, want one range and four (7 % at 24 sequences of 8,000).
 
     12 and 16 ranges (clusters beyond the portable size, for one or two long sequences: 16,384 keys of one sequence 13.3 us against 18.3
     with 8) only from 16,384 keys on and while the CTAs leave a quarter of the places free (9 ranges of 4
@@ -538,7 +538,7 @@ def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: i
         rounds = -(-base * s // places)
         if s in (3, 5, 6, 7, 8) and base * s * 16 > rounds * places * (13 if per_sm > 1 else 12):
             continue
-        cost = rounds * (1150 + keys * hd / 64 / s) + 40 * s + (200 if s > 1 else 0)
+        cost = rounds * (1150 + keys * hd / 64 / s) + (52 if hd == 64 else 40) * s + (200 if s > 1 else 0)
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
