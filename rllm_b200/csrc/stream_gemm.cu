@@ -387,12 +387,11 @@ int launch(const Params& p, int ctas, cudaStream_t s) {
 // 9.7 | 9.3), as is the head (80.8 | 81.5). At 9 tokens the lines lie at the same places.
 // Four groups (17 to 32 tokens, K 2,048) lose with the norm in front: a CTA then reads as many bytes of float rows as of
 // weights (gate/up 19.7 | 17.8 at 32 tokens, q/k/v 10.1 | 9.4; a step of 24 requests 1,065 us | 997).
-constexpr int SMS = 148;                         // of the one GPU that this is built for
 constexpr bool has_16(int epi) { return epi == EPI_ACCUM_F32 || epi == EPI_SWIGLU || epi == EPI_QKV_ROPE; }
-bool streams_16(int epi, bool norm, int N, int nchw, int hd) {
+bool streams_16(int epi, bool norm, int N, int nchw, int hd, int sm_count) {
   if (!has_16(epi) || (epi == EPI_QKV_ROPE && 128 % hd)) return false;    // heads that the tcgen05 kernel takes as well
-  if (nchw > (norm ? 1 : 2)) return epi == EPI_ACCUM_F32 && N / 16 <= SMS && nchw <= MAX_RESIDENT;
-  return !(norm && epi == EPI_SWIGLU) || N <= 64 * SMS;
+  if (nchw > (norm ? 1 : 2)) return epi == EPI_ACCUM_F32 && N / 16 <= sm_count && nchw <= MAX_RESIDENT;
+  return !(norm && epi == EPI_SWIGLU) || N <= 64 * sm_count;
 }
 
 template <int EPI, bool NORM>
@@ -418,16 +417,16 @@ int launch_nch(const Params& p, int ctas, cudaStream_t s) {
 int chunks_per_warp(int K) { return ((K + CK - 1) / CK + Cfg::WARPS - 1) / Cfg::WARPS; }
 
 // Can the kernel take this problem? The rules the launchers below enforce.
-int supported(int epi, bool norm, int T, int N, int K, int hd) {
+int supported(int epi, bool norm, int T, int N, int K, int hd, int sm_count) {
   if (T < 1 || T > 2 * NT || N < 16 || N % 16 || K < 32 || K % 32) return 0;
   if (epi < 0 || epi > EPI_QKV_ROPE) return 0;
   if (norm && (epi == EPI_ACCUM_F32 || chunks_per_warp(K) > MAX_RESIDENT)) return 0;
   if (epi == EPI_QKV_ROPE && (hd < 32 || hd % 32 || N % hd)) return 0;
-  return T <= NT || streams_16(epi, norm, N, chunks_per_warp(K), hd);
+  return T <= NT || streams_16(epi, norm, N, chunks_per_warp(K), hd, sm_count);
 }
 
 int run(int epi, bool norm, Params& p, int sm_count, cudaStream_t s) {
-  if (!supported(epi, norm, p.T, p.N, p.K, p.rope.hd)) return ERR_BAD_SIZE;
+  if (!supported(epi, norm, p.T, p.N, p.K, p.rope.hd, sm_count)) return ERR_BAD_SIZE;
   if ((uintptr_t)p.W & 15) return ERR_BAD_ALIGN;
   if (norm) {
     if (p.ldh % 4 || ((uintptr_t)p.h & 15) || ((uintptr_t)p.g & 15)) return ERR_BAD_ALIGN;
@@ -461,9 +460,9 @@ int run(int epi, bool norm, Params& p, int sm_count, cudaStream_t s) {
 }  // namespace
 
 // 1 when rllm_stream_gemm / rllm_stream_gemm_qkv_rope take the problem (T tokens, N output features
-// (of one half with SwiGLU), inner size K, norm in front or not; hd: head size, rotary epilogue only).
-RLLM_API int rllm_stream_gemm_supported(int epi, int norm, int T, int N, int K, int hd) {
-  return supported(epi, norm != 0, T, N, K, hd);
+// (of one half with SwiGLU), inner size K, norm in front or not; hd: head size, rotary epilogue only) on a GPU of sm_count SMs.
+RLLM_API int rllm_stream_gemm_supported(int epi, int norm, int T, int N, int K, int hd, int sm_count) {
+  return supported(epi, norm != 0, T, N, K, hd, sm_count);
 }
 
 // C[T, N] = X W^T for T <= 8, or 16 where `streams_16` says so. X: bf16 [T, K] with row stride ldx, or null: then X = rmsnorm(h[rows]; g, eps)

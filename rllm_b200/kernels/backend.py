@@ -123,7 +123,7 @@ class Backend:
         # the kernel for steps of at most 8 tokens builds the normalised rows once per CTA whatever
         # the width (a CTA walks many slabs of the weight)
         return (w.shape[0] + 127) // 128 <= self._sm100.init(self.device).sm_count or \
-            self._sm100.stream_supported(ops.EPI_STORE_F32, True, x.shape[0], w.shape[0], w.shape[1])
+            self._sm100.stream_supported(ops.EPI_STORE_F32, True, x.shape[0], w.shape[0], w.shape[1], sm_count=self.sm_count)
 
     def fuses_norm(self, T):
         """May a product of a step of T tokens take the norm in front of it into its own kernel?"""

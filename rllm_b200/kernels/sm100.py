@@ -21,7 +21,7 @@ ops.register_signatures("sm100", {
     "rllm_tc_gemm_norm_max_tokens": [],
     "rllm_tc_gemm_qkv_rope": [_P, c_longlong, _P, c_longlong, _P, c_int, c_float, _P, _P, c_longlong, c_int, c_int,
                               _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P],
-    "rllm_stream_gemm_supported": [c_int, c_int, c_int, c_int, c_int, c_int],
+    "rllm_stream_gemm_supported": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
     "rllm_stream_gemm": [c_int, _P, c_longlong, _P, c_longlong, _P, _P, c_int, c_float, _P, _P, c_longlong, c_int,
                          c_int, c_int, c_int, _P],
     "rllm_stream_gemm_mixes": [_P, c_longlong, c_int, c_longlong, _P, _P, c_longlong, c_int, c_int, c_int, c_int, _P],
@@ -94,15 +94,17 @@ STREAM = os.environ.get("RLLM_B200_NO_STREAM_GEMM") != "1"
 _stream_ok: dict[tuple, bool] = {}
 
 
-def stream_supported(epilogue: int, norm: bool, T: int, N: int, K: int, hd: int = 0) -> bool:
+def stream_supported(epilogue: int, norm: bool, T: int, N: int, K: int, hd: int = 0, sm_count: int | None = None) -> bool:
     """Does the weight-streaming kernel for steps of at most 8 tokens, some products of up to 16, take this product? (N:
-    output features, of one half with the SwiGLU epilogue.)"""
+    output features, of one half with the SwiGLU epilogue; `sm_count`: of the GPU it runs on, None: the current one's.)"""
     if not STREAM or T > 16:
         return False
-    key = (epilogue, norm, T, N, K, hd)
+    if sm_count is None:
+        sm_count = init("cuda").sm_count
+    key = (epilogue, norm, T, N, K, hd, sm_count)
     ok = _stream_ok.get(key)
     if ok is None:
-        ok = _stream_ok[key] = bool(ops._fn("sm100", "rllm_stream_gemm_supported")(epilogue, int(norm), T, N, K, hd))
+        ok = _stream_ok[key] = bool(ops._fn("sm100", "rllm_stream_gemm_supported")(epilogue, int(norm), T, N, K, hd, sm_count))
     return ok
 
 
@@ -191,7 +193,7 @@ def _product(x, w, epilogue, code, out, split):
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
     if out.dtype != out_dtype or out.shape != (T, N) or out.stride(1) != 1:
         raise ops.KernelError(f"tc gemm out must be [{T}, {N}] of {out_dtype}")
-    if split and stream_supported(epilogue, False, T, N, K):
+    if split and stream_supported(epilogue, False, T, N, K, sm_count=st.sm_count):
         rc = ops._fn("sm100", "rllm_stream_gemm")(
             code, x.data_ptr(), x.stride(0), None, 0, None, None, 0, 0.0, w.data_ptr(), out.data_ptr(),
             out.stride(0), T, N, K, st.sm_count, ops._stream())
@@ -219,7 +221,7 @@ def gemm_mixes(x: torch.Tensor, w: torch.Tensor, rows_each: int, out: torch.Tens
             x.data_ptr(), x.stride(0), int(rows_each), x.stride(1), w.data_ptr(), out.data_ptr(), out.stride(0), T, N, K,
             st.err.data_ptr(), st.sm_count, ops._stream()), "tc_gemm_mixes")
         return True
-    if rows_each % 16 or not stream_supported(ops.EPI_STORE, False, T, N, K):
+    if rows_each % 16 or not stream_supported(ops.EPI_STORE, False, T, N, K, sm_count=st.sm_count):
         return False
     ops._check(ops._fn("sm100", "rllm_stream_gemm_mixes")(
         x.data_ptr(), x.stride(0), int(rows_each), x.stride(1), w.data_ptr(), out.data_ptr(), out.stride(0), T, N, K, st.sm_count,
@@ -270,7 +272,7 @@ def gemm_norm(h: torch.Tensor, g: torch.Tensor, eps: float, w: torch.Tensor, epi
     N = w.shape[0] // 2 if epilogue == ops.EPI_SWIGLU else w.shape[0]
     out = torch.empty((T, N), dtype=torch.float32 if epilogue == ops.EPI_STORE_F32 else torch.bfloat16,
                       device=h.device)
-    if split and stream_supported(epilogue, True, T, N, K):
+    if split and stream_supported(epilogue, True, T, N, K, sm_count=st.sm_count):
         rc = ops._fn("sm100", "rllm_stream_gemm")(
             code, None, 0, h.data_ptr(), h.stride(0), ops._ptr(rows), g.data_ptr(), ops._dt(g, "norm weight"),
             float(eps), w.data_ptr(), out.data_ptr(), out.stride(0), T, N, K, st.sm_count, ops._stream())
@@ -306,18 +308,18 @@ def gemm_qkv_rope(x: torch.Tensor | None, w_qkv: torch.Tensor, positions: torch.
     has just asked `qkv_rope_supported` about x, w_qkv and kcache. `w_fixed` as in `gemm`."""
     T, K = norm[0].shape if norm is not None else x.shape
     # steps of at most 8 tokens: the weight-streaming kernel (any head size that is a multiple of 32), up to 16 for some K
-    streamed = split and rot_dim == hd and stream_supported(EPI_QKV_ROPE, norm is not None, T, (nh + 2 * nkv) * hd, K, hd)
+    dev = (x if norm is None else norm[0]).device
+    streamed = split and rot_dim == hd and dev.type == "cuda" and \
+        stream_supported(EPI_QKV_ROPE, norm is not None, T, (nh + 2 * nkv) * hd, K, hd, init(dev).sm_count)
     if norm is not None:
         h, g, eps = norm
         if not norm_supported(h, g, w_qkv) or (128 % hd and not streamed) or \
                 (kcache is not None and kcache.dtype != torch.bfloat16):
             raise ops.KernelError("tc gemm with norm and rotary epilogue: sizes not supported")
-        dev = h.device
     else:
         if not asked and not (gemm_supported(x, w_qkv) and (128 % hd == 0 or streamed)
                 and (kcache is None or kcache.dtype == torch.bfloat16)):
             raise ops.KernelError("tc gemm with rotary epilogue: bfloat16 operands and a head size dividing 128")
-        dev = x.device
     st = init(dev)
     N = (nh + 2 * nkv) * hd
     if w_qkv.shape[0] != N:

@@ -52,3 +52,12 @@ def test_pairs_take_tiles_in_steps_of_32_tokens():
             assert sm100.launch_plan(STORE, 1000, 2048, 2048, SMS) == (width, 1, True)
     finally:
         sm100.set_pairs(False)
+
+
+def test_which_products_of_9_to_16_tokens_are_streamed_goes_with_the_gpus_sms():
+    """A long K is streamed where a CTA has one job (16 features), a norm's gate/up pair where it leaves a tcgen05 tile no SM."""
+    for sms in (100, 132, SMS):
+        assert sm100.stream_supported(ACCUM, False, 12, 16 * sms, 8192, sm_count=sms)
+        assert not sm100.stream_supported(ACCUM, False, 12, 16 * sms + 16, 8192, sm_count=sms)
+        assert sm100.stream_supported(SWIGLU, True, 12, 64 * sms, 2048, sm_count=sms)
+        assert not sm100.stream_supported(SWIGLU, True, 12, 64 * sms + 16, 2048, sm_count=sms)
