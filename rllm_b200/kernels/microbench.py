@@ -736,7 +736,9 @@ def main(argv=None) -> int:
             p.add_argument("--no-split", action="store_true")
             p.add_argument("--weight-rows", action="store_true",
                            help="gate/up of long portions with the weight rows on the accumulator's rows (default: the tokens)")
-            p.add_argument("--pairs", action="store_true", help="more than 64 tokens on pairs of CTAs (tcgen05.mma.cta_group::2) always; else where the rule says so")
+            p.add_argument("--pairs", nargs="?", type=int, default=0, const=1,
+                           help="products on pairs of CTAs (tcgen05.mma.cta_group::2): 0 where the rule says so (default), 1 all that pairs take, "
+                                "-1 none, 32 to 256 all with that many tokens a tile")
             p.add_argument("--ranges", type=int, default=0, help="ranges of K to force on the tcgen05 small-tile kernel")
         else:
             p.add_argument("--heads", type=int, default=32)

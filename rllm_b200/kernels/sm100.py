@@ -109,8 +109,9 @@ def stream_supported(epilogue: int, norm: bool, T: int, N: int, K: int, hd: int 
 
 
 def set_pairs(on: bool | int) -> None:
-    """Products of more than 64 tokens on pairs of CTAs (`tcgen05.mma.cta_group::2`): True all that pairs take, False (the
-    default) those that are faster there by the launcher's rule, -1 none; 32 to 256: all, with that many tokens a tile."""
+    """Products on pairs of CTAs (`tcgen05.mma.cta_group::2`): False (the default) those of more than 128 tokens that are faster
+    there by the launcher's rule, True all that pairs take (more than 64 tokens), -1 none; 32 to 256: all, with that many tokens a tile
+    (steps of 32)."""
     ops._fn("sm100", "rllm_tc_gemm_set_pairs")(int(on))
 
 
