@@ -30,11 +30,12 @@
 //               has grown by more than 2^8 since (P then stays below 2^8, which bf16 holds as
 //               well as values below 1); when it moves, the thread scales its row of the output
 //               in TMEM (tcgen05.ld / st) before the next PV is added.
-// The (row tile, K tile) steps are numbered k = 0, 1, ... in the order A0 B0 A1 B1 ...; S of step k
-// lands in accumulator k % 3 (heads of 128: see Shape) once PV of step k - 3, whose P lay there, is complete, so while both row tiles are in their softmax the scores of the step
+// The (row tile, K tile) steps are numbered k = 0, 1, ... in the order A0 B0 A1 B1 ... With heads of 64, and wherever scores are bounded, S of step k
+// lands in accumulator k % 3 once PV of step k - 3, whose P lay there, is complete; keys of 128 and more with unbounded scores have an accumulator a row
+// tile and P beside it (Shape). Either way, while both row tiles are in their softmax the scores of the step
 // after are computed already, and a row tile that has written its P goes on at once: the four warp
 // schedulers always have a warp with work (two warps each, one of either tile).
-// TMEM: three S accumulators and PV of both tiles, 512 columns.
+// TMEM: the S accumulators (and P) and PV of both tiles, 512 columns.
 // Where a work item's two row tiles lie: next to each other, or (`fold`) as far from one end of the sequence's rows as from the other. Items of
 // neighbours are as long as the keys they see, which balances where every CTA gets several; where the items are no more than the
 // SMs, the longest is the launch, and folded ones are all alike. 16 / 4 heads of 128 over

@@ -355,8 +355,8 @@ __global__ void __launch_bounds__(THREADS) talk_attention_mma_kernel(const Args 
 // the outputs of the heads that use kv head c, HB of them at a time, each sum in the order of the heads. Bound by the parts'
 // bytes (2,048 tokens x 16 heads x 512: 29 us with a column a thread). Single tokens over SPLITS ranges of keys are a few CTAs, whose
 // time is their chain of loads: with the ranges counted at compile time those of several heads are on their way together
-// (8 tokens, 16 heads
-// of 128 over 4 kv heads, three ranges: the decode step of two such layers and two others 359 -> 323 us).
+// (8 tokens, 16 heads of 128 over 4 kv heads, three ranges: with the sum of a layer's terms for few rows (row_mix.cu) the decode step
+// of two such layers and two others 368 -> 339 us).
 constexpr int HB = 4;
 template <int SPLITS>
 __global__ void __launch_bounds__(128) talk_mix_kernel(const float* __restrict__ parts, const float* __restrict__ mix,

@@ -5,9 +5,10 @@
 // The weight tile is the MMA's A operand (M = 128 weight rows) and the token tile is its B
 // operand (N = BN tokens), so a decode step with a handful of tokens still fills the 128-row MMA
 // and streams every weight byte exactly once. Steps of up to 64 tokens (128 for a narrow weight)
-// run token tiles of 16 or 32 in the first kernel below; more tokens run in the persistent kernel
-// further down, whose token tile is any multiple of 16 up to 256 (128 with the gate/up pair),
-// chosen so that the tiles fill whole waves of CTAs. The accumulator D[weight row (TMEM lane),
+// run token tiles of 16 or 32 in the first kernel below, which also shares tiles of 64 and 128 tokens between ranges
+// of K where a weight of few rows meets 33 to 256 tokens (`plan_ranges`); more tokens run in the persistent kernels
+// further down, on single CTAs, whose token tile is any multiple of 16 up to 256 (128 with the gate/up pair),
+// chosen so that the tiles fill whole waves of CTAs, or on pairs of them (`plan_pairs`). `choose` decides. The accumulator D[weight row (TMEM lane),
 // token (TMEM column)] is read back with tcgen05.ld by the epilogue warps, thread = weight row, and
 // written as C[token][row]. Gate/up pairs of 33 tokens and more (with no norm in front) exchange the
 // roles: tokens on the accumulator's rows, the tile's 128 gate and 128 up weight rows one operand of
@@ -712,13 +713,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------- many tokens
-// The same product for steps of more than 64 tokens (prompt portions). One CTA per SM walks the
+// The same product for steps of more than 64 tokens (prompt portions; gate/up pairs from 33 on). One CTA per SM walks the
 // output tiles (token tiles fastest, so the CTAs of a wave share their weight tiles in L2 and a
 // weight byte comes from DRAM once) and keeps two accumulators in TMEM: while the epilogue warps
 // read tile i out of one, the MMA warp already fills the other with tile i + 1, so the tensor
-// cores do not wait for the epilogue. No ranges of K and no norm in front here; the rotary epilogue
-// exists but is chosen only up to 128 tokens (beyond, the row-parallel rotation kernel is faster
-// than rotating in four epilogue warps).
+// cores do not wait for the epilogue. No ranges of K and no norm in front here.
 // WR: weight rows of a tile per accumulator. 128, or 64 for the kernel with the tokens on the accumulator's
 // rows when the 128-row tiles would leave most SMs without one (few tokens).
 template <int BN, bool DUAL, int WR = BM> struct PCfg {
@@ -1452,10 +1451,9 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
     const int forced = allow_split > 1 ? allow_split : 0;
     if (forced > 0) splits = forced < kb / 2 ? (forced < MAX_CLUSTER ? forced : MAX_CLUSTER) : (kb / 2 > 0 ? kb / 2 : 1);
   }
-  // A step of few tokens: token tiles of 16 or 32 (33 to 64 tokens: two tiles of 32 land their
-  // parts faster than one of 64, which reads the weights once but has three stages and one issuing
-  // thread: at 64 tokens gate/up 20.8 against 19.3 us, down 13.7 against 12.2, O 8.3 against 7.3),
-  // and ranges of K until every SM has a CTA. Up to 128 tokens the
+  // A step of few tokens: token tiles of 16 or 32 and ranges of K until every SM has a CTA. 33 to 64 tokens take two tiles of 32, which land
+  // their parts faster than one of 64 that reads the weights once (64 tokens, 2,048 x 8,192: 12.7 against 14.2 us); where they do not,
+  // `plan_ranges` says so afterwards. Up to 128 tokens the
   // same holds for a narrow weight that would give the persistent kernel under a quarter of the SMs.
   // (33 to 64 tokens against a weight of many tiles, the output head: one token tile of 64 in the persistent
   // kernel reads the weight once, two tiles of 32 read it twice)
@@ -1468,8 +1466,7 @@ void plan(int epi, int T, int N, int K, int sm_count, int allow_split, int* bn_o
     bn = T <= 16 ? 16 : 32;
     if (bn >= 32) while (splits & (splits - 1)) splits &= splits - 1;     // wider tiles: a power of two
   } else {
-    // More tokens: no ranges of K (a partial tile of 128+ columns costs more to merge than it saves), and
-    // the persistent kernel, whose tile takes any number of tokens in steps of 16. A CTA's time goes with
+    // More tokens: no ranges of K (but see `plan_ranges`), and the persistent kernel, whose tile takes any number of tokens in steps of 16. A CTA's time goes with
     // its tiles x the operand rows a tile takes in per 64 of K (128 or 256 weight rows + the tokens): the
     // width that makes this smallest fills whole waves (2,048 tokens x 24 weight tiles: 176 tokens a tile
     // are 288 tiles, 1.95 waves of 148, where 256 are 192 tiles, 1.3 waves that cost 2); of equals the wider.
