@@ -524,19 +524,18 @@ def decode_splits(num_seqs: int, nkv: int, max_kv_len: int, sm_count: int, hd: i
     1,346 measurements (1 to 64 sequences, 200 to 8,000 keys, heads of 64 and 128 over 4 and 8 kv heads) the choice is 0.3 % behind the best number
     of each on average, and at most 6 % where contexts of 550 and of 1,000 keys, under one bound, want one range and four (7 % at 24 sequences of 8,000).
 
-    12 and 16 ranges (clusters beyond the portable size, for one or two long sequences: 16,384 keys of one sequence 13.3 us against 18.3
-    with 8) only from 16,384 keys on and while the CTAs leave a quarter of the places free (9 ranges of 4
-    sequences, 288 CTAs on 296 places: 16.7 us against 10.8 with 8); inside a decode step, behind a
-    kernel whose CTAs fill whole SMs, such a cluster starts later than a small one (4,096 keys: 6.3 us against 6.9
-    alone, but the step at batch 1 0.621 ms against 0.615, at batch 2 0.692 against 0.642)."""
+    16 ranges (a cluster beyond the portable size) only from 16,384 keys on and while their CTAs take no more than two thirds of the places:
+    the steps above with contexts of 9,000, 1 sequence 632 with 8, 594 with 16; 2 sequences 659 with 8, 742 with 16 (256 of 296 places), 730 with 12; 3 sequences over 4 kv heads of 128
+    404 with 8, 344 with 16; 2 over 4 kv heads with one CTA an SM 416 with 8, 429 with 16, 441 with 12. At 4,096 keys such a cluster is faster alone (6.3 us against 6.9) but starts
+    later inside a step, behind a kernel whose CTAs fill whole SMs (the step at batch 1 0.621 ms against 0.615)."""
     base = max(1, num_seqs * nkv)
     places = per_sm * sm_count
     keys = max_kv_len * 3 // 4 if captured else max_kv_len
     best, best_cost = 1, None
-    for s in (1, 2, 3, 4, 5, 6, 7, 8, 12, 16):
+    for s in (1, 2, 3, 4, 5, 6, 7, 8, 16):
         if s > 1 and keys // s < 64:
             break
-        if s > 8 and (base * s * 4 > places * 3 or max_kv_len < 16384):
+        if s > 8 and (base * s * 3 > places * 2 or max_kv_len < 16384):
             break
         rounds = -(-base * s // places)
         if s in (3, 5, 6, 7, 8) and base * s * 16 > rounds * places * (13 if per_sm > 1 else 12):
